@@ -11,7 +11,22 @@
 
 #include <cstdint>
 
+#include "tlq_softfp.cuh"
+
 namespace tlq {
+
+// Quotient and square root of the step's arithmetic: in FP64 on the integer
+// pipe (tlq_softfp.cuh: the hardware operations' bits; a division on GB300's
+// FP64 pipe takes 133 SM cycles a warp, 29 there, a square root 139 and 35),
+// in FP32 the hardware's.
+__device__ __forceinline__ double quot(double a, double b) { return sf::div(a, b); }
+__device__ __forceinline__ float quot(float a, float b) { return a / b; }
+__device__ __forceinline__ double root(double a) { return sf::sqrt_rn(a); }
+__device__ __forceinline__ float root(float a) { return sqrt(a); }
+// Several quotients by one divisor.
+__device__ __forceinline__ sf::Divisor divisor(double b) { return sf::divisor(b); }
+__device__ __forceinline__ float divisor(float b) { return b; }
+__device__ __forceinline__ double quot(double a, const sf::Divisor& b) { return sf::div(a, b); }
 
 // source/constants.f90:6-15 (cgs).  PI is the reference's truncated value.
 constexpr double AMU = 1.660538782e-24;
@@ -111,16 +126,17 @@ __device__ __forceinline__ double zcoord(const Params& p, int k) { return (p.zl 
 // ---------------------------------------------------------------------------
 template <class R>
 __device__ __forceinline__ void cons2prim(R g, const R* u, R* w) {
+  const auto r = divisor(u[0]);
   w[0] = u[0];
-  w[1] = u[1] / u[0];
-  w[2] = u[2] / u[0];
-  w[3] = u[3] / u[0];
-  w[4] = (g - R(1.0)) * (u[4] - R(0.5) * ((u[1] * u[1] + u[2] * u[2]) + u[3] * u[3]) / u[0]);
+  w[1] = quot(u[1], r);
+  w[2] = quot(u[2], r);
+  w[3] = quot(u[3], r);
+  w[4] = (g - R(1.0)) * (u[4] - quot(R(0.5) * ((u[1] * u[1] + u[2] * u[2]) + u[3] * u[3]), r));
   w[4] = mx(w[4], R(1e-20));
 }
 
 // csound, source/HydroCore.f90:157-168.
-template <class R> __device__ __forceinline__ R csound(R g, R pres, R den) { return sqrt(g * pres / den); }
+template <class R> __device__ __forceinline__ R csound(R g, R pres, R den) { return root(quot(g * pres, den)); }
 
 // ---------------------------------------------------------------------------
 // limiter / average, source/HLLC.f90:560-638 (HLL.f90:319-397 is identical).
@@ -147,7 +163,7 @@ __device__ __forceinline__ R average(R a, R b, int opt) {
         return __fdividef(xy * (x + y), fmaf(x, x, y * y)) * __uint_as_float(eb);
       } else {
         if (a * b <= R(0.0)) return R(0.0);
-        return a * b * (a + b) / (a * a + b * b);
+        return quot(a * b * (a + b), a * a + b * b);
       }
     case LIM_MINMOD:
       s = sgn1(a);
@@ -235,13 +251,14 @@ __device__ __forceinline__ bool riemann(int solver, R g, R g1, R* ff, const R* w
       R fl[5], fr[5];
       prim2f(g1, fl, wl, d);
       prim2f(g1, fr, wr, d);
+      const auto ds = divisor(sr - sl);
 #pragma unroll
-      for (int e = 0; e < 5; ++e) ff[e] = (sr * fl[e] - sl * fr[e] + sl * sr * (UR[e] - UL[e])) / (sr - sl);
+      for (int e = 0; e < 5; ++e) ff[e] = quot(sr * fl[e] - sl * fr[e] + sl * sr * (UR[e] - UL[e]), ds);
     }
     return true;  // NaN speeds take the HLL average branch, as in the reference
   }
-  const R sst = (wr[4] - wl[4] + wl[0] * ul * (sl - ul) - wr[0] * ur * (sr - ur)) /
-                (wl[0] * (sl - ul) - wr[0] * (sr - ur));
+  const R sst = quot(wr[4] - wl[4] + wl[0] * ul * (sl - ul) - wr[0] * ur * (sr - ur),
+                     wl[0] * (sl - ul) - wr[0] * (sr - ur));
   // Branch order of the reference: sl>=0, sr<=0, sst>=0, sst<=0.  The two
   // star branches share one code path on the selected side.
   bool star, left;
@@ -263,12 +280,12 @@ __device__ __forceinline__ bool riemann(int solver, R g, R g1, R* ff, const R* w
     const R s = left ? sl : sr;
     const R un = left ? ul : ur;
     const R a = w[0] * (s - un);
-    const R rhostr = a / (s - sst);
+    const R rhostr = quot(a, s - sst);
     R us[5];
     us[0] = rhostr;
 #pragma unroll
     for (int e = 1; e <= 3; ++e) us[e] = (e == d) ? rhostr * sst : rhostr * w[e];
-    us[4] = rhostr * (uc[4] / w[0] + (sst - un) * (sst + w[4] / a));
+    us[4] = rhostr * (quot(uc[4], w[0]) + (sst - un) * (sst + quot(w[4], a)));
 #pragma unroll
     for (int e = 0; e < 5; ++e) ff[e] = ff[e] + s * (us[e] - uc[e]);
   }
@@ -383,7 +400,7 @@ __device__ __forceinline__ double cool_coef(const CoolTable& t, double temp) {
   if (lo >= t.n) return pow(10.0, t.C[t.n - 1]);
   const double T0 = t.logT[lo - 1], C0 = t.C[lo - 1];
   const double T1 = t.logT[lo], C1 = t.C[lo];
-  return pow(10.0, (C1 - C0) / (T1 - T0) * (log10(temp) - T0) + C0);
+  return pow(10.0, quot(C1 - C0, T1 - T0) * (log10(temp) - T0) + C0);
 }
 
 // The exact integrator (COOL_EXACT): the temperature after a step of
@@ -430,48 +447,49 @@ __device__ __forceinline__ double cool_exact_T(const CoolTable& t, double temp, 
 __device__ __forceinline__ void cool_cell(const Params& p, double* w, double& u4, double dt) {
   const double g = p.gamma;
   const double Tmin = p.cool.T[0];
-  double temp = w[4] * p.mu0 * AMU / (w[0] * KB);
+  double temp = quot(w[4] * p.mu0 * AMU, w[0] * KB);
   if (!(temp >= Tmin)) return;
-  double ETH = w[4] / (g - 1.0);
+  const auto gm1 = divisor(g - 1.0);
+  double ETH = quot(w[4], gm1);
   const double vel2 = w[1] * w[1] + w[2] * w[2] + w[3] * w[3];
   const double EK = 0.5 * w[0] * vel2;
   double aloss = cool_coef(p.cool, temp);
-  const double numdens = w[0] / (p.mu0 * AMU);
-  double ce = aloss * (numdens * numdens) / ETH;
+  const double numdens = quot(w[0], p.mu0 * AMU);
+  double ce = quot(aloss * (numdens * numdens), ETH);
   if (p.cooling == COOL_EXACT && ce * dt > p.cool_sub_frac) {
     const double Tn = cool_exact_T(p.cool, temp, aloss, ce * dt);
-    w[4] = w[4] * (Tn / temp);
-    ETH = w[4] / (g - 1.0);
+    w[4] = w[4] * quot(Tn, temp);
+    ETH = quot(w[4], gm1);
     u4 = EK + ETH;
     return;
   }
   int nsub = 1;
   if (p.cooling == COOL_SUBCYCLE && ce * dt > p.cool_sub_frac) {
-    const double q = ceil(ce * dt / p.cool_sub_frac);
+    const double q = ceil(quot(ce * dt, p.cool_sub_frac));
     nsub = (q > (double)p.cool_max_sub) ? p.cool_max_sub : (int)q;
     if (nsub < 1) nsub = 1;
   }
-  const double h = (nsub == 1) ? dt : dt / (double)nsub;
+  const double h = (nsub == 1) ? dt : quot(dt, (double)nsub);
   for (int s = 0; s < nsub; ++s) {
     if (s > 0) {
-      temp = w[4] * p.mu0 * AMU / (w[0] * KB);
+      temp = quot(w[4] * p.mu0 * AMU, w[0] * KB);
       if (!(temp >= Tmin)) break;
-      ETH = w[4] / (g - 1.0);
+      ETH = quot(w[4], gm1);
       aloss = cool_coef(p.cool, temp);
-      ce = aloss * (numdens * numdens) / ETH;
+      ce = quot(aloss * (numdens * numdens), ETH);
     }
     double cool_factor = exp(-ce * (h));
     if (cool_factor < 1.0 - p.cooling_limit) cool_factor = 1.0 - p.cooling_limit;
     const double new_temp = temp * cool_factor;
     bool floored = false;
     if (new_temp < T_FLOOR) {
-      cool_factor = T_FLOOR / temp;
+      cool_factor = quot(T_FLOOR, temp);
       floored = true;
     }
     w[4] = w[4] * cool_factor;
     if (floored) break;
   }
-  ETH = w[4] / (g - 1.0);
+  ETH = quot(w[4], gm1);
   u4 = EK + ETH;
 }
 
@@ -479,9 +497,9 @@ __device__ __forceinline__ void cool_cell(const Params& p, double* w, double& u4
 // centred potential differences phi(+1) - phi(-1) per axis.
 __device__ __forceinline__ void gravity_cell(const Params& p, const double* w, double dpx, double dpy, double dpz,
                                              double* s) {
-  const double fg1 = dpx / (2.0 * p.dx);
-  const double fg2 = dpy / (2.0 * p.dy);
-  const double fg3 = dpz / (2.0 * p.dz);
+  const double fg1 = quot(dpx, 2.0 * p.dx);
+  const double fg2 = quot(dpy, 2.0 * p.dy);
+  const double fg3 = quot(dpz, 2.0 * p.dz);
   s[0] = 0.0;
   s[1] = -w[0] * fg1;
   s[2] = -w[0] * fg2;
