@@ -30,9 +30,9 @@
 #else
 #include <cmath>
 #define TLQ_SF static inline
+#endif
 #ifndef TLQ_SF_HOST_SEED  // compiled for the host: lets a caller move the seeds within the GPU's error
 #define TLQ_SF_HOST_SEED(y) (y)
-#endif
 #endif
 
 namespace tlq {
