@@ -56,9 +56,9 @@ PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
 
 // 4-D map {x, y, z, var} over a SoA array with `nvar` planes of elements of
 // `esize` bytes (8: FP64, 4: FP32); box = the tile plus the halo its kernel
-// reads: the plain form's halo-2 box; in the mixed form stage 1's box of U
-// (2 cells in x, 1 in y: halo1 = true) and stage 2's halo-2 box of UPP's
-// FP32 primitives.
+// reads: stage 1's box of U (2 cells in x, 1 in y: halo1 = true; in the plain
+// form the carried pressure's too) and stage 2's halo-2 box of UPP (in the
+// mixed form its FP32 primitives).
 int make_map(tlq_ctx* ctx, CUtensorMap* m, void* base, int nvar, int esize = 8, bool halo1 = false) {
   auto fn = encode_fn();
   if (!fn) return fail(ctx, TLQ_ERR_CUDA, "cuTensorMapEncodeTiled is unavailable");
@@ -68,8 +68,8 @@ int make_map(tlq_ctx* ctx, CUtensorMap* m, void* base, int nvar, int esize = 8, 
   const cuuint64_t es = (cuuint64_t)esize;
   cuuint64_t strides[3] = {(cuuint64_t)L.px * es, (cuuint64_t)L.px * L.nyg * es, (cuuint64_t)L.plane * es};
   const bool mixed = ctx->cfg.precision == TLQ_PREC_MIXED;
-  const cuuint32_t bx = (cuuint32_t)(mixed ? MHX : HX);
-  const cuuint32_t by = (cuuint32_t)(mixed ? (halo1 ? MTY + 2 : MHY) : HY);
+  const cuuint32_t bx = (cuuint32_t)((mixed ? MTX : TX) + 4);
+  const cuuint32_t by = (cuuint32_t)((mixed ? MTY : TY) + (halo1 ? 2 : 4));
   cuuint32_t box[4] = {bx, by, 1, (cuuint32_t)nvar};
   cuuint32_t estr[4] = {1, 1, 1, 1};
   CUresult r = fn(m, esize == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, base, dims,
@@ -230,7 +230,7 @@ int enqueue_step(tlq_ctx* ctx, int par, bool timed) {
   if (mixed)
     CK(launch_stage_mixed(1, ctx->tm_U[par], a, ctx->grid, ctx->stream));
   else
-    CK(launch_stage(1, ctx->cfg.precision, ctx->tm_U[par], ctx->tm_P, a, ctx->grid, ctx->stream));
+    CK(launch_stage(1, ctx->tm_U[par], ctx->tm_P, a, ctx->grid, ctx->stream));
   if (timed) CK(cudaEventRecordWithFlags(ctx->ev[1], ctx->stream, cudaEventRecordExternal));
   // stage 2: UPP (+ U[par]) -> U[par^1]
   if (ctx->cfg.self_gravity) CK(enqueue_multigrid_soa(ctx, ctx->U[par], ctx->stream));
@@ -244,7 +244,7 @@ int enqueue_step(tlq_ctx* ctx, int par, bool timed) {
   if (mixed)
     CK(launch_stage_mixed(2, ctx->tm_UPP, a, ctx->grid, ctx->stream));
   else
-    CK(launch_stage(2, ctx->cfg.precision, ctx->tm_UPP, ctx->tm_P, a, ctx->grid, ctx->stream));
+    CK(launch_stage(2, ctx->tm_UPP, ctx->tm_P, a, ctx->grid, ctx->stream));
   if (timed) CK(cudaEventRecordWithFlags(ctx->ev[2], ctx->stream, cudaEventRecordExternal));
   // surrogate cooling + the dt reduction (stage 2 leaves both to it)
   if (ctx->cfg.cooling == TLQ_COOL_MLP)
@@ -447,10 +447,10 @@ int tlq_create(const tlq_config* cfg, tlq_ctx** out) {
   if (prepare_stage_kernels() != cudaSuccess) return bail(TLQ_ERR_CUDA);
   if (cfg->precision == TLQ_PREC_MIXED && prepare_mixed_kernels() != cudaSuccess) return bail(TLQ_ERR_CUDA);
   const bool mixed = cfg->precision == TLQ_PREC_MIXED;
-  int r = make_map(ctx, &ctx->tm_U[0], ctx->U[0], 5, 8, mixed);
-  if (!r) r = make_map(ctx, &ctx->tm_U[1], ctx->U[1], 5, 8, mixed);
+  int r = make_map(ctx, &ctx->tm_U[0], ctx->U[0], 5, 8, true);
+  if (!r) r = make_map(ctx, &ctx->tm_U[1], ctx->U[1], 5, 8, true);
   if (!r) r = make_map(ctx, &ctx->tm_UPP, ctx->UPP, 5, mixed ? 4 : 8);
-  if (!r) r = make_map(ctx, &ctx->tm_P, ctx->Pc, 1);
+  if (!r) r = make_map(ctx, &ctx->tm_P, ctx->Pc, 1, 8, true);
   if (r) return bail(r);
   for (int q = 0; q < 6; ++q) cudaEventCreate(&ctx->ev[q]);
   if (cudaDeviceSynchronize() != cudaSuccess) return bail(TLQ_ERR_CUDA);

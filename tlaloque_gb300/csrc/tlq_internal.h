@@ -32,9 +32,8 @@ constexpr int RED_THREADS = 256;  // block size of the reduction kernels
 
 // Fused step (FP64 instantiations in tlq_kernels.cu).
 cudaError_t prepare_stage_kernels();
-size_t stage_smem_bytes(int precision);
-cudaError_t launch_stage(int stage, int precision, const CUtensorMap& tm_in, const CUtensorMap& tm_p,
-                         const StageArgs& a, dim3 grid, cudaStream_t s);
+cudaError_t launch_stage(int stage, const CUtensorMap& tm_in, const CUtensorMap& tm_p, const StageArgs& a, dim3 grid,
+                         cudaStream_t s);
 
 // Mixed-precision stage kernels (tlq_mixed.cu).
 cudaError_t prepare_mixed_kernels();

@@ -19,22 +19,34 @@ constexpr int BT = 256;  // block size of the simple kernels
 // ===========================================================================
 // Fused stage kernels
 // ===========================================================================
-size_t stage_smem_bytes(int /*precision*/) { return sizeof(StageSmem<double>); }
-
+// The specialised instance: van Leer with HLLC, the reference's default
+// pairing (user/parameters.f90); every other pairing runs the generic one.
 cudaError_t prepare_stage_kernels() {
-  const int smem = (int)sizeof(StageSmem<double>);
-  cudaError_t e = cudaFuncSetAttribute(stage_kernel<1, double>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  if (e != cudaSuccess) return e;
-  return cudaFuncSetAttribute(stage_kernel<2, double>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  const void* ks[4] = {(const void*)stage_kernel<1, -1, -1>, (const void*)stage_kernel<2, -1, -1>,
+                       (const void*)stage_kernel<1, LIM_VANLEER, SOLVER_HLLC>,
+                       (const void*)stage_kernel<2, LIM_VANLEER, SOLVER_HLLC>};
+  for (int q = 0; q < 4; ++q) {
+    const int smem = q % 2 == 0 ? (int)sizeof(StageSmem<1>) : (int)sizeof(StageSmem<2>);
+    const cudaError_t e = cudaFuncSetAttribute(ks[q], cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
 }
 
-cudaError_t launch_stage(int stage, int /*precision*/, const CUtensorMap& tm_in, const CUtensorMap& tm_p,
-                         const StageArgs& a, dim3 grid, cudaStream_t s) {
-  const size_t smem = sizeof(StageSmem<double>);
-  if (stage == 1)
-    stage_kernel<1, double><<<grid, NT, smem, s>>>(tm_in, tm_p, a);
-  else
-    stage_kernel<2, double><<<grid, NT, smem, s>>>(tm_in, tm_p, a);
+cudaError_t launch_stage(int stage, const CUtensorMap& tm_in, const CUtensorMap& tm_p, const StageArgs& a, dim3 grid,
+                         cudaStream_t s) {
+  const bool spec = a.p.limiter == LIM_VANLEER && a.p.solver == SOLVER_HLLC;
+  if (stage == 1) {
+    if (spec)
+      stage_kernel<1, LIM_VANLEER, SOLVER_HLLC><<<grid, NT, sizeof(StageSmem<1>), s>>>(tm_in, tm_p, a);
+    else
+      stage_kernel<1, -1, -1><<<grid, NT, sizeof(StageSmem<1>), s>>>(tm_in, tm_p, a);
+  } else {
+    if (spec)
+      stage_kernel<2, LIM_VANLEER, SOLVER_HLLC><<<grid, NT, sizeof(StageSmem<2>), s>>>(tm_in, tm_p, a);
+    else
+      stage_kernel<2, -1, -1><<<grid, NT, sizeof(StageSmem<2>), s>>>(tm_in, tm_p, a);
+  }
   return cudaGetLastError();
 }
 

@@ -15,12 +15,14 @@
 
 namespace tlq {
 
-// Quotient and square root of the step's arithmetic: in FP64 on the integer
-// pipe (tlq_softfp.cuh: the hardware operations' bits; a division on GB300's
-// FP64 pipe takes 133 SM cycles a warp, 29 there, a square root 139 and 35),
-// in FP32 the hardware's.
+// Quotient, square root and (where the FP64 pipe is the busier one) product of
+// the step's arithmetic: in FP64 on the integer pipe (tlq_softfp.cuh: the
+// hardware operations' bits; a division on GB300's FP64 pipe takes 133 SM
+// cycles a warp, 23 there, a square root 139 and 33), in FP32 the hardware's.
 __device__ __forceinline__ double quot(double a, double b) { return sf::div(a, b); }
 __device__ __forceinline__ float quot(float a, float b) { return a / b; }
+__device__ __forceinline__ double prod(double a, double b) { return sf::mul(a, b); }
+__device__ __forceinline__ float prod(float a, float b) { return a * b; }
 __device__ __forceinline__ double root(double a) { return sf::sqrt_rn(a); }
 __device__ __forceinline__ float root(float a) { return sqrt(a); }
 // Several quotients by one divisor.
@@ -126,12 +128,17 @@ __device__ __forceinline__ double zcoord(const Params& p, int k) { return (p.zl 
 // ---------------------------------------------------------------------------
 template <class R>
 __device__ __forceinline__ void cons2prim(R g, const R* u, R* w) {
-  const auto r = divisor(u[0]);
+  const auto r = divisor(u[0]);  // (one reciprocal for the four quotients)
   w[0] = u[0];
   w[1] = quot(u[1], r);
   w[2] = quot(u[2], r);
   w[3] = quot(u[3], r);
-  w[4] = (g - R(1.0)) * (u[4] - quot(R(0.5) * ((u[1] * u[1] + u[2] * u[2]) + u[3] * u[3]), r));
+  const R k2 = (u[1] * u[1] + u[2] * u[2]) + u[3] * u[3];
+  if constexpr (sizeof(R) == 8) {  // halving is exact: (0.5 k2)/rho = 0.5 (k2/rho), taken with the difference in one FMA
+    w[4] = (g - 1.0) * __fma_rn(-0.5, quot(k2, r), u[4]);
+  } else {
+    w[4] = (g - R(1.0)) * (u[4] - R(0.5) * k2 / u[0]);
+  }
   w[4] = mx(w[4], R(1e-20));
 }
 
@@ -162,8 +169,9 @@ __device__ __forceinline__ R average(R a, R b, int opt) {
         if (!(xy > 0.0f)) return R(0.0);
         return __fdividef(xy * (x + y), fmaf(x, x, y * y)) * __uint_as_float(eb);
       } else {
-        if (a * b <= R(0.0)) return R(0.0);
-        return quot(a * b * (a + b), a * a + b * b);
+        const R ab = prod(a, b);
+        if (ab <= R(0.0)) return R(0.0);
+        return quot(prod(ab, a + b), prod(a, a) + prod(b, b));
       }
     case LIM_MINMOD:
       s = sgn1(a);

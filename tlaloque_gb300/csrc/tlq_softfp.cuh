@@ -5,10 +5,11 @@
 // Why: GB300 runs FP64 at 1/64 of the FP32 rate.  Measured with 16 warps per
 // SM of independent chains, an addition, multiplication or FMA takes 18.6 SM
 // cycles per warp, a division 133 and a square root 139 (their Newton steps
-// are FMAs on the same pipe); below, a division takes 29, a square root 35
-// and a multiplication 17.5, on pipes that run beside the FP64 one (4
-// multiplications here beside 4 FP64 additions: 82 cycles, the additions
-// alone 76).
+// are FMAs on the same pipe); below, a division takes 23, a square root 33
+// and a multiplication 15, on pipes that run beside the FP64 one (4
+// multiplications here beside 4 FP64 additions: 75 cycles, the additions
+// alone 72).  Dependent: a division 103 ns (280 on the FP64 pipe), a square
+// root 148 (299), a multiplication 75 (39).
 //
 // How: schoolbook long division and digit-by-digit square root on the
 // 53-bit significands with ~30-bit digits.  An FP32 reciprocal (square
@@ -116,6 +117,31 @@ TLQ_SF float rsqrt_seed(float x) {
 #else
   return TLQ_SF_HOST_SEED((float)(1.0 / std::sqrt((double)x)));
 #endif
+}
+
+// The upper word of (hi:lo) << n, 0 < n < 32.
+TLQ_SF uint32_t shl2(uint32_t hi, uint32_t lo, uint32_t n) {
+#if defined(__CUDA_ARCH__)
+  return __funnelshift_l(lo, hi, n);
+#else
+  return (hi << n) | (lo >> (32u - n));
+#endif
+}
+// (h:l) rounded to nearest even by the 32 bits f that follow (their lowest
+// sticky): plus the carry of f + (2^31 - 1) + odd.
+TLQ_SF double round_up(uint32_t h, uint32_t l, uint32_t f) {
+  const uint32_t c = 0x7fffffffu + (l & 1u);
+#if defined(__CUDA_ARCH__)
+  asm("{\n\t.reg .u32 t;\n\tadd.cc.u32 t, %2, %3;\n\taddc.cc.u32 %1, %1, 0;\n\taddc.u32 %0, %0, 0;\n\t}"
+      : "+r"(h), "+r"(l)
+      : "r"(f), "r"(c));
+#else
+  const uint64_t up = ((uint64_t)f + c) >> 32;
+  const uint64_t v = (((uint64_t)h << 32) | l) + up;
+  h = (uint32_t)(v >> 32);
+  l = (uint32_t)v;
+#endif
+  return make(h, l);
 }
 
 // Reciprocal of a normal double's significand: V ~ 2^63 / Bt, Bt = the
@@ -232,31 +258,31 @@ TLQ_SF double sqrt_rn(double a) {
 // a * b.
 TLQ_SF double mul(double a, double b) {
   const uint32_t ah = hi32(a), al = lo32(a), bh = hi32(b), bl = lo32(b);
-  const int ea = (int)((ah >> 20) & 0x7ffu), eb = (int)((bh >> 20) & 0x7ffu);
-  int e = ea + eb - 1023;
   const uint32_t sign = (ah ^ bh) & 0x80000000u;
-  const bool aok = (uint32_t)(ea - 1) < 2046u, bok = (uint32_t)(eb - 1) < 2046u;
-  if (!(aok && bok && (uint32_t)(e - 2) < 2043u)) {
-    const bool az = ((ah & 0x7fffffffu) | al) == 0u, bz = ((bh & 0x7fffffffu) | bl) == 0u;
-    if ((az && (bok || bz)) || (bz && aok)) return make(sign, 0u);
+  // exponent fields less 512: in range while below 2^10, the product's too
+  // while their sum stays below 2045
+  const uint32_t ea = (ah & 0x7ff00000u) - 0x20000000u, eb = (bh & 0x7ff00000u) - 0x20000000u;
+  if (((ea | eb) & 0xc0000000u) || ea + eb >= 0x7fd00000u) {
+    const uint32_t za = (ah & 0x7fffffffu) | al, zb = (bh & 0x7fffffffu) | bl;
+    if ((za == 0u && (bh & 0x7ff00000u) != 0x7ff00000u) || (zb == 0u && (ah & 0x7ff00000u) != 0x7ff00000u))
+      return make(sign, 0u);  // 0 * finite
     return mul_slow(a, b);
   }
-  const uint32_t mh = (ah & 0xfffffu) | 0x100000u, nm = (bh & 0xfffffu) | 0x100000u;
-  const uint32_t nh = (nm << 11) | (bl >> 21), nl = bl << 11;
-  const uint64_t p0 = mulw(al, nl);
-  const uint64_t m1 = mulw(al, nh) + (p0 >> 32);
-  const uint64_t m2 = mulw(mh, nl) + (uint32_t)m1;
-  uint64_t h = mulw(mh, nh) + (m1 >> 32) + (m2 >> 32);  // the product's bits from 2^64 on: [2^51, 2^53)
-  uint32_t f = (uint32_t)m2;                            // the next 32
-  const uint32_t st = (uint32_t)p0 != 0u ? 1u : 0u;
-  if (!((uint32_t)(h >> 32) & 0x100000u)) {
-    h = (h << 1) | (f >> 31);
-    f <<= 1;
-    e -= 1;
-  }
-  const bool up = (f | st) > 0x80000000u - ((uint32_t)h & 1u);
-  h += up ? 1u : 0u;
-  return make((uint32_t)(h >> 32) + ((uint32_t)e << 20) + sign, (uint32_t)h);
+  const uint32_t mh = (ah & 0xfffffu) | 0x100000u, nh = (bh & 0xfffffu) | 0x100000u;
+  // the product's words w0..w3 (106 bits, the leading one at bit 104 or 105)
+  const uint64_t p0 = mulw(al, bl);
+  const uint64_t p1 = mulw(al, nh) + (p0 >> 32);
+  const uint64_t p2 = mulw(mh, bl) + (uint32_t)p1;
+  const uint64_t p3 = mulw(mh, nh) + (p1 >> 32) + (p2 >> 32);
+  const uint32_t w0 = (uint32_t)p0, w1 = (uint32_t)p2, w2 = (uint32_t)p3, w3 = (uint32_t)(p3 >> 32);
+  const uint32_t one = w3 >> 9;  // 1: the product of the significands is 2 or more
+  const uint32_t sh = 12u - one;
+  const uint32_t h = shl2(w3, w2, sh), l = shl2(w2, w1, sh);
+  // the next 32 bits, the rest as a sticky bit (w0's bits that moved into f
+  // are zero wherever f is the tie 2^31, so w0 != 0 says the same)
+  const uint32_t f = shl2(w1, w0, sh) | (w0 != 0u ? 1u : 0u);
+  const uint32_t e = ea + eb + (one << 20) + sign;  // (h holds the leading one)
+  return round_up(h + e, l, f);
 }
 
 }  // namespace sf

@@ -20,8 +20,6 @@
 namespace tlq {
 
 constexpr int TX = 16, TY = 8, NT = TX * TY;
-constexpr int HX = TX + 4, HY = TY + 4;  // halo-2 box
-constexpr int PLANE_BOX = HY * HX;
 
 // Tile of the mixed-form kernels (its own constants, so that it can be tuned
 // apart from the plain form's): MTX x MTY columns on MNT threads, a multiple
@@ -36,10 +34,9 @@ constexpr int PLANE_BOX = HY * HX;
 #define TLQ_MNT 128
 #endif
 constexpr int MTX = TLQ_MTX, MTY = TLQ_MTY, MNT = TLQ_MNT;
-constexpr int MHX = MTX + 4, MHY = MTY + 4;  // halo-2 box
 static_assert(MTX * MTY <= MNT, "one cell per thread");
 static_assert(MTX % 16 == 0 && MNT % 32 == 0, "tile shape");
-constexpr int NRING = 4;
+constexpr int NRING = 3;
 constexpr long long WAIT_LIMIT = 1LL << 24;  // mbarrier polls before giving up
 
 struct StageArgs {
@@ -60,44 +57,62 @@ struct StageArgs {
   unsigned long long* cool_counts;  // [2]: the cells stage 2 cooled in a single step
 };
 
-template <class R>
+// Geometry of the planes the plain form stages in shared memory (x fastest,
+// tile cell (tx, ty) at (OY + ty, 2 + tx)): 2 halo cells in x (a TMA box of
+// FP64 values starts on an even cell), in y the faces' own reach (1 in stage
+// 1, 2 in stage 2).
+template <int S>
+struct Geo {
+  static constexpr int OY = S, PX = TX + 4, PY = TY + 2 * OY, PB = PX * PY;
+};
+
+// Shared memory of the plain form's kernels: three planes of conserved
+// values (the TMA's landing slots), the primitives of the plane whose x and y
+// faces are evaluated, and the x and y fluxes.  What the z faces need of
+// their own column lives in the column's thread, so a block takes 62 KB and
+// 3 blocks fit an SM (107 KB and 2 with four planes of both forms and every
+// flux in shared memory).
+template <int S>
 struct StageSmem {
-  double raw[NRING][5 * PLANE_BOX];  // TMA landing zone (conserved, FP64)
-  double praw[NRING][PLANE_BOX];     // TMA landing zone (carried pressure)
-  R prm[NRING][5][HY][HX];           // primitives of the ring planes
-  R fx[5][TY][TX + 1];               // x-face fluxes of the current plane
-  R fy[5][TY + 1][TX];               // y-face fluxes of the current plane
-  R fz[2][5][TY][TX];                // z-face fluxes k-1/2, k+1/2
+  static constexpr int NP = (S == 1) ? 8 : 5;  // stage 1 adds the cell's sound speed, E/rho and enthalpy
+  // (slots padded to 128 bytes, the TMA's destination alignment)
+  double raw[NRING][(5 * Geo<S>::PB + 15) / 16 * 16];
+  double praw[S == 1 ? NRING : 1][S == 1 ? (Geo<S>::PB + 15) / 16 * 16 : 16];  // the carried pressure (stage 1 with cooling)
+  double prm[NP][Geo<S>::PB];
+  double sx[S == 2 ? 5 : 1][S == 2 ? TY * (TX + 2) : 1];  // x and y slopes of the plane's cells
+  double sy[S == 2 ? 5 : 1][S == 2 ? (TY + 2) * TX : 1];
+  double fx[5][TY][TX + 1];
+  double fy[5][TY + 1][TX];
   uint64_t bar[NRING];
   double red[96];
   int flag;
   int abort;
 };
 
-// Ghost targets of one interior cell along one axis (boundaries.f90 non-MPI
-// branches).  layers = 1: boundariesI (:183-257); layers = 2: boundariesII
-// (:433-531).  Returns the number of (target index, flip) pairs.
-__device__ __forceinline__ int ghost_targets(int layers, int bclo, int bchi, int c, int n, int* tgt, int* flip) {
-  int m = 0;
-  if (bclo == BC_OUTFLOW) {
-    if (c == 1) { tgt[m] = 0; flip[m++] = 0; if (layers == 2) { tgt[m] = -1; flip[m++] = 0; } }
-  } else if (bclo == BC_REFLECTIVE) {
-    if (c == 1) { tgt[m] = 0; flip[m++] = 1; }
-    if (layers == 2 && c == 2) { tgt[m] = -1; flip[m++] = 1; }
-  } else if (bclo == BC_PERIODIC) {
-    if (c == n) { tgt[m] = 0; flip[m++] = 0; }
-    if (layers == 2 && c == n - 1) { tgt[m] = -1; flip[m++] = 0; }
+// The face-ghost images of interior cell (i, j, k) (boundaries.f90 non-MPI
+// branches; layers = 1: boundariesI :183-257, layers = 2: boundariesII
+// :433-531): put(axis, flip, gi, gj, gk) for each ghost cell that takes this
+// cell's value (flip: with the momentum along the axis negated).  Rolled
+// loops: few cells come here, and unrolled this code (with what put inlines)
+// was most of a stage kernel's 0.5-0.9 MB of instructions (now 0.12-0.36).
+// (Stage 1 of the mixed form keeps its unrolled ghost_targets: rolled, its
+// plane loop compiled 5 % slower on the 256^3 bubble.)
+template <class Put>
+__device__ __forceinline__ void ghost_images(const Params& p, int layers, int i, int j, int k, Put put) {
+#pragma unroll 1
+  for (int f = 0; f < 6; ++f) {
+    const int ax = f >> 1, hi = f & 1, bc = p.bc[f];
+    const int c = ax == 0 ? i : (ax == 1 ? j : k), n = ax == 0 ? p.nx : (ax == 1 ? p.ny : p.nz);
+#pragma unroll 1
+    for (int l = 0; l < layers; ++l) {
+      // the interior cell ghost layer l of this side copies
+      const bool from_hi = (bc == BC_PERIODIC) != (hi != 0);
+      const int off = bc == BC_OUTFLOW ? 0 : l;
+      if (c != (from_hi ? n - off : 1 + off)) continue;
+      const int g = hi ? n + 1 + l : -l;
+      put(ax, bc == BC_REFLECTIVE, ax == 0 ? g : i, ax == 1 ? g : j, ax == 2 ? g : k);
+    }
   }
-  if (bchi == BC_OUTFLOW) {
-    if (c == n) { tgt[m] = n + 1; flip[m++] = 0; if (layers == 2) { tgt[m] = n + 2; flip[m++] = 0; } }
-  } else if (bchi == BC_REFLECTIVE) {
-    if (c == n) { tgt[m] = n + 1; flip[m++] = 1; }
-    if (layers == 2 && c == n - 1) { tgt[m] = n + 2; flip[m++] = 1; }
-  } else if (bchi == BC_PERIODIC) {
-    if (c == 1) { tgt[m] = n + 1; flip[m++] = 0; }
-    if (layers == 2 && c == 2) { tgt[m] = n + 2; flip[m++] = 0; }
-  }
-  return m;
 }
 
 // Write the face-ghost images of cell (i, j, k), whose value (before the
@@ -105,32 +120,138 @@ __device__ __forceinline__ int ghost_targets(int layers, int bclo, int bchi, int
 // (borders applies user_boundaries after the face fill).
 __device__ __forceinline__ void write_ghosts(const Params& p, const Layout& L, double* out, int layers, int i, int j,
                                              int k, const double* v) {
-  const int c3[3] = {i, j, k};
-  const int n3[3] = {p.nx, p.ny, p.nz};
+  ghost_images(p, layers, i, j, k, [&](int ax, bool flip, int gi, int gj, int gk) {
+    double g[5];
 #pragma unroll
-  for (int ax = 0; ax < 3; ++ax) {
-    int tgt[4], flp[4];
-    const int m = ghost_targets(layers, p.bc[2 * ax], p.bc[2 * ax + 1], c3[ax], n3[ax], tgt, flp);
-    for (int q = 0; q < m; ++q) {
-      int g3[3] = {i, j, k};
-      g3[ax] = tgt[q];
-      double g[5];
+    for (int e = 0; e < 5; ++e) g[e] = (flip && e == ax + 1) ? -v[e] : v[e];
+    winds_cell(p, gi, gj, gk, g);
+    const long long o = L.at(gi, gj, gk);
 #pragma unroll
-      for (int e = 0; e < 5; ++e) g[e] = (flp[q] && e == ax + 1) ? -v[e] : v[e];
-      winds_cell(p, g3[0], g3[1], g3[2], g);
-      const long long o = L.at(g3[0], g3[1], g3[2]);
+    for (int e = 0; e < 5; ++e) out[e * L.plane + o] = g[e];
+  });
+}
+
+// ---------------------------------------------------------------------------
+// One face's flux in direction d from the states beside it: HLL[C] of
+// riemann (tlq_physics.cuh) operation for operation, with what the cells
+// share formed once per cell instead of once per face.  cl, cr: the sound
+// speeds; el, er: E/rho of the two sides (0.0 in stage 2, which forms the
+// chosen side's); hl, hr: (1/2) rho v^2 + g1 p, likewise; UL, UR: the
+// cell-centred conserved states, `us` doubles between variables.
+//   Every 0.5 x is exact, so its sum with the next term takes one FMA, the
+// rounding unchanged.  prod: a multiplication on the integer pipe.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ double enthalpy(double g1, const double* w) {
+  return __fma_rn(0.5, w[0] * ((w[1] * w[1] + w[2] * w[2]) + w[3] * w[3]), g1 * w[4]);
+}
+
+// prim2f of tlq_physics.cuh with the mass flux m = rho un and h given.
+__device__ __forceinline__ void flux_of(double* ff, const double* w, double un, double m, double h, int d) {
+  ff[0] = m;
 #pragma unroll
-      for (int e = 0; e < 5; ++e) out[e * L.plane + o] = g[e];
+  for (int e = 1; e <= 3; ++e) {
+    // (rho u_lo) u_hi, lo < hi the two component indices
+    const double t = ((e < d) ? w[0] * w[e] : m) * ((e < d) ? un : w[e]);
+    ff[e] = (e == d) ? t + w[4] : t;
+  }
+  ff[4] = un * h;
+}
+
+template <int STAGE, int SOLV>
+__device__ __forceinline__ void face_flux(const Params& p, double* ff, const double* wl, const double* wr, double cl,
+                                          double cr, double el, double er, double hl, double hr, const double* UL,
+                                          const double* UR, int us, int d) {
+  const double ul = comp(wl, d), ur = comp(wr, d);
+  const double sl = mn(ul - cl, ur - cr);
+  const double sr = mx(ul + cl, ur + cr);
+  const double ml = prod(wl[0], ul), mr = prod(wr[0], ur);
+  if (SOLV == SOLVER_HLL || (SOLV < 0 && p.solver == SOLVER_HLL)) {
+    if (sl >= 0.0 || sr <= 0.0) {
+      const bool left = sl >= 0.0;
+      double w[5];
+#pragma unroll
+      for (int e = 0; e < 5; ++e) w[e] = left ? wl[e] : wr[e];
+      flux_of(ff, w, left ? ul : ur, left ? ml : mr, STAGE == 1 ? (left ? hl : hr) : enthalpy(p.g1, w), d);
+    } else {
+      double fl[5], fr[5];
+      flux_of(fl, wl, ul, ml, STAGE == 1 ? hl : enthalpy(p.g1, wl), d);
+      flux_of(fr, wr, ur, mr, STAGE == 1 ? hr : enthalpy(p.g1, wr), d);
+      const auto ds = divisor(sr - sl);
+      const double ss = prod(sl, sr);
+#pragma unroll
+      for (int e = 0; e < 5; ++e) 
+        ff[e] = quot(prod(sr, fl[e]) - prod(sl, fr[e]) + prod(ss, UR[e * us] - UL[e * us]), ds);
     }
+    return;  // NaN speeds take the HLL average branch, as in the reference
+  }
+  const double dl = sl - ul, dr = sr - ur;
+  const double al = prod(wl[0], dl), ar = prod(wr[0], dr);
+  const double sst = quot(wr[4] - wl[4] + prod(ml, dl) - prod(mr, dr), al - ar);
+  // Branch order of the reference: sl>=0, sr<=0, sst>=0, sst<=0; a face with
+  // NaN speeds takes none (NaN here)
+  bool star, left;
+  if (sl >= 0.0) { star = false; left = true; }
+  else if (sr <= 0.0) { star = false; left = false; }
+  else if (sst >= 0.0) { star = true; left = true; }
+  else if (sst <= 0.0) { star = true; left = false; }
+  else {
+#pragma unroll
+    for (int e = 0; e < 5; ++e) ff[e] = NAN;
+    return;
+  }
+  double w[5];
+#pragma unroll
+  for (int e = 0; e < 5; ++e) w[e] = left ? wl[e] : wr[e];
+  const double un = left ? ul : ur;
+  flux_of(ff, w, un, left ? ml : mr, STAGE == 1 ? (left ? hl : hr) : enthalpy(p.g1, w), d);
+  if (star) {
+    const double* uc = left ? UL : UR;
+    const double s = left ? sl : sr;
+    const double a = left ? al : ar;  // rho (s - un)
+    const double rhostr = quot(a, s - sst);
+    const double eor = STAGE == 1 ? (left ? el : er) : quot(uc[4 * us], w[0]);
+    double u[5];
+    u[0] = rhostr;
+#pragma unroll
+    for (int e = 1; e <= 3; ++e) u[e] = prod(rhostr, (e == d) ? sst : w[e]);
+    u[4] = prod(rhostr, eor + prod(sst - un, sst + quot(w[4], a)));
+#pragma unroll
+    for (int e = 0; e < 5; ++e) ff[e] = ff[e] + prod(s, u[e] - uc[e * us]);
   }
 }
 
-template <int STAGE, class R>
-__global__ void __launch_bounds__(NT, 2)
-    stage_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant__ CUtensorMap tm_p, StageArgs a) {
-  constexpr int H = STAGE;  // reconstruction halo: 1st order needs 1 cell, 2nd order 2
+// The plain FP64 step's kernels.  What bounds them: the FP64 pipe (18.6 SM
+// cycles per warp instruction), so every operation whose result another face
+// or cell also needs is done once --
+//   stage 1: the sound speed, E/rho and enthalpy per cell (each was formed
+//     for all six faces of a cell);
+//   stage 2: the limited slopes per cell (the slope right of a face is the
+//     one left of the next face: one per cell and direction instead of two
+//     per face);
+// divisions and square roots run on the integer pipe (tlq_softfp.cuh).
+//   A thread owns a column of the tile.  Per plane: it converts the column's
+// next plane (kept in registers for the z direction), the block converts the
+// plane's halo, then (stage 2) the slopes, then the faces -- each thread its
+// cell's left x, lower y and upper z face, one warp in turn the tile's right
+// and upper edges -- through one copy of the code, then the cells' update.
+// The z flux stays in its thread.
+//   Measured, Sedov 128^3, 8-plane chunks: stage 1 2.90 -> 1.02 ms, stage 2
+// 5.09 -> 2.12 ms per launch against one face task list with the limiter and
+// sound speeds per face and hardware divisions (1.86 and 2.98 ms with those
+// off the FP64 pipe).  Now 159 FP64 operations per cell in stage 1 and 365 in
+// stage 2 at 75-80 % of that pipe's rate, beside 5,400 and 9,300 integer and
+// other instructions per warp of cells.  Which multiplications go to the
+// integer pipe is measured too: all of them, or none, is 3-12 % slower than
+// the star state's, the wave speeds', the limiter's and the update's.
+template <int STAGE, int LIM, int SOLV>
+__global__ void __launch_bounds__(NT, STAGE == 1 ? 4 : 3)
+    stage_kernel(const __grid_constant__ CUtensorMap tm_in, const __grid_constant__ CUtensorMap tm_p,
+                 const __grid_constant__ StageArgs a) {
+  using G = Geo<STAGE>;
+  using Smem = StageSmem<STAGE>;
+  constexpr int H = STAGE, OY = G::OY, PX = G::PX, PB = G::PB, NP = Smem::NP;
   extern __shared__ __align__(128) unsigned char smem_bytes[];
-  StageSmem<R>& s = *reinterpret_cast<StageSmem<R>*>(smem_bytes);
+  Smem& s = *reinterpret_cast<Smem*>(smem_bytes);
   const Params& p = a.p;
   const Layout& L = a.L;
   const int tid = threadIdx.x;
@@ -138,13 +259,15 @@ __global__ void __launch_bounds__(NT, 2)
   const int i0 = 1 + bx * TX, j0 = 1 + by * TY;
   const int k0 = 1 + (int)blockIdx.z * a.zlen;
   const int k1 = min(p.nz, k0 + a.zlen - 1);
+  const int lim = LIM >= 0 ? LIM : p.limiter;
   Clock* clk = a.clk;
 
   if (!(clk->t < clk->tfin)) return;  // the loop condition of mainHD.f90:61 (uniform)
   const double dtstep = clk->dt;
   const double dt = (STAGE == 1) ? dtstep / 2.0 : dtstep;  // dth = dt/2.0 (mainHD.f90:78)
   const double dtdx = dt / p.dx, dtdy = dt / p.dy, dtdz = dt / p.dz;
-  const uint32_t box_bytes = 5u * PLANE_BOX * 8u + (a.use_p ? PLANE_BOX * 8u : 0u);
+  const bool use_p = STAGE == 1 && a.use_p;
+  const uint32_t box_bytes = 5u * PB * 8u + (use_p ? PB * 8u : 0u);
   const int last_plane = k1 + H;
 
   if (tid == 0) {
@@ -154,13 +277,15 @@ __global__ void __launch_bounds__(NT, 2)
   }
   __syncthreads();
 
+  // Plane q lives in slot (q - (k0 - H)) mod 3.
+  auto slot_of = [&](int q) { return (unsigned)(q - (k0 - H)) % (unsigned)NRING; };
   int issued = k0 - H - 1;  // last plane issued (meaningful in thread 0)
-  auto issue = [&](int q) {  // thread 0: plane q of the input into slot q & 3
-    const int slot = q & 3;
+  auto issue = [&](int q) {  // thread 0
+    const int slot = slot_of(q);
     fence_proxy_async();
     mbar_arrive_expect_tx(&s.bar[slot], box_bytes);
-    tma_load_4d(s.raw[slot], &tm_in, &s.bar[slot], bx * TX, by * TY, q + 1, 0);
-    if (a.use_p) tma_load_4d(s.praw[slot], &tm_p, &s.bar[slot], bx * TX, by * TY, q + 1, 0);
+    tma_load_4d(s.raw[slot], &tm_in, &s.bar[slot], bx * TX, by * TY + 2 - OY, q + 1, 0);
+    if (use_p) tma_load_4d(s.praw[slot], &tm_p, &s.bar[slot], bx * TX, by * TY + 2 - OY, q + 1, 0);
     issued = q;
   };
   // Every thread waits for every plane in order and tracks the slot phases.
@@ -169,7 +294,7 @@ __global__ void __launch_bounds__(NT, 2)
   bool failed = false;
   auto wait_plane = [&](int q) {
     if (failed) return;
-    const int slot = q & 3;
+    const int slot = slot_of(q);
     if (!mbar_wait_bounded(&s.bar[slot], (phase >> slot) & 1u, WAIT_LIMIT)) {
       failed = true;
       s.abort = 1;
@@ -179,166 +304,221 @@ __global__ void __launch_bounds__(NT, 2)
     waited = q;
   };
 
-  // Primitives of plane q on the cross-shaped region the faces read.
-  auto convert = [&](int q) {
-    const int slot = q & 3;
-    constexpr int RW = TX + 2 * H;
-    constexpr int NROW = RW * TY, NCOL = TX * 2 * H;
-    for (int t = tid; t < NROW + NCOL; t += NT) {
-      int lx, ly;
-      if (t < NROW) {
-        lx = 2 - H + t % RW;
-        ly = 2 + t / RW;
-      } else {
-        const int u = t - NROW, r2 = u / TX;
-        lx = 2 + u % TX;
-        ly = (r2 < H) ? (2 - H + r2) : (TY + 2 + r2 - H);
-      }
-      const double* r = &s.raw[slot][ly * HX + lx];
-      R u[5], w[5];
-#pragma unroll
-      for (int e = 0; e < 5; ++e) u[e] = (R)r[e * PLANE_BOX];
-      cons2prim(R(p.gamma), u, w);
-      if (a.use_p) {
-        const int i = i0 - 2 + lx, j = j0 - 2 + ly;
-        if (i >= 1 && i <= p.nx && j >= 1 && j <= p.ny && q >= 1 && q <= p.nz) w[4] = (R)s.praw[slot][ly * HX + lx];
-      }
-#pragma unroll
-      for (int e = 0; e < 5; ++e) s.prm[slot][e][ly][lx] = w[e];
-    }
-  };
-
-  // Face fluxes: x and y faces of plane k (when xy) and the z face k+1/2.
-  auto faces = [&](int k, bool xy) {
-    constexpr int NXF = (TX + 1) * TY, NYF = TX * (TY + 1), NZF = TX * TY;
-    const int tbeg = xy ? 0 : NXF + NYF;
-    const int sk = k & 3;
-    constexpr int VS = PLANE_BOX;  // variable stride in prm and raw
-    for (int t = tbeg + tid; t < NXF + NYF + NZF; t += NT) {
-      int d, fxl, fyl;
-      const R *w0, *w1, *w2, *w3;
-      const double *uL, *uR;
-      bool valid;
-      if (t < NXF) {
-        d = 1;
-        fxl = t % (TX + 1);
-        fyl = t / (TX + 1);
-        const int ly = fyl + 2;
-        w0 = &s.prm[sk][0][ly][fxl];
-        w1 = w0 + 1; w2 = w0 + 2; w3 = w0 + 3;
-        uL = &s.raw[sk][ly * HX + fxl + 1];
-        uR = uL + 1;
-        valid = (i0 - 1 + fxl <= p.nx) && (j0 + fyl <= p.ny);
-      } else if (t < NXF + NYF) {
-        d = 2;
-        const int u = t - NXF;
-        fxl = u % TX;
-        fyl = u / TX;
-        const int lx = fxl + 2;
-        w0 = &s.prm[sk][0][fyl][lx];
-        w1 = w0 + HX; w2 = w0 + 2 * HX; w3 = w0 + 3 * HX;
-        uL = &s.raw[sk][(fyl + 1) * HX + lx];
-        uR = uL + HX;
-        valid = (i0 + fxl <= p.nx) && (j0 - 1 + fyl <= p.ny);
-      } else {
-        d = 3;
-        const int u = t - NXF - NYF;
-        fxl = u % TX;
-        fyl = u / TX;
-        const int lx = fxl + 2, ly = fyl + 2;
-        w0 = &s.prm[(k - 1) & 3][0][ly][lx];
-        w1 = &s.prm[k & 3][0][ly][lx];
-        w2 = &s.prm[(k + 1) & 3][0][ly][lx];
-        w3 = &s.prm[(k + 2) & 3][0][ly][lx];
-        uL = &s.raw[k & 3][ly * HX + lx];
-        uR = &s.raw[(k + 1) & 3][ly * HX + lx];
-        valid = (i0 + fxl <= p.nx) && (j0 + fyl <= p.ny);
-      }
-      if (!valid) continue;
-      R wll[5], wl[5], wr[5], wrr[5], UL[5], UR[5], ff[5];
-#pragma unroll
-      for (int e = 0; e < 5; ++e) {
-        wl[e] = w1[e * VS];
-        wr[e] = w2[e * VS];
-        UL[e] = (R)uL[e * VS];
-        UR[e] = (R)uR[e * VS];
-      }
-      if (STAGE == 2) {
-#pragma unroll
-        for (int e = 0; e < 5; ++e) {
-          wll[e] = w0[e * VS];
-          wrr[e] = w3[e * VS];
-        }
-        limiter(wll, wl, wr, wrr, p.limiter);
-      }
-      if (!riemann(p.solver, R(p.gamma), R(p.g1), ff, wl, wr, UL, UR, d)) {
-#pragma unroll
-        for (int e = 0; e < 5; ++e) ff[e] = R(NAN);
-      }
-      if (d == 1) {
-#pragma unroll
-        for (int e = 0; e < 5; ++e) s.fx[e][fyl][fxl] = ff[e];
-      } else if (d == 2) {
-#pragma unroll
-        for (int e = 0; e < 5; ++e) s.fy[e][fyl][fxl] = ff[e];
-      } else {
-#pragma unroll
-        for (int e = 0; e < 5; ++e) s.fz[(k + 1) & 1][e][fyl][fxl] = ff[e];
-      }
-    }
-  };
-
-  // ---- prologue: planes k0-H .. k0+H-1 and the z face k0-1/2 ---------------
-  if (tid == 0)
-    for (int q = k0 - H; q <= min(k0 - H + 3, last_plane); ++q) issue(q);
-  for (int q = k0 - H; q <= k0 + H - 1; ++q) wait_plane(q);
-  __syncthreads();
-  const bool aborted0 = s.abort != 0;
-  if (!aborted0)
-    for (int q = k0 - H; q <= k0 + H - 1; ++q) convert(q);
-  __syncthreads();
-  if (!aborted0) faces(k0 - 1, false);
-  __syncthreads();
-  if (STAGE == 2 && tid == 0 && !aborted0 && k0 + 2 <= last_plane) issue(k0 + 2);
-
   const int tx = tid % TX, ty = tid / TX;
   const int i = i0 + tx, j = j0 + ty;
   const bool cell_ok = (i <= p.nx) && (j <= p.ny);
-  double m0 = 0.0, m1 = 0.0, m2 = 0.0;  // CFL maxima (STAGE 2)
+  const int oc = (ty + OY) * PX + tx + 2;
 
-  bool aborted = aborted0;
-  for (int k = k0; k <= k1 && !aborted; ++k) {
+  // Primitives (and stage 1's derived values) of the cell at offset o of
+  // landed plane q, mesh indices (ii, jj).
+  auto convert = [&](int q, int o, int ii, int jj, double* w) {
+    if (ii > p.nx + 2 || jj > p.ny + 2) {  // beyond the mesh: no face reads it
+#pragma unroll
+      for (int e = 0; e < NP; ++e) w[e] = 1.0;
+      return;
+    }
+    const int slot = slot_of(q);
+    double u[5];
+#pragma unroll
+    for (int e = 0; e < 5; ++e) u[e] = s.raw[slot][e * PB + o];
+    cons2prim(p.gamma, u, w);
+    if constexpr (STAGE == 1) {
+      if (use_p && ii >= 1 && ii <= p.nx && jj >= 1 && jj <= p.ny && q >= 1 && q <= p.nz) w[4] = s.praw[slot][o];
+      const auto r = divisor(u[0]);
+      w[5] = root(quot(p.gamma * w[4], r));
+      w[6] = quot(u[4], r);
+      w[7] = enthalpy(p.g1, w);
+    }
+  };
+
+  // ---- prologue: the column's first planes ---------------------------------
+  if (tid == 0)
+    for (int q = k0 - H; q < k0 - H + NRING && q <= last_plane; ++q) issue(q);
+  // the column's primitives of plane k and k+1, its slope of plane k in z
+  // (stage 2) and its lower z flux
+  double w0[NP], w1[NP], sz[5], fz[5];
+#pragma unroll
+  for (int e = 0; e < 5; ++e) sz[e] = fz[e] = 0.0;
+  bool aborted = false;
+  for (int q = k0 - H; q < k0; ++q) {  // (stage 1: k0-1; stage 2: k0-2, k0-1)
+#pragma unroll
+    for (int e = 0; e < NP; ++e) w0[e] = w1[e];
+    wait_plane(q);
+    convert(q, oc, i, j, w1);
+  }
+  if (STAGE == 1) {
+#pragma unroll
+    for (int e = 0; e < NP; ++e) w0[e] = w1[e];
+  }
+  unsigned long long m0 = 0ull, m1 = 0ull, m2 = 0ull;  // CFL maxima as max_key keys (STAGE 2)
+
+  // Stage 1 starts at k0-1 (its z face k0-1/2), stage 2 at k0-2 (the z slope
+  // of k0-1).  At plane k: w0 = plane k (stage 2: w1 = plane k+1).
+  for (int k = k0 - H; k <= k1; ++k) {
+    const bool cells = k >= k0, zface = k >= k0 - 1;
+    const int slot = slot_of(k), slot1 = slot_of(k + 1);
+    double w2[NP];  // plane k + H
     wait_plane(k + H);
-    convert(k + H);   // reads garbage only if the wait gave up; discarded below
-    __syncthreads();  // S1
+    convert(k + H, oc, i, j, w2);  // (garbage if the wait gave up; discarded below)
+    if (cells) {
+#pragma unroll
+      for (int e = 0; e < NP; ++e) s.prm[e][oc] = w0[e];
+      constexpr int NROW = 2 * H * TY, NCOL = 2 * H * TX;
+      if (tid < NROW + NCOL) {  // the plane's halo
+        int lx, ly;
+        if (tid < NROW) {
+          const int c = tid / TY;
+          lx = c < H ? 2 - H + c : TX + 2 + c - H;
+          ly = OY + tid % TY;
+        } else {
+          const int u = tid - NROW, c = u / TX;
+          lx = 2 + u % TX;
+          ly = c < H ? OY - H + c : TY + OY + c - H;
+        }
+        double w[NP];
+        convert(k, ly * PX + lx, i0 - 2 + lx, j0 - OY + ly, w);
+#pragma unroll
+        for (int e = 0; e < NP; ++e) s.prm[e][ly * PX + lx] = w[e];
+      }
+    }
+    __syncthreads();  // the plane's primitives
     if (s.abort) { aborted = true; break; }
-    if (tid == 0 && k + 3 <= last_plane && k + 3 > issued) issue(k + 3);
-    faces(k, true);
-    __syncthreads();  // S2
+    if (STAGE == 1 && tid == 0 && k + 2 <= last_plane && k + 2 > issued) issue(k + 2);  // plane k-1's slot
 
-    if (cell_ok) {
-      const int cur = (k + 1) & 1, prv = k & 1;
+    double sz1[5];  // the z slope of plane k+1
+    if constexpr (STAGE == 2) {
+#pragma unroll 1
+      for (int r = cells ? 0 : 3; r < 4; ++r) {
+        double dm[5], dp[5];
+        double* out = nullptr;
+        int os = 0;
+        if (r == 3) {
+#pragma unroll
+          for (int e = 0; e < 5; ++e) {
+            dm[e] = w1[e] - w0[e];
+            dp[e] = w2[e] - w1[e];
+          }
+        } else {
+          // the own cell's x, its y, and the cells beside the tile (48 tasks,
+          // on the upper warps when k is odd)
+          int o, st, t = (k & 1) ? NT - 1 - tid : tid;
+          if (r == 0) { o = oc; st = 1; out = &s.sx[0][ty * (TX + 2) + tx + 1]; }
+          else if (r == 1) { o = oc; st = PX; out = &s.sy[0][(ty + 1) * TX + tx]; }
+          else if (t < 2 * TY) {
+            const int lx = t < TY ? 1 : TX + 2, row = t % TY;
+            o = (row + OY) * PX + lx; st = 1; out = &s.sx[0][row * (TX + 2) + lx - 1];
+          } else if (t < 2 * TY + 2 * TX) {
+            const int u = t - 2 * TY, ly = u < TX ? 1 : TY + 2;
+            o = ly * PX + 2 + u % TX; st = PX; out = &s.sy[0][(ly - 1) * TX + u % TX];
+          } else continue;
+          os = st == 1 ? TY * (TX + 2) : (TY + 2) * TX;
+#pragma unroll
+          for (int e = 0; e < 5; ++e) {
+            const double* c = &s.prm[e][o];
+            const double v = c[0];
+            dm[e] = v - c[-st];
+            dp[e] = c[st] - v;
+          }
+        }
+#pragma unroll
+        for (int e = 0; e < 5; ++e) {
+          const double v = average(dm[e], dp[e], lim);
+          if (r == 3) sz1[e] = v; else out[e * os] = v;
+        }
+      }
+      if (cells) __syncthreads();  // the plane's slopes
+    }
+
+    double fz1[5];
+    if (zface) {
+#pragma unroll 1
+      for (int r = cells ? 0 : 2; r < 4; ++r) {
+        double wl[NP], wr[NP], ff[5];
+        const double *uL, *uR;
+        double* out = nullptr;
+        int d, fs = 0;
+        if (r == 2) {
+          d = 3;
+          if (!cell_ok) continue;
+          if constexpr (STAGE == 1) {
+#pragma unroll
+            for (int e = 0; e < NP; ++e) { wl[e] = w0[e]; wr[e] = w2[e]; }
+          } else {
+#pragma unroll
+            for (int e = 0; e < 5; ++e) {
+              wl[e] = __fma_rn(0.5, sz[e], w0[e]);
+              wr[e] = __fma_rn(-0.5, sz1[e], w1[e]);
+            }
+          }
+          uL = &s.raw[slot][oc];
+          uR = &s.raw[slot1][oc];
+        } else {
+          // the left x face, the lower y face; the edges: x = TX (8 faces), y
+          // = TY (16), on warp k mod 4
+          int fxl = tx, fyl = ty;
+          d = r + 1;
+          if (r == 3) {
+            const int t = tid - 32 * (k & 3);
+            if (t < 0 || t >= TY + TX || !cells) continue;
+            d = t < TY ? 1 : 2;
+            fxl = t < TY ? TX : t - TY;
+            fyl = t < TY ? t : TY;
+          }
+          const int ii = i0 + fxl, jj = j0 + fyl;  // the cell right of (above) the face
+          if (!(d == 1 ? (ii - 1 <= p.nx && jj <= p.ny) : (ii <= p.nx && jj - 1 <= p.ny))) continue;
+          const int st = d == 1 ? 1 : PX, oR = (fyl + OY) * PX + fxl + 2, oL = oR - st;
+#pragma unroll
+          for (int e = 0; e < NP; ++e) {
+            wl[e] = s.prm[e][oL];
+            wr[e] = s.prm[e][oR];
+          }
+          if constexpr (STAGE == 2) {
+            const double* sp = d == 1 ? &s.sx[0][fyl * (TX + 2) + fxl] : &s.sy[0][fyl * TX + fxl];
+            const int one = d == 1 ? 1 : TX, ss = d == 1 ? TY * (TX + 2) : (TY + 2) * TX;
+#pragma unroll
+            for (int e = 0; e < 5; ++e) {
+              wl[e] = __fma_rn(0.5, sp[e * ss], wl[e]);
+              wr[e] = __fma_rn(-0.5, sp[e * ss + one], wr[e]);
+            }
+          }
+          uL = &s.raw[slot][oL];
+          uR = &s.raw[slot][oR];
+          out = d == 1 ? &s.fx[0][fyl][fxl] : &s.fy[0][fyl][fxl];
+          fs = d == 1 ? TY * (TX + 1) : (TY + 1) * TX;
+        }
+        if constexpr (STAGE == 1)
+          face_flux<1, SOLV>(p, ff, wl, wr, wl[5], wr[5], wl[6], wr[6], wl[7], wr[7], uL, uR, PB, d);
+        else
+          face_flux<2, SOLV>(p, ff, wl, wr, csound(p.gamma, wl[4], wl[0]), csound(p.gamma, wr[4], wr[0]), 0.0, 0.0,
+                             0.0, 0.0, uL, uR, PB, d);
+#pragma unroll
+        for (int e = 0; e < 5; ++e) {
+          if (r == 2) fz1[e] = ff[e]; else out[e * fs] = ff[e];
+        }
+      }
+    }
+    __syncthreads();  // the plane's fluxes; (stage 2) plane k's slot is free
+    if (STAGE == 2 && tid == 0 && k + 3 <= last_plane && k + 3 > issued) issue(k + 3);
+
+    if (cells && cell_ok) {
       const long long c = L.at(i, j, k);
       double uc[5], up[5];
       if (STAGE == 1) {
 #pragma unroll
-        for (int e = 0; e < 5; ++e) uc[e] = s.raw[k & 3][e * PLANE_BOX + (ty + 2) * HX + tx + 2];
+        for (int e = 0; e < 5; ++e) uc[e] = s.raw[slot][e * PB + oc];
       } else {
 #pragma unroll
         for (int e = 0; e < 5; ++e) uc[e] = a.uold[e * L.plane + c];
       }
 #pragma unroll
       for (int e = 0; e < 5; ++e)
-        up[e] = uc[e] - dtdx * ((double)s.fx[e][ty][tx + 1] - (double)s.fx[e][ty][tx]) -
-                dtdy * ((double)s.fy[e][ty + 1][tx] - (double)s.fy[e][ty][tx]) -
-                dtdz * ((double)s.fz[cur][e][ty][tx] - (double)s.fz[prv][e][ty][tx]);
+        up[e] = uc[e] - prod(dtdx, s.fx[e][ty][tx + 1] - s.fx[e][ty][tx]) -
+                prod(dtdy, s.fy[e][ty + 1][tx] - s.fy[e][ty][tx]) - prod(dtdz, fz1[e] - fz[e]);
       if (p.gravity) {  // Godunov's + dt*S (source/HLLC.f90:39-41)
         const double* ph = a.phi;
         const long long pxy = (long long)L.px * L.nyg;
-        double w[5], sv[5];
-#pragma unroll
-        for (int e = 0; e < 5; ++e) w[e] = (double)s.prm[k & 3][e][ty + 2][tx + 2];
-        gravity_cell(p, w, ph[c + 1] - ph[c - 1], ph[c + L.px] - ph[c - L.px], ph[c + pxy] - ph[c - pxy], sv);
+        double sv[5];
+        gravity_cell(p, w0, ph[c + 1] - ph[c - 1], ph[c + L.px] - ph[c - L.px], ph[c + pxy] - ph[c - pxy], sv);
 #pragma unroll
         for (int e = 0; e < 5; ++e) up[e] = up[e] + dt * sv[e];
       }
@@ -359,7 +539,7 @@ __global__ void __launch_bounds__(NT, 2)
 #pragma unroll
         for (int e = 0; e < 5; ++e) {
           const double* uo = a.uold + e * L.plane + c;
-          un[e] = up[e] + p.eta * (uo[1] + uo[-1] + uo[L.px] + uo[-L.px] + uo[pxy] + uo[-pxy] - 6.0 * uc[e]);
+          un[e] = up[e] + prod(p.eta, uo[1] + uo[-1] + uo[L.px] + uo[-L.px] + uo[pxy] + uo[-pxy] - 6.0 * uc[e]);
         }
         cons2prim(p.gamma, un, w);  // calc_prims(UPrim, U)
         if (p.cooling != COOL_NONE) {
@@ -371,10 +551,25 @@ __global__ void __launch_bounds__(NT, 2)
         for (int e = 0; e < 5; ++e) a.out[e * L.plane + c] = un[e];
         double v3[3];
         signal_speeds(p.gamma, w, v3);
-        m0 = max_nan(m0, v3[0]);
-        m1 = max_nan(m1, v3[1]);
-        m2 = max_nan(m2, v3[2]);
+        m0 = max(m0, max_key(v3[0]));
+        m1 = max(m1, max_key(v3[1]));
+        m2 = max(m2, max_key(v3[2]));
       }
+    }
+    if constexpr (STAGE == 2) {
+#pragma unroll
+      for (int e = 0; e < 5; ++e) {
+        w0[e] = w1[e];
+        w1[e] = w2[e];
+        sz[e] = sz1[e];
+      }
+    } else {
+#pragma unroll
+      for (int e = 0; e < NP; ++e) w0[e] = w2[e];
+    }
+    if (zface) {
+#pragma unroll
+      for (int e = 0; e < 5; ++e) fz[e] = fz1[e];
     }
   }
 
@@ -384,14 +579,14 @@ __global__ void __launch_bounds__(NT, 2)
     if (tid == 0) {
       atomicOr(&clk->status, ST_TIMEOUT);
       for (int q = waited + 1; q <= issued; ++q) {
-        const int slot = q & 3;
+        const int slot = slot_of(q);
         mbar_wait_bounded(&s.bar[slot], (phase >> slot) & 1u, WAIT_LIMIT);
         phase ^= 1u << slot;
       }
     }
-    m0 = m1 = m2 = NAN;
+    m0 = m1 = m2 = ~0ull;
   }
-  if (STAGE == 2) cfl_reduce_finalize<NT>(m0, m1, m2, clk, p, true, s.red, &s.flag);
+  if (STAGE == 2) cfl_reduce_finalize<NT>(key_value(m0), key_value(m1), key_value(m2), clk, p, true, s.red, &s.flag);
 }
 
 }  // namespace tlq

@@ -324,6 +324,32 @@ __device__ __forceinline__ void cool_cell_f(const Params& p, float cT, float inv
   cool_cell_known(p, cT, inv_muamu, gm1, w, u4, dt, temp, aloss, seg);
 }
 
+// Ghost targets of one interior cell along one axis (boundaries.f90 non-MPI
+// branches).  layers = 1: boundariesI (:183-257); layers = 2: boundariesII
+// (:433-531).  Returns the number of (target index, flip) pairs.
+__device__ __forceinline__ int ghost_targets(int layers, int bclo, int bchi, int c, int n, int* tgt, int* flip) {
+  int m = 0;
+  if (bclo == BC_OUTFLOW) {
+    if (c == 1) { tgt[m] = 0; flip[m++] = 0; if (layers == 2) { tgt[m] = -1; flip[m++] = 0; } }
+  } else if (bclo == BC_REFLECTIVE) {
+    if (c == 1) { tgt[m] = 0; flip[m++] = 1; }
+    if (layers == 2 && c == 2) { tgt[m] = -1; flip[m++] = 1; }
+  } else if (bclo == BC_PERIODIC) {
+    if (c == n) { tgt[m] = 0; flip[m++] = 0; }
+    if (layers == 2 && c == n - 1) { tgt[m] = -1; flip[m++] = 0; }
+  }
+  if (bchi == BC_OUTFLOW) {
+    if (c == n) { tgt[m] = n + 1; flip[m++] = 0; if (layers == 2) { tgt[m] = n + 2; flip[m++] = 0; } }
+  } else if (bchi == BC_REFLECTIVE) {
+    if (c == n) { tgt[m] = n + 1; flip[m++] = 1; }
+    if (layers == 2 && c == n - 1) { tgt[m] = n + 2; flip[m++] = 1; }
+  } else if (bchi == BC_PERIODIC) {
+    if (c == 1) { tgt[m] = n + 1; flip[m++] = 0; }
+    if (layers == 2 && c == 2) { tgt[m] = n + 2; flip[m++] = 0; }
+  }
+  return m;
+}
+
 // The face-ghost images of a stage-1 cell (borders(UPP, 2), boundaries.f90
 // non-MPI branches) as FP32 primitives of UPP: the FP64 image of v (normal
 // momentum negated at a reflective face) with the winds applied at the ghost
