@@ -7,6 +7,7 @@
 
 #include <cstdint>
 
+#include "tlq_convert.cuh"
 #include "tlq_physics.cuh"
 
 namespace tlq {
@@ -108,17 +109,43 @@ __device__ __forceinline__ double ld_cg(const double* p) { return __ldcg(p); }
 // `advance` is set, as `step` does at HydroCore.f90:208-209).  No block ever
 // waits for another, and the maximum is exact whatever the order.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ double warp_max_nan(double v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v = max_nan(v, __shfl_xor_sync(0xffffffffu, v, o));
-  return v;
+// A signal speed as an unsigned key whose integer order is max_nan's order
+// from 0: the bits of a positive value order like it, a NaN takes the largest
+// key (it wins, as max_nan lets it), and values <= 0 the key 0 (they never
+// beat the reduction's starting 0).  Key 0 reads back as +0.0 and the largest
+// key as a NaN.  FP32 speeds (the mixed form) have 32-bit keys, which order
+// like the FP64 values they convert to.
+__device__ __forceinline__ unsigned long long max_key(double x) {
+  if (x != x) return ~0ull;
+  return x > 0.0 ? (unsigned long long)__double_as_longlong(x) : 0ull;
+}
+__device__ __forceinline__ unsigned max_key(float x) {
+  if (x != x) return 0x7fffffffu;
+  return x > 0.0f ? __float_as_uint(x) : 0u;
+}
+__device__ __forceinline__ double key_value(unsigned long long k) { return __longlong_as_double((long long)k); }
+__device__ __forceinline__ unsigned long long key64(unsigned long long k) { return k; }
+__device__ __forceinline__ unsigned long long key64(unsigned k) { return max_key(f2d(__uint_as_float(k))); }
+
+// The warp's largest key (redux.sync on 32-bit words; a 64-bit key takes its
+// upper word's maximum, then the lower words that go with it).
+__device__ __forceinline__ unsigned warp_max(unsigned k) { return __reduce_max_sync(0xffffffffu, k); }
+__device__ __forceinline__ unsigned long long warp_max(unsigned long long k) {
+  const unsigned hi = (unsigned)(k >> 32), top = __reduce_max_sync(0xffffffffu, hi);
+  const unsigned lo = __reduce_max_sync(0xffffffffu, hi == top ? (unsigned)k : 0u);
+  return ((unsigned long long)top << 32) | lo;
 }
 
-template <int NTHREADS>
-__device__ __forceinline__ void block_max3(double& a, double& b, double& c, double* red /*3*32*/) {
-  a = warp_max_nan(a);
-  b = warp_max_nan(b);
-  c = warp_max_nan(c);
+// A block's maxima of three keys, in thread 0.  Integer maxima: the same
+// reduction with FP64 compares and shuffles was a tail of 11,000 to 24,000
+// cycles per block (each compare a slot of the FP64 pipe).  red: 3 x 32 words
+// of 8 bytes.
+template <int NTHREADS, class K>
+__device__ __forceinline__ void block_max3(K& a, K& b, K& c, double* red_) {
+  K* red = reinterpret_cast<K*>(red_);
+  a = warp_max(a);
+  b = warp_max(b);
+  c = warp_max(c);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   constexpr int NW = NTHREADS / 32;
   __syncthreads();
@@ -129,51 +156,42 @@ __device__ __forceinline__ void block_max3(double& a, double& b, double& c, doub
   }
   __syncthreads();
   if (warp == 0) {
-    a = lane < NW ? red[lane] : 0.0;
-    b = lane < NW ? red[32 + lane] : 0.0;
-    c = lane < NW ? red[64 + lane] : 0.0;
-    a = warp_max_nan(a);
-    b = warp_max_nan(b);
-    c = warp_max_nan(c);
+    a = warp_max(lane < NW ? red[lane] : K(0));
+    b = warp_max(lane < NW ? red[32 + lane] : K(0));
+    c = warp_max(lane < NW ? red[64 + lane] : K(0));
   }
 }
 
-// A maximum of signal speeds as an unsigned key whose integer order is
-// max_nan's order from 0: the bits of a positive double order like its value,
-// a NaN takes the largest key (it wins, as max_nan lets it), and values <= 0
-// the key 0 (they never beat the reduction's starting 0).  Key 0 reads back
-// as +0.0 and the largest key as a NaN.
-__device__ __forceinline__ unsigned long long max_key(double x) {
-  if (x != x) return ~0ull;
-  return x > 0.0 ? (unsigned long long)__double_as_longlong(x) : 0ull;
-}
-__device__ __forceinline__ double key_value(unsigned long long k) { return __longlong_as_double((long long)k); }
-
 // Thread 0 folds a block's maxima (from block_max3) into the clock's.
-__device__ __forceinline__ void cfl_fold(double a, double b, double c, Clock* clk) {
-  atomicMax(&clk->vmax[0], max_key(a));
-  atomicMax(&clk->vmax[1], max_key(b));
-  atomicMax(&clk->vmax[2], max_key(c));
+template <class K>
+__device__ __forceinline__ void cfl_fold(K a, K b, K c, Clock* clk) {
+  // (0 changes nothing: a block without cells saves the three atomics)
+  if (a) atomicMax(&clk->vmax[0], key64(a));
+  if (b) atomicMax(&clk->vmax[1], key64(b));
+  if (c) atomicMax(&clk->vmax[2], key64(c));
 }
 
 // A block's maxima without finishing the reduction (a later kernel of the
-// same step, stream-ordered after this one, finishes it).
-template <int NTHREADS>
-__device__ __forceinline__ void cfl_contribute(double a, double b, double c, Clock* clk, double* red) {
-  block_max3<NTHREADS>(a, b, c, red);
-  if (threadIdx.x == 0) cfl_fold(a, b, c, clk);
+// same step, stream-ordered after this one, finishes it).  R: float or double
+// speeds.
+template <int NTHREADS, class R>
+__device__ __forceinline__ void cfl_contribute(R a, R b, R c, Clock* clk, double* red) {
+  auto ka = max_key(a), kb = max_key(b), kc = max_key(c);
+  block_max3<NTHREADS>(ka, kb, kc, red);
+  if (threadIdx.x == 0) cfl_fold(ka, kb, kc, clk);
 }
 
 // nblocks: the blocks (tiles) of this reduction, each arriving once (a
 // persistent kernel reduces per mesh over the tiles it works through).
 // Maxima that earlier kernels of the step folded in (cfl_contribute) take
 // part.  *s_flag is set in the block that finished.
-template <int NTHREADS>
-__device__ void cfl_reduce_finalize_n(double a, double b, double c, Clock* clk, const Params& p, bool advance,
-                                      double* red, int* s_flag, unsigned nblocks) {
-  block_max3<NTHREADS>(a, b, c, red);
+template <int NTHREADS, class R>
+__device__ void cfl_reduce_finalize_n(R a, R b, R c, Clock* clk, const Params& p, bool advance, double* red,
+                                      int* s_flag, unsigned nblocks) {
+  auto ka = max_key(a), kb = max_key(b), kc = max_key(c);
+  block_max3<NTHREADS>(ka, kb, kc, red);
   if (threadIdx.x == 0) {
-    cfl_fold(a, b, c, clk);
+    cfl_fold(ka, kb, kc, clk);
     __threadfence();
     const unsigned t = atomicAdd(&clk->ticket, 1u);
     *s_flag = (t == nblocks - 1);
@@ -196,8 +214,8 @@ __device__ void cfl_reduce_finalize_n(double a, double b, double c, Clock* clk, 
   __threadfence();
 }
 
-template <int NTHREADS>
-__device__ __forceinline__ void cfl_reduce_finalize(double a, double b, double c, Clock* clk, const Params& p,
+template <int NTHREADS, class R>
+__device__ __forceinline__ void cfl_reduce_finalize(R a, R b, R c, Clock* clk, const Params& p,
                                                     bool advance, double* red, int* s_flag) {
   cfl_reduce_finalize_n<NTHREADS>(a, b, c, clk, p, advance, red, s_flag, gridDim.x * gridDim.y * gridDim.z);
 }

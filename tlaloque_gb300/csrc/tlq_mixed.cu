@@ -71,7 +71,7 @@ __global__ void __launch_bounds__(RED_THREADS) k_init_dt_mixed(Params p, Layout 
     m1 = (v1 != v1 || v1 > m1) ? v1 : m1;
     m2 = (v2 != v2 || v2 > m2) ? v2 : m2;
   }
-  cfl_reduce_finalize<RED_THREADS>(f2d(m0), f2d(m1), f2d(m2), clk, p, false, red, &flag);
+  cfl_reduce_finalize<RED_THREADS>(m0, m1, m2, clk, p, false, red, &flag);
 }
 
 cudaError_t launch_init_dt_mixed(const Params& p, const Layout& L, const double* U, Clock* clk, int nblocks,

@@ -528,10 +528,10 @@ __device__ __forceinline__ void signal_speeds(double g, const double* w, double*
 __device__ __forceinline__ double max_nan(double a, double b) { return (a != a || a > b) ? a : b; }
 
 // dt from the three maxima, source/HydroCore.f90:144.
-__host__ __device__ __forceinline__ double cfl_dt(double cfl, double dx, double dy, double dz, double mvx, double mvy,
+__device__ __forceinline__ double cfl_dt(double cfl, double dx, double dy, double dz, double mvx, double mvy,
                                                   double mvz) {
-  const double m = mn(mn(dx / mvx, dy / mvy), dz / mvz);
-  return cfl * m / sqrt(3.0);
+  const double m = mn(mn(quot(dx, mvx), quot(dy, mvy)), quot(dz, mvz));
+  return quot(cfl * m, sqrt(3.0));
 }
 
 }  // namespace tlq

@@ -237,7 +237,7 @@ __device__ __forceinline__ void face_flux(const Params& p, double* ff, const dou
 // The z flux stays in its thread.
 //   Measured, Sedov 128^3, 8-plane chunks: stage 1 2.90 -> 1.02 ms, stage 2
 // 5.09 -> 2.12 ms per launch against one face task list with the limiter and
-// sound speeds per face and hardware divisions (1.86 and 2.98 ms with those
+// sound speeds per face and hardware divisions (1.44 and 2.80 ms with those
 // off the FP64 pipe).  Now 159 FP64 operations per cell in stage 1 and 365 in
 // stage 2 at 75-80 % of that pipe's rate, beside 5,400 and 9,300 integer and
 // other instructions per warp of cells.  Which multiplications go to the

@@ -996,30 +996,24 @@ __device__ __forceinline__ void mixed_tile2(const CUtensorMap* tm, const StageAr
   }
 
   cp_async_wait_all();  // (a tile that gave up leaves no copy of its own in flight)
-  double d0 = f2d(m0), d1 = f2d(m1), d2 = f2d(m2);
   if (aborted) {
     if (tid == 0) {
       atomicOr(&clk->status, ST_TIMEOUT);
       pw.drain(s.bar, 4, issued);
     }
-    d0 = d1 = d2 = NAN;
+    m0 = m1 = m2 = NAN;
   }
   if (p.cooling == COOL_MLP && a.cool_counts) {
-    unsigned v = nsingle, f = nfloor;
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-      v += __shfl_xor_sync(0xffffffffu, v, off);
-      f += __shfl_xor_sync(0xffffffffu, f, off);
-    }
+    const unsigned v = __reduce_add_sync(0xffffffffu, nsingle), f = __reduce_add_sync(0xffffffffu, nfloor);
     if ((tid & 31) == 0 && v) atomicAdd(&a.cool_counts[2], (unsigned long long)v);
     if ((tid & 31) == 0 && f) atomicAdd(&a.cool_counts[1], (unsigned long long)f);  // the exact integrator's
   }
   if (p.cooling != COOL_MLP) {
-    cfl_reduce_finalize_n<MNT>(d0, d1, d2, clk, p, true, s.red, &s.flag, nblk);
+    cfl_reduce_finalize_n<MNT>(m0, m1, m2, clk, p, true, s.red, &s.flag, nblk);
   } else {
     // with the surrogate the cooling passes finish the reduction over
     // these block maxima and their own
-    cfl_contribute<MNT>(d0, d1, d2, clk, s.red);
+    cfl_contribute<MNT>(m0, m1, m2, clk, s.red);
   }
 }
 
@@ -1037,6 +1031,8 @@ __global__ void __launch_bounds__(MNT, MixedBlocks<STAGE>::value)
     stage_kernel_mixed(const __grid_constant__ CUtensorMap tm_in, const __grid_constant__ StageArgs a) {
   extern __shared__ __align__(128) unsigned char smem_bytes[];
   MixedSmem<STAGE>& s = *reinterpret_cast<MixedSmem<STAGE>*>(smem_bytes);
+  // (the surrogate's cooling pass may set up beside the last wave)
+  if (STAGE == 2) cudaTriggerProgrammaticLaunchCompletion();
   mixed_tile<STAGE, LIM, SOLV>(&tm_in, a, s, blockIdx.x, blockIdx.y, blockIdx.z, gridDim.x * gridDim.y * gridDim.z,
                                blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z));
 }

@@ -100,11 +100,9 @@ struct CoolJob {
   unsigned blk0, nblk;  // this mesh's blocks of each pass: [blk0, blk0 + nblk)
 };
 
-// The mesh block b of a pass works on: `one` for a single mesh (jobs null),
-// else the job whose block range holds b (ranges ascending, back to back).
-__device__ __forceinline__ const CoolJob* job_of_block(const CoolJob& one, const CoolJob* jobs, int njobs,
-                                                      unsigned b) {
-  if (!jobs) return &one;
+// The mesh block b of a pass works on: the job whose block range holds b
+// (ranges ascending, back to back).
+__device__ __forceinline__ const CoolJob* job_of_block(const CoolJob* jobs, int njobs, unsigned b) {
   int lo = 0, hi = njobs - 1;
   while (lo < hi) {
     const int mid = (lo + hi + 1) >> 1;
@@ -139,26 +137,28 @@ __device__ __forceinline__ void cell_cool(const Params& p, const SurrogateArgs& 
   const float gm1 = p.f_gamma - 1.0f;
   float cf[5];
   mixed_cell(gm1, u, 1, cf, c.w);
-  c.T = (c.w[4] / c.w[0]) * p.f_cT;
+  // (divisions and products as intrinsics: every kernel that inlines this
+  // gets the same bits)
+  c.T = __fmul_rn(__fdividef(c.w[4], c.w[0]), p.f_cT);
   c.need = cools_at(p, c.T, u);
   c.tau = 0.f;
   c.lam = 0.f;
   c.feat[0] = c.feat[1] = c.feat[2] = 0.f;
   c.inbox = false;
   if (c.need) {
-    const float nd = c.w[0] * p.f_inv_muamu;
-    const float eth = c.w[4] / gm1;
+    const float nd = __fmul_rn(c.w[0], p.f_inv_muamu);
+    const float eth = __fdividef(c.w[4], gm1);
     c.lam = cool_coef_f(p.cool, c.T);
-    c.tau = (c.lam * nd) * (nd / eth) * dtf;
+    c.tau = __fmul_rn(__fmul_rn(__fmul_rn(c.lam, nd), __fdividef(nd, eth)), dtf);
     const float f0 = log10f(nd), f1 = log10f(c.T), f2 = log10f(c.tau);
     // inclusive, with 1e-4 dex of slack for the FP32 logarithms of cells on
     // a face of the box (e.g. a medium at the table's first temperature)
     constexpr float SL = 1e-4f;
     c.inbox = f0 >= sa.box[0] - SL && f0 <= sa.box[1] + SL && f1 >= sa.box[2] - SL && f1 <= sa.box[3] + SL &&
               f2 >= sa.box[4] - SL && f2 <= sa.box[5] + SL;
-    c.feat[0] = (f0 - sa.norm[0]) / sa.norm[1];
-    c.feat[1] = (f1 - sa.norm[2]) / sa.norm[3];
-    c.feat[2] = (f2 - sa.norm[4]) / sa.norm[5];
+    c.feat[0] = __fdividef(__fsub_rn(f0, sa.norm[0]), sa.norm[1]);
+    c.feat[1] = __fdividef(__fsub_rn(f1, sa.norm[2]), sa.norm[3]);
+    c.feat[2] = __fdividef(__fmaf_rn(__log2f(c.tau), 0.301029996f, -sa.norm[4]), sa.norm[5]);  // (f2 - centre, fused)
   }
 }
 
@@ -174,18 +174,14 @@ __device__ __forceinline__ void warp_append(bool take, unsigned v, unsigned* que
 }
 
 // The counters of the three outcomes (network, fallback, single step).
-__device__ __forceinline__ void add_counts(const SurrogateArgs& sa, unsigned long long used, unsigned long long fell,
-                                           unsigned long long one) {
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) {
-    used += __shfl_xor_sync(0xffffffffu, used, off);
-    fell += __shfl_xor_sync(0xffffffffu, fell, off);
-    one += __shfl_xor_sync(0xffffffffu, one, off);
-  }
+__device__ __forceinline__ void add_counts(const SurrogateArgs& sa, unsigned used, unsigned fell, unsigned one) {
+  used = __reduce_add_sync(0xffffffffu, used);
+  fell = __reduce_add_sync(0xffffffffu, fell);
+  one = __reduce_add_sync(0xffffffffu, one);
   if ((threadIdx.x & 31) == 0) {
-    if (used) atomicAdd(&sa.counts[0], used);
-    if (fell) atomicAdd(&sa.counts[1], fell);
-    if (one) atomicAdd(&sa.counts[2], one);
+    if (used) atomicAdd(&sa.counts[0], (unsigned long long)used);
+    if (fell) atomicAdd(&sa.counts[1], (unsigned long long)fell);
+    if (one) atomicAdd(&sa.counts[2], (unsigned long long)one);
   }
 }
 
@@ -200,7 +196,7 @@ __device__ void cool_sort_mesh(const CoolJob& j, double* red, unsigned nblocks, 
   const float gm1 = p.f_gamma - 1.0f, gf = p.f_gamma;
   const float dtf = d2f(clk->dt);
   float m0 = 0.f, m1 = 0.f, m2 = 0.f;
-  unsigned long long fell = 0, one = 0;
+  unsigned fell = 0, one = 0;
   // warp-uniform trip count (the appends are warp-wide)
   for (long long base = (long long)bid * CT; base < n; base += (long long)nblocks * CT) {
     const long long q = base + threadIdx.x;
@@ -233,7 +229,34 @@ __device__ void cool_sort_mesh(const CoolJob& j, double* red, unsigned nblocks, 
     one += single ? 1 : 0;
   }
   add_counts(j.sa, 0, fell, one);
-  cfl_contribute<CT>(f2d(m0), f2d(m1), f2d(m2), j.clk, red);
+  cfl_contribute<CT>(m0, m1, m2, j.clk, red);
+}
+
+// A network cell: the prediction y's change where the residual check accepts
+// it, else the exact integrator's; u[4] and the primitives updated.  tc: the
+// tensor-core path is healthy.
+__device__ __forceinline__ bool cool_net_cell(const Params& p, CellCool& c, double* u, float y, bool tc, float dtf) {
+  const CoolTable& tab = p.cool;
+  const float T = c.T, tau = c.tau, gm1 = p.f_gamma - 1.0f;
+  // the exact integrator's change and the network's, T_new/T - 1 (the
+  // network's r: ln(T_new/T) = -(tau + tau^2 r); clamped at the table's
+  // first temperature, where cooling stops).  A cell whose cooling
+  // reaches that temperature within the step (the exact change is the
+  // floor's, T_0/T - 1) takes the exact integrator: training leaves those
+  // pairs out, and the network's prediction, clamped at the floor, could
+  // only err on one side.
+  const float qfloor = __fsub_rn(__fdividef(tab.Tf[0], T), 1.0f);
+  const float qx = cool_exact_dropf(tab, T, c.lam, tau);
+  const float qf = fmaxf(expm1f(__fmul_rn(-__fmaf_rn(tau, y, 1.0f), tau)), qfloor);
+  const bool ok = tc && qx > qfloor && fabsf(qf - qx) <= p.f_mlp_tol;
+  if (ok) {
+    const float dp = __fmul_rn(c.w[4], qf);
+    c.w[4] = __fadd_rn(c.w[4], dp);
+    u[4] = u[4] + f2d(__fdividef(dp, gm1));
+  } else {
+    cool_cell_f(p, p.f_cT, p.f_inv_muamu, gm1, c.w, u[4], dtf, u);
+  }
+  return ok;
 }
 
 __device__ void cool_net_mesh(const CoolJob& j, umma::Smem& S, double* red, unsigned nblocks, unsigned bid) {
@@ -247,11 +270,10 @@ __device__ void cool_net_mesh(const CoolJob& j, umma::Smem& S, double* red, unsi
   double* __restrict__ U = step_output(j.U0, j.U1, clk, j.it_base);
   umma::load_weights(sa.img, S);
   umma::setup(S);
-  const CoolTable& tab = p.cool;
-  const float gm1 = p.f_gamma - 1.0f, gf = p.f_gamma;
+  const float gf = p.f_gamma;
   const float dtf = d2f(clk->dt);
   float m0 = 0.f, m1 = 0.f, m2 = 0.f;
-  unsigned long long used = 0, fell = 0;
+  unsigned used = 0, fell = 0;
   uint32_t phase = 0;
   bool tc = true;  // the tensor-core path is healthy (block-wide)
   // block-uniform trip count: one 128-row MMA tile per iteration
@@ -273,26 +295,8 @@ __device__ void cool_net_mesh(const CoolJob& j, umma::Smem& S, double* red, unsi
     if (tc) tc = umma::forward(S, c.feat, y, phase);
     bool ok = false;
     if (valid) {
-      const float T = c.T, tau = c.tau;
-      // the exact integrator's change and the network's, T_new/T - 1 (the
-      // network's r: ln(T_new/T) = -(tau + tau^2 r); clamped at the table's
-      // first temperature, where cooling stops).  A cell whose cooling
-      // reaches that temperature within the step (the exact change is the
-      // floor's, T_0/T - 1) takes the exact integrator: training leaves those
-      // pairs out, and the network's prediction, clamped at the floor, could
-      // only err on one side.
-      const float qfloor = __fsub_rn(tab.Tf[0] / T, 1.0f);
-      const float qx = cool_exact_dropf(tab, T, c.lam, tau);
-      const float qf = fmaxf(expm1f(-(1.0f + tau * y) * tau), qfloor);
-      ok = tc && qx > qfloor && fabsf(qf - qx) <= p.f_mlp_tol;
-      if (ok) {
-        const float dp = __fmul_rn(c.w[4], qf);
-        c.w[4] = __fadd_rn(c.w[4], dp);
-        U[4 * L.plane + o] = u[4] + f2d(dp / gm1);
-      } else {
-        cool_cell_f(p, p.f_cT, p.f_inv_muamu, gm1, c.w, u[4], dtf, u);  // the exact integrator
-        U[4 * L.plane + o] = u[4];
-      }
+      ok = cool_net_cell(p, c, u, y, tc, dtf);
+      U[4 * L.plane + o] = u[4];
       speeds_max(c.w, gf, m0, m1, m2);
     }
     used += ok ? 1 : 0;
@@ -306,34 +310,30 @@ __device__ void cool_net_mesh(const CoolJob& j, umma::Smem& S, double* red, unsi
   }
   umma::teardown(S);
   add_counts(sa, used, fell, 0);
-  cfl_contribute<CT>(f2d(m0), f2d(m1), f2d(m2), j.clk, red);
+  cfl_contribute<CT>(m0, m1, m2, j.clk, red);
 }
 
-// The sort and network passes of one mesh (jobs null: `one`) or of njobs
-// meshes, each on its own range of the grid's blocks.  One kernel, one call
-// site each: the single-mesh and batched steps run the same instructions,
-// so their FP32 results agree bit for bit.
-__global__ void __launch_bounds__(CT) k_cool_sort(const __grid_constant__ CoolJob one,
-                                                  const CoolJob* __restrict__ jobs, int njobs) {
+// The sort and network passes of njobs meshes, each on its own range of the
+// grid's blocks.
+__global__ void __launch_bounds__(CT) k_cool_sort(const CoolJob* __restrict__ jobs, int njobs) {
   __shared__ double red[96];
   __shared__ SmemJob sj;
-  const CoolJob& j = stage_job(sj, job_of_block(one, jobs, njobs, blockIdx.x));
+  const CoolJob& j = stage_job(sj, job_of_block(jobs, njobs, blockIdx.x));
   cool_sort_mesh(j, red, j.nblk, blockIdx.x - j.blk0);
 }
 
-__global__ void __launch_bounds__(CT, 3) k_cool_net(const __grid_constant__ CoolJob one,
-                                                 const CoolJob* __restrict__ jobs, int njobs) {
+__global__ void __launch_bounds__(CT, 3) k_cool_net(const CoolJob* __restrict__ jobs, int njobs) {
   __shared__ umma::Smem S;
   __shared__ double red[96];
   __shared__ SmemJob sj;
-  const CoolJob& j = stage_job(sj, job_of_block(one, jobs, njobs, blockIdx.x));
+  const CoolJob& j = stage_job(sj, job_of_block(jobs, njobs, blockIdx.x));
   cool_net_mesh(j, S, red, j.nblk, blockIdx.x - j.blk0);
 }
 
 __device__ void cool_dt_mesh(const CoolJob& j, double* red, int* flag, unsigned nblocks) {
   Clock* clk = j.clk;
   if (!(clk->t < clk->tfin)) return;
-  cfl_reduce_finalize_n<FT>(0.0, 0.0, 0.0, clk, j.p, true, red, flag, nblocks);
+  cfl_reduce_finalize_n<FT>(0.0f, 0.0f, 0.0f, clk, j.p, true, red, flag, nblocks);
   if (*flag && threadIdx.x == 0) {
     *j.cqcount = 0u;
     *j.nqcount = 0u;
@@ -342,15 +342,107 @@ __device__ void cool_dt_mesh(const CoolJob& j, double* red, int* flag, unsigned 
 
 // Pass 3: the dt reduction over the block maxima of stage 2 and the two
 // cooling passes (this pass's blocks only take their tickets); the last
-// block of a mesh empties its queues.  One mesh (jobs null: `one`) or njobs
-// meshes, as the other passes.
-__global__ void __launch_bounds__(FT) k_cool_dt(const __grid_constant__ CoolJob one, const CoolJob* __restrict__ jobs,
-                                                int njobs) {
+// block of a mesh empties its queues.
+__global__ void __launch_bounds__(FT) k_cool_dt(const CoolJob* __restrict__ jobs, int njobs) {
   __shared__ double red[96];
   __shared__ int flag;
   __shared__ SmemJob sj;
-  const CoolJob& j = stage_job(sj, job_of_block(one, jobs, njobs, blockIdx.x));
+  const CoolJob& j = stage_job(sj, job_of_block(jobs, njobs, blockIdx.x));
   cool_dt_mesh(j, red, &flag, j.nblk);
+}
+
+// The single-mesh step's cooling in one launch: the three passes' work on
+// stage 2's queue directly, the last block to finish closing the dt reduction
+// and emptying the queue.  Nearly every queued cell is the network's (stage 2
+// cools the others), so sorting them first gains no density here, and the
+// passes were latency: three launches of a few tiles each, 49 us of a 48^3
+// clumpy step (the stages take 56) and 72 us at 128^3.  (The batched step
+// keeps the three passes: its members' queues differ widely in length.)
+__global__ void __launch_bounds__(2 * CT, 2) k_cool_all(const __grid_constant__ CoolJob j) {
+  __shared__ umma::Smem S;
+  __shared__ float x3[3][CT], acc[CT];
+  __shared__ double red[96];
+  __shared__ int flag;
+  const Params& p = j.p;
+  const Layout& L = j.L;
+  Clock* clk = j.clk;
+  const SurrogateArgs& sa = j.sa;
+  // launched before stage 2 has ended (programmatic dependent launch): the
+  // weights and the TMEM columns come in beside its last wave
+  umma::load_weights(sa.img, S);
+  umma::setup(S);
+  // and the cooling table's FP32 columns into L1 (a cell walks them in a dozen
+  // dependent loads)
+  {
+    const CoolTable& t = p.cool;
+    const float* cols[5] = {t.Tf, t.logTf, t.Cf, t.slopef, t.gcumf};
+#pragma unroll
+    for (int e = 0; e < 5; ++e)
+      for (int q = 32 * (int)threadIdx.x; q < t.n; q += 32 * 2 * CT)
+        asm volatile("prefetch.global.L1 [%0];" ::"l"(cols[e] + q));
+  }
+  cudaGridDependencySynchronize();
+  if (!(clk->t < clk->tfin)) {  // the step did not run (mainHD.f90:61)
+    umma::teardown(S);
+    return;
+  }
+  const long long n = (long long)*j.cqcount;
+  double* __restrict__ U = step_output(j.U0, j.U1, clk, j.it_base);
+  const float gm1 = p.f_gamma - 1.0f, gf = p.f_gamma;
+  const float dtf = d2f(clk->dt);
+  float m0 = 0.f, m1 = 0.f, m2 = 0.f;
+  unsigned used = 0, fell = 0, one = 0;
+  uint32_t phase = 0;
+  bool tc = true;
+  for (long long base = (long long)blockIdx.x * CT; base < n; base += (long long)gridDim.x * CT) {
+    // the lower 128 threads hold a cell each, the upper ones help with the network
+    const long long q = base + threadIdx.x;
+    const bool valid = threadIdx.x < CT && q < n;
+    long long o = 0;
+    double u[5] = {1.0, 0.0, 0.0, 0.0, 1.0};
+    if (valid) {
+      o = interior_offset(p, L, j.cqueue[q]);
+#pragma unroll
+      for (int e = 0; e < 5; ++e) u[e] = U[e * L.plane + o];
+    }
+    CellCool c;
+    c.need = false;
+    if (threadIdx.x < CT) {
+      cell_cool(p, sa, u, dtf, c);
+#pragma unroll
+      for (int e = 0; e < 3; ++e) x3[e][threadIdx.x] = c.feat[e];
+    }
+    const bool need = valid && c.need;
+    const bool single = need && !(c.tau > p.f_cool_sub_frac);
+    const bool net = need && !single && c.inbox;
+    if (__syncthreads_or(net) && tc) {
+      tc = umma::forward2(S, x3, acc, phase);
+      __syncthreads();
+    }
+    if (need) {
+      const float y = acc[threadIdx.x];
+      bool ok = false;
+      if (net)
+        ok = cool_net_cell(p, c, u, y, tc, dtf);
+      else
+        cool_cell_f(p, p.f_cT, p.f_inv_muamu, gm1, c.w, u[4], dtf, u);
+      U[4 * L.plane + o] = u[4];
+      speeds_max(c.w, gf, m0, m1, m2);
+      used += ok ? 1 : 0;
+      one += single ? 1 : 0;
+      fell += (!ok && !single) ? 1 : 0;
+    }
+  }
+  if (!tc) {
+    // an MMA wait ran out: the cells took the exact integrator; the step
+    // reports the timeout
+    if (threadIdx.x == 0) atomicOr(&clk->status, ST_TIMEOUT);
+    umma::drain(S, phase);
+  }
+  umma::teardown(S);
+  add_counts(sa, used, fell, one);
+  cfl_reduce_finalize_n<2 * CT>(m0, m1, m2, clk, p, true, red, &flag, gridDim.x);
+  if (flag && threadIdx.x == 0) *j.cqcount = 0u;
 }
 
 }  // namespace
@@ -388,31 +480,35 @@ cudaError_t launch_cool_mlp_dt(const Params& p, const Layout& L, double* U0, dou
                                Clock* clk, const void* img, const float norm[6], const double box[6],
                                unsigned long long* counts, const unsigned* cqueue, unsigned* cqcount,
                                unsigned* nqueue, unsigned* nqcount, cudaStream_t s) {
-  const int nb = pass_blocks(p);
+  // a 128-cell tile for every 512 cells (a tenth to a quarter of a clumpy
+  // medium is queued), at most one resident wave (2 blocks per SM)
+  const long long n = (long long)p.nx * p.ny * p.nz;
+  const int nb = (int)std::min<long long>((n + 511) / 512, 152 * 2);
   CoolJob j;
   fill_cool_job(&j, p, L, U0, U1, it_base, clk, img, norm, box, counts, cqueue, cqcount, nqueue, nqcount, 0, nb);
-  k_cool_sort<<<nb, CT, 0, s>>>(j, nullptr, 1);
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  k_cool_net<<<nb, CT, 0, s>>>(j, nullptr, 1);
-  e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  k_cool_dt<<<nb, FT, 0, s>>>(j, nullptr, 1);
-  return cudaGetLastError();
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(nb);
+  cfg.blockDim = dim3(2 * CT);
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, k_cool_all, j);
 }
 
 int cool_pass_blocks(const Params& p) { return pass_blocks(p); }
 
 cudaError_t launch_cool_mlp_dt_batch(const void* jobs, int njobs, int nblocks, cudaStream_t s) {
   const CoolJob* d = static_cast<const CoolJob*>(jobs);
-  const CoolJob none{};
-  k_cool_sort<<<nblocks, CT, 0, s>>>(none, d, njobs);
+  k_cool_sort<<<nblocks, CT, 0, s>>>(d, njobs);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  k_cool_net<<<nblocks, CT, 0, s>>>(none, d, njobs);
+  k_cool_net<<<nblocks, CT, 0, s>>>(d, njobs);
   e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  k_cool_dt<<<nblocks, FT, 0, s>>>(none, d, njobs);
+  k_cool_dt<<<nblocks, FT, 0, s>>>(d, njobs);
   return cudaGetLastError();
 }
 

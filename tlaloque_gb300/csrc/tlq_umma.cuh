@@ -220,7 +220,8 @@ __device__ __forceinline__ bool layer_mma(Smem& s, const __nv_bfloat16* w, uint3
 // The network on this thread's cell: features x (normalised) -> y.  All
 // 128 threads of the block call it together.  The row is streamed in
 // pieces (8 columns of layer 1, 32 TMEM columns of layers 2-3), so that a
-// thread never holds all 64 activations.  Returns false (and the block
+// thread never holds all 64 activations.  Sums as explicit-rounding
+// intrinsics: the kernels that inline this get the same bits.  Returns false (and the block
 // stops using the tensor cores) when an MMA wait ran out.
 __device__ __forceinline__ bool forward(Smem& s, const float* x, float& y, uint32_t& phase) {
   const int r = threadIdx.x;
@@ -230,7 +231,7 @@ __device__ __forceinline__ bool forward(Smem& s, const float* x, float& y, uint3
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
       const float4 w = *reinterpret_cast<const float4*>(s.w1[8 * c + q]);
-      h8[q] = mlp::silu_f(s.b1[8 * c + q] + w.x * x[0] + w.y * x[1] + w.z * x[2]);
+      h8[q] = mlp::silu_f(__fmaf_rn(w.z, x[2], __fmaf_rn(w.y, x[1], __fmaf_rn(w.x, x[0], s.b1[8 * c + q]))));
     }
     store_chunk(s, r, c, h8);
   }
@@ -245,7 +246,7 @@ __device__ __forceinline__ bool forward(Smem& s, const float* x, float& y, uint3
     for (int c = 0; c < 4; ++c) {
       float h8[8];
 #pragma unroll
-      for (int q = 0; q < 8; ++q) h8[q] = mlp::silu_f(v[8 * c + q] + s.b2[32 * half + 8 * c + q]);
+      for (int q = 0; q < 8; ++q) h8[q] = mlp::silu_f(__fadd_rn(v[8 * c + q], s.b2[32 * half + 8 * c + q]));
       store_chunk(s, r, 4 * half + c, h8);
     }
   }
@@ -256,9 +257,63 @@ __device__ __forceinline__ bool forward(Smem& s, const float* x, float& y, uint3
     float v[32];
     ld32(lane_base + 32u * half, v);
 #pragma unroll
-    for (int q = 0; q < 32; ++q) acc += s.w4[32 * half + q] * mlp::silu_f(v[q] + s.b3[32 * half + q]);
+    for (int q = 0; q < 32; ++q) 
+      acc = __fmaf_rn(s.w4[32 * half + q], mlp::silu_f(__fadd_rn(v[q], s.b3[32 * half + q])), acc);
   }
-  y = s.b4 + acc;
+  y = __fadd_rn(s.b4, acc);
+  return true;
+}
+
+// The same network on 256 threads, two per cell (row t & 127): each thread
+// takes half of a layer's columns (thread half 0: 0-31), which halves the
+// latency of the 192 SiLUs per cell where few tiles are in flight.  x3: the
+// rows' features (3 x 128, written and synchronised by the caller); acc: 128
+// floats.  Layer 4's sum runs through both halves in column order, so y is
+// forward's, bit for bit; half 1's threads leave it in acc[row] (read it
+// after a barrier).
+__device__ __forceinline__ bool forward2(Smem& s, const float (*x3)[ROWS], float* acc, uint32_t& phase) {
+  const int r = threadIdx.x & (ROWS - 1), half = threadIdx.x / ROWS;
+  const float x0 = x3[0][r], x1 = x3[1][r], x2 = x3[2][r];
+#pragma unroll
+  for (int cc = 0; cc < 4; ++cc) {
+    const int c = 4 * half + cc;
+    float h8[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const float4 w = *reinterpret_cast<const float4*>(s.w1[8 * c + q]);
+      h8[q] = mlp::silu_f(__fmaf_rn(w.z, x2, __fmaf_rn(w.y, x1, __fmaf_rn(w.x, x0, s.b1[8 * c + q]))));
+    }
+    store_chunk(s, r, c, h8);
+  }
+  // (warps w and w + 4 reach the same TMEM lanes)
+  const uint32_t addr = s.tmem + ((uint32_t)(threadIdx.x & 96u) << 16) + 32u * half;
+  if (!layer_mma(s, s.w2, phase)) return false;
+  float v[32];
+  ld32(addr, v);
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    float h8[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) h8[q] = mlp::silu_f(__fadd_rn(v[8 * c + q], s.b2[32 * half + 8 * c + q]));
+    store_chunk(s, r, 4 * half + c, h8);
+  }
+  if (!layer_mma(s, s.w3, phase)) return false;
+  ld32(addr, v);
+#pragma unroll
+  for (int q = 0; q < 32; ++q) v[q] = mlp::silu_f(__fadd_rn(v[q], s.b3[32 * half + q]));
+  float a = 0.0f;
+  if (half == 0) {
+#pragma unroll
+    for (int q = 0; q < 32; ++q) a = __fmaf_rn(s.w4[q], v[q], a);
+    acc[r] = a;
+  }
+  __syncthreads();
+  if (half == 1) {
+    a = acc[r];
+#pragma unroll
+    for (int q = 0; q < 32; ++q) a = __fmaf_rn(s.w4[32 + q], v[q], a);
+    acc[r] = __fadd_rn(s.b4, a);
+  }
   return true;
 }
 
