@@ -274,8 +274,10 @@ int tlq_output(tlq_ctx* ctx, int format, const char* outputpath, int nout, int r
 int tlq_output_wait(tlq_ctx* ctx);
 
 /* Stage tiling (no counterpart in the reference): the z-chunk length of the
- * stage grid (>= 8 planes, or nz; default 64 for nz >= 128, 32 for nz >= 32,
- * else nz), and the measuring autotuner that picks it -- from the cache file
+ * stage grid (>= 8 planes, or nz; the default follows from a cost model of the
+ * mesh's tiles and the resident blocks; a mesh too small to fill the GPU with
+ * chunks of 8 planes runs shorter ones whatever the choice; results do not
+ * depend on it), and the measuring autotuner that picks it -- from the cache file
  * (JSON keyed by GPU name, mesh size and form; NULL = no cache) or timed now
  * over `steps` steps per candidate (8, 16, 32, 64, 128) from the current
  * state, which is restored afterwards. */
@@ -310,7 +312,8 @@ int tlq_batch_create(const tlq_config* cfgs, int nmembers, tlq_batch** out);
 int tlq_batch_destroy(tlq_batch* b);
 int tlq_batch_size(const tlq_batch* b);
 tlq_ctx* tlq_batch_member(tlq_batch* b, int i);
-/* z-chunk length (planes per tile, >= 8) of member i; default by nz. */
+/* z-chunk length (planes per tile, >= 8) of member i; the default by the same
+ * model over all members' tiles. */
 int tlq_batch_set_tiling(tlq_batch* b, int i, int zlen);
 int tlq_batch_get_tiling(const tlq_batch* b, int i, int* zlen);
 /* Autotuner: per distinct mesh size, the z-chunk length from the cache file

@@ -210,7 +210,7 @@ int enqueue_step(tlq_ctx* ctx, int par, bool timed) {
   a.p = ctx->P;
   a.L = ctx->L;
   a.clk = ctx->clk;
-  a.zlen = ctx->zlen;
+  a.zlen = ctx->zrun;
   a.phi = ctx->cfg.self_gravity ? ctx->phit : ctx->phi;
   a.phif = ctx->phif;
   a.lapf = ctx->lapf;
@@ -320,12 +320,52 @@ int read_clock(tlq_ctx* ctx) {
 
 }  // namespace
 
+// The chunk length for meshes of tiles[q] column tiles x nz[q] planes that
+// step together.  A block costs its planes plus its prologue (1.8 planes in
+// the mixed form, 1.5 in the plain one); blocks beyond one resident wave (5
+// per SM mixed; the plain form's pipes are full at about 2.4) add up, and the
+// last wave is half empty on average: cost = (z + prologue) (1 + waves), a
+// wave that is not full adding 0.65 of its share in the mixed form.  Fitted to
+// sweeps of 24^3..300^3 meshes in both forms: the choice is within 6 % of
+// the sweep's best (mixed bubble 48^3: 0.066 ms a step, 0.43 with 32-plane
+// chunks; 128^3 0.43 and 1.03; plain Sod tube 256x4x4 0.12 and 0.33, Sedov
+// 128^3 3.1 and 4.1 with 64-plane chunks).
+int rule_zlen(const int* tiles, const int* nz, int n, bool mixed) {
+  const double wave = mixed ? 152.0 * 5.0 : 152.0 * 2.4, prologue = mixed ? 1.8 : 1.5;
+  int nzmax = 1;
+  for (int q = 0; q < n; ++q) nzmax = std::max(nzmax, nz[q]);
+  int best = 1;
+  double cost = std::numeric_limits<double>::infinity();
+  for (int z = 1; z <= std::min(nzmax, 64); ++z) {
+    double blocks = 0.0;
+    for (int q = 0; q < n; ++q) blocks += (double)tiles[q] * (double)((nz[q] + z - 1) / z);
+    const double w = blocks / wave;
+    const double c = (z + prologue) * (1.0 + (mixed && w <= 1.0 ? 0.65 * w : w));
+    if (c <= cost) {
+      cost = c;
+      best = z;
+    }
+  }
+  return best;
+}
+
+// The chunk length that runs for a chosen one: the choice, except that a mesh
+// too small to fill the GPU with chunks of 8 planes (the shortest choice) is
+// split to the rule's length; chunks of equal length.
+int split_zlen(int zlen, int rule, int nz) {
+  const int z = rule < 8 ? std::min(zlen, rule) : zlen;
+  const int chunks = (nz + z - 1) / z;
+  return (nz + chunks - 1) / chunks;
+}
+
 int ctx_set_zlen(tlq_ctx* ctx, int zlen) {
   const int nz = ctx->cfg.nz;
   zlen = std::min(zlen, nz);
   if (zlen < 8 && zlen != nz) return fail(ctx, TLQ_ERR_ARG, "z-chunk length must be >= 8 planes (or nz)");
   ctx->zlen = zlen;
-  ctx->grid.z = (unsigned)((nz + zlen - 1) / zlen);
+  const int tiles = (int)(ctx->grid.x * ctx->grid.y);
+  ctx->zrun = split_zlen(zlen, rule_zlen(&tiles, &nz, 1, ctx->cfg.precision == TLQ_PREC_MIXED), nz);
+  ctx->grid.z = (unsigned)((nz + ctx->zrun - 1) / ctx->zrun);
   invalidate_graphs(ctx);
   return TLQ_OK;
 }
@@ -435,12 +475,12 @@ int tlq_create(const tlq_config* cfg, tlq_ctx** out) {
   ctx->clk_host->tfin = std::numeric_limits<double>::infinity();
   cudaMemcpy(ctx->clk, ctx->clk_host, sizeof(Clock), cudaMemcpyHostToDevice);
   // stage grid: column tiles (TX x TY plain, MTX x MTY mixed), z split into
-  // chunks of zlen planes
+  // chunks
   const int tx_ = cfg->precision == TLQ_PREC_MIXED ? MTX : TX, ty_ = cfg->precision == TLQ_PREC_MIXED ? MTY : TY;
   const int gx = (cfg->nx + tx_ - 1) / tx_, gy = (cfg->ny + ty_ - 1) / ty_;
-  ctx->zlen = cfg->nz >= 128 ? 64 : (cfg->nz >= 32 ? 32 : cfg->nz);
-  const int gz = (cfg->nz + ctx->zlen - 1) / ctx->zlen;
-  ctx->grid = dim3(gx, gy, gz);
+  ctx->grid = dim3(gx, gy, 1);
+  const int tiles = gx * gy;
+  ctx_set_zlen(ctx, std::max(8, rule_zlen(&tiles, &cfg->nz, 1, cfg->precision == TLQ_PREC_MIXED)));
   const int nb = init_blocks(ctx->P);
   if (cudaMalloc(&ctx->sums_partials, sizeof(double) * 5 * (size_t)nb) || cudaMalloc(&ctx->sums_out, sizeof(double) * 5))
     return bail(TLQ_ERR_NOMEM);

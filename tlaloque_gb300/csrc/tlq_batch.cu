@@ -117,7 +117,8 @@ using tlq::MemberDesc;
 
 struct tlq_batch {
   std::vector<tlq_ctx*> m;
-  std::vector<int> zlen;            // z-chunk length per member
+  std::vector<int> zlen;            // chosen z-chunk length per member
+  std::vector<int> zrun;            // the one that runs (set_zrun)
   std::vector<unsigned> gen_seen;   // member set-up generation the graph was built for
   cudaStream_t stream = nullptr;
   std::vector<MemberDesc> h_desc;
@@ -151,6 +152,27 @@ int bfail(tlq_batch* b, int code, const std::string& m) {
 
 int tiles_z(const tlq_ctx* c, int zlen) { return (c->cfg.nz + zlen - 1) / zlen; }
 
+int member_tiles(const tlq_ctx* c) {
+  return ((c->cfg.nx + tlq::MTX - 1) / tlq::MTX) * ((c->cfg.ny + tlq::MTY - 1) / tlq::MTY);
+}
+
+// The rule's chunk length for the batch: its members share the persistent
+// launches (the autotuner, which runs one size's members at a time, keeps it
+// too, so that what it times is what the batch runs).
+int batch_rule(const tlq_batch* b) {
+  std::vector<int> tiles, nz;
+  for (const tlq_ctx* c : b->m) {
+    tiles.push_back(member_tiles(c));
+    nz.push_back(c->cfg.nz);
+  }
+  return rule_zlen(tiles.data(), nz.data(), (int)tiles.size(), true);
+}
+
+void set_zrun(tlq_batch* b) {
+  const int rule = batch_rule(b);
+  for (size_t i = 0; i < b->m.size(); ++i) b->zrun[i] = split_zlen(b->zlen[i], rule, b->m[i]->cfg.nz);
+}
+
 void fill_desc(tlq_batch* b, int i) {
   tlq_ctx* c = b->m[i];
   MemberDesc& d = b->h_desc[i];
@@ -164,7 +186,7 @@ void fill_desc(tlq_batch* b, int i) {
       a.p = c->P;
       a.L = c->L;
       a.clk = c->clk;
-      a.zlen = b->zlen[i];
+      a.zlen = b->zrun[i];
       a.phi = c->phi;
       a.phif = c->phif;
       a.lapf = c->lapf;
@@ -180,7 +202,7 @@ void fill_desc(tlq_batch* b, int i) {
   d.it_base = c->it_base;
   d.gx = (c->cfg.nx + tlq::MTX - 1) / tlq::MTX;
   d.gy = (c->cfg.ny + tlq::MTY - 1) / tlq::MTY;
-  d.gz = tiles_z(c, b->zlen[i]);
+  d.gz = tiles_z(c, b->zrun[i]);
 }
 
 // Work list of the members in `which` (all when empty), most planes per tile
@@ -191,11 +213,11 @@ std::vector<Item> make_items(const tlq_batch* b, const std::vector<int>& which) 
   std::vector<int> ms = which;
   if (ms.empty())
     for (int i = 0; i < (int)b->m.size(); ++i) ms.push_back(i);
-  std::stable_sort(ms.begin(), ms.end(), [&](int x, int y) { return b->zlen[x] > b->zlen[y]; });
+  std::stable_sort(ms.begin(), ms.end(), [&](int x, int y) { return b->zrun[x] > b->zrun[y]; });
   for (int i : ms) {
     const tlq_ctx* c = b->m[i];
     const int gx = (c->cfg.nx + tlq::MTX - 1) / tlq::MTX, gy = (c->cfg.ny + tlq::MTY - 1) / tlq::MTY;
-    const int gz = tiles_z(c, b->zlen[i]);
+    const int gz = tiles_z(c, b->zrun[i]);
     for (int bz = 0; bz < gz; ++bz)
       for (int by = 0; by < gy; ++by)
         for (int bx = 0; bx < gx; ++bx) v.push_back(Item{i, bx, by, bz});
@@ -229,6 +251,7 @@ int upload_items(tlq_batch* b, const std::vector<Item>& v) {
 // Descriptors of all members, and the cooling-pass arguments of the
 // surrogate members in `which` (all when empty).
 int refresh_desc(tlq_batch* b, const std::vector<int>& which = {}) {
+  set_zrun(b);
   for (int i = 0; i < (int)b->m.size(); ++i) fill_desc(b, i);
   BCK(cudaMemcpyAsync(b->d_desc, b->h_desc.data(), b->h_desc.size() * sizeof(MemberDesc), cudaMemcpyHostToDevice,
                       b->stream));
@@ -383,8 +406,12 @@ int tlq_batch_create(const tlq_config* cfgs, int n, tlq_batch** out) {
     const int rc = tlq_create(&cfgs[i], &c);
     if (rc != TLQ_OK) return bail(rc);
     b->m.push_back(c);
-    b->zlen.push_back(c->zlen);
     b->gen_seen.push_back(~0u);
+  }
+  const int rule = std::max(8, batch_rule(b));
+  for (tlq_ctx* c : b->m) {
+    b->zlen.push_back(std::min(rule, c->cfg.nz));
+    b->zrun.push_back(b->zlen.back());
   }
   if (cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) != cudaSuccess) return bail(TLQ_ERR_CUDA);
   for (tlq_ctx* c : b->m)
