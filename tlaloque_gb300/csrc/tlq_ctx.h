@@ -29,6 +29,8 @@ struct tlq_ctx {
   void* mg_work = nullptr;
   void* mg_ctl = nullptr;
   void* mg_mom = nullptr;
+  void* mg_exch = nullptr;  // the levels' exchange arrays between planes
+  void* mg_sched = nullptr;  // and the relax's schedules
   cudaStream_t mg_body = nullptr;  // captures a V-cycle into a graph's loop body
   double* phig = nullptr;
   double* phit = nullptr;

@@ -18,11 +18,12 @@
 // and j.  A block walks a plane's anti-diagonals i + j = d in order, and
 // every other neighbour (east, north, the k planes, the source) still holds
 // its value from before the half-sweep.  A relax's ten half-sweeps run in one
-// cooperative launch, skewed by a few diagonals per half-sweep, each plane's
-// block checking its neighbour planes' progress (k_mg_relax_plane with the
-// plane in shared memory up to 128 cells, k_mg_relax_pipe from the level
-// arrays above; k_mg_half, one launch per half-sweep, where the planes cannot
-// all be resident).  With the order kept and FP64 without contraction, every
+// cooperative launch, skewed by a few diagonals per half-sweep
+// (k_mg_relax_plane, up to 128 cells: the plane in shared memory, values
+// tagged with their half-sweep exchanged between planes; k_mg_relax_pipe,
+// above: from the level arrays, each plane's block checking its neighbour
+// planes' progress; k_mg_half, one launch per half-sweep, where the planes
+// cannot all be resident).  With the order kept and FP64 without contraction, every
 // level is bit-identical to a sequential restatement; only the stopping
 // test's sum |dphi| is summed in another order (it decides only whether the
 // next V-cycle runs).
@@ -65,6 +66,8 @@ struct MgLevel {
   double* E;
   double* R;
   double* T;   // source(i,j,k)*dxl**2 of the smoother, formed once with R
+  void* X;     // the shared-memory relax's exchange between planes (Tagged; null: level too large)
+  const void* sched;  // and its schedule (MgSched)
   double dxl;  // (xr - xl) / n (sources.f90:232; x extent for every axis, as there)
 };
 
@@ -77,6 +80,7 @@ struct MgCtl {
   double c0[5], cm[5][5], sm[5][5];  // multipole moments (sources.f90:599-681)
   double part[2 * 1024];             // per-plane partial sums of the last pass's |change|
   int abort;                         // a pipelined relax gave up waiting (sticky for the call)
+  unsigned call;                     // MultiGrid calls begun (tags of the exchange arrays)
   int prog[1026];                    // pipelined relax: plane k's last finished diagonal, hs*(2n+2) + d
   long long wait_limit;              // polls of a neighbour's progress before giving up (set at allocation)
 };
@@ -286,6 +290,7 @@ __global__ void k_mg_begin(MgCtl* c, const Clock* clk) {
   c->iter = 0;
   c->dif = 1.e28;
   c->abort = 0;
+  c->call = c->call + 1u;
 }
 
 // Residue(0) = 4 pi G dens, Error(0) = phi (sources.f90:136-137).
@@ -372,7 +377,9 @@ __global__ void k_mg_end(const MgCtl* c, Clock* clk, int n, const double* E0, do
 // bit for bit unless that is a signed zero or old is not finite (then the
 // 0*old term can change the sign or give a NaN): those take the literal
 // expression, every other update saves its three FP64 operations (the FP64
-// pipe bounds the smoother).
+// pipe bounds the smoother).  SOFT: the product on the integer pipe, where
+// the FP64 pipe is the limit.
+template <bool SOFT = false>
 __device__ __forceinline__ double mg_new(double east, double west, double north, double south, double up, double down,
                                          double sdx, double old) {
   double a = east + west;
@@ -381,7 +388,7 @@ __device__ __forceinline__ double mg_new(double east, double west, double north,
   a = a + up;
   a = a + down;
   a = a - sdx;
-  double v = (1.0 / 6.0) * a;
+  double v = SOFT ? sf::mul(1.0 / 6.0, a) : (1.0 / 6.0) * a;
   const long long vb = __double_as_longlong(v), ob = __double_as_longlong(old);
   if ((vb & 0x7fffffffffffffffLL) == 0 || ((ob >> 52) & 0x7ff) == 0x7ff) {
     const double w = 1.0;
@@ -675,105 +682,274 @@ __global__ void __launch_bounds__(NT, MINB) k_mg_relax_pipe(MgCtl* c, MgLevel lv
 }
 
 // ---------------------------------------------------------------------------
-// The same skewed relax with the block's plane held in shared memory (levels
-// up to 128 cells: (n+2)^2 doubles, 135 KB at 128).  Only plane k's block
-// writes plane k during a relax, so its copy in shared memory is the current
-// one: an update reads its old value and its four in-plane neighbours there
-// (no L2 round trip per step and no diagonal buffers; the values are the
-// same ones the reference's order gives, by the argument above), and
-// writes the new value there and to the level array, where the neighbour
-// planes read it.  The ghost rows and columns (i or j = 0, n+1) do not
-// change during a relax.  Layout: column parity, row, column / 2, so that a
-// warp's cells of one diagonal (consecutive columns of one parity) fall on
+// The skewed relax with the block's plane in shared memory (levels of 8 to
+// 128 cells: (N+2)^2 doubles, 135 KB at 128).  Only plane k's block writes
+// plane k during a relax, so its copy in shared memory is the current one: an
+// update reads its old value and its four in-plane neighbours there.  The
+// ghost rows and columns do not change during a relax; the level array takes
+// the plane back at the end.  Layout: column parity, row, column / 2, so that
+// a warp's cells of one diagonal (consecutive columns of one parity) fall on
 // distinct banks.
+//
+// Time step t processes diagonal t - S hs of half-sweep hs, S = MG_SKEW.  In
+// half-sweeps 2g and 2g+1 (group g) plane k changes the cells s = 0 (the
+// wave) in one and the cells i even, j odd in the other.  S is even, so both
+// lie on rows of one parity at any step: an odd column has a wave cell every
+// step, an even column a wave cell and one of the other kind in turn.  The
+// step's cells of all five groups are dealt to the block's first threads: the
+// FP64 pipe charges a warp instruction the same whatever its active lanes
+// (a thread per column and group keeps 20 warps of a 128-cell plane busy with
+// 9 warps' worth of cells on average).  Which cell a thread has at a step, and
+// its offsets, come from a schedule formed once per context (MgSched): worked
+// out in the kernel it was most of a step's instructions.
+//
+// The planes above and below exchange values through X, 16 bytes a cell: the
+// value and a tag that names this relax and the half-sweep which formed it
+// (the values from before the relax, the ghost planes' among them, have the
+// tag MG_INITIAL), written and read in one 128-bit access.  A reader uses a
+// value when its tag is the one it needs, else loads again (a bounded number
+// of times): no fence, no flag, no block-wide poll.  The value cannot be overwritten early: the neighbour's
+// next update of that cell needs this plane's.  X is laid out by diagonal, so
+// a warp's cells are contiguous.
+//
+// Half as many helper threads as there are cells run ahead of the workers:
+// during step t they check the values that step t + 1 needs (loaded during
+// step t - 1), leave them in shared memory with the source, and issue the
+// loads of step t + 2.  The workers only read shared memory: with loads, tag
+// checks and address arithmetic in their path a step took 1,600 cycles,
+// of which the update's seven dependent FP64 operations are 570.
+//
+// What bounds a step: those operations and the barrier; on 128 cells the
+// FP64 pipe.  Measured per launch on the 128^3 cloud (ncu), against a thread
+// per column and group with loads one step ahead and a fence and a poll by
+// the whole block every few steps: 128 cells 743 -> 380 us, 64: 260 -> 130,
+// 32: 143 -> 65, 16: 98 -> 43, 8: 60 -> 34.
 // ---------------------------------------------------------------------------
-__host__ __device__ __forceinline__ int plane_slot(int n, int i, int j) {
-  return ((i & 1) * (n + 2) + j) * ((n >> 1) + 1) + (i >> 1);
-}
-size_t plane_smem(int n) { return (size_t)(n + 2) * (n + 2) * sizeof(double); }
+constexpr int MG_SKEW = 4;  // (6: 4 % slower, 2 more steps per half-sweep; 2 leaves a value no time to arrive)
+constexpr unsigned MG_INITIAL = 15;
 
-template <int NT, int HG, int CH, bool TRACK>
-__global__ void __launch_bounds__(NT, 1) k_mg_relax_plane(MgCtl* c, MgLevel lv, double* part) {
-  constexpr int K = 10 / HG;
-  constexpr int SKEW = CH + 1;
-  static_assert(K * HG == 10, "HG divides the ten half-sweeps");
+template <int N>
+struct PlaneGeo {
+  static constexpr int NT = (5 * N + 31) / 32 * 32;       // workers: the most cells of a step, whole warps
+  static constexpr int NH = (NT / 2 + 31) / 32 * 32;      // helpers, two cells each
+  static constexpr int R = N / 2 + 1, PS = (N + 2) * R;
+  static constexpr int STEPS = (2 * N + 9 * MG_SKEW) / 2 * 2;  // t = 2 .. 2N + 9 S (an even number of steps)
+  static constexpr int ROWS = STEPS + 4;                       // and those the helpers look ahead to
+  // the plane, and two steps' values from above, below and the source per worker
+  static constexpr size_t smem = ((size_t)(N + 2) * (N + 2) + 2 * 3 * (size_t)NT) * sizeof(double);
+};
+// Cells of a level's exchange array: planes 0..N+1 of diagonals 0..2N+1 by column.
+bool exch_level(int n) { return n > MG_COARSE_N && n <= 128; }
+long long exch_cells(int n) { return (long long)(n + 2) * (2 * n + 2) * n; }
+
+using Tagged = unsigned __int128;  // the double's bits, the tag above them
+__device__ __forceinline__ double tagged_value(Tagged r) { return __longlong_as_double((long long)r); }
+__device__ __forceinline__ unsigned long long tagged_tag(Tagged r) { return (unsigned long long)(r >> 64); }
+// Loaded where `take`; asynchronous: nothing here waits for the value.
+__device__ __forceinline__ void ld_tagged(Tagged& r, const Tagged* p, bool take) {
+  asm volatile(
+      "{\n\t.reg .pred t;\n\tsetp.ne.b32 t, %2, 0;\n\t@t ld.relaxed.gpu.global.b128 %0, [%1];\n\t}"
+      : "+q"(r)
+      : "l"(p), "r"((int)take)
+      : "memory");
+}
+__device__ __forceinline__ void st_tagged(Tagged* p, double v, unsigned long long tag) {
+  const Tagged r = (Tagged)tag << 64 | (unsigned long long)__double_as_longlong(v);
+  asm volatile("st.relaxed.gpu.global.b128 [%0], %1;" ::"l"(p), "q"(r) : "memory");
+}
+__device__ __forceinline__ void ld_pred(double& r, const double* p, bool take) {
+  asm volatile("{\n\t.reg .pred t;\n\tsetp.ne.b32 t, %2, 0;\n\t@t ld.global.f64 %0, [%1];\n\t}"
+               : "+d"(r)
+               : "l"(p), "r"((int)take));
+}
+
+// One entry of a level's schedule, [plane parity][step - 2][thread]: the
+// cell's offset in the shared plane and its half-sweep, its offsets in a
+// plane of X and of the level arrays; og = 0: no cell.
+struct alignas(8) MgSched {
+  unsigned short o, hs, x, og;
+};
+long long sched_entries(int n) {  // per plane parity
+  const long long rows = (2 * n + 9 * MG_SKEW) / 2 * 2 + 4, nt = (5 * n + 31) / 32 * 32;  // PlaneGeo's
+  return rows * nt;
+}
+__host__ __device__ __forceinline__ int mg_xcol(int n, int i) { return (i & 1) ? i >> 1 : n / 2 + (i >> 1) - 1; }
+
+// The schedule of an n-cell level: one thread per entry.  Group g's own time
+// is t - 2 S g; its wave's diagonal there holds the odd columns lo..hi, and
+// the even columns' turn (the wave's on even steps) the even ones.
+__global__ void k_mg_sched(int n, MgSched* out, int rows, int nt) {
+  const long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (q >= 2LL * rows * nt) return;
+  const int f0 = (int)(q % nt), t = 2 + (int)((q / nt) % rows), kp = (int)(q / ((long long)rows * nt));
+  MgSched e = {0, 0, 0, 0};
+  int f = f0;
+  for (int g = 0; g < 5; ++g) {
+    const int tau = t - 2 * MG_SKEW * g;
+    const int dw = tau - MG_SKEW * kp, d = (tau & 1) ? tau - MG_SKEW * (1 - kp) : dw;
+    const int lo = max(1, dw - n) | 1, hi = min(n, dw - 1), le = (max(2, d - n) + 1) & ~1, he = min(n, d - 1);
+    const int no = hi >= lo ? (hi - lo) / 2 + 1 : 0, ne = he >= le ? (he - le) / 2 + 1 : 0;
+    if (f < no + ne) {
+      const bool odd = f < no;
+      const int i = odd ? lo + 2 * f : le + 2 * (f - no);
+      const int hs = 2 * g + ((odd || !(t & 1)) ? kp : 1 - kp), j = t - MG_SKEW * hs - i;
+      e.o = (unsigned short)(((i & 1) * (n + 2) + j) * (n / 2 + 1) + (i >> 1));
+      e.hs = (unsigned short)hs;
+      e.x = (unsigned short)((i + j) * n + mg_xcol(n, i));
+      e.og = (unsigned short)(i + (n + 2) * j);
+      break;
+    }
+    f -= no + ne;
+  }
+  out[q] = e;
+}
+
+template <int N, bool TRACK>
+__global__ void __launch_bounds__(PlaneGeo<N>::NT + PlaneGeo<N>::NH, 1)
+    k_mg_relax_plane(MgCtl* c, MgLevel lv, int leg, double* part) {
+  using G = PlaneGeo<N>;
+  constexpr int R = G::R, PS = G::PS, NT = G::NT, NH = G::NH;
+  constexpr int s1 = N + 2, s2 = (N + 2) * (N + 2);
+  constexpr int XP = (2 * N + 2) * N;  // X: plane stride
+  static_assert(MG_SKEW % 2 == 0, "rows of one parity per step");
+  static_assert(XP <= 65536 && s2 <= 65536, "schedule entries of 16 bits");
   extern __shared__ double P[];
   __shared__ double red[32];
-  __shared__ int s_ok;
+  __shared__ int s_gave_up[2];  // by parity of a pair of steps: set in the pair, read after it
   if (!c->active) return;
-  const int n = lv.n, k = blockIdx.x + 1;
-  const long long s2 = (long long)(n + 2) * (n + 2), base = s2 * k;
-  double* __restrict__ E = lv.E;
-  const double* __restrict__ Sd = lv.T;
-  for (int q = threadIdx.x; q < (n + 2) * (n + 2); q += blockDim.x)
-    P[plane_slot(n, q % (n + 2), q / (n + 2))] = E[base + q];
-  __syncthreads();
-  const bool live = (int)threadIdx.x < n * HG;
-  const int col = (int)(threadIdx.x % n), hn = n >> 1;
-  const int i = col < hn ? 2 * col + 1 : 2 * (col - hn) + 2;  // odd columns first (whole idle warps)
-  const int h0 = live ? (int)(threadIdx.x / n) * K : 0;
-  const int R = hn + 1, PS = (n + 2) * R;  // row stride and size of one parity's array
-  const int de = (i & 1) ? 1 - PS : PS, dw = (i & 1) ? -PS : PS - 1;  // east, west: the other parity
-  const int tmax = 2 * n + 9 * SKEW;
-  // one half-sweep's cell of a step: whether it changes, where it lies, and
-  // its values from the level arrays (the planes above and below, the source)
-  struct Fetch {
-    double ru, rd, rs;
-    long long og;
-    int os;
-    bool up;
-  };
-  auto fetch = [&](int t, Fetch* f) {
-#pragma unroll
-    for (int q = 0; q < K; ++q) {
-      const int hs = h0 + q, d = t - SKEW * hs, j = d - i;
-      const bool par = ((k & 1) ^ (hs & 1)) != 0;  // cells (i even, j odd) of this plane
-      f[q].up = live && d >= 2 && d <= 2 * n && j >= 1 && j <= n &&
-                (par ? (!(i & 1) && (j & 1)) : ((i & 1) || !(j & 1)));
-      if (f[q].up) {
-        f[q].og = base + i + (long long)(n + 2) * j;
-        f[q].os = plane_slot(n, i, j);
-        f[q].ru = ldcg(E + f[q].og + s2);
-        f[q].rd = ldcg(E + f[q].og - s2);
-        f[q].rs = Sd[f[q].og];
+  double* const B = P + s2;  // [step parity][above, below, source][worker]
+  const int k = blockIdx.x + 1, tid = threadIdx.x;
+  double* __restrict__ E = lv.E + (long long)s2 * k;
+  Tagged* X = static_cast<Tagged*>(lv.X) + (long long)XP * k;
+  const uint2* __restrict__ sched =
+      reinterpret_cast<const uint2*>(static_cast<const MgSched*>(lv.sched)) + (long long)(k & 1) * G::ROWS * NT;
+  const unsigned long long seq = (unsigned long long)(c->call * 64u + 2u * (unsigned)c->iter + (unsigned)leg) << 4;
+  // the plane into shared memory and, tagged, into X; the ghost planes by
+  // their neighbours' blocks
+  for (int j = tid / 32; j < N + 2; j += (NT + NH) / 32)
+    for (int i = tid % 32; i < N + 2; i += 32) {
+      const int o = i + s1 * j;
+      const double v = E[o];
+      P[((i & 1) * (N + 2) + j) * R + (i >> 1)] = v;
+      if (i >= 1 && i <= N && j >= 1 && j <= N) {
+        const int x = (i + j) * N + mg_xcol(N, i);
+        st_tagged(X + x, v, seq | MG_INITIAL);
+        if (k == 1) st_tagged(X - XP + x, E[o - s2], seq | MG_INITIAL);
+        if (k == N) st_tagged(X + XP + x, E[o + s2], seq | MG_INITIAL);
       }
     }
-  };
+  if (tid < 2) s_gave_up[tid] = 0;
   double acc8 = 0.0, acc9 = 0.0;
-  for (int t0 = 2; t0 <= tmax; t0 += CH) {
-    const int t1 = min(t0 + CH - 1, tmax);
-    const int need = t1 + 1 - SKEW;  // the neighbours' last step this chunk reads
-    if (need >= 2 && !mg_wait(c, k, n, need, &s_ok)) return;
-    // The other planes' values and the source of step t + 1 load while step
-    // t computes: the chunk's wait covers every step of the chunk, and a
-    // neighbour cannot get SKEW steps ahead of this plane's published
-    // progress, so none of them changes before its use.
-    Fetch cur[K], nxt[K];
-    fetch(t0, cur);
-    for (int t = t0; t <= t1; ++t) {
-      if (t < t1) fetch(t + 1, nxt);
+  if (tid < NT) {
+    // ---- workers: one cell a step ------------------------------------------
+    sched += tid;
+    uint2 m = __ldg(sched), next = __ldg(sched + NT);  // (x: o | hs << 16, y: x | og << 16)
+    sched += 2 * NT;
+    __syncthreads();
+    __syncthreads();  // step 2's values
+    for (int t0 = 2; t0 < 2 + G::STEPS; t0 += 2) {
 #pragma unroll
-      for (int q = 0; q < K; ++q) {
-        if (!cur[q].up) continue;
-        const int hs = h0 + q, o = cur[q].os;
-        const double old = P[o];
-        const double v = mg_new(P[o + de], P[o + dw], P[o + R], P[o - R], cur[q].ru, cur[q].rd, cur[q].rs, old);
-        P[o] = v;
-        E[cur[q].og] = v;
-        if (TRACK && hs == 8) acc8 += fabs(v - old);
-        if (TRACK && hs == 9) acc9 += fabs(v - old);
+      for (int q = 0; q < 2; ++q) {  // step t0 + q
+        if (m.y != 0u) {
+          const int o = (int)(m.x & 0xffffu);
+          double* pc = P + o;
+          // east and west lie in the other parity's half
+          const double* pe = pc + (o >= PS ? 1 - PS : PS);
+          const double* b = B + q * 3 * NT + tid;
+          const double old = pc[0];
+          const double v = mg_new<(N >= 128)>(pe[0], pe[-1], pc[R], pc[-R], b[0], b[NT], b[2 * NT], old);
+          pc[0] = v;
+          st_tagged(X + (m.y & 0xffffu), v, seq | (m.x >> 16));
+          if (TRACK) {
+            if ((m.x >> 16) == 8u) acc8 += fabs(v - old);
+            if ((m.x >> 16) == 9u) acc9 += fabs(v - old);
+          }
+        }
+        m = next;
+        next = __ldg(sched);
+        sched += NT;
+        __syncthreads();
       }
-      __syncthreads();
-#pragma unroll
-      for (int q = 0; q < K; ++q) cur[q] = nxt[q];
+      if (*(volatile int*)&s_gave_up[(t0 >> 1) & 1]) return;
     }
-    mg_publish(c, k, t1);
+  } else {
+    // ---- helpers: two cells each -------------------------------------------
+    const double* __restrict__ Sd = lv.T + (long long)s2 * k;
+    const int h = tid - NT;
+    const bool two = h + NH < NT, top = k == N, bottom = k == 1;
+    sched += h;
+    uint2 cell[2], ahead[2];  // the entries of the step whose loads are in flight, and of the one after
+    Tagged ru[2] = {0, 0}, rd[2] = {0, 0};
+    double rs[2] = {0.0, 0.0};
+    auto entries = [&](uint2* e) {
+      e[0] = __ldg(sched);
+      e[1] = two ? __ldg(sched + NH) : make_uint2(0u, 0u);
+      sched += NT;
+    };
+    auto fetch = [&]() {
+#pragma unroll
+      for (int w = 0; w < 2; ++w) {
+        const Tagged* x = X + (cell[w].y & 0xffffu);
+        ld_tagged(ru[w], x + XP, cell[w].y != 0u);
+        ld_tagged(rd[w], x - XP, cell[w].y != 0u);
+        ld_pred(rs[w], Sd + (cell[w].y >> 16), cell[w].y != 0u);
+      }
+    };
+    // the values in flight, checked, into slot s of B
+    auto deliver = [&](int s, int* gave_up) {
+#pragma unroll
+      for (int w = 0; w < 2; ++w) {
+        if (cell[w].y == 0u) continue;
+        const unsigned hs = cell[w].x >> 16, prev = hs == 0u ? MG_INITIAL : hs - 1u;
+        const unsigned long long wu = seq | (top ? MG_INITIAL : prev), wd = seq | (bottom ? MG_INITIAL : prev);
+        const Tagged* x = X + (cell[w].y & 0xffffu);
+        long long tries = 0;
+        while (tagged_tag(ru[w]) != wu || tagged_tag(rd[w]) != wd) {
+          if (++tries > c->wait_limit || *(volatile int*)&c->abort) {
+            *gave_up = 1;
+            atomicOr(&c->status, MG_ST_TIMEOUT);
+            atomicExch(&c->abort, 1);
+            break;
+          }
+          ld_tagged(ru[w], x + XP, true);
+          ld_tagged(rd[w], x - XP, true);
+        }
+        double* b = B + s * 3 * NT + h + w * NH;
+        b[0] = tagged_value(ru[w]);
+        b[NT] = tagged_value(rd[w]);
+        b[2 * NT] = rs[w];
+      }
+    };
+    entries(cell);
+    entries(ahead);
+    __syncthreads();
+    fetch();
+    deliver(0, &s_gave_up[1]);  // step 2's (t0 = 2: pair parity 1)
+    cell[0] = ahead[0];
+    cell[1] = ahead[1];
+    entries(ahead);
+    fetch();
+    __syncthreads();
+    for (int t0 = 2; t0 < 2 + G::STEPS; t0 += 2) {
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {  // during step t0 + q
+        deliver(q ^ 1, &s_gave_up[(t0 >> 1) & 1]);
+        cell[0] = ahead[0];
+        cell[1] = ahead[1];
+        entries(ahead);
+        fetch();
+        __syncthreads();
+      }
+      if (*(volatile int*)&s_gave_up[(t0 >> 1) & 1]) return;
+    }
   }
+  for (int j = 1 + tid / 32; j <= N; j += (NT + NH) / 32)
+    for (int i = 1 + tid % 32; i <= N; i += 32) E[i + s1 * j] = P[((i & 1) * (N + 2) + j) * R + (i >> 1)];
   if (TRACK) {
     const double a = block_sum(acc8, red);
-    if (threadIdx.x == 0) part[blockIdx.x] = a;
+    if (tid == 0) part[blockIdx.x] = a;
     const double b = block_sum(acc9, red);
-    if (threadIdx.x == 0) part[n + blockIdx.x] = b;
+    if (tid == 0) part[N + blockIdx.x] = b;
   }
 }
 
@@ -1035,47 +1211,44 @@ bool launch_pipe(MgCtl* c, const MgLevel& lv, double* part, cudaStream_t s) {
   return cudaLaunchKernelEx(&cfg, k_mg_relax_pipe<NT, MINB, HG, G, CH, TRACK>, c, lv, part) == cudaSuccess;
 }
 
-// The shared-memory-plane relax: one block of NT threads per plane, all
-// resident at once (with the plane's dynamic shared memory).
-template <int NT, int HG, int CH, bool TRACK>
-bool launch_plane(MgCtl* c, const MgLevel& lv, double* part, cudaStream_t s) {
-  const int n = lv.n;
-  const int nt = (n * HG + 31) / 32 * 32;
-  static int state = 0;  // 0 unknown, 1 fits, 2 does not (one level size per instantiation)
+// The shared-memory-plane relax: one block per plane, all resident at once.
+template <int N, bool TRACK>
+bool launch_plane(MgCtl* c, const MgLevel& lv, int leg, double* part, cudaStream_t s) {
+  using G = PlaneGeo<N>;
+  static int state = 0;  // 0 unknown, 1 fits, 2 does not
   if (!state) {
     int dev = 0, sms = 0, per = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    bool ok = cudaFuncSetAttribute(k_mg_relax_plane<NT, HG, CH, TRACK>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)plane_smem(n)) == cudaSuccess;
-    ok = ok && cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_mg_relax_plane<NT, HG, CH, TRACK>, nt,
-                                                             plane_smem(n)) == cudaSuccess;
+    bool ok = cudaFuncSetAttribute(k_mg_relax_plane<N, TRACK>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)G::smem) == cudaSuccess;
+    ok = ok && cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_mg_relax_plane<N, TRACK>, G::NT + G::NH, G::smem) ==
+                   cudaSuccess;
     if (!ok) cudaGetLastError();
-    state = (ok && (long long)per * sms >= n) ? 1 : 2;
+    state = (ok && (long long)per * sms >= N) ? 1 : 2;
   }
-  if (state != 1) return false;
-  k_mg_prog_reset<<<1, 256, 0, s>>>(c, n);
+  if (state != 1 || !lv.X) return false;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(n);
-  cfg.blockDim = dim3(nt);
-  cfg.dynamicSmemBytes = plane_smem(n);
+  cfg.gridDim = dim3(N);
+  cfg.blockDim = dim3(G::NT + G::NH);
+  cfg.dynamicSmemBytes = G::smem;
   cfg.stream = s;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeCooperative;
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, k_mg_relax_plane<NT, HG, CH, TRACK>, c, lv, part) == cudaSuccess;
+  return cudaLaunchKernelEx(&cfg, k_mg_relax_plane<N, TRACK>, c, lv, leg, part) == cudaSuccess;
 }
 
 template <bool TRACK>
-bool launch_plane_any(MgCtl* c, const MgLevel& lv, double* part, cudaStream_t s) {
+bool launch_plane_any(MgCtl* c, const MgLevel& lv, int leg, double* part, cudaStream_t s) {
   switch (lv.n) {
-    case 8: return launch_plane<96, 10, 2, TRACK>(c, lv, part, s);
-    case 16: return launch_plane<160, 10, 2, TRACK>(c, lv, part, s);
-    case 32: return launch_plane<320, 10, 4, TRACK>(c, lv, part, s);
-    case 64: return launch_plane<640, 10, 8, TRACK>(c, lv, part, s);
-    case 128: return launch_plane<640, 5, 8, TRACK>(c, lv, part, s);
+    case 8: return launch_plane<8, TRACK>(c, lv, leg, part, s);
+    case 16: return launch_plane<16, TRACK>(c, lv, leg, part, s);
+    case 32: return launch_plane<32, TRACK>(c, lv, leg, part, s);
+    case 64: return launch_plane<64, TRACK>(c, lv, leg, part, s);
+    case 128: return launch_plane<128, TRACK>(c, lv, leg, part, s);
     default: return false;
   }
 }
@@ -1085,16 +1258,15 @@ bool launch_plane_any(MgCtl* c, const MgLevel& lv, double* part, cudaStream_t s)
 // Levels up to 128 cells hold their planes in shared memory
 // (k_mg_relax_plane) unless TLQ_MG_PLANE=0; the others, and those, then use
 // k_mg_relax_pipe.  Its threads per plane (measured on the gravitating
-// cloud): 128-cell levels
-// 5 x 128 (two half-sweeps each), 64 down to 8: 10 x n; neighbour checks
-// every 8 steps on 128 and 64 cells, 4 on 32, 2 below (a relax takes
-// 2n + 9 (CH + 1) steps); 256-cell levels need two blocks per SM: 2 x 256,
-// checks every 4 steps.
+// cloud): 128-cell levels 5 x 128 (two half-sweeps each), 64 down to 8:
+// 10 x n; neighbour checks every 8 steps on 128 and 64 cells, 4 on 32, 2
+// below (a relax takes 2n + 9 (CH + 1) steps); 256-cell levels need two
+// blocks per SM: 2 x 256, checks every 4 steps.
 template <bool TRACK>
-bool launch_pipe_any(MgCtl* c, const MgLevel& lv, double* part, cudaStream_t s) {
+bool launch_pipe_any(MgCtl* c, const MgLevel& lv, int leg, double* part, cudaStream_t s) {
   const char* env = std::getenv("TLQ_MG_PLANE");
   const bool plane = !(env && env[0] == '0');
-  if (plane && launch_plane_any<TRACK>(c, lv, part, s)) return true;
+  if (plane && launch_plane_any<TRACK>(c, lv, leg, part, s)) return true;
   switch (lv.n) {
     case 8: return launch_pipe<96, 1, 10, 1, 2, TRACK>(c, lv, part, s);
     case 16: return launch_pipe<160, 1, 10, 1, 2, TRACK>(c, lv, part, s);
@@ -1106,10 +1278,11 @@ bool launch_pipe_any(MgCtl* c, const MgLevel& lv, double* part, cudaStream_t s) 
   }
 }
 
-void launch_relax(MgCtl* c, const MgLevel& lv, double* part, cudaStream_t s) {
+// leg: 0 on the way down, 1 on the way up.
+void launch_relax(MgCtl* c, const MgLevel& lv, int leg, double* part, cudaStream_t s) {
   const char* env = std::getenv("TLQ_MG_PIPELINE");
   const bool pipe = !(env && env[0] == '0');
-  if (pipe && (part ? launch_pipe_any<true>(c, lv, part, s) : launch_pipe_any<false>(c, lv, part, s))) return;
+  if (pipe && (part ? launch_pipe_any<true>(c, lv, leg, part, s) : launch_pipe_any<false>(c, lv, leg, part, s))) return;
   for (int h = 0; h < 10; ++h) launch_half(c, lv, h & 1, (part && h >= 8) ? part + (h - 8) * lv.n : nullptr, s);
 }
 
@@ -1154,6 +1327,30 @@ cudaError_t mg_alloc(tlq_ctx* ctx) {
   e = cudaMemcpy(reinterpret_cast<char*>(ctx->mg_ctl) + offsetof(MgCtl, wait_limit), &limit, sizeof limit,
                  cudaMemcpyHostToDevice);
   if (e != cudaSuccess) return e;
+  long long xc = 0, sc = 0;
+  for (int l = 0; l <= L; ++l)
+    if (exch_level(ctx->cfg.nx >> l)) {
+      xc += exch_cells(ctx->cfg.nx >> l);
+      sc += 2 * sched_entries(ctx->cfg.nx >> l);
+    }
+  if (xc) {
+    e = cudaMalloc(&ctx->mg_sched, (size_t)sc * sizeof(MgSched));
+    if (e != cudaSuccess) return e;
+    MgSched* at = static_cast<MgSched*>(ctx->mg_sched);
+    for (int l = 0; l <= L; ++l) {
+      const int n = ctx->cfg.nx >> l;
+      if (!exch_level(n)) continue;
+      const int nt = (5 * n + 31) / 32 * 32, rows = (int)(sched_entries(n) / nt);
+      k_mg_sched<<<(unsigned)((2 * sched_entries(n) + 255) / 256), 256>>>(n, at, rows, nt);
+      e = cudaGetLastError();
+      if (e != cudaSuccess) return e;
+      at += 2 * sched_entries(n);
+    }
+    e = cudaMalloc(&ctx->mg_exch, (size_t)xc * sizeof(Tagged));
+    if (e != cudaSuccess) return e;
+    e = cudaMemset(ctx->mg_exch, 0, (size_t)xc * sizeof(Tagged));  // (no call's tag)
+    if (e != cudaSuccess) return e;
+  }
   e = cudaMalloc(&ctx->mg_mom, (size_t)MG_MOM_BLOCKS * 25 * sizeof(double));
   if (e != cudaSuccess) return e;
   e = cudaStreamCreateWithFlags(&ctx->mg_body, cudaStreamNonBlocking);
@@ -1171,6 +1368,8 @@ cudaError_t mg_alloc(tlq_ctx* ctx) {
 }
 
 void mg_free(tlq_ctx* ctx) {
+  cudaFree(ctx->mg_exch); cudaFree(ctx->mg_sched);
+  ctx->mg_exch = nullptr; ctx->mg_sched = nullptr;
   cudaFree(ctx->mg_work); cudaFree(ctx->mg_ctl); cudaFree(ctx->mg_mom); cudaFree(ctx->phig); cudaFree(ctx->phit);
   if (ctx->mg_body) cudaStreamDestroy(ctx->mg_body);
   ctx->mg_work = nullptr; ctx->mg_ctl = nullptr; ctx->mg_mom = nullptr; ctx->phig = nullptr; ctx->phit = nullptr;
@@ -1187,11 +1386,17 @@ MgLevels mg_plan(const tlq_ctx* ctx, int L) {
     total += m * m * m;
   }
   double* base = static_cast<double*>(ctx->mg_work);
-  long long off = 0;
+  long long off = 0, xoff = 0, soff = 0;
   for (int l = 0; l <= L; ++l) {
     const int n = ctx->cfg.nx >> l;
     const long long m = n + 2;
     v.lv[l].n = n;
+    v.lv[l].X = exch_level(n) ? static_cast<Tagged*>(ctx->mg_exch) + xoff : nullptr;
+    v.lv[l].sched = exch_level(n) ? static_cast<MgSched*>(ctx->mg_sched) + soff : nullptr;
+    if (exch_level(n)) {
+      xoff += exch_cells(n);
+      soff += 2 * sched_entries(n);
+    }
     v.lv[l].E = base + off;
     v.lv[l].R = base + total + off;
     v.lv[l].T = base + 2 * total + off;
@@ -1238,7 +1443,7 @@ cudaError_t enqueue_mg(tlq_ctx* ctx, Dens rho, const Clock* clk, double* phit, c
     // down: level 0 .. lc-1 on the large kernels
     for (int l = 0; l < lc; ++l) {
       if (l > 0) k_mg_ghosts<<<1, 1024, 0, st>>>(c, v.lv[l], multipole ? 1 : 0);
-      launch_relax(c, v.lv[l], nullptr, st);
+      launch_relax(c, v.lv[l], 0, nullptr, st);
       k_mg_resid_restrict<<<grid_for((long long)v.lv[l + 1].n * v.lv[l + 1].n * v.lv[l + 1].n, 256), 256, 0, st>>>(
           c, v.lv[l], v.lv[l + 1]);
     }
@@ -1249,7 +1454,7 @@ cudaError_t enqueue_mg(tlq_ctx* ctx, Dens rho, const Clock* clk, double* phit, c
       k_mg_prolong_add<<<grid_for(mf * mf * mf, 256), 256, 0, st>>>(c, v.lv[l + 1], v.lv[l]);
       if (l > 0) k_mg_ghosts<<<1, 1024, 0, st>>>(c, v.lv[l], multipole ? 1 : 0);
       // the last pass of the level-0 relax forms Dif (sources.f90:465-471)
-      launch_relax(c, v.lv[l], l == 0 ? part : nullptr, st);
+      launch_relax(c, v.lv[l], 1, l == 0 ? part : nullptr, st);
     }
     k_mg_cycle_end<<<1, 1, 0, st>>>(c, 2 * n);
   };
