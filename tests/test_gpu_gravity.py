@@ -52,6 +52,20 @@ def test_multigrid_bit_exact_zero_faces(gpu_lib, n):
     np.testing.assert_array_equal(g, o)
 
 
+@pytest.mark.parametrize("n,bc", [(2, tlq.GBC_ZERO), (4, tlq.GBC_ZERO), (4, tlq.GBC_MULTIPOLE)])
+def test_multigrid_whole_mesh_in_one_block(gpu_lib, n, bc):
+    """Meshes of fewer than 8 cells a side: the whole cycle in the one-block
+    kernel (n = 8 is among the cases above), twice from a perturbed
+    potential whose faces hold values, bit for bit."""
+    cfg, U0 = problems.gravitating_cloud(n, grav_bc=bc)
+    start = 1e9 * np.random.default_rng(n).standard_normal(cfg.phi_shape)
+    for it in (1, 2):  # (no face update: it % 10 != 0)
+        g, gc, o, oc = one_call(cfg, U0, np.asfortranarray(start), it)
+        assert gc == oc
+        np.testing.assert_array_equal(g, o)
+        start = o
+
+
 def test_multigrid_bit_exact_256(gpu_lib):
     """A 256^3 mesh: its finest level relaxes in the 512-thread, two blocks
     per SM variant of the pipelined kernel (256 planes resident at once)."""

@@ -31,6 +31,7 @@ struct tlq_ctx {
   void* mg_mom = nullptr;
   void* mg_exch = nullptr;  // the levels' exchange arrays between planes
   void* mg_sched = nullptr;  // and the relax's schedules
+  void* mg_coarse = nullptr;  // the one-block levels' schedule
   cudaStream_t mg_body = nullptr;  // captures a V-cycle into a graph's loop body
   double* phig = nullptr;
   double* phit = nullptr;

@@ -32,7 +32,7 @@
 // device, so the solve needs no host round trip: in a CUDA graph the
 // V-cycles are the body of a while node whose condition that test sets; run
 // directly, a fixed sequence of 31 cycle slots whose launches return once
-// the test failed.  Levels of at most 4 cells run inside one block (one
+// the test failed.  Levels of at most 8 cells run inside one block (one
 // launch per cycle).
 //
 // Built with -fmad=false (FP64 as the restatement evaluates it).
@@ -41,6 +41,7 @@
 #include <cstddef>
 #include <cstdlib>
 #include <cstring>
+#include <memory>
 #include <string>
 
 #include "tlq_convert.cuh"
@@ -50,7 +51,7 @@ namespace tlq {
 namespace {
 
 constexpr int MG_MAXL = 11;         // levels 0..10: meshes up to 1024^3
-constexpr int MG_COARSE_N = 4;      // levels of at most this many cells run in the one-block kernel
+constexpr int MG_COARSE_N = 8;      // levels of at most this many cells run in the one-block kernel
 constexpr int MG_CYCLES = 31;       // the reference's V-cycle cap (sources.f90:140)
 constexpr int MG_PF = 4;            // diagonal steps the smoother's loads run ahead
 constexpr int MG_MOM_THREADS = 256;
@@ -104,16 +105,6 @@ struct DensAoS {
 // ---------------------------------------------------------------------------
 // Multipole boundary values (sources.f90:9-96, 558-787)
 // ---------------------------------------------------------------------------
-__device__ double powi(double x, int n) {  // x**n, run-time n: the binary method, as gfortran
-  unsigned m = n < 0 ? (unsigned)(-n) : (unsigned)n;
-  double y = (m % 2) ? x : 1.0;
-  while (m >>= 1) {
-    x = x * x;
-    if (m % 2) y = y * x;
-  }
-  return n < 0 ? 1.0 / y : y;
-}
-
 __device__ double legendre(double x, int l) {
   const double x2 = x * x;
   switch (l) {
@@ -129,7 +120,7 @@ __device__ double legendre(double x, int l) {
 // reference raises to the real powers 1/2 and 3/2; equal up to rounding).
 // |x| <= 1 here (x = z/r with r >= |z| in rounded arithmetic), so 1 - x^2 >= 0.
 __device__ double alegendre(double x, int l, int m) {
-  const double x2 = x * x, s = 1.0 - x2, q = sqrt(s);
+  const double x2 = x * x, s = 1.0 - x2, q = sf::sqrt_rn(s);
   switch (l) {
     case 0: return 1.0;
     case 1: return m == 0 ? x : -q;
@@ -157,7 +148,8 @@ __device__ double alegendre(double x, int l, int m) {
 // cos(acos(z/r))), and cos(m phi), sin(m phi) from cos phi = x/rho, sin phi
 // = y/rho, rho = |(x, y)|, by the Chebyshev recurrence (it takes cos and sin
 // of m atan2(y, x)).  Equal up to rounding; on the FP64 pipe these are a few
-// operations instead of eleven transcendental functions per cell.
+// operations instead of eleven transcendental functions per cell, the roots
+// and divisions on the integer pipe beside them.
 struct Sph {
   double coth, r, c[5], s[5];
 };
@@ -167,10 +159,10 @@ __device__ Sph sph_terms(const Params& p, int i, int j, int k) {
   const double z = (p.zl + p.dz * (double)k) - p.dz / 2.0;
   Sph o;
   const double rho2 = x * x + y * y;
-  o.r = sqrt(rho2 + z * z);
-  o.coth = z / o.r;
-  const double rho = sqrt(rho2);
-  const double c1 = rho > 0.0 ? x / rho : 1.0, s1 = rho > 0.0 ? y / rho : 0.0;
+  o.r = sf::sqrt_rn(rho2 + z * z);
+  o.coth = sf::div(z, o.r);
+  const double rho = sf::sqrt_rn(rho2);
+  const double c1 = rho > 0.0 ? sf::div(x, rho) : 1.0, s1 = rho > 0.0 ? sf::div(y, rho) : 0.0;
   o.c[0] = 1.0;
   o.s[0] = 0.0;
   o.c[1] = c1;
@@ -184,6 +176,7 @@ __device__ Sph sph_terms(const Params& p, int i, int j, int k) {
 }
 
 // 25 sums per block: c0 l = 0..4, then cm and sm for l = 1..4, m = 1..l.
+// FP64 pipe (128^3: 765 us with the roots and divisions on it, 586 without).
 template <class Dens>
 __global__ void __launch_bounds__(MG_MOM_THREADS) k_mg_moments(const MgCtl* c, const Clock* clk, Params p, Dens rho,
                                                              double* part) {
@@ -234,20 +227,24 @@ __global__ void __launch_bounds__(MG_MOM_THREADS) k_mg_moments(const MgCtl* c, c
   }
 }
 
-__global__ void k_mg_moments_final(MgCtl* c, const Clock* clk, const double* part, int nblocks) {
+// The moments from the blocks' sums, a warp per moment.
+__global__ void __launch_bounds__(25 * 32) k_mg_moments_final(MgCtl* c, const Clock* clk, const double* part,
+                                                            int nblocks) {
   // slots 5..14 (cm) and 15..24 (sm): (l, m) = (1,1) (2,1) (2,2) (3,1) .. (4,4)
   constexpr int LS[10] = {1, 2, 2, 3, 3, 3, 4, 4, 4, 4}, MS[10] = {1, 1, 2, 1, 2, 3, 1, 2, 3, 4};
   if (!c->run || clk->it % 10 != 0) return;
-  const int q = threadIdx.x;
-  if (q >= 25) return;
+  const int q = threadIdx.x / 32;
   double v = 0.0;
-  for (int b = 0; b < nblocks; ++b) v += part[b * 25 + q];
+  for (int b = threadIdx.x % 32; b < nblocks; b += 32) v += part[b * 25 + q];
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+  if (threadIdx.x % 32) return;
   if (q < 5) {
     c->c0[q] = v;
     return;
   }
   const int r = q < 15 ? q - 5 : q - 15, l = LS[r], m = MS[r];
-  const double cf = 2.0 * tgamma((double)(l - m) + 1.0) / tgamma((double)(l + m) + 1.0);
+  double cf = 2.0;  // 2 (l - m)! / (l + m)!
+  for (int f = l - m + 1; f <= l + m; ++f) cf = cf / (double)f;
   if (q < 15)
     c->cm[l][m] = cf * v;
   else
@@ -270,12 +267,15 @@ __global__ void k_mg_faces(const MgCtl* c, const Clock* clk, Params p, double* p
     else { i = a; j = b; k = bnd; }
     const Sph sp = sph_terms(p, i, j, k);
     const double coth = sp.coth, rb = sp.r;
-    double v = 0.0;
-    v = v - c->c0[0] / rb;
-    for (int l = 1; l <= 4; ++l) {
-      v = v - c->c0[l] * legendre(coth, l) / powi(rb, l + 1);
+    double v = sf::div(-c->c0[0], rb), rp = rb;
+#pragma unroll
+    for (int l = 1; l <= 4; ++l) {  // (degree l's terms over r**(l+1) at once)
+      rp = rp * rb;
+      double t = c->c0[l] * legendre(coth, l);
+#pragma unroll
       for (int m = 1; m <= l; ++m)
-        v = v - 2.0 * (c->cm[l][m] * sp.c[m] + c->sm[l][m] * sp.s[m]) * alegendre(coth, l, m) / powi(rb, l + 1);
+        t = t + 2.0 * (c->cm[l][m] * sp.c[m] + c->sm[l][m] * sp.s[m]) * alegendre(coth, l, m);
+      v = v - sf::div(t, rp);
     }
     phi[mgi(n, i, j, k)] = 6.67430e-8 * v;
   }
@@ -284,13 +284,36 @@ __global__ void k_mg_faces(const MgCtl* c, const Clock* clk, Params p, double* p
 // ---------------------------------------------------------------------------
 // Cycle control
 // ---------------------------------------------------------------------------
-__global__ void k_mg_begin(MgCtl* c, const Clock* clk) {
+// The loop test of the V-cycles (sources.f90:140): another cycle while
+// Dif > 10 and fewer than 31 ran.  As the condition of a graph's loop node
+// where the V-cycles are the body of one (loop), so that cycles after
+// convergence are not launched at all.
+__device__ void mg_loop_test(MgCtl* c, bool loop, cudaGraphConditionalHandle h) {
+  const int go = c->run && c->dif > 10.0 && c->iter < MG_CYCLES;
+  c->active = go;
+  if (go) c->iter = c->iter + 1;
+  if (loop) cudaGraphSetConditional(h, go ? 1u : 0u);
+}
+
+__global__ void k_mg_begin(MgCtl* c, const Clock* clk, bool loop, cudaGraphConditionalHandle h) {
   c->run = clk->t < clk->tfin;  // the loop test of mainHD.f90:61 (the step's)
-  c->active = 0;
   c->iter = 0;
   c->dif = 1.e28;
   c->abort = 0;
   c->call = c->call + 1u;
+  mg_loop_test(c, loop, h);
+}
+
+// One warp: Dif from the planes' sums (256 of them on 128 cells: 19 us as
+// one thread's chain of FP64 additions), and the next loop test.
+__global__ void k_mg_cycle_end(MgCtl* c, int nparts, bool loop, cudaGraphConditionalHandle h) {
+  if (!c->active) return;
+  double v = 0.0;
+  for (int q = threadIdx.x; q < nparts; q += 32) v += c->part[q];
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+  if (threadIdx.x) return;
+  c->dif = v;
+  mg_loop_test(c, loop, h);
 }
 
 // Residue(0) = 4 pi G dens, Error(0) = phi (sources.f90:136-137).
@@ -307,43 +330,6 @@ __global__ void k_mg_init(const MgCtl* c, Dens rho, int n, const double* phi, do
     T0[q] = r * (dxl * dxl);
     E0[q] = phi[q];
   }
-}
-
-// The loop test of the V-cycles (sources.f90:140): another cycle while
-// Dif > 10 and fewer than 31 ran; the error of every coarse level restarts
-// at 0 (:146-148).
-// (Every block decides from the same inputs; k_mg_cycle_flag updates them
-// after this launch.)
-__global__ void k_mg_cycle_begin(const MgCtl* c, double* Ecoarse, long long ncoarse) {
-  __shared__ int go;
-  if (threadIdx.x == 0) go = c->run && c->dif > 10.0 && c->iter < MG_CYCLES;
-  __syncthreads();
-  if (!go) return;
-  for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < ncoarse;
-       q += (long long)gridDim.x * blockDim.x)
-    Ecoarse[q] = 0.0;
-}
-
-// The flag and the count, after every block of k_mg_cycle_begin has read
-// the previous values.
-__global__ void k_mg_cycle_flag(MgCtl* c) {
-  const int go = c->run && c->dif > 10.0 && c->iter < MG_CYCLES;
-  c->active = go;
-  if (go) c->iter = c->iter + 1;
-}
-
-// The same loop test as the condition of a graph's loop node: the step's
-// graph runs the V-cycles as the body of a while node, so that cycles after
-// convergence are not launched at all.
-__global__ void k_mg_loop_test(const MgCtl* c, cudaGraphConditionalHandle h) {
-  cudaGraphSetConditional(h, (c->run && c->dif > 10.0 && c->iter < MG_CYCLES) ? 1u : 0u);
-}
-
-__global__ void k_mg_cycle_end(MgCtl* c, int nparts) {
-  if (!c->active) return;
-  double v = 0.0;
-  for (int q = 0; q < nparts; ++q) v += c->part[q];
-  c->dif = v;
 }
 
 // phi = Error(0) (sources.f90:189); PHIT = PHIP + PHI into the stage's
@@ -682,7 +668,7 @@ __global__ void __launch_bounds__(NT, MINB) k_mg_relax_pipe(MgCtl* c, MgLevel lv
 }
 
 // ---------------------------------------------------------------------------
-// The skewed relax with the block's plane in shared memory (levels of 8 to
+// The skewed relax with the block's plane in shared memory (levels of 16 to
 // 128 cells: (N+2)^2 doubles, 135 KB at 128).  Only plane k's block writes
 // plane k during a relax, so its copy in shared memory is the current one: an
 // update reads its old value and its four in-plane neighbours there.  The
@@ -723,7 +709,7 @@ __global__ void __launch_bounds__(NT, MINB) k_mg_relax_pipe(MgCtl* c, MgLevel lv
 // FP64 pipe.  Measured per launch on the 128^3 cloud (ncu), against a thread
 // per column and group with loads one step ahead and a fence and a poll by
 // the whole block every few steps: 128 cells 743 -> 380 us, 64: 260 -> 130,
-// 32: 143 -> 65, 16: 98 -> 43, 8: 60 -> 34.
+// 32: 143 -> 65, 16: 98 -> 43.
 // ---------------------------------------------------------------------------
 constexpr int MG_SKEW = 4;  // (6: 4 % slower, 2 more steps per half-sweep; 2 leaves a value no time to arrive)
 constexpr unsigned MG_INITIAL = 15;
@@ -959,144 +945,212 @@ __global__ void k_mg_prog_reset(MgCtl* c, int n) {
   for (int q = threadIdx.x; q <= n + 1; q += blockDim.x) c->prog[q] = -1;
 }
 
-// The error's ghosts on a coarse level: -(first interior layer) per face in
-// each build's statement order (sources.f90:262-283, 285-290); one block.
-__device__ void mg_ghosts(const MgLevel& lv, int bc_multipole) {
-  const int n = lv.n, m = n + 2;
-  double* E = lv.E;
-  const int order_mpi[6] = {0, 1, 2, 3, 4, 5};  // x-, x+, y-, y+, z-, z+
-  const int order_ser[6] = {0, 2, 4, 1, 3, 5};  // x-, y-, z-, x+, y+, z+
-  for (int s = 0; s < 6; ++s) {
-    const int f = bc_multipole ? order_mpi[s] : order_ser[s];
-    const int axis = f >> 1, hi = f & 1;
-    const int g = hi ? n + 1 : 0, src = hi ? n : 1;
-    for (int q = threadIdx.x; q < m * m; q += blockDim.x) {
-      const int a = q % m, b = q / m;
-      long long to, from;
-      if (axis == 0) { to = mgi(n, g, a, b); from = mgi(n, src, a, b); }
-      else if (axis == 1) { to = mgi(n, a, g, b); from = mgi(n, a, src, b); }
-      else { to = mgi(n, a, b, g); from = mgi(n, a, b, src); }
-      E[to] = -E[from];
-    }
-    __syncthreads();
+// A coarse level's error at cell (i, j, k) and, where the cell lies at the
+// level's edge, in its ghosts.  The reference sets each face's ghosts to
+// -(first interior layer) over the whole face, face after face (sources.f90:
+// 262-283, 285-290): whatever the order of the faces, a ghost then holds the
+// nearest interior cell's value, negated once per coordinate out of range.
+__device__ __forceinline__ void mg_put(double* E, int n, int i, int j, int k, double v) {
+  double* p = E + mgi(n, i, j, k);
+  if (n == 1) {
+    for (int q = 0; q < 27; ++q) E[q] = (q == 13 || ((q % 3 != 1) + (q / 3 % 3 != 1) + (q / 9 != 1)) == 2) ? v : -v;
+    return;
   }
-}
-
-__global__ void __launch_bounds__(1024) k_mg_ghosts(const MgCtl* c, MgLevel lv, int bc_multipole) {
-  if (!c->active) return;
-  mg_ghosts(lv, bc_multipole);
+  const int s1 = n + 2, s2 = s1 * s1;
+  const int x = i == 1 ? -1 : i == n ? 1 : 0, y = j == 1 ? -s1 : j == n ? s1 : 0, z = k == 1 ? -s2 : k == n ? s2 : 0;
+  p[0] = v;
+  if (x) p[x] = -v;
+  if (y) p[y] = -v;
+  if (z) p[z] = -v;
+  if (x && y) p[x + y] = v;
+  if (x && z) p[x + z] = v;
+  if (y && z) p[y + z] = v;
+  if (x && y && z) p[x + y + z] = -v;
 }
 
 // resid on the fine level (sources.f90:196-216) and restriction onto the
-// coarse one (:118-137), fused: each coarse cell forms its 8 children's
-// residuals.  (The reference's ret array of the fine level is not kept: it
-// is overwritten before anything reads it.)
-__device__ __forceinline__ double mg_resid_cell(const MgLevel& f, int i, int j, int k) {
-  const int n = f.n;
-  const long long o = mgi(n, i, j, k), s1 = n + 2, s2 = (long long)(n + 2) * (n + 2);
-  const double* E = f.E;
-  double g = E[o - 1] + E[o + 1];
-  g = g + E[o - s1];
-  g = g + E[o + s1];
-  g = g + E[o - s2];
-  g = g + E[o + s2];
-  g = (g - 6.0 * E[o]) / (f.dxl * f.dxl);
-  return f.R[o] - g;
-}
-
-__device__ void mg_resid_restrict(const MgLevel& f, const MgLevel& c, long long t, long long nt) {
-  const int nc = c.n;
-  for (long long q = t; q < (long long)nc * nc * nc; q += nt) {
-    const int i = 1 + (int)(q % nc), j = 1 + (int)((q / nc) % nc), k = 1 + (int)(q / ((long long)nc * nc));
-    const int i1 = 2 * i - 1, j1 = 2 * j - 1, k1 = 2 * k - 1;
-    double a = mg_resid_cell(f, i1, j1, k1) + mg_resid_cell(f, i1 + 1, j1, k1);
-    a = a + mg_resid_cell(f, i1, j1 + 1, k1);
-    a = a + mg_resid_cell(f, i1, j1, k1 + 1);
-    a = a + mg_resid_cell(f, i1 + 1, j1 + 1, k1);
-    a = a + mg_resid_cell(f, i1 + 1, j1, k1 + 1);
-    a = a + mg_resid_cell(f, i1, j1 + 1, k1 + 1);
-    a = a + mg_resid_cell(f, i1 + 1, j1 + 1, k1 + 1);
-    const double r = (1.0 / 8.0) * a;
-    c.R[mgi(nc, i, j, k)] = r;
-    c.T[mgi(nc, i, j, k)] = r * (c.dxl * c.dxl);
-  }
+// coarse one (:118-137), fused: each coarse cell q forms its 8 children's
+// residuals; its own error starts the cycle's way down at 0 (:146-148).
+// (The reference's ret array of the fine level is not kept: it is
+// overwritten before anything reads it.)  The FP64 pipe bounds it: 8
+// operations a fine cell are left on it, the division by dxl**2 and the
+// product 6 E run on the integer pipe beside them.  128^3 fine cells: 72 -> 30 us.
+__device__ __forceinline__ void mg_resid_restrict(const double* __restrict__ E, const double* __restrict__ Rf, int n,
+                                                  double dxl, double* Ec, double* Rc, double* Tc, int q) {
+  const int nc = n / 2, s1 = n + 2, s2 = (n + 2) * (n + 2);
+  const int i = 1 + q % nc, j = 1 + (q / nc) % nc, k = 1 + q / (nc * nc);
+  const long long o0 = mgi(n, 2 * i - 1, 2 * j - 1, 2 * k - 1);
+  const double d2 = dxl * dxl;
+  auto cell = [&](int di, int dj, int dk) {
+    const long long o = o0 + di + s1 * dj + s2 * dk;
+    double g = E[o - 1] + E[o + 1];
+    g = g + E[o - s1];
+    g = g + E[o + s1];
+    g = g + E[o - s2];
+    g = g + E[o + s2];
+    g = sf::div(g - sf::mul(6.0, E[o]), d2);
+    return Rf[o] - g;
+  };
+  double a = cell(0, 0, 0) + cell(1, 0, 0);
+  a = a + cell(0, 1, 0);
+  a = a + cell(0, 0, 1);
+  a = a + cell(1, 1, 0);
+  a = a + cell(1, 0, 1);
+  a = a + cell(0, 1, 1);
+  a = a + cell(1, 1, 1);
+  const double r = (1.0 / 8.0) * a, dc = dxl * 2.0;  // (the coarse level's dxl: (xr - xl) / (n/2), exactly twice)
+  Rc[mgi(nc, i, j, k)] = r;
+  Tc[mgi(nc, i, j, k)] = r * (dc * dc);
+  mg_put(Ec, nc, i, j, k, 0.0);
 }
 
 __global__ void k_mg_resid_restrict(const MgCtl* c, MgLevel f, MgLevel co) {
   if (!c->active) return;
-  mg_resid_restrict(f, co, blockIdx.x * (long long)blockDim.x + threadIdx.x, (long long)gridDim.x * blockDim.x);
+  const int q = blockIdx.x * blockDim.x + threadIdx.x;
+  if (q < co.n * co.n * co.n) mg_resid_restrict(f.E, f.R, f.n, f.dxl, co.E, co.R, co.T, q);
 }
 
-// prolongation (sources.f90:139-194) onto a zeroed ret, then
-// Error = Error + ret over the whole array (:181): interior cells add their
-// trilinear child value, ghosts add 0.
-__device__ void mg_prolong_add(const MgLevel& c, const MgLevel& f, long long t, long long nt) {
-  const int nf = f.n, nc = c.n, m = nf + 2;
+// prolongation (sources.f90:139-194), then Error = Error + ret (:181) and,
+// on a coarse level (ghosts), the error's ghosts: each coarse cell q serves
+// its 8 children, whose sums begin alike (27 V + 9 Vx for four of them, with
+// 9 Vy for two): 54 additions and 19 products where 8 separate sums take 64
+// and 64, the products on the integer pipe beside the additions, which
+// bound it.  The last two operations are one fused one: (1/64) r is exact
+// (unless it is subnormal: then as two).  128^3 fine cells: 72 -> 34 us (and
+// 12.6 us less per coarse level, the launch that set the ghosts).
+__device__ __forceinline__ void mg_prolong_add(const double* __restrict__ V, double* E, int nc, int q, bool ghosts) {
+  const int n = 2 * nc;
   const long long s1 = nc + 2, s2 = (long long)(nc + 2) * (nc + 2);
-  for (long long q = t; q < (long long)m * m * m; q += nt) {
-    const int fi = (int)(q % m), fj = (int)((q / m) % m), fk = (int)(q / ((long long)m * m));
-    double r = 0.0;
-    if (fi >= 1 && fi <= nf && fj >= 1 && fj <= nf && fk >= 1 && fk <= nf) {
-      const int i = (fi + 1) >> 1, j = (fj + 1) >> 1, k = (fk + 1) >> 1;
-      const long long di = (fi & 1) ? -1 : 1, dj = (fj & 1) ? -s1 : s1, dk = (fk & 1) ? -s2 : s2;
-      const long long o = mgi(nc, i, j, k);
-      const double* V = c.E;
-      double a = 27.0 * V[o] + 9.0 * V[o + di];
-      a = a + 9.0 * V[o + dj];
-      a = a + 9.0 * V[o + dk];
-      a = a + 3.0 * V[o + di + dj];
-      a = a + 3.0 * V[o + di + dk];
-      a = a + 3.0 * V[o + dj + dk];
-      a = a + V[o + di + dj + dk];
-      r = (1.0 / 64.0) * a;
+  const int i = 1 + q % nc, j = 1 + (q / nc) % nc, k = 1 + q / (nc * nc);
+  const long long o = mgi(nc, i, j, k);
+  const double v27 = sf::mul(27.0, V[o]);
+  double vy[2], vz[2], vyz[2][2];
+#pragma unroll
+  for (int b = 0; b < 2; ++b) {
+    vy[b] = sf::mul(9.0, V[o + (b ? s1 : -s1)]);
+    vz[b] = sf::mul(9.0, V[o + (b ? s2 : -s2)]);
+#pragma unroll
+    for (int g = 0; g < 2; ++g) vyz[b][g] = sf::mul(3.0, V[o + (b ? s1 : -s1) + (g ? s2 : -s2)]);
+  }
+#pragma unroll
+  for (int a = 0; a < 2; ++a) {
+    const long long ox = o + (a ? 1 : -1);
+    const double ax = v27 + sf::mul(9.0, V[ox]);
+    double vxz[2];
+#pragma unroll
+    for (int g = 0; g < 2; ++g) vxz[g] = sf::mul(3.0, V[ox + (g ? s2 : -s2)]);
+#pragma unroll
+    for (int b = 0; b < 2; ++b) {
+      const long long oxy = ox + (b ? s1 : -s1);
+      const double axy = ax + vy[b], vxy = sf::mul(3.0, V[oxy]);
+#pragma unroll
+      for (int g = 0; g < 2; ++g) {
+        double r = axy + vz[g];
+        r = r + vxy;
+        r = r + vxz[g];
+        r = r + vyz[b][g];
+        r = r + V[oxy + (g ? s2 : -s2)];
+        const int fi = 2 * i - 1 + a, fj = 2 * j - 1 + b, fk = 2 * k - 1 + g;
+        const double old = E[mgi(n, fi, fj, fk)];
+        const bool small = ((unsigned)__double2hiint(r) & 0x7fffffffu) < 0x00800000u;  // |r| < 2^-1015
+        const double v = small ? old + (1.0 / 64.0) * r : fma(1.0 / 64.0, r, old);
+        if (ghosts)
+          mg_put(E, n, fi, fj, fk, v);
+        else
+          E[mgi(n, fi, fj, fk)] = v;
+      }
     }
-    f.E[q] = f.E[q] + r;
   }
 }
 
-__global__ void k_mg_prolong_add(const MgCtl* c, MgLevel co, MgLevel f) {
+__global__ void k_mg_prolong_add(const MgCtl* c, MgLevel co, MgLevel f, bool ghosts) {
   if (!c->active) return;
-  mg_prolong_add(co, f, blockIdx.x * (long long)blockDim.x + threadIdx.x, (long long)gridDim.x * blockDim.x);
+  const int q = blockIdx.x * blockDim.x + threadIdx.x;
+  if (q < co.n * co.n * co.n) mg_prolong_add(co.E, f.E, co.n, q, ghosts);
 }
 
 // ---------------------------------------------------------------------------
-// Levels lc..L (n <= MG_COARSE_N) of one V-cycle in one block
+// Levels of at most MG_COARSE_N cells of one V-cycle in one block, in shared
+// memory.  A relax's ten half-sweeps overlap as in k_mg_relax_plane, a skew
+// of two diagonals apart (a value is there after the step's barrier): step t
+// holds the cells of half-sweep hs on diagonal i + j = 2 + t - 2 hs of every
+// plane, 2n + 17 steps instead of ten waves of 2n - 1.  The steps' cells lie
+// in a table, packed: at most 128 of them on 8 cells, one per thread, so
+// that four warps' FP64 operations (8 x 4 x 19 cycles a step) take no longer
+// than one cell's chain of eight (8 x 79), which bounds it.  Levels 8 to 1:
+// 140 us a cycle (from level arrays, wave after wave: 195 us for 4 to 1
+// alone, and 68 us and four launches more for the 8-cell level's relaxes).
 // ---------------------------------------------------------------------------
-constexpr int MG_CT = 128;  // threads: (n/2 planes) x n <= 4 x 8, and the level-wide loops
+constexpr int MG_CT = 128;
+static_assert(MG_CT == 2 * MG_COARSE_N * MG_COARSE_N, "a step's cells, one per thread");
 
-// Relax (5 passes of 2 half-sweeps) on a level of at most 32 cells; the
-// wave planes of a half-sweep advance together, thread t <-> (plane slot
-// t / n, i = t % n + 1), the parallel planes' cells first (no plane of one
-// kind reads a cell of the other kind that the half-sweep writes).
-__device__ double mg_relax_block(const MgLevel& lv, double* pub, double* red, bool track) {
-  const int n = lv.n;
-  double last = 0.0;
-  for (int pass = 0; pass < 5; ++pass) {
-    double acc = 0.0;
-    for (int half = 0; half < 2; ++half) {
-      // parallel planes: (k & 1) != half
-      for (int k = 1; k <= n; ++k)
-        if (((k & 1) ^ half) == 1 && n >= 2) acc += mg_parallel_plane<true>(lv, k, threadIdx.x, blockDim.x);
-      const int ps = threadIdx.x / n, i = threadIdx.x % n + 1;
-      const int k = 2 * ps + (half ? 1 : 2);  // (k & 1) == half
-      const bool mine = ps < n / 2 && k <= n;
-      // every thread runs the diagonal loop (uniform barriers); others idle
-      const double a = mg_wave_plane<true>(lv, mine ? k : 1, mine ? i : n + 1, pub + (mine ? ps : 0) * 2 * (n + 1));
-      acc += mine ? a : 0.0;
-      __syncthreads();
+struct alignas(16) MgCoarseSched {
+  unsigned short first[3][40];               // per level size (8, 4, 2): the first entry of each step, and the end
+  unsigned short cell[(512 + 64 + 8) * 5];   // offset in the level's array; bit 15: the last pass
+};
+
+void mg_coarse_sched(MgCoarseSched* s) {
+  int at = 0;
+  for (int lv = 0; lv < 3; ++lv) {
+    const int n = 8 >> lv;
+    for (int t = 0; t < 2 * n + 17; ++t) {
+      s->first[lv][t] = (unsigned short)at;
+      for (int hs = 0; hs < 10; ++hs)
+        for (int k = 1; k <= n; ++k)
+          for (int i = 1; i <= n; ++i) {
+            const int j = 2 + t - 2 * hs - i;
+            const bool s1 = !(i & 1) && (j & 1);
+            if (j < 1 || j > n || s1 != (((k ^ hs) & 1) == 1)) continue;
+            s->cell[at++] = (unsigned short)(mgi(n, i, j, k) | (hs >= 8 ? 0x8000 : 0));
+          }
     }
-    if (track && pass == 4) last = block_sum(acc, red);
+    s->first[lv][2 * n + 17] = (unsigned short)at;
   }
-  return last;  // (thread 0)
 }
 
-// Gauss-Seidel in i, j, k order until the summed change is <= 0.001
-// (sources.f90:337-396); one thread, the coarsest level is tiny.
-__device__ void mg_solve_block(const MgLevel& lv, MgCtl* c) {
+struct MgCoarseMem {
+  double E[1307], R[1307], T[1307];  // levels of 8, 4, 2 and 1 cells
+  MgCoarseSched sched;
+};
+template <int N>
+constexpr int MG_COARSE_AT = N == 8 ? 0 : N == 4 ? 1000 : N == 2 ? 1216 : 1280;
+
+// 5 passes of 2 half-sweeps; returns the thread's part of the last pass's
+// |change| (track).
+template <int N>
+__device__ __forceinline__ double mg_relax_shared(MgCoarseMem& m, bool track) {
+  constexpr int LV = N == 8 ? 0 : N == 4 ? 1 : 2, STEPS = 2 * N + 17, s1 = N + 2, s2 = s1 * s1;
+  double* E = m.E + MG_COARSE_AT<N>;
+  const double* T = m.T + MG_COARSE_AT<N>;
+  const unsigned short* first = m.sched.first[LV];
+  double acc = 0.0;
+  int at = first[0] + (int)threadIdx.x, end = first[1];
+  int e = at < end ? m.sched.cell[at] : -1;
+  for (int t = 0; t < STEPS; ++t) {
+    const int cur = e;
+    if (t + 1 < STEPS) {
+      at = end + (int)threadIdx.x;
+      end = first[t + 2];
+      e = at < end ? m.sched.cell[at] : -1;
+    }
+    if (cur >= 0) {
+      double* p = E + (cur & 0x7fff);
+      const double old = p[0];
+      const double v = mg_new(p[1], p[-1], p[s1], p[-s1], p[s2], p[-s2], T[cur & 0x7fff], old);
+      p[0] = v;
+      if (track && (cur & 0x8000)) acc += fabs(v - old);
+    }
+    __syncthreads();
+  }
+  return acc;
+}
+
+// Gauss-Seidel on the coarsest level, one cell, until the change is
+// <= 0.001 (sources.f90:337-396); its ghosts are not set anew.
+__device__ void mg_solve_shared(MgCoarseMem& m, MgCtl* c) {
   if (threadIdx.x == 0) {
-    const int n = lv.n;
-    const long long s1 = n + 2, s2 = (long long)(n + 2) * (n + 2);
-    const double dxl2 = lv.dxl * lv.dxl;
+    double* p = m.E + MG_COARSE_AT<1> + 13;
+    const double sdx = m.T[MG_COARSE_AT<1> + 13];
     double Dif = 1000.0;
     int passes = 0;
     while (Dif > 0.001) {
@@ -1104,58 +1158,64 @@ __device__ void mg_solve_block(const MgLevel& lv, MgCtl* c) {
         atomicOr(&c->status, MG_ST_SOLVE);
         break;
       }
-      double difp = 0.0;
-      for (int i = 1; i <= n; ++i)
-        for (int j = 1; j <= n; ++j)
-          for (int k = 1; k <= n; ++k) {
-            const long long o = mgi(n, i, j, k);
-            const double old = lv.E[o];
-            const double v = mg_new(lv.E[o + 1], lv.E[o - 1], lv.E[o + s1], lv.E[o - s1], lv.E[o + s2], lv.E[o - s2],
-                                    lv.R[o] * dxl2, old);
-            lv.E[o] = v;
-            difp = difp + fabs(v - old);
-          }
-      Dif = difp;
+      const double old = p[0];
+      p[0] = mg_new(p[1], p[-1], p[3], p[-3], p[9], p[-9], sdx, old);
+      Dif = fabs(p[0] - old);
     }
   }
   __syncthreads();
 }
 
-struct MgLevels {
-  MgLevel lv[MG_MAXL];
-};
+// Levels N .. 1 of one V-cycle: relax, residual + restriction, the levels
+// below, prolongation + add, relax.
+template <int N>
+__device__ __forceinline__ double mg_cycle_shared(MgCoarseMem& m, MgCtl* c, double dxl, bool whole) {
+  if constexpr (N == 1) {
+    mg_solve_shared(m, c);
+    return 0.0;
+  } else {
+    constexpr int f = MG_COARSE_AT<N>, g = MG_COARSE_AT<N / 2>, CELLS = N * N * N / 8;
+    mg_relax_shared<N>(m, false);
+    if (threadIdx.x < CELLS)
+      mg_resid_restrict(m.E + f, m.R + f, N, dxl, m.E + g, m.R + g, m.T + g, (int)threadIdx.x);
+    __syncthreads();
+    mg_cycle_shared<N / 2>(m, c, 2.0 * dxl, false);
+    if (threadIdx.x < CELLS) mg_prolong_add(m.E + g, m.E + f, N / 2, (int)threadIdx.x, !whole);
+    __syncthreads();
+    return mg_relax_shared<N>(m, whole);
+  }
+}
 
-// The part of one V-cycle on levels lc..L: down (relax lc; then per level
-// residual + restriction, ghosts, relax or, on L, solve) and up (per level
-// prolongation + add, ghosts, relax).  With lc = 0 it is the whole cycle
-// and also forms Dif.
-__global__ void __launch_bounds__(MG_CT) k_mg_coarse(MgCtl* c, MgLevels levels, int lc, int L, int bc_multipole) {
-  __shared__ double pub[16 * 2 * 33];
+// WHOLE: the mesh itself has N cells; the kernel is the cycle and also forms
+// Dif's sum.
+template <int N, bool WHOLE>
+__global__ void __launch_bounds__(MG_CT) k_mg_coarse(MgCtl* c, MgLevel top, const MgCoarseSched* sched) {
+  __shared__ MgCoarseMem m;
   __shared__ double red[32];
   if (!c->active) return;
-  const long long t = threadIdx.x, nt = blockDim.x;
-  // down
-  if (lc > 0) mg_ghosts(levels.lv[lc], bc_multipole);
-  if (lc == L)
-    mg_solve_block(levels.lv[L], c);
-  else
-    mg_relax_block(levels.lv[lc], pub, red, false);
-  for (int l = lc + 1; l <= L; ++l) {
-    mg_resid_restrict(levels.lv[l - 1], levels.lv[l], t, nt);
-    __syncthreads();
-    mg_ghosts(levels.lv[l], bc_multipole);
-    if (l == L)
-      mg_solve_block(levels.lv[l], c);
-    else
-      mg_relax_block(levels.lv[l], pub, red, false);
+  constexpr int f = MG_COARSE_AT<N>, CELLS = (N + 2) * (N + 2) * (N + 2);
+  for (int q = threadIdx.x; q < (int)(sizeof(MgCoarseSched) / 16); q += MG_CT)
+    reinterpret_cast<uint4*>(&m.sched)[q] = reinterpret_cast<const uint4*>(sched)[q];
+  for (int q = threadIdx.x; q < CELLS; q += MG_CT) {
+    m.E[f + q] = top.E[q];
+    m.R[f + q] = top.R[q];
+    m.T[f + q] = top.T[q];
   }
-  // up
-  for (int l = L - 1; l >= lc; --l) {
-    mg_prolong_add(levels.lv[l + 1], levels.lv[l], t, nt);
-    __syncthreads();
-    if (l > 0) mg_ghosts(levels.lv[l], bc_multipole);
-    const double d = mg_relax_block(levels.lv[l], pub, red, l == 0);
-    if (l == 0 && threadIdx.x == 0) c->part[0] = d;
+  __syncthreads();
+  const double acc = mg_cycle_shared<N>(m, c, top.dxl, WHOLE);
+  for (int q = threadIdx.x; q < CELLS; q += MG_CT) top.E[q] = m.E[f + q];
+  if (WHOLE) {
+    const double d = block_sum(acc, red);
+    if (threadIdx.x == 0) c->part[0] = d;
+  }
+}
+
+void launch_coarse(MgCtl* c, const MgLevel& top, const void* sched, cudaStream_t s) {
+  const MgCoarseSched* t = static_cast<const MgCoarseSched*>(sched);
+  switch (top.n) {
+    case 8: k_mg_coarse<8, true><<<1, MG_CT, 0, s>>>(c, top, t); break;
+    case 4: k_mg_coarse<4, true><<<1, MG_CT, 0, s>>>(c, top, t); break;
+    default: k_mg_coarse<2, true><<<1, MG_CT, 0, s>>>(c, top, t);
   }
 }
 
@@ -1244,7 +1304,6 @@ bool launch_plane(MgCtl* c, const MgLevel& lv, int leg, double* part, cudaStream
 template <bool TRACK>
 bool launch_plane_any(MgCtl* c, const MgLevel& lv, int leg, double* part, cudaStream_t s) {
   switch (lv.n) {
-    case 8: return launch_plane<8, TRACK>(c, lv, leg, part, s);
     case 16: return launch_plane<16, TRACK>(c, lv, leg, part, s);
     case 32: return launch_plane<32, TRACK>(c, lv, leg, part, s);
     case 64: return launch_plane<64, TRACK>(c, lv, leg, part, s);
@@ -1258,9 +1317,9 @@ bool launch_plane_any(MgCtl* c, const MgLevel& lv, int leg, double* part, cudaSt
 // Levels up to 128 cells hold their planes in shared memory
 // (k_mg_relax_plane) unless TLQ_MG_PLANE=0; the others, and those, then use
 // k_mg_relax_pipe.  Its threads per plane (measured on the gravitating
-// cloud): 128-cell levels 5 x 128 (two half-sweeps each), 64 down to 8:
+// cloud): 128-cell levels 5 x 128 (two half-sweeps each), 64 down to 16:
 // 10 x n; neighbour checks every 8 steps on 128 and 64 cells, 4 on 32, 2
-// below (a relax takes 2n + 9 (CH + 1) steps); 256-cell levels need two
+// on 16 (a relax takes 2n + 9 (CH + 1) steps); 256-cell levels need two
 // blocks per SM: 2 x 256, checks every 4 steps.
 template <bool TRACK>
 bool launch_pipe_any(MgCtl* c, const MgLevel& lv, int leg, double* part, cudaStream_t s) {
@@ -1268,7 +1327,6 @@ bool launch_pipe_any(MgCtl* c, const MgLevel& lv, int leg, double* part, cudaStr
   const bool plane = !(env && env[0] == '0');
   if (plane && launch_plane_any<TRACK>(c, lv, leg, part, s)) return true;
   switch (lv.n) {
-    case 8: return launch_pipe<96, 1, 10, 1, 2, TRACK>(c, lv, part, s);
     case 16: return launch_pipe<160, 1, 10, 1, 2, TRACK>(c, lv, part, s);
     case 32: return launch_pipe<320, 1, 10, 1, 4, TRACK>(c, lv, part, s);
     case 64: return launch_pipe<640, 1, 10, 1, 8, TRACK>(c, lv, part, s);
@@ -1327,6 +1385,12 @@ cudaError_t mg_alloc(tlq_ctx* ctx) {
   e = cudaMemcpy(reinterpret_cast<char*>(ctx->mg_ctl) + offsetof(MgCtl, wait_limit), &limit, sizeof limit,
                  cudaMemcpyHostToDevice);
   if (e != cudaSuccess) return e;
+  const auto coarse = std::make_unique<MgCoarseSched>();
+  mg_coarse_sched(coarse.get());
+  e = cudaMalloc(&ctx->mg_coarse, sizeof(MgCoarseSched));
+  if (e != cudaSuccess) return e;
+  e = cudaMemcpy(ctx->mg_coarse, coarse.get(), sizeof(MgCoarseSched), cudaMemcpyHostToDevice);
+  if (e != cudaSuccess) return e;
   long long xc = 0, sc = 0;
   for (int l = 0; l <= L; ++l)
     if (exch_level(ctx->cfg.nx >> l)) {
@@ -1368,8 +1432,8 @@ cudaError_t mg_alloc(tlq_ctx* ctx) {
 }
 
 void mg_free(tlq_ctx* ctx) {
-  cudaFree(ctx->mg_exch); cudaFree(ctx->mg_sched);
-  ctx->mg_exch = nullptr; ctx->mg_sched = nullptr;
+  cudaFree(ctx->mg_exch); cudaFree(ctx->mg_sched); cudaFree(ctx->mg_coarse);
+  ctx->mg_exch = nullptr; ctx->mg_coarse = nullptr; ctx->mg_sched = nullptr;
   cudaFree(ctx->mg_work); cudaFree(ctx->mg_ctl); cudaFree(ctx->mg_mom); cudaFree(ctx->phig); cudaFree(ctx->phit);
   if (ctx->mg_body) cudaStreamDestroy(ctx->mg_body);
   ctx->mg_work = nullptr; ctx->mg_ctl = nullptr; ctx->mg_mom = nullptr; ctx->phig = nullptr; ctx->phit = nullptr;
@@ -1377,6 +1441,10 @@ void mg_free(tlq_ctx* ctx) {
 }
 
 namespace {
+
+struct MgLevels {
+  MgLevel lv[MG_MAXL];
+};
 
 MgLevels mg_plan(const tlq_ctx* ctx, int L) {
   MgLevels v{};
@@ -1415,49 +1483,7 @@ cudaError_t enqueue_mg(tlq_ctx* ctx, Dens rho, const Clock* clk, double* phit, c
   const bool multipole = ctx->cfg.grav_bc == TLQ_GBC_MULTIPOLE;
   int lc = 0;
   while (lc < L && v.lv[lc].n > MG_COARSE_N) ++lc;
-  long long ncoarse = 0;  // E of levels 1..L, contiguous after E of level 0
-  for (int l = 1; l <= L; ++l) {
-    const long long m = v.lv[l].n + 2;
-    ncoarse += m * m * m;
-  }
   const long long m0 = n + 2;
-  k_mg_begin<<<1, 1, 0, s>>>(c, clk);
-  if (multipole) {
-    k_mg_moments<<<MG_MOM_BLOCKS, MG_MOM_THREADS, 0, s>>>(c, clk, ctx->P, rho, static_cast<double*>(ctx->mg_mom));
-    k_mg_moments_final<<<1, 32, 0, s>>>(c, clk, static_cast<const double*>(ctx->mg_mom), MG_MOM_BLOCKS);
-    k_mg_faces<<<grid_for(6LL * n * n, 256), 256, 0, s>>>(c, clk, ctx->P, ctx->phig);
-  }
-  k_mg_init<<<grid_for(m0 * m0 * m0, 256), 256, 0, s>>>(c, rho, n, ctx->phig, v.lv[0].E, v.lv[0].R, v.lv[0].T,
-                                                        v.lv[0].dxl);
-  double* part = reinterpret_cast<double*>(reinterpret_cast<char*>(c) + offsetof(MgCtl, part));
-  // One V-cycle slot (sources.f90:140-187): its first kernels evaluate the
-  // loop test, and every later kernel of a slot that does not run returns.
-  auto cycle = [&](cudaStream_t st) {
-    k_mg_cycle_begin<<<grid_for(ncoarse, 256), 256, 0, st>>>(c, v.lv[0].E + m0 * m0 * m0, ncoarse);
-    k_mg_cycle_flag<<<1, 1, 0, st>>>(c);
-    if (lc == 0) {
-      k_mg_coarse<<<1, MG_CT, 0, st>>>(c, v, 0, L, multipole ? 1 : 0);
-      k_mg_cycle_end<<<1, 1, 0, st>>>(c, 1);
-      return;
-    }
-    // down: level 0 .. lc-1 on the large kernels
-    for (int l = 0; l < lc; ++l) {
-      if (l > 0) k_mg_ghosts<<<1, 1024, 0, st>>>(c, v.lv[l], multipole ? 1 : 0);
-      launch_relax(c, v.lv[l], 0, nullptr, st);
-      k_mg_resid_restrict<<<grid_for((long long)v.lv[l + 1].n * v.lv[l + 1].n * v.lv[l + 1].n, 256), 256, 0, st>>>(
-          c, v.lv[l], v.lv[l + 1]);
-    }
-    k_mg_coarse<<<1, MG_CT, 0, st>>>(c, v, lc, L, multipole ? 1 : 0);
-    // up: level lc-1 .. 0
-    for (int l = lc - 1; l >= 0; --l) {
-      const long long mf = v.lv[l].n + 2;
-      k_mg_prolong_add<<<grid_for(mf * mf * mf, 256), 256, 0, st>>>(c, v.lv[l + 1], v.lv[l]);
-      if (l > 0) k_mg_ghosts<<<1, 1024, 0, st>>>(c, v.lv[l], multipole ? 1 : 0);
-      // the last pass of the level-0 relax forms Dif (sources.f90:465-471)
-      launch_relax(c, v.lv[l], 1, l == 0 ? part : nullptr, st);
-    }
-    k_mg_cycle_end<<<1, 1, 0, st>>>(c, 2 * n);
-  };
   // Captured into a graph: the cycles are the body of a while node whose
   // condition the loop test sets on the device (before the node and at the
   // end of each cycle), captured on the context's second stream.  Run
@@ -1469,11 +1495,51 @@ cudaError_t enqueue_mg(tlq_ctx* ctx, Dens rho, const Clock* clk, double* phit, c
   cudaError_t e = cudaStreamGetCaptureInfo(s, &cst, nullptr, &cg, &deps, nullptr, &nd);
   if (e != cudaSuccess) return e;
   const char* env = std::getenv("TLQ_MG_GRAPH_LOOP");
-  if (cst == cudaStreamCaptureStatusActive && ctx->mg_body && !(env && env[0] == '0')) {
-    cudaGraphConditionalHandle h;
+  const bool loop = cst == cudaStreamCaptureStatusActive && ctx->mg_body && !(env && env[0] == '0');
+  cudaGraphConditionalHandle h = {};
+  if (loop) {
     e = cudaGraphConditionalHandleCreate(&h, cg, 0, 0);
     if (e != cudaSuccess) return e;
-    k_mg_loop_test<<<1, 1, 0, s>>>(c, h);
+  }
+  k_mg_begin<<<1, 1, 0, s>>>(c, clk, loop, h);
+  if (multipole) {
+    k_mg_moments<<<MG_MOM_BLOCKS, MG_MOM_THREADS, 0, s>>>(c, clk, ctx->P, rho, static_cast<double*>(ctx->mg_mom));
+    k_mg_moments_final<<<1, 25 * 32, 0, s>>>(c, clk, static_cast<const double*>(ctx->mg_mom), MG_MOM_BLOCKS);
+    k_mg_faces<<<grid_for(6LL * n * n, 256), 256, 0, s>>>(c, clk, ctx->P, ctx->phig);
+  }
+  k_mg_init<<<grid_for(m0 * m0 * m0, 256), 256, 0, s>>>(c, rho, n, ctx->phig, v.lv[0].E, v.lv[0].R, v.lv[0].T,
+                                                        v.lv[0].dxl);
+  double* part = reinterpret_cast<double*>(reinterpret_cast<char*>(c) + offsetof(MgCtl, part));
+  // a level operator's launch: a thread per coarse cell; blocks of one warp
+  // where 128 threads would leave most SMs without one
+  auto blocks = [](int nc) { return nc >= 64 ? 128 : 32; };
+  // One V-cycle slot (sources.f90:140-187): k_mg_begin or the cycle before
+  // evaluated the loop test, and every kernel of a slot that does not run
+  // returns.
+  auto cycle = [&](cudaStream_t st) {
+    if (lc == 0) {
+      launch_coarse(c, v.lv[0], ctx->mg_coarse, st);
+      k_mg_cycle_end<<<1, 32, 0, st>>>(c, 1, loop, h);
+      return;
+    }
+    // down: level 0 .. lc-1 on the large kernels
+    for (int l = 0; l < lc; ++l) {
+      launch_relax(c, v.lv[l], 0, nullptr, st);
+      const int nc = v.lv[l + 1].n, nt = blocks(nc);
+      k_mg_resid_restrict<<<(nc * nc * nc + nt - 1) / nt, nt, 0, st>>>(c, v.lv[l], v.lv[l + 1]);
+    }
+    k_mg_coarse<MG_COARSE_N, false><<<1, MG_CT, 0, st>>>(c, v.lv[lc],
+                                                         static_cast<const MgCoarseSched*>(ctx->mg_coarse));
+    // up: level lc-1 .. 0
+    for (int l = lc - 1; l >= 0; --l) {
+      const int nc = v.lv[l + 1].n, nt = blocks(nc);
+      k_mg_prolong_add<<<(nc * nc * nc + nt - 1) / nt, nt, 0, st>>>(c, v.lv[l + 1], v.lv[l], l > 0);
+      // the last pass of the level-0 relax forms Dif (sources.f90:465-471)
+      launch_relax(c, v.lv[l], 1, l == 0 ? part : nullptr, st);
+    }
+    k_mg_cycle_end<<<1, 32, 0, st>>>(c, 2 * n, loop, h);
+  };
+  if (loop) {
     e = cudaStreamGetCaptureInfo(s, &cst, nullptr, &cg, &deps, nullptr, &nd);
     if (e != cudaSuccess) return e;
     cudaGraphNodeParams np = {};
@@ -1488,7 +1554,6 @@ cudaError_t enqueue_mg(tlq_ctx* ctx, Dens rho, const Clock* clk, double* phit, c
                                       cudaStreamCaptureModeThreadLocal);
     if (e != cudaSuccess) return e;
     cycle(ctx->mg_body);
-    k_mg_loop_test<<<1, 1, 0, ctx->mg_body>>>(c, h);
     cudaGraph_t body = nullptr;
     e = cudaStreamEndCapture(ctx->mg_body, &body);
     if (e != cudaSuccess) return e;
