@@ -364,7 +364,13 @@ __global__ void k_mg_end(const MgCtl* c, Clock* clk, int n, const double* E0, do
 // 0*old term can change the sign or give a NaN): those take the literal
 // expression, every other update saves its three FP64 operations (the FP64
 // pipe bounds the smoother).  SOFT: the product on the integer pipe, where
-// the FP64 pipe is the limit.
+// the FP64 pipe is the limit (64 and 128 cells: 1 and 3 % of a step).
+// (mg_tail is a call: inlined, its three operations ran for every update and
+// their result was dropped, 10 warp instructions of the FP64 pipe for 7.)
+__device__ __noinline__ double mg_tail(double v, double old) {
+  const double w = 1.0;
+  return v * w + (1.0 - w) * old;
+}
 template <bool SOFT = false>
 __device__ __forceinline__ double mg_new(double east, double west, double north, double south, double up, double down,
                                          double sdx, double old) {
@@ -376,10 +382,7 @@ __device__ __forceinline__ double mg_new(double east, double west, double north,
   a = a - sdx;
   double v = SOFT ? sf::mul(1.0 / 6.0, a) : (1.0 / 6.0) * a;
   const long long vb = __double_as_longlong(v), ob = __double_as_longlong(old);
-  if ((vb & 0x7fffffffffffffffLL) == 0 || ((ob >> 52) & 0x7ff) == 0x7ff) {
-    const double w = 1.0;
-    v = v * w + (1.0 - w) * old;
-  }
+  if ((vb & 0x7fffffffffffffffLL) == 0 || ((ob >> 52) & 0x7ff) == 0x7ff) v = mg_tail(v, old);
   return v;
 }
 
@@ -709,7 +712,8 @@ __global__ void __launch_bounds__(NT, MINB) k_mg_relax_pipe(MgCtl* c, MgLevel lv
 // FP64 pipe.  Measured per launch on the 128^3 cloud (ncu), against a thread
 // per column and group with loads one step ahead and a fence and a poll by
 // the whole block every few steps: 128 cells 743 -> 380 us, 64: 260 -> 130,
-// 32: 143 -> 65, 16: 98 -> 43.
+// 32: 143 -> 65, 16: 98 -> 43; with mg_tail's operations out of every update
+// 316, 115, 62 and 41.
 // ---------------------------------------------------------------------------
 constexpr int MG_SKEW = 4;  // (6: 4 % slower, 2 more steps per half-sweep; 2 leaves a value no time to arrive)
 constexpr unsigned MG_INITIAL = 15;
@@ -843,7 +847,7 @@ __global__ void __launch_bounds__(PlaneGeo<N>::NT + PlaneGeo<N>::NH, 1)
           const double* pe = pc + (o >= PS ? 1 - PS : PS);
           const double* b = B + q * 3 * NT + tid;
           const double old = pc[0];
-          const double v = mg_new<(N >= 128)>(pe[0], pe[-1], pc[R], pc[-R], b[0], b[NT], b[2 * NT], old);
+          const double v = mg_new<(N >= 64)>(pe[0], pe[-1], pc[R], pc[-R], b[0], b[NT], b[2 * NT], old);
           pc[0] = v;
           st_tagged(X + (m.y & 0xffffu), v, seq | (m.x >> 16));
           if (TRACK) {
