@@ -31,6 +31,8 @@ struct tlq_ctx {
   void* mg_mom = nullptr;
   void* mg_exch = nullptr;  // the levels' exchange arrays between planes
   void* mg_sched = nullptr;  // and the relax's schedules
+  int* mg_go = nullptr;       // pinned: whether the cycle after an enqueued one runs, by its parity
+  cudaEvent_t mg_seen[2] = {};
   void* mg_coarse = nullptr;  // the one-block levels' schedule
   cudaStream_t mg_body = nullptr;  // captures a V-cycle into a graph's loop body
   double* phig = nullptr;

@@ -31,8 +31,7 @@
 // The reference's loop test (Dif > 10 and fewer than 31 cycles) runs on the
 // device, so the solve needs no host round trip: in a CUDA graph the
 // V-cycles are the body of a while node whose condition that test sets; run
-// directly, a fixed sequence of 31 cycle slots whose launches return once
-// the test failed.  Levels of at most 8 cells run inside one block (one
+// directly, up to 31 cycle slots whose launches return once the test failed.  Levels of at most 8 cells run inside one block (one
 // launch per cycle).
 //
 // Built with -fmad=false (FP64 as the restatement evaluates it).
@@ -1421,6 +1420,12 @@ cudaError_t mg_alloc(tlq_ctx* ctx) {
   }
   e = cudaMalloc(&ctx->mg_mom, (size_t)MG_MOM_BLOCKS * 25 * sizeof(double));
   if (e != cudaSuccess) return e;
+  e = cudaMallocHost(&ctx->mg_go, 2 * sizeof(int));
+  if (e != cudaSuccess) return e;
+  for (cudaEvent_t& ev : ctx->mg_seen) {
+    e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
+    if (e != cudaSuccess) return e;
+  }
   e = cudaStreamCreateWithFlags(&ctx->mg_body, cudaStreamNonBlocking);
   if (e != cudaSuccess) return e;
   const long long m0 = ctx->cfg.nx + 2;
@@ -1440,6 +1445,12 @@ void mg_free(tlq_ctx* ctx) {
   ctx->mg_exch = nullptr; ctx->mg_coarse = nullptr; ctx->mg_sched = nullptr;
   cudaFree(ctx->mg_work); cudaFree(ctx->mg_ctl); cudaFree(ctx->mg_mom); cudaFree(ctx->phig); cudaFree(ctx->phit);
   if (ctx->mg_body) cudaStreamDestroy(ctx->mg_body);
+  for (cudaEvent_t& ev : ctx->mg_seen) {
+    if (ev) cudaEventDestroy(ev);
+    ev = nullptr;
+  }
+  cudaFreeHost(ctx->mg_go);
+  ctx->mg_go = nullptr;
   ctx->mg_work = nullptr; ctx->mg_ctl = nullptr; ctx->mg_mom = nullptr; ctx->phig = nullptr; ctx->phit = nullptr;
   ctx->mg_body = nullptr;
 }
@@ -1491,7 +1502,7 @@ cudaError_t enqueue_mg(tlq_ctx* ctx, Dens rho, const Clock* clk, double* phit, c
   // Captured into a graph: the cycles are the body of a while node whose
   // condition the loop test sets on the device (before the node and at the
   // end of each cycle), captured on the context's second stream.  Run
-  // directly (or with TLQ_MG_GRAPH_LOOP=0): the fixed sequence of 31 slots.
+  // directly (or with TLQ_MG_GRAPH_LOOP=0): a sequence of up to 31 slots.
   cudaStreamCaptureStatus cst = cudaStreamCaptureStatusNone;
   cudaGraph_t cg = nullptr;
   const cudaGraphNode_t* deps = nullptr;
@@ -1564,7 +1575,23 @@ cudaError_t enqueue_mg(tlq_ctx* ctx, Dens rho, const Clock* clk, double* phit, c
     e = cudaStreamUpdateCaptureDependencies(s, &node, nullptr, 1, cudaStreamSetCaptureDependencies);
     if (e != cudaSuccess) return e;
   } else {
-    for (int cyc = 0; cyc < MG_CYCLES; ++cyc) cycle(s);
+    // Outside a capture the slots are enqueued two ahead of the cycle that the
+    // host has seen to go on, so that at most two slots run empty (of about
+    // 17 launches each, 1.5 us a launch; its callers wait for the result).
+    const bool look = cst == cudaStreamCaptureStatusNone;
+    for (int cyc = 0; cyc < MG_CYCLES; ++cyc) {
+      if (look && cyc >= 2) {
+        e = cudaEventSynchronize(ctx->mg_seen[cyc & 1]);
+        if (e != cudaSuccess) return e;
+        if (!ctx->mg_go[cyc & 1]) break;
+      }
+      cycle(s);
+      if (!look) continue;
+      e = cudaMemcpyAsync(ctx->mg_go + (cyc & 1), &c->active, sizeof(int), cudaMemcpyDeviceToHost, s);
+      if (e != cudaSuccess) return e;
+      e = cudaEventRecord(ctx->mg_seen[cyc & 1], s);
+      if (e != cudaSuccess) return e;
+    }
   }
   k_mg_end<<<grid_for(m0 * m0 * m0, 256), 256, 0, s>>>(c, const_cast<Clock*>(clk), n, v.lv[0].E, ctx->phig, ctx->phi,
                                                        phit, phit ? ctx->phif : nullptr, ctx->L);
