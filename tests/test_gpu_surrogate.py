@@ -66,6 +66,23 @@ def test_gradient_matches_oracle(gpu_lib):
     assert np.linalg.norm(g - g64) / np.linalg.norm(g64) < 0.05
 
 
+@pytest.mark.parametrize("n", [1, 16, 17, 128, 129, 152 * 128 + 17])
+def test_gradient_tile_edges(gpu_lib, n):
+    """Sample counts around a warp's tile (16), a block's (128) and the
+    blocks' first turn (152 of them).  Bound: a BF16 rounding flip moves one
+    operand by 2^-8, so a block of parameters by at most that."""
+    rng = np.random.default_rng(n)
+    P = mo.init_params(7)
+    X = rng.uniform(-1, 1, (n, 3)).astype(np.float32)
+    Y = rng.uniform(2, 4, n).astype(np.float32)  # (errors of one sign: no cancelling sums)
+    loss, g = tlq.mlp_loss_grad(P, X, Y)
+    loss_o, g_o = mo.loss_grad(P, X, Y, bf16_round=True)
+    assert abs(loss - loss_o) <= 1e-4 * loss_o
+    cuts = [mo.OFF_W1, mo.OFF_B1, mo.OFF_W2, mo.OFF_B2, mo.OFF_W3, mo.OFF_B3, mo.OFF_W4, mo.OFF_B4, mo.NPARAM]
+    for a, b in zip(cuts, cuts[1:]):
+        assert np.linalg.norm(g[a:b] - g_o[a:b]) <= 2.0**-8 * np.linalg.norm(g_o[a:b]), (a, b)
+
+
 def test_inference_matches_oracle(gpu_lib):
     rng = np.random.default_rng(1)
     P = mo.init_params(6)

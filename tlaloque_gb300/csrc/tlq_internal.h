@@ -65,9 +65,8 @@ cudaError_t launch_conserved_sums(const Params& p, const Layout& L, const double
                                   double* out5, cudaStream_t s);
 
 // Cooling surrogate (tlq_mlp.cu).
-size_t mlp_train_smem();
 cudaError_t launch_mlp_grad(const float* P, const float* X, const float* Y, const float* Wt, int nb, float* grad,
-                            float* loss, int nblocks, cudaStream_t s);
+                            float* loss, cudaStream_t s);
 cudaError_t launch_adam(float* P, float* m, float* v, const float* grad, int n, float lr, float b1, float b2,
                         float eps, int t, cudaStream_t s);
 cudaError_t launch_mlp_infer(const float* P, const float* X, int n, float* Y, cudaStream_t s);

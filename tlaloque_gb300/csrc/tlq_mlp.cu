@@ -7,6 +7,8 @@
 // product are rounded to BF16; products accumulate in FP32; the input and
 // output layers, biases, pre-activations, SiLU derivatives, the loss
 // gradient, the layer-1 and layer-4 weight gradients are FP32.
+#include <algorithm>
+
 #include "tlq_internal.h"
 #include "tlq_mlp.cuh"
 #include "tlq_umma.cuh"
@@ -14,19 +16,72 @@
 namespace tlq {
 namespace mlp {
 
-constexpr int TW = 4;        // warps per training block
+constexpr int TW = 8;        // warps per training block: one per (layer, 16 rows) of the two 64 x 64 gradients
 constexpr int TT = TW * 32;  // threads per training block
 constexpr int TS = 16;       // samples per warp tile
-constexpr int LDS = TS + 8;  // padded row length of the transposed staging tiles
+constexpr int NVEC = 7;      // 64-wide gradients: W4, b3, b2, b1 and W1's three columns
 
 struct TrainSmem {
   SmemWeights W;
-  SmemWeightsT WT;
-  __nv_bfloat16 stA[TW][HID][LDS];  // dZ^T of the tile (features x samples)
-  __nv_bfloat16 stB[TW][HID][LDS];  // H^T of the tile
-  float g[NPARAM];                  // this block's gradient
-  float loss;
+  // Each warp's tile for the weight gradients, sample by feature: dZ3, H2, dZ2, H1
+  alignas(16) __nv_bfloat16 st[4][TW][TS][LD];
+  float vec[TW][NVEC][HID];
+  float b4[TW], loss[TW];
 };
+
+__device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+template <bool TRANS>
+__device__ __forceinline__ void ldmatrix4(uint32_t r[4], uint32_t addr) {
+  if (TRANS)
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(addr)
+                 : "memory");
+  else
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(addr)
+                 : "memory");
+}
+
+// acc = bias + A W^T (the layer), or A W (BACK: the layer's transpose), 64 x
+// 64, for one m16 tile; the operand fragments two k-tiles at a time, the
+// eight column tiles' products of a k-tile one after another (independent).
+template <bool BACK>
+__device__ __forceinline__ void train_dense(float acc[8][4], const uint32_t a[4][4], const __nv_bfloat16 (*w)[LD],
+                                            const float* bias, int lane) {
+  const int tig = lane & 3;
+  // lane l gives the address of row l % 8 of 8 x 8 matrix l / 8
+  const uint32_t base = smem_addr(BACK ? &w[lane][0] : &w[lane & 7][8 * (lane >> 3)]);
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const float b0 = bias ? bias[8 * j + 2 * tig] : 0.0f, b1 = bias ? bias[8 * j + 2 * tig + 1] : 0.0f;
+    acc[j][0] = b0; acc[j][1] = b1; acc[j][2] = b0; acc[j][3] = b1;
+  }
+#pragma unroll
+  for (int kp = 0; kp < 2; ++kp) {
+    uint32_t b[8][4];
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      ldmatrix4<BACK>(b[j], base + (uint32_t)sizeof(__nv_bfloat16) *
+                                       (BACK ? 32 * kp * LD + 8 * j : 8 * j * LD + 32 * kp));
+#pragma unroll
+    for (int k = 0; k < 2; ++k)
+#pragma unroll
+      for (int j = 0; j < 8; ++j) mma_bf16(acc[j], a[2 * kp + k], b[j][2 * k], b[j][2 * k + 1]);
+  }
+}
+
+// A fragment set (rows g, g+8; 64 columns) into a staging tile.
+__device__ __forceinline__ void stage(__nv_bfloat16 (*dst)[LD], const uint32_t a[4][4], int g, int tig) {
+#pragma unroll
+  for (int kt = 0; kt < 4; ++kt) {
+    *reinterpret_cast<uint32_t*>(&dst[g][16 * kt + 2 * tig]) = a[kt][0];
+    *reinterpret_cast<uint32_t*>(&dst[g + 8][16 * kt + 2 * tig]) = a[kt][1];
+    *reinterpret_cast<uint32_t*>(&dst[g][16 * kt + 8 + 2 * tig]) = a[kt][2];
+    *reinterpret_cast<uint32_t*>(&dst[g + 8][16 * kt + 8 + 2 * tig]) = a[kt][3];
+  }
+}
 
 __device__ __forceinline__ void frag_plain(uint32_t a[4][4], const float d[8][4]) {
 #pragma unroll
@@ -38,175 +93,226 @@ __device__ __forceinline__ void frag_plain(uint32_t a[4][4], const float d[8][4]
   }
 }
 
-// Sum over the 8 lanes that share tig (rows g = 0..7 of a fragment).
-__device__ __forceinline__ float sum_over_g(float v) {
-  v += __shfl_xor_sync(0xffffffffu, v, 4);
-  v += __shfl_xor_sync(0xffffffffu, v, 8);
-  v += __shfl_xor_sync(0xffffffffu, v, 16);
-  return v;
+// 1 / x for x >= 1 without the division's branch, which kept a thread's 32
+// sigmoids of a layer from overlapping: the approximate reciprocal and one
+// Newton step in fused arithmetic (correctly rounded but for rare ties,
+// Markstein 1990).  Where 1 / x is subnormal, and for infinity, the
+// approximation alone (0).
+__device__ __forceinline__ float recip_ge1(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return x < 0x1p126f ? fmaf(r, fmaf(-x, r, 1.0f), r) : r;
 }
 
-// dW_layer (64 x 64, out x in) += dZ^T H over the warp's 16 samples, from the
-// transposed BF16 staging tiles, into the block gradient (shared atomics).
-__device__ __forceinline__ void weight_grad64(float* gW, const __nv_bfloat16 (*dzT)[LDS],
-                                              const __nv_bfloat16 (*hT)[LDS], int g, int tig) {
+// z -> silu(z) and silu'(z), with one sigmoid.
+__device__ __forceinline__ void silu_both(float h[8][4], float ds[8][4], const float z[8][4]) {
 #pragma unroll
-  for (int mt = 0; mt < 4; ++mt) {  // output-feature tile (rows of dW)
-    uint32_t a[4];
-    a[0] = *reinterpret_cast<const uint32_t*>(&dzT[16 * mt + g][2 * tig]);
-    a[1] = *reinterpret_cast<const uint32_t*>(&dzT[16 * mt + g + 8][2 * tig]);
-    a[2] = *reinterpret_cast<const uint32_t*>(&dzT[16 * mt + g][2 * tig + 8]);
-    a[3] = *reinterpret_cast<const uint32_t*>(&dzT[16 * mt + g + 8][2 * tig + 8]);
+  for (int j = 0; j < 8; ++j)
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {  // input-feature tile (columns of dW)
-      float acc[4] = {0.f, 0.f, 0.f, 0.f};
-      const uint32_t b0 = *reinterpret_cast<const uint32_t*>(&hT[8 * j + g][2 * tig]);
-      const uint32_t b1 = *reinterpret_cast<const uint32_t*>(&hT[8 * j + g][2 * tig + 8]);
-      mma_bf16(acc, a, b0, b1);
-      const int r0 = 16 * mt + g, c0 = 8 * j + 2 * tig;
-      atomicAdd(&gW[r0 * HID + c0], acc[0]);
-      atomicAdd(&gW[r0 * HID + c0 + 1], acc[1]);
-      atomicAdd(&gW[(r0 + 8) * HID + c0], acc[2]);
-      atomicAdd(&gW[(r0 + 8) * HID + c0 + 1], acc[3]);
+    for (int q = 0; q < 4; ++q) {
+      const float sg = recip_ge1(1.0f + __expf(-z[j][q]));
+      h[j][q] = z[j][q] * sg;
+      ds[j][q] = sg * (1.0f + z[j][q] * (1.0f - sg));
     }
-  }
 }
 
-// Stage a C-layout fragment set (rows = samples g, g+8; 64 features) as the
-// transposed BF16 tile [feature][sample].
-__device__ __forceinline__ void stage_T(__nv_bfloat16 (*dst)[LDS], const float v[8][4], int g, int tig) {
+// v[2 j + h] over the 8 lanes that share tig, each adding its column sums 8 j
+// + 2 tig + h: lane g keeps j = g (14 exchanges for 16 sums, where a sum
+// per column takes 48), added to acc[0..1].
+__device__ __forceinline__ void add_column_sums(float acc[2], const float v[16], int lane) {
+  float a[8], b[4];
+  const bool h4 = lane & 16, h3 = lane & 8, h2 = lane & 4;
 #pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    const int c = 8 * j + 2 * tig;
-    dst[c][g] = __float2bfloat16_rn(v[j][0]);
-    dst[c + 1][g] = __float2bfloat16_rn(v[j][1]);
-    dst[c][g + 8] = __float2bfloat16_rn(v[j][2]);
-    dst[c + 1][g + 8] = __float2bfloat16_rn(v[j][3]);
-  }
+  for (int q = 0; q < 8; ++q)
+    a[q] = (h4 ? v[8 + q] : v[q]) + __shfl_xor_sync(0xffffffffu, h4 ? v[q] : v[8 + q], 16);
+#pragma unroll
+  for (int q = 0; q < 4; ++q)
+    b[q] = (h3 ? a[4 + q] : a[q]) + __shfl_xor_sync(0xffffffffu, h3 ? a[q] : a[4 + q], 8);
+#pragma unroll
+  for (int q = 0; q < 2; ++q)
+    acc[q] += (h2 ? b[2 + q] : b[q]) + __shfl_xor_sync(0xffffffffu, h2 ? b[q] : b[2 + q], 4);
 }
 
 // One pass over a minibatch: loss sum_i |w_i| e_i^2 / nb and its gradient
 // w.r.t. the FP32 parameters P, on features X (3 per sample, normalised),
 // targets Y and weights Wt (all 1 when null), e_i = y_i - t_i, or
 // min(y_i - t_i, 0) where w_i < 0 (a one-sided target: y_i >= t_i).  grad and
-// loss are accumulated with global atomics.
+// loss are accumulated with global atomics, once per block.
+//
+// A warp takes 16 samples through the forward and the backward pass in
+// registers and stages dZ and H of the two 64 x 64 layers; the block's eight
+// warps then share those layers' weight gradients, 16 rows of one layer
+// each over the block's 128 samples, and hold them in registers until the
+// end (added with FP32 additions every 16 samples, as the products' own
+// accumulator starts at zero).  Each pre-activation's sigmoid is evaluated
+// once, for the activation and its derivative.  262,144 samples: 637 us with
+// shared-memory atomics for every 16 samples' gradient, a sum over lanes per
+// column and three sigmoids, 105 us now, bound by issue (sigmoids and their
+// divisions, products, column sums).
 __global__ void __launch_bounds__(TT) k_mlp_grad(const float* __restrict__ P, const float* __restrict__ X,
                                                  const float* __restrict__ Y, const float* __restrict__ Wt, int nb,
                                                  float* grad, float* loss) {
   extern __shared__ __align__(16) unsigned char sm_[];
   TrainSmem& s = *reinterpret_cast<TrainSmem*>(sm_);
-  load_weights(P, s.W, &s.WT);
-  for (int q = threadIdx.x; q < NPARAM; q += TT) s.g[q] = 0.0f;
-  if (threadIdx.x == 0) s.loss = 0.0f;
+  load_weights(P, s.W);
   __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, tig = lane & 3;
   const float inv_nb = 1.0f / (float)nb;
   const int ntiles = (nb + TS - 1) / TS;
-  for (int tile = blockIdx.x * TW + warp; tile < ntiles; tile += gridDim.x * TW) {
-    const int r0 = tile * TS + g, r1 = r0 + 8;
-    const bool v0 = r0 < nb, v1 = r1 < nb;
-    float xg[3] = {0.f, 0.f, 0.f}, xg8[3] = {0.f, 0.f, 0.f};
-    if (v0) for (int f = 0; f < 3; ++f) xg[f] = X[3 * r0 + f];
-    if (v1) for (int f = 0; f < 3; ++f) xg8[f] = X[3 * r1 + f];
-    float z1[8][4], z2[8][4], z3[8][4], y[2];
-    forward_tile(s.W, xg, xg8, g, tig, y, z1, z2, z3);
-    // d loss / d y = 2 w (y - t) / nb (rows outside the batch contribute 0)
-    float dy0 = 0.f, dy1 = 0.f;
-    if (tig == 0) {
-      float w0 = v0 ? (Wt ? Wt[r0] : 1.0f) : 0.0f, w1 = v1 ? (Wt ? Wt[r1] : 1.0f) : 0.0f;
-      float e0 = v0 ? y[0] - Y[r0] : 0.0f, e1 = v1 ? y[1] - Y[r1] : 0.0f;
-      if (w0 < 0.0f) { w0 = -w0; e0 = fminf(e0, 0.0f); }
-      if (w1 < 0.0f) { w1 = -w1; e1 = fminf(e1, 0.0f); }
-      dy0 = 2.0f * w0 * e0 * inv_nb;
-      dy1 = 2.0f * w1 * e1 * inv_nb;
-      atomicAdd(&s.loss, (w0 * e0 * e0 + w1 * e1 * e1) * inv_nb);
-    }
-    dy0 = __shfl_sync(0xffffffffu, dy0, lane & ~3);
-    dy1 = __shfl_sync(0xffffffffu, dy1, lane & ~3);
-    // layer 4: dW4 = dy H3, db4 = sum dy, dZ3 = dy W4 * silu'(z3)
-    float d[8][4];
-    float db4p = (tig == 0) ? dy0 + dy1 : 0.0f;
-    db4p = sum_over_g(db4p);
-    if (lane == 0) atomicAdd(&s.g[OFF_B4], db4p);
+  float gw[8][4], vec[NVEC][2], gb4 = 0.0f, part = 0.0f;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const int c = 8 * j + 2 * tig;
-      const float w0 = s.W.w4[c], w1v = s.W.w4[c + 1];
-      const float h00 = silu_f(z3[j][0]), h01 = silu_f(z3[j][1]);
-      const float h10 = silu_f(z3[j][2]), h11 = silu_f(z3[j][3]);
-      float gw0 = sum_over_g(dy0 * h00 + dy1 * h10);
-      float gw1 = sum_over_g(dy0 * h01 + dy1 * h11);
-      if (g == 0) {
-        atomicAdd(&s.g[OFF_W4 + c], gw0);
-        atomicAdd(&s.g[OFF_W4 + c + 1], gw1);
-      }
-      d[j][0] = dy0 * w0 * dsilu_f(z3[j][0]);
-      d[j][1] = dy0 * w1v * dsilu_f(z3[j][1]);
-      d[j][2] = dy1 * w0 * dsilu_f(z3[j][2]);
-      d[j][3] = dy1 * w1v * dsilu_f(z3[j][3]);
-    }
-    // layers 3 and 2: db = sum dZ; dW = dZ^T H (tensor cores); dH = dZ W (tensor cores)
-    const int offW[2] = {OFF_W3, OFF_W2}, offB[2] = {OFF_B3, OFF_B2};
+  for (int j = 0; j < 8; ++j)
 #pragma unroll
-    for (int L = 0; L < 2; ++L) {
-      float (*zin)[4] = (L == 0) ? z2 : z1;  // pre-activation feeding this layer
+    for (int q = 0; q < 4; ++q) gw[j][q] = 0.0f;
+#pragma unroll
+  for (int q = 0; q < NVEC; ++q) vec[q][0] = vec[q][1] = 0.0f;
+  for (int tile0 = blockIdx.x * TW; tile0 < ntiles; tile0 += gridDim.x * TW) {
+    const int tile = tile0 + warp;
+    if (tile < ntiles) {
+      const int r0 = tile * TS + g, r1 = r0 + 8;
+      const bool v0 = r0 < nb, v1 = r1 < nb;
+      float xg[3] = {0.f, 0.f, 0.f}, xg8[3] = {0.f, 0.f, 0.f};
+      if (v0) for (int f = 0; f < 3; ++f) xg[f] = X[3 * (size_t)r0 + f];
+      if (v1) for (int f = 0; f < 3; ++f) xg8[f] = X[3 * (size_t)r1 + f];
+      float d[8][4], h[8][4], ds1[8][4], ds2[8][4], ds3[8][4], v[16];
+      uint32_t a[4][4];
+      input_layer(d, s.W, xg, xg8, tig);
+      silu_both(h, ds1, d);
+      frag_plain(a, h);
+      stage(s.st[3][warp], a, g, tig);
+      train_dense<false>(d, a, s.W.w2, s.W.b2, lane);
+      silu_both(h, ds2, d);
+      frag_plain(a, h);
+      stage(s.st[1][warp], a, g, tig);
+      train_dense<false>(d, a, s.W.w3, s.W.b3, lane);
+      silu_both(h, ds3, d);
+      // output layer in FP32: this lane's 16 columns, then the sum over tig
+      float y0 = 0.0f, y1 = 0.0f;
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
         const int c = 8 * j + 2 * tig;
-        const float s0 = sum_over_g(d[j][0] + d[j][2]);
-        const float s1 = sum_over_g(d[j][1] + d[j][3]);
-        if (g == 0) {
-          atomicAdd(&s.g[offB[L] + c], s0);
-          atomicAdd(&s.g[offB[L] + c + 1], s1);
+        y0 += s.W.w4[c] * h[j][0] + s.W.w4[c + 1] * h[j][1];
+        y1 += s.W.w4[c] * h[j][2] + s.W.w4[c + 1] * h[j][3];
+      }
+      y0 += __shfl_xor_sync(0xffffffffu, y0, 1);
+      y1 += __shfl_xor_sync(0xffffffffu, y1, 1);
+      y0 += __shfl_xor_sync(0xffffffffu, y0, 2);
+      y1 += __shfl_xor_sync(0xffffffffu, y1, 2);
+      y0 = s.W.b4 + y0;  // row g
+      y1 = s.W.b4 + y1;  // row g + 8
+      // d loss / d y = 2 w (y - t) / nb (rows outside the batch contribute 0)
+      float dy0 = 0.f, dy1 = 0.f;
+      if (tig == 0) {
+        float w0 = v0 ? (Wt ? Wt[r0] : 1.0f) : 0.0f, w1 = v1 ? (Wt ? Wt[r1] : 1.0f) : 0.0f;
+        float e0 = v0 ? y0 - Y[r0] : 0.0f, e1 = v1 ? y1 - Y[r1] : 0.0f;
+        if (w0 < 0.0f) { w0 = -w0; e0 = fminf(e0, 0.0f); }
+        if (w1 < 0.0f) { w1 = -w1; e1 = fminf(e1, 0.0f); }
+        dy0 = 2.0f * w0 * e0 * inv_nb;
+        dy1 = 2.0f * w1 * e1 * inv_nb;
+        part += (w0 * e0 * e0 + w1 * e1 * e1) * inv_nb;
+        gb4 += dy0 + dy1;
+      }
+      dy0 = __shfl_sync(0xffffffffu, dy0, lane & ~3);
+      dy1 = __shfl_sync(0xffffffffu, dy1, lane & ~3);
+      // layer 4: dW4 = dy H3, dZ3 = dy W4 * silu'(z3)
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const int c = 8 * j + 2 * tig;
+        const float w0 = s.W.w4[c], w1 = s.W.w4[c + 1];
+        v[2 * j] = dy0 * h[j][0] + dy1 * h[j][2];
+        v[2 * j + 1] = dy0 * h[j][1] + dy1 * h[j][3];
+        d[j][0] = dy0 * w0 * ds3[j][0];
+        d[j][1] = dy0 * w1 * ds3[j][1];
+        d[j][2] = dy1 * w0 * ds3[j][2];
+        d[j][3] = dy1 * w1 * ds3[j][3];
+      }
+      add_column_sums(vec[0], v, lane);
+      // layers 3 and 2: db = sum dZ; dH = dZ W (tensor cores)
+#pragma unroll
+      for (int L = 0; L < 2; ++L) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          v[2 * j] = d[j][0] + d[j][2];
+          v[2 * j + 1] = d[j][1] + d[j][3];
+        }
+        add_column_sums(vec[1 + L], v, lane);
+        frag_plain(a, d);
+        stage(s.st[2 * L][warp], a, g, tig);
+        train_dense<true>(h, a, L == 0 ? s.W.w3 : s.W.w2, nullptr, lane);
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+#pragma unroll
+          for (int q = 0; q < 4; ++q) d[j][q] = h[j][q] * (L == 0 ? ds2[j][q] : ds1[j][q]);
+      }
+      // layer 1: db1 = sum dZ1, dW1 = dZ1^T X (K = 3, FP32)
+#pragma unroll
+      for (int f = -1; f < 3; ++f) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          v[2 * j] = f < 0 ? d[j][0] + d[j][2] : d[j][0] * xg[f] + d[j][2] * xg8[f];
+          v[2 * j + 1] = f < 0 ? d[j][1] + d[j][3] : d[j][1] * xg[f] + d[j][3] * xg8[f];
+        }
+        add_column_sums(vec[4 + f], v, lane);
+      }
+    }
+    __syncthreads();
+    // dW = dZ^T H (tensor cores) of layer 3 (warps 0-3) or 2, rows 16 (warp & 3) ..
+    const int nt = min(TW, ntiles - tile0), L = warp >> 2, mt = warp & 3;
+    for (int t = 0; t < nt; ++t) {
+      uint32_t a[4];
+      // (matrices: samples 0-7 of features 0-7, 0-7 of 8-15, 8-15 of 0-7, 8-15 of 8-15)
+      ldmatrix4<true>(a, smem_addr(&s.st[2 * L][t][(lane & 7) + 8 * (lane >> 4)][16 * mt + 8 * ((lane >> 3) & 1)]));
+#pragma unroll
+      for (int jp = 0; jp < 4; ++jp) {
+        uint32_t b[4];
+        ldmatrix4<true>(b, smem_addr(&s.st[2 * L + 1][t][(lane & 7) + 8 * ((lane >> 3) & 1)][16 * jp + 8 * (lane >> 4)]));
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          float acc[4] = {0.f, 0.f, 0.f, 0.f};
+          mma_bf16(acc, a, b[2 * q], b[2 * q + 1]);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) gw[2 * jp + q][e] += acc[e];
         }
       }
-      float h[8][4];
-#pragma unroll
-      for (int j = 0; j < 8; ++j)
-#pragma unroll
-        for (int q = 0; q < 4; ++q) h[j][q] = silu_f(zin[j][q]);
-      __syncwarp();
-      stage_T(s.stA[warp], d, g, tig);
-      stage_T(s.stB[warp], h, g, tig);
-      __syncwarp();
-      weight_grad64(&s.g[offW[L]], s.stA[warp], s.stB[warp], g, tig);
-      __syncwarp();
-      uint32_t a[4][4];
-      frag_plain(a, d);
-      float dh[8][4];
-      if (L == 0)
-        dense64<4, LD>(dh, a, s.WT.w3t, nullptr, g, tig);
-      else
-        dense64<4, LD>(dh, a, s.WT.w2t, nullptr, g, tig);
-#pragma unroll
-      for (int j = 0; j < 8; ++j)
-#pragma unroll
-        for (int q = 0; q < 4; ++q) d[j][q] = dh[j][q] * dsilu_f(zin[j][q]);
     }
-    // layer 1: db1 = sum dZ1, dW1 = dZ1^T X (K = 3, FP32)
+    __syncthreads();
+  }
+  float* gW = grad + ((warp >> 2) ? OFF_W2 : OFF_W3) + (16 * (warp & 3) + g) * HID + 2 * tig;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const int c = 8 * j + 2 * tig;
-      const float s0 = sum_over_g(d[j][0] + d[j][2]);
-      const float s1 = sum_over_g(d[j][1] + d[j][3]);
-      if (g == 0) {
-        atomicAdd(&s.g[OFF_B1 + c], s0);
-        atomicAdd(&s.g[OFF_B1 + c + 1], s1);
-      }
+  for (int j = 0; j < 8; ++j) {
+    atomicAdd(reinterpret_cast<float2*>(gW + 8 * j), make_float2(gw[j][0], gw[j][1]));
+    atomicAdd(reinterpret_cast<float2*>(gW + 8 * HID + 8 * j), make_float2(gw[j][2], gw[j][3]));
+  }
 #pragma unroll
-      for (int f = 0; f < 3; ++f) {
-        const float w0 = sum_over_g(d[j][0] * xg[f] + d[j][2] * xg8[f]);
-        const float w1v = sum_over_g(d[j][1] * xg[f] + d[j][3] * xg8[f]);
-        if (g == 0) {
-          atomicAdd(&s.g[OFF_W1 + c * IN + f], w0);
-          atomicAdd(&s.g[OFF_W1 + (c + 1) * IN + f], w1v);
-        }
-      }
-    }
+  for (int q = 0; q < NVEC; ++q) {
+    s.vec[warp][q][8 * g + 2 * tig] = vec[q][0];
+    s.vec[warp][q][8 * g + 2 * tig + 1] = vec[q][1];
+  }
+  for (int o = 16; o > 0; o >>= 1) {
+    gb4 += __shfl_xor_sync(0xffffffffu, gb4, o);
+    part += __shfl_xor_sync(0xffffffffu, part, o);
+  }
+  if (lane == 0) {
+    s.b4[warp] = gb4;
+    s.loss[warp] = part;
   }
   __syncthreads();
-  for (int q = threadIdx.x; q < NPARAM; q += TT) atomicAdd(&grad[q], s.g[q]);
-  if (threadIdx.x == 0) atomicAdd(loss, s.loss);
+  for (int q = threadIdx.x; q < NVEC * HID + 2; q += TT) {
+    float sum = 0.0f;
+    for (int w = 0; w < TW; ++w)
+      sum += q < NVEC * HID ? s.vec[w][q / HID][q % HID] : q == NVEC * HID ? s.b4[w] : s.loss[w];
+    const int c = q % HID, k = q / HID;
+    if (q == NVEC * HID + 1)
+      atomicAdd(loss, sum);
+    else
+      atomicAdd(&grad[q == NVEC * HID ? OFF_B4
+                      : k == 0       ? OFF_W4 + c
+                      : k == 1       ? OFF_B3 + c
+                      : k == 2       ? OFF_B2 + c
+                      : k == 3       ? OFF_B1 + c
+                                     : OFF_W1 + c * IN + (k - 4)],
+                sum);
+  }
 }
 
 // Adam on the FP32 master parameters.
@@ -226,7 +332,7 @@ __global__ void k_adam(float* P, float* m, float* v, const float* grad, int n, f
 __global__ void __launch_bounds__(TT) k_mlp_infer(const float* __restrict__ P, const float* __restrict__ X, int n,
                                                   float* __restrict__ Yout) {
   __shared__ SmemWeights W;
-  load_weights(P, W, nullptr);
+  load_weights(P, W);
   __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, tig = lane & 3;
   const int ntiles = (n + TS - 1) / TS;
@@ -406,14 +512,14 @@ cudaError_t launch_normalise(float* X, long long N, const float norm[6], cudaStr
   return cudaGetLastError();
 }
 
-size_t mlp_train_smem() { return sizeof(mlp::TrainSmem); }
-
 cudaError_t launch_mlp_grad(const float* P, const float* X, const float* Y, const float* Wt, int nb, float* grad,
-                            float* loss, int nblocks, cudaStream_t s) {
+                            float* loss, cudaStream_t s) {
   // (set on every call: the attribute belongs to the current device)
   const cudaError_t e = cudaFuncSetAttribute(mlp::k_mlp_grad, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)sizeof(mlp::TrainSmem));
   if (e != cudaSuccess) return e;
+  // a warp per 16 samples, at most a block per SM (98 KB and 256 threads of up to 255 registers)
+  const int nblocks = std::max(1, std::min(152, (nb + mlp::TS * mlp::TW - 1) / (mlp::TS * mlp::TW)));
   mlp::k_mlp_grad<<<nblocks, mlp::TT, sizeof(mlp::TrainSmem), s>>>(P, X, Y, Wt, nb, grad, loss);
   return cudaGetLastError();
 }
@@ -426,7 +532,7 @@ cudaError_t launch_adam(float* P, float* m, float* v, const float* grad, int n, 
 }
 
 namespace {
-__global__ void k_pack_weights(const float* __restrict__ P, mlp::SmemWeights* img) { mlp::load_weights(P, *img, nullptr); }
+__global__ void k_pack_weights(const float* __restrict__ P, mlp::SmemWeights* img) { mlp::load_weights(P, *img); }
 }  // namespace
 
 size_t mlp_image_bytes() { return sizeof(mlp::SmemWeights); }

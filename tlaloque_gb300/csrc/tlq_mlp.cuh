@@ -35,12 +35,6 @@ struct alignas(16) SmemWeights {
   float w4[HID];                // output layer, FP32
   float b1[HID], b2[HID], b3[HID], b4;
 };
-// Transposed copies for the backward pass (dH = dZ W).
-struct SmemWeightsT {
-  __nv_bfloat16 w2t[HID][LD];
-  __nv_bfloat16 w3t[HID][LD];
-};
-
 __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
   const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);  // .x = lo (low 16 bits)
   return *reinterpret_cast<const uint32_t*>(&v);
@@ -57,13 +51,8 @@ __device__ __forceinline__ void mma_bf16(float* d, const uint32_t* a, uint32_t b
 
 __device__ __forceinline__ float sigmoid_f(float z) { return 1.0f / (1.0f + __expf(-z)); }
 __device__ __forceinline__ float silu_f(float z) { return z * sigmoid_f(z); }
-__device__ __forceinline__ float dsilu_f(float z) {
-  const float s = sigmoid_f(z);
-  return s * (1.0f + z * (1.0f - s));
-}
-
 // Load the FP32 master parameters into the BF16 shared layout (all threads).
-__device__ inline void load_weights(const float* __restrict__ P, SmemWeights& W, SmemWeightsT* WT) {
+__device__ inline void load_weights(const float* __restrict__ P, SmemWeights& W) {
   for (int q = threadIdx.x; q < HID * 4; q += blockDim.x) {
     const int n = q / 4, k = q % 4;
     W.w1[n][k] = k < IN ? P[OFF_W1 + n * IN + k] : 0.0f;
@@ -73,10 +62,6 @@ __device__ inline void load_weights(const float* __restrict__ P, SmemWeights& W,
     const bool in = k < HID;
     W.w2[n][k] = __float2bfloat16_rn(in ? P[OFF_W2 + n * HID + k] : 0.0f);
     W.w3[n][k] = __float2bfloat16_rn(in ? P[OFF_W3 + n * HID + k] : 0.0f);
-    if (WT) {
-      WT->w2t[n][k] = __float2bfloat16_rn(in ? P[OFF_W2 + k * HID + n] : 0.0f);
-      WT->w3t[n][k] = __float2bfloat16_rn(in ? P[OFF_W3 + k * HID + n] : 0.0f);
-    }
   }
   for (int q = threadIdx.x; q < HID; q += blockDim.x) {
     W.w4[q] = P[OFF_W4 + q];
@@ -158,36 +143,16 @@ __device__ __forceinline__ void act_to_frag(uint32_t a[4][4], const float z[8][4
 }
 
 // Forward pass of one m16 tile; returns the outputs of rows g and g+8 in
-// y[0], y[1] (in all four lanes of the group g).  Optionally keeps the
-// pre-activations of the three hidden layers (training).
+// y[0], y[1] (in all four lanes of the group g).
 __device__ __forceinline__ void forward_tile(const SmemWeights& W, const float* xg, const float* xg8, int g, int tig,
-                                             float* y, float (*z1)[4] = nullptr, float (*z2)[4] = nullptr,
-                                             float (*z3)[4] = nullptr) {
+                                             float* y) {
   float acc[8][4];
   input_layer(acc, W, xg, xg8, tig);
-  if (z1) {
-#pragma unroll
-    for (int j = 0; j < 8; ++j)
-#pragma unroll
-      for (int q = 0; q < 4; ++q) z1[j][q] = acc[j][q];
-  }
   uint32_t a[4][4];
   act_to_frag(a, acc);
   dense64<4, LD>(acc, a, W.w2, W.b2, g, tig);
-  if (z2) {
-#pragma unroll
-    for (int j = 0; j < 8; ++j)
-#pragma unroll
-      for (int q = 0; q < 4; ++q) z2[j][q] = acc[j][q];
-  }
   act_to_frag(a, acc);
   dense64<4, LD>(acc, a, W.w3, W.b3, g, tig);
-  if (z3) {
-#pragma unroll
-    for (int j = 0; j < 8; ++j)
-#pragma unroll
-      for (int q = 0; q < 4; ++q) z3[j][q] = acc[j][q];
-  }
   // output layer in FP32: this lane's 16 columns, then the sum over tig
   float s0 = 0.0f, s1 = 0.0f;
 #pragma unroll

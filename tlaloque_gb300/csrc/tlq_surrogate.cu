@@ -668,7 +668,6 @@ int tlq_train_cooling_surrogate(tlq_ctx* ctx, const tlq_surrogate_opts* opts, tl
   TCK(cudaMemsetAsync(v, 0, NPARAM * sizeof(float), s));
   const long long steps_per_epoch = Ntr / o.batch;
   const long long total = steps_per_epoch * o.epochs;
-  const int gblocks = std::max(1, std::min(152 * 2, (o.batch / 16 + 3) / 4));  // 16-sample tiles, 4 warps a block
   float lfirst = 0.f, llast = 0.f;
   long long t = 0;
   for (int ep = 0; ep < o.epochs; ++ep) {
@@ -677,8 +676,7 @@ int tlq_train_cooling_surrogate(tlq_ctx* ctx, const tlq_surrogate_opts* opts, tl
       const float lr = o.lr * (0.05f + 0.95f * 0.5f * (1.0f + std::cos(3.14159265f * (float)(t - 1) / (float)total)));
       TCK(cudaMemsetAsync(grad, 0, NPARAM * sizeof(float), s));
       TCK(cudaMemsetAsync(loss, 0, sizeof(float), s));
-      TCK(launch_mlp_grad(P, X2 + 3 * b * o.batch, Y2 + b * o.batch, Wt2 + b * o.batch, o.batch, grad, loss,
-                          gblocks, s));
+      TCK(launch_mlp_grad(P, X2 + 3 * b * o.batch, Y2 + b * o.batch, Wt2 + b * o.batch, o.batch, grad, loss, s));
       TCK(launch_adam(P, m, v, grad, NPARAM, lr, 0.9f, 0.999f, 1e-8f, (int)t, s));
       if (t == 1) {
         TCK(cudaMemcpyAsync(&lfirst, loss, sizeof(float), cudaMemcpyDeviceToHost, s));
@@ -789,7 +787,7 @@ int tlq_mlp_loss_grad(const float* params, const float* X, const float* Y, const
   if (e == cudaSuccess) e = cudaMemset(dg, 0, tlq::mlp::NPARAM * sizeof(float));
   if (e == cudaSuccess) e = cudaMemset(dl, 0, sizeof(float));
   if (e == cudaSuccess)
-    e = launch_mlp_grad(dP, dX, dY, dW, n, dg, dl, std::max(1, std::min(152 * 2, (n / 16 + 3) / 4)), 0);
+    e = launch_mlp_grad(dP, dX, dY, dW, n, dg, dl, 0);
   if (e == cudaSuccess) e = cudaMemcpy(grad, dg, tlq::mlp::NPARAM * sizeof(float), cudaMemcpyDeviceToHost);
   if (e == cudaSuccess) e = cudaMemcpy(loss, dl, sizeof(float), cudaMemcpyDeviceToHost);
   cudaFree(dP); cudaFree(dX); cudaFree(dY); cudaFree(dW); cudaFree(dg); cudaFree(dl);
