@@ -307,18 +307,19 @@ __device__ __forceinline__ bool riemann(int solver, R g, R g1, R* ff, const R* w
 __device__ __forceinline__ bool wind_cell(const Params& p, const Wind& w, int i, int j, int k, double* u) {
   if (i < w.ilo || i > w.ihi || j < w.jlo || j > w.jhi || k < w.klo || k > w.khi) return false;
   const double x = xcoord(p, i), y = ycoord(p, j), z = zcoord(p, k);
-  const double dist = sqrt((x - w.xc) * (x - w.xc) + (y - w.yc) * (y - w.yc) + (z - w.zc) * (z - w.zc));
+  const double dist = root((x - w.xc) * (x - w.xc) + (y - w.yc) * (y - w.yc) + (z - w.zc) * (z - w.zc));
   if (!(dist < w.radius)) return false;
-  const double dens = w.mdot / (w.vinf * dist * dist * 4.0 * PI_REF);
-  const double vx = w.vinf * (x - w.xc) / dist + w.vx;
-  const double vy = w.vinf * (y - w.yc) / dist + w.vy;
-  const double vz = w.vinf * (z - w.zc) / dist + w.vz;
-  const double pres = dens * KB * w.temp / (w.mu * AMU);
+  const double dens = quot(w.mdot, w.vinf * dist * dist * 4.0 * PI_REF);
+  const auto dd = divisor(dist);
+  const double vx = quot(w.vinf * (x - w.xc), dd) + w.vx;
+  const double vy = quot(w.vinf * (y - w.yc), dd) + w.vy;
+  const double vz = quot(w.vinf * (z - w.zc), dd) + w.vz;
+  const double pres = quot(dens * KB * w.temp, w.mu * AMU);
   u[0] = dens;
   u[1] = dens * vx;
   u[2] = dens * vy;
   u[3] = dens * vz;
-  u[4] = 0.5 * dens * ((vx * vx + vy * vy) + vz * vz) + pres / (p.gamma - 1.0);
+  u[4] = 0.5 * dens * ((vx * vx + vy * vy) + vz * vz) + quot(pres, p.gamma - 1.0);
   return true;
 }
 
@@ -363,25 +364,29 @@ __device__ __forceinline__ bool near_boundary_or_wind(const Params& p, int i, in
 // face, and the z range [klo, khi] of the spherical winds whose index boxes
 // meet the tile's columns.  Formed once per tile (the winds' boxes are read
 // from memory there, not per cell); plane k of the tile may hold a cell for
-// which near_boundary_or_wind is true only if may_be_special(k).
+// which near_boundary_or_wind is true only if may_be_special(k), and a cell
+// that a wind sets, or a ghost image that one overwrites, only if windy(k).
 struct TileSpecial {
-  bool ij;
+  bool ij, ghost_wind;
   int klo, khi;
   __device__ __forceinline__ bool may_be_special(const Params& p, int k) const {
     return ij || k <= 2 || k >= p.nz - 1 || (p.nplanes > 0 && k >= p.nz) || (k >= klo && k <= khi);
   }
+  __device__ __forceinline__ bool windy(int k) const { return ghost_wind || (k >= klo && k <= khi); }
 };
 __device__ __forceinline__ TileSpecial tile_special(const Params& p, int i0, int i1, int j0, int j1) {
   TileSpecial t;
   t.ij = i0 <= 2 || j0 <= 2 || i1 >= p.nx - 1 || j1 >= p.ny - 1;
   t.klo = 1 << 30;
   t.khi = -(1 << 30);
+  t.ghost_wind = p.nplanes > 0;
   for (int s = 0; s < p.nwinds; ++s) {
     const Wind& w = p.winds[s];
     if (i1 >= w.ilo && i0 <= w.ihi && j1 >= w.jlo && j0 <= w.jhi) {
       t.klo = min(t.klo, w.klo);
       t.khi = max(t.khi, w.khi);
     }
+    if (w.ilo < 1 || w.jlo < 1 || w.klo < 1 || w.ihi > p.nx || w.jhi > p.ny || w.khi > p.nz) t.ghost_wind = true;
   }
   return t;
 }

@@ -95,8 +95,6 @@ struct StageSmem {
 // cell's value (flip: with the momentum along the axis negated).  Rolled
 // loops: few cells come here, and unrolled this code (with what put inlines)
 // was most of a stage kernel's 0.5-0.9 MB of instructions (now 0.12-0.36).
-// (Stage 1 of the mixed form keeps its unrolled ghost_targets: rolled, its
-// plane loop compiled 5 % slower on the 256^3 bubble.)
 template <class Put>
 __device__ __forceinline__ void ghost_images(const Params& p, int layers, int i, int j, int k, Put put) {
 #pragma unroll 1

@@ -103,6 +103,14 @@ template <int S>
 using MixedSmem = typename MixedSmemSel<S>::type;
 
 
+// The pressure of a cell from its FP64 conserved values (a call: few cells
+// take it, and inlined it lengthened every conversion loop, whose kernels
+// wait on instruction fetch: stage 1 of the bubble 256^3 0.966 -> 0.938 ms).
+static __device__ __noinline__ float kinetic_pressure(float gm1, double r, double m1, double m2, double m3, double E) {
+  const double k2 = __fma_rn(m3, m3, __fma_rn(m2, m2, __dmul_rn(m1, m1)));
+  return d2f(__dmul_rn((double)gm1, __dsub_rn(E, sf::div(__dmul_rn(0.5, k2), r))));
+}
+
 // One cell: FP64 conserved (stride vs) -> FP32 conserved and primitives.
 // The pressure of a cell whose kinetic energy exceeds 0.99 of its total
 // energy is recovered in FP64 (FP32 would lose it to cancellation).  The
@@ -122,13 +130,9 @@ __device__ __forceinline__ void mixed_cell(float gm1, const double* u, long long
   const bool kin = ek > __fmul_rn(0.99f, cf[4]);
   float p = __fmul_rn(gm1, __fsub_rn(cf[4], ek));
   // a branch the whole warp skips unless one of its cells needs FP64 (the
-  // FP64 division would otherwise be evaluated for every cell)
+  // FP64 operations would otherwise run for every cell)
   if (__any_sync(__activemask(), kin)) {
-    if (kin) {
-      const double r = u[0], m1 = u[vs], m2 = u[2 * vs], m3 = u[3 * vs], E = u[4 * vs];
-      const double k2 = __fma_rn(m3, m3, __fma_rn(m2, m2, __dmul_rn(m1, m1)));
-      p = d2f(__dmul_rn((double)gm1, __dsub_rn(E, __ddiv_rn(__dmul_rn(0.5, k2), r))));
-    }
+    if (kin) p = kinetic_pressure(gm1, u[0], u[vs], u[2 * vs], u[3 * vs], u[4 * vs]);
   }
   w[4] = fmaxf(p, 1e-20f);
 }
@@ -324,58 +328,69 @@ __device__ __forceinline__ void cool_cell_f(const Params& p, float cT, float inv
   cool_cell_known(p, cT, inv_muamu, gm1, w, u4, dt, temp, aloss, seg);
 }
 
-// Ghost targets of one interior cell along one axis (boundaries.f90 non-MPI
-// branches).  layers = 1: boundariesI (:183-257); layers = 2: boundariesII
-// (:433-531).  Returns the number of (target index, flip) pairs.
-__device__ __forceinline__ int ghost_targets(int layers, int bclo, int bchi, int c, int n, int* tgt, int* flip) {
-  int m = 0;
-  if (bclo == BC_OUTFLOW) {
-    if (c == 1) { tgt[m] = 0; flip[m++] = 0; if (layers == 2) { tgt[m] = -1; flip[m++] = 0; } }
-  } else if (bclo == BC_REFLECTIVE) {
-    if (c == 1) { tgt[m] = 0; flip[m++] = 1; }
-    if (layers == 2 && c == 2) { tgt[m] = -1; flip[m++] = 1; }
-  } else if (bclo == BC_PERIODIC) {
-    if (c == n) { tgt[m] = 0; flip[m++] = 0; }
-    if (layers == 2 && c == n - 1) { tgt[m] = -1; flip[m++] = 0; }
-  }
-  if (bchi == BC_OUTFLOW) {
-    if (c == n) { tgt[m] = n + 1; flip[m++] = 0; if (layers == 2) { tgt[m] = n + 2; flip[m++] = 0; } }
-  } else if (bchi == BC_REFLECTIVE) {
-    if (c == n) { tgt[m] = n + 1; flip[m++] = 1; }
-    if (layers == 2 && c == n - 1) { tgt[m] = n + 2; flip[m++] = 1; }
-  } else if (bchi == BC_PERIODIC) {
-    if (c == 1) { tgt[m] = n + 1; flip[m++] = 0; }
-    if (layers == 2 && c == 2) { tgt[m] = n + 2; flip[m++] = 0; }
-  }
-  return m;
-}
-
-// The face-ghost images of a stage-1 cell (borders(UPP, 2), boundaries.f90
-// non-MPI branches) as FP32 primitives of UPP: the FP64 image of v (normal
-// momentum negated at a reflective face) with the winds applied at the ghost
-// cell, through mixed_cell -- what stage 2 forms from UPP.
-__device__ __forceinline__ void write_ghost_prims(const Params& p, const Layout& L, float* out, float gm1, int i,
-                                                  int j, int k, const double* v) {
-  const int c3[3] = {i, j, k};
-  const int n3[3] = {p.nx, p.ny, p.nz};
-#pragma unroll
+// The face-ghost images (ghost_images) of the interior cell (i, j, k) at c
+// where no wind reaches a ghost cell: its value v, the momentum along the
+// axis negated at a reflective face.  FP32 primitives as well: negating a
+// momentum negates its velocity and leaves the others, so they are what
+// mixed_cell would form of the image.
+//   A tile at an x or y face has such cells in every warp and plane: with
+// each image formed anew from FP64 (winds, mixed_cell) it took twice an
+// interior tile's time in stage 1 and 1.45 times in stage 2 (16-plane chunks,
+// 290 k and 142 k cycles, 340 k and 235 k); now 1.3 and 1.15 times.  Bubble
+// 256^3: stage 1 0.97 -> 0.83 ms, stage 2 1.42 -> 1.34; diagonal Sod 150^3:
+// 0.235 -> 0.198 and 0.281 -> 0.265.  The axes rolled in stage 1 (less code:
+// 3 % on the bubble), unrolled in stage 2 (1 %).
+template <int LAYERS, class T>
+__device__ __forceinline__ void store_ghosts(const Params& p, const Layout& L, T* out, int i, int j, int k,
+                                             long long c, const T* v) {
+#pragma unroll(LAYERS == 2 ? 1 : 3)
   for (int ax = 0; ax < 3; ++ax) {
-    int tgt[4], flp[4];
-    const int m = ghost_targets(2, p.bc[2 * ax], p.bc[2 * ax + 1], c3[ax], n3[ax], tgt, flp);
-    for (int q = 0; q < m; ++q) {
-      int g3[3] = {i, j, k};
-      g3[ax] = tgt[q];
-      double g[5];
+    const int q = ax == 0 ? i : ax == 1 ? j : k, n = ax == 0 ? p.nx : ax == 1 ? p.ny : p.nz;
+    if (q > LAYERS && q <= n - LAYERS) continue;
+    const long long st = ax == 0 ? 1 : ax == 1 ? (long long)L.px : (long long)L.px * L.nyg;
+#pragma unroll 1
+    for (int side = 0; side < 2; ++side) {
+      const int bc = p.bc[2 * ax + side];
+      const bool flip = bc == BC_REFLECTIVE, from_hi = (bc == BC_PERIODIC) != (side != 0);
 #pragma unroll
-      for (int e = 0; e < 5; ++e) g[e] = (flp[q] && e == ax + 1) ? -v[e] : v[e];
-      winds_cell(p, g3[0], g3[1], g3[2], g);
-      float cf[5], w[5];
-      mixed_cell(gm1, g, 1, cf, w);
-      const long long o = L.at(g3[0], g3[1], g3[2]);
+      for (int l = 0; l < LAYERS; ++l) {
+        const int off = bc == BC_OUTFLOW ? 0 : l;  // the cell that layer l copies
+        if (q != (from_hi ? n - off : 1 + off)) continue;
+        T* o = out + c + (long long)((side ? n + 1 + l : -l) - q) * st;
 #pragma unroll
-      for (int e = 0; e < 5; ++e) out[e * L.plane + o] = w[e];
+        for (int e = 0; e < 5; ++e) o[e * L.plane] = (flip && e == ax + 1) ? -v[e] : v[e];
+      }
     }
   }
+}
+
+// Where a wind may reach the cell or its ghost images: the images of v (the
+// value before the winds) with the winds applied at the ghost cells, and v
+// with the winds.  Calls: few tiles come here.
+struct Cons {
+  double u[5];
+};
+static __device__ __noinline__ Cons windy_ghosts(const Params& p, const Layout& L, double* out, int i, int j, int k, Cons v) {
+  write_ghosts(p, L, out, 1, i, j, k, v.u);
+  winds_cell(p, i, j, k, v.u);
+  return v;
+}
+// (stage 1: the images as FP32 primitives of UPP, what stage 2 forms from it)
+static __device__ __noinline__ Cons windy_ghost_prims(const Params& p, const Layout& L, float* out, float gm1, int i, int j,
+                                               int k, Cons v) {
+  ghost_images(p, 2, i, j, k, [&](int ax, bool flip, int gi, int gj, int gk) {
+    double g[5];
+#pragma unroll
+    for (int e = 0; e < 5; ++e) g[e] = (flip && e == ax + 1) ? -v.u[e] : v.u[e];
+    winds_cell(p, gi, gj, gk, g);
+    float cf[5], w[5];
+    mixed_cell(gm1, g, 1, cf, w);
+    const long long o = L.at(gi, gj, gk);
+#pragma unroll
+    for (int e = 0; e < 5; ++e) out[e * L.plane + o] = w[e];
+  });
+  winds_cell(p, i, j, k, v.u);
+  return v;
 }
 
 // The conserved values of a cell from its FP32 primitives: what HLLC takes
@@ -784,15 +799,14 @@ __device__ __forceinline__ void mixed_tile1(const CUtensorMap* tm, const StageAr
       w[4] = fmaxf(__fmul_rn(gm1, __fsub_rn(uf[4], ek)), 1e-20f);
     }
     if (__any_sync(__activemask(), fp64) && fp64) {
-      double up[5];
+      Cons up;
 #pragma unroll
-      for (int e = 0; e < 5; ++e) up[e] = a.uold[e * L.plane + c] - f2d(dU[e]);
-      if (nb) {
-        write_ghost_prims(p, L, a.uppf, gm1, i, j, k, up);  // borders(UPP, 2)
-        winds_cell(p, i, j, k, up);
-      }
+      for (int e = 0; e < 5; ++e) up.u[e] = a.uold[e * L.plane + c] - f2d(dU[e]);
+      const bool windy = ts.windy(k);  // (the tile's)
+      if (nb && windy) up = windy_ghost_prims(p, L, a.uppf, gm1, i, j, k, up);  // borders(UPP, 2)
       float cf[5];
-      mixed_cell(gm1, up, 1, cf, w);
+      mixed_cell(gm1, up.u, 1, cf, w);
+      if (nb && !windy) store_ghosts<2>(p, L, a.uppf, i, j, k, c, w);
     }
 #pragma unroll
     for (int e = 0; e < 5; ++e) a.uppf[e * L.plane + c] = w[e];
@@ -918,14 +932,17 @@ __device__ __forceinline__ void mixed_tile2(const CUtensorMap* tm, const StageAr
 #pragma unroll
         for (int e = 0; e < 5; ++e) un[e] = uc[e] + f2d(lv[e] - dU[e]);
       } else {
-        double up[5];
+        Cons up;
 #pragma unroll
-        for (int e = 0; e < 5; ++e) up[e] = uc[e] - f2d(dU[e]);
-        write_ghosts(p, L, a.out, 1, i, j, k, up);  // borders(UP, 1) with the winds
-        winds_cell(p, i, j, k, up);
+        for (int e = 0; e < 5; ++e) up.u[e] = uc[e] - f2d(dU[e]);
+        // borders(UP, 1), with the winds
+        if (s.tspec.windy(k))
+          up = windy_ghosts(p, L, a.out, i, j, k, up);
+        else
+          store_ghosts<1>(p, L, a.out, i, j, k, c, up.u);
         // step: U = UP + eta * (Laplacian of the old U), from stage 1
 #pragma unroll
-        for (int e = 0; e < 5; ++e) un[e] = up[e] + f2d(lv[e]);
+        for (int e = 0; e < 5; ++e) un[e] = up.u[e] + f2d(lv[e]);
       }
       float cf[5], w[5];
       mixed_cell(gm1, un, 1, cf, w);  // calc_prims(UPrim, U)
