@@ -106,6 +106,43 @@ def test_step_gravity_and_winds_bit_exact(gpu_lib):
     assert_bit_exact(cfg, run, hist, Ug, Wg)
 
 
+def test_step_wind_too_large_for_a_table(gpu_lib):
+    """A wind whose index box (71^3 cells) is beyond the tables' size is
+    evaluated in the stages, one beside it comes from its table."""
+    cfg, U0 = problems.wind_bubble(72, cooling=tlq.COOL_NONE)
+    cfg.winds[0].radius = 33.0 * cfg.dx
+    cfg.winds.append(tlq.Wind(xc=cfg.xr - 1.5 * cfg.dx, yc=0.0, zc=0.0, radius=3.0 * cfg.dx, mdot=cfg.winds[0].mdot,
+                              vinf=5e7, temp=1e4, mu=1.3))
+    run, hist, Ug, Wg = run_both(cfg, U0, 2)
+    assert_bit_exact(cfg, run, hist, Ug, Wg)
+
+
+@pytest.mark.parametrize("precision", [tlq.PREC_FP64, tlq.PREC_MIXED])
+@pytest.mark.parametrize("bc", [BC3, (tlq.BC_OUTFLOW,) * 6, (tlq.BC_REFLECTIVE,) * 6, (tlq.BC_PERIODIC,) * 6])
+@pytest.mark.parametrize("n3", [(19, 13, 11), (16, 8, 9), (2, 2, 2), (33, 3, 4)])
+def test_ghost_images_as_the_general_path(gpu_lib, n3, bc, precision):
+    """The ghost images stored as copies of the cell's values against the
+    general path (each image formed anew, with the winds), which a wind that
+    holds no cell centre but whose index box crosses a face selects: the
+    same bits."""
+    def run(winds):
+        cfg = tlq.Config(nx=n3[0], ny=n3[1], nz=n3[2], xl=0.0, xr=1.0, yl=0.0, yr=0.8, zl=0.0, zr=0.6, bc=bc,
+                         eta=0.01, precision=precision)
+        cfg.winds = winds(cfg)
+        U = smooth_state(cfg, seed=n3[0], mach=1.5)
+        with tlq.Context(cfg) as ctx:
+            ctx.borders(U, 1)
+            ctx.upload(U)
+            hist = [ctx.step() for _ in range(4)]
+            return hist, ctx.state()[0][:, face_ghost_mask(cfg)]
+
+    h0, U0 = run(lambda cfg: [])
+    h1, U1 = run(lambda cfg: [tlq.Wind(xc=cfg.xl, yc=cfg.yl, zc=cfg.zl, radius=1e-3 * cfg.dx, mdot=1.0, vinf=1.0,
+                                       temp=1.0, mu=1.0)])
+    assert h0 == h1
+    np.testing.assert_array_equal(U0, U1)
+
+
 def test_step_plane_wind_bit_exact(gpu_lib):
     """A plane wind (imposePlaneWind, winds.f90:92-147: the top three
     z-planes, every i, j) with a spherical wind and point gravity, as the

@@ -513,7 +513,7 @@ int tlq_destroy(tlq_ctx* ctx) {
   cudaFree(ctx->mlp_cqueue); cudaFree(ctx->mlp_nqueue); cudaFree(ctx->mlp_qcount);
   cudaFree(ctx->clk); cudaFree(ctx->sums_partials); cudaFree(ctx->sums_out);
   cudaFree(ctx->staging);
-  cudaFree(ctx->dT); cudaFree(ctx->dlogT); cudaFree(ctx->dC); cudaFree(ctx->dwinds); cudaFree(ctx->dmasses);
+  cudaFree(ctx->dT); cudaFree(ctx->dlogT); cudaFree(ctx->dC); cudaFree(ctx->dwinds); cudaFree(ctx->dwind_tab); cudaFree(ctx->dmasses);
   cudaFree(ctx->dTf); cudaFree(ctx->dlogTf); cudaFree(ctx->dCf);
   cudaFree(ctx->dslope); cudaFree(ctx->dgcum); cudaFree(ctx->dslopef); cudaFree(ctx->dgcumf);
   for (int q = 0; q < 6; ++q) cudaFree(ctx->rb[q]);
@@ -635,7 +635,9 @@ int tlq_set_plane_winds(tlq_ctx* ctx, const tlq_plane_wind* w, int n) {
 int tlq_set_winds(tlq_ctx* ctx, const tlq_wind* w, int n) {
   if (!ctx || n < 0 || (n > 0 && !w)) return TLQ_ERR_ARG;
   cudaFree(ctx->dwinds);
+  cudaFree(ctx->dwind_tab);
   ctx->dwinds = nullptr;
+  ctx->dwind_tab = nullptr;
   ctx->P.nwinds = 0;
   ctx->P.winds = nullptr;
   if (n > 0) {
@@ -654,6 +656,28 @@ int tlq_set_winds(tlq_ctx* ctx, const tlq_wind* w, int n) {
       d.jlo = std::max(-1, lo(d.yc, d.radius, p.yl, p.dy)); d.jhi = std::min(p.ny + 2, hi(d.yc, d.radius, p.yl, p.dy));
       d.klo = std::max(-1, lo(d.zc, d.radius, p.zl, p.dz)); d.khi = std::min(p.nz + 2, hi(d.zc, d.radius, p.zl, p.dz));
     }
+    // the tables of the winds' cells, until their common size is reached
+    auto tabled = [](const Wind& d) {
+      return d.ihi >= d.ilo && d.jhi >= d.jlo && d.khi >= d.klo &&
+             (long long)(d.ihi - d.ilo + 1) * (d.jhi - d.jlo + 1) * (d.khi - d.klo + 1) <= tlq::WIND_TABLE_CELLS;
+    };
+    long long cells = 0;
+    for (Wind& d : hw) {
+      d.tab = nullptr;
+      if (tabled(d) && cells + d.cells() <= tlq::WIND_TABLE_CELLS) cells += d.cells();
+    }
+    const bool room = cells > 0 && cudaMalloc(&ctx->dwind_tab, 6 * cells * sizeof(double)) == cudaSuccess;
+    if (!room) cudaGetLastError();  // (without tables the stages evaluate the winds)
+    cells = 0;
+    for (Wind& d : hw) {
+      if (!room || !tabled(d) || cells + d.cells() > tlq::WIND_TABLE_CELLS) continue;
+      double* t = ctx->dwind_tab + 6 * cells;
+      CK(ctx->cfg.precision == TLQ_PREC_MIXED ? launch_wind_table_mixed(p, d, t, ctx->stream)
+                                              : launch_wind_table(p, d, t, ctx->stream));
+      d.tab = t;
+      cells += d.cells();
+    }
+    CK(cudaStreamSynchronize(ctx->stream));
     CK(cudaMalloc(&ctx->dwinds, n * sizeof(Wind)));
     CK(cudaMemcpy(ctx->dwinds, hw.data(), n * sizeof(Wind), cudaMemcpyHostToDevice));
     ctx->P.nwinds = n;

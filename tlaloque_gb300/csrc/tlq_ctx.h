@@ -49,6 +49,7 @@ struct tlq_ctx {
   double *dslope = nullptr, *dgcum = nullptr;  // the exact integrator's closed form (CoolTable)
   float *dslopef = nullptr, *dgcumf = nullptr;
   Wind* dwinds = nullptr;
+  double* dwind_tab = nullptr;  // the winds' tables (Wind::tab)
   double* dmasses = nullptr;
   int nmasses = 0;
   std::vector<double> masses_host;

@@ -599,6 +599,16 @@ cudaError_t launch_borders_aos(const Params& p, const Aos& A, double* U, int ord
   if (p.nwinds > 0) k_winds_aos<<<grid_for(A.cells()), BT, 0, s>>>(p, A, U);
   return cudaGetLastError();
 }
+namespace {
+__global__ void __launch_bounds__(BT) k_wind_table(Params p, Wind w, double* tab) {
+  const int q = blockIdx.x * BT + threadIdx.x;
+  if (q < w.cells()) wind_table_cell(p, w, q, tab);
+}
+}  // namespace
+cudaError_t launch_wind_table(const Params& p, const Wind& w, double* tab, cudaStream_t s) {
+  k_wind_table<<<(w.cells() + BT - 1) / BT, BT, 0, s>>>(p, w, tab);
+  return cudaGetLastError();
+}
 cudaError_t launch_winds_aos(const Params& p, const Aos& A, double* U, cudaStream_t s) {
   if (p.nwinds > 0) k_winds_aos<<<grid_for(A.cells()), BT, 0, s>>>(p, A, U);
   return cudaGetLastError();

@@ -74,6 +74,17 @@ __global__ void __launch_bounds__(RED_THREADS) k_init_dt_mixed(Params p, Layout 
   cfl_reduce_finalize<RED_THREADS>(m0, m1, m2, clk, p, false, red, &flag);
 }
 
+namespace {
+__global__ void __launch_bounds__(128) k_wind_table_mixed(Params p, Wind w, double* tab) {
+  const int q = blockIdx.x * 128 + threadIdx.x;
+  if (q < w.cells()) wind_table_cell(p, w, q, tab);
+}
+}  // namespace
+cudaError_t launch_wind_table_mixed(const Params& p, const Wind& w, double* tab, cudaStream_t s) {
+  k_wind_table_mixed<<<(w.cells() + 127) / 128, 128, 0, s>>>(p, w, tab);
+  return cudaGetLastError();
+}
+
 cudaError_t launch_init_dt_mixed(const Params& p, const Layout& L, const double* U, Clock* clk, int nblocks,
                                  cudaStream_t s) {
   k_init_dt_mixed<<<nblocks, RED_THREADS, 0, s>>>(p, L, U, clk);
