@@ -328,54 +328,8 @@ __device__ __forceinline__ void cool_cell_f(const Params& p, float cT, float inv
   cool_cell_known(p, cT, inv_muamu, gm1, w, u4, dt, temp, aloss, seg);
 }
 
-// The face-ghost images (ghost_images) of the interior cell (i, j, k) at c
-// where no wind reaches a ghost cell: its value v, the momentum along the
-// axis negated at a reflective face.  FP32 primitives as well: negating a
-// momentum negates its velocity and leaves the others, so they are what
-// mixed_cell would form of the image.
-//   A tile at an x or y face has such cells in every warp and plane: with
-// each image formed anew from FP64 (winds, mixed_cell) it took twice an
-// interior tile's time in stage 1 and 1.45 times in stage 2 (16-plane chunks,
-// 290 k and 142 k cycles, 340 k and 235 k); now 1.3 and 1.15 times.  Bubble
-// 256^3: stage 1 0.97 -> 0.83 ms, stage 2 1.42 -> 1.34; diagonal Sod 150^3:
-// 0.235 -> 0.198 and 0.281 -> 0.265.  The axes rolled in stage 1 (less code:
-// 3 % on the bubble), unrolled in stage 2 (1 %).
-template <int LAYERS, class T>
-__device__ __forceinline__ void store_ghosts(const Params& p, const Layout& L, T* out, int i, int j, int k,
-                                             long long c, const T* v) {
-#pragma unroll(LAYERS == 2 ? 1 : 3)
-  for (int ax = 0; ax < 3; ++ax) {
-    const int q = ax == 0 ? i : ax == 1 ? j : k, n = ax == 0 ? p.nx : ax == 1 ? p.ny : p.nz;
-    if (q > LAYERS && q <= n - LAYERS) continue;
-    const long long st = ax == 0 ? 1 : ax == 1 ? (long long)L.px : (long long)L.px * L.nyg;
-#pragma unroll 1
-    for (int side = 0; side < 2; ++side) {
-      const int bc = p.bc[2 * ax + side];
-      const bool flip = bc == BC_REFLECTIVE, from_hi = (bc == BC_PERIODIC) != (side != 0);
-#pragma unroll
-      for (int l = 0; l < LAYERS; ++l) {
-        const int off = bc == BC_OUTFLOW ? 0 : l;  // the cell that layer l copies
-        if (q != (from_hi ? n - off : 1 + off)) continue;
-        T* o = out + c + (long long)((side ? n + 1 + l : -l) - q) * st;
-#pragma unroll
-        for (int e = 0; e < 5; ++e) o[e * L.plane] = (flip && e == ax + 1) ? -v[e] : v[e];
-      }
-    }
-  }
-}
-
-// Where a wind may reach the cell or its ghost images: the images of v (the
-// value before the winds) with the winds applied at the ghost cells, and v
-// with the winds.  Calls: few tiles come here.
-struct Cons {
-  double u[5];
-};
-static __device__ __noinline__ Cons windy_ghosts(const Params& p, const Layout& L, double* out, int i, int j, int k, Cons v) {
-  write_ghosts(p, L, out, 1, i, j, k, v.u);
-  winds_cell(p, i, j, k, v.u);
-  return v;
-}
-// (stage 1: the images as FP32 primitives of UPP, what stage 2 forms from it)
+// windy_ghosts of stage 1: the images as FP32 primitives of UPP, what stage 2
+// forms from it.
 static __device__ __noinline__ Cons windy_ghost_prims(const Params& p, const Layout& L, float* out, float gm1, int i, int j,
                                                int k, Cons v) {
   ghost_images(p, 2, i, j, k, [&](int ax, bool flip, int gi, int gj, int gk) {
@@ -937,7 +891,7 @@ __device__ __forceinline__ void mixed_tile2(const CUtensorMap* tm, const StageAr
         for (int e = 0; e < 5; ++e) up.u[e] = uc[e] - f2d(dU[e]);
         // borders(UP, 1), with the winds
         if (s.tspec.windy(k))
-          up = windy_ghosts(p, L, a.out, i, j, k, up);
+          up = windy_ghosts(p, L, a.out, 1, i, j, k, up);
         else
           store_ghosts<1>(p, L, a.out, i, j, k, c, up.u);
         // step: U = UP + eta * (Laplacian of the old U), from stage 1
