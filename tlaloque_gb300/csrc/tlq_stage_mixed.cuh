@@ -118,8 +118,7 @@ static __device__ __noinline__ float kinetic_pressure(float gm1, double r, doubl
 // contract them differently in the kernels that inline this (the stages,
 // the surrogate's passes): every kernel gets the same bits for a cell.
 __device__ __forceinline__ void mixed_cell(float gm1, const double* u, long long vs, float* cf, float* w) {
-#pragma unroll
-  for (int e = 0; e < 5; ++e) cf[e] = d2f(u[e * vs]);
+  d2f5(u, vs, cf);
   const float inv = 1.0f / cf[0];
   w[0] = cf[0];
   w[1] = cf[1] * inv;
