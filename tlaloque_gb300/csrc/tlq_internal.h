@@ -96,9 +96,9 @@ cudaError_t launch_cool_mlp_dt(const Params& p, const Layout& L, double* U0, dou
                                unsigned* nqueue, unsigned* nqcount, cudaStream_t s);
 // The same three passes for several meshes in three launches: fill_cool_job
 // writes one mesh's arguments (cool_job_bytes() of them) into a host array
-// that is copied to the device; mesh m runs on blocks [blk0, blk0 + nblk) of
-// each pass (ranges ascending and back to back from 0, nblk between 1 and
-// cool_pass_blocks, nblocks their total).
+// that is copied to the device; mesh m's blocks of the dt pass are [blk0,
+// blk0 + nblk) (ranges ascending and back to back from 0, nblk between 1 and
+// cool_pass_blocks, nblocks their total and the grid of each pass).
 size_t cool_job_bytes();
 int cool_pass_blocks(const Params& p);
 void fill_cool_job(void* dst, const Params& p, const Layout& L, double* U0, double* U1, long long it_base, Clock* clk,

@@ -35,6 +35,7 @@ struct SurrogateArgs {
 };
 
 constexpr int CT = 128;      // threads per block of the network pass
+constexpr int ST = 512;      // threads per block of the sort pass
 constexpr int FT = 128;      // threads per block of the dt pass
 constexpr int PB = 152 * 3;  // blocks of each pass (at most): one resident wave of the network pass
 
@@ -53,12 +54,12 @@ __device__ __forceinline__ void speeds_max(const float* w, float gf, float& m0, 
   m2 = (v2 != v2 || v2 > m2) ? v2 : m2;
 }
 
-__device__ __forceinline__ long long interior_offset(const Params& p, const Layout& L, long long cidx) {
-  const int i = 1 + (int)(cidx % p.nx);
-  const long long r = cidx / p.nx;
-  const int j = 1 + (int)(r % p.ny);
-  const int k = 1 + (int)(r / p.ny);
-  return L.at(i, j, k);
+// (32-bit divisions: a queue entry is one word; 64-bit ones were a third of a
+// pass's instructions)
+__device__ __forceinline__ long long interior_offset(const Params& p, const Layout& L, unsigned cidx) {
+  const unsigned nx = (unsigned)p.nx, ny = (unsigned)p.ny;
+  const unsigned r = cidx / nx, k = r / ny;
+  return L.at(1 + (int)(cidx - r * nx), 1 + (int)(r - k * ny), 1 + (int)k);
 }
 
 // Pass 1 (sort): stage 2 queued the interior cells that cool (temp >= the
@@ -97,7 +98,7 @@ struct CoolJob {
   unsigned* cqcount;
   unsigned* nqueue;  // cells for the network
   unsigned* nqcount;
-  unsigned blk0, nblk;  // this mesh's blocks of each pass: [blk0, blk0 + nblk)
+  unsigned blk0, nblk;  // this mesh's blocks of the dt pass: [blk0, blk0 + nblk)
 };
 
 // The mesh block b of a pass works on: the job whose block range holds b
@@ -162,15 +163,33 @@ __device__ __forceinline__ void cell_cool(const Params& p, const SurrogateArgs& 
   }
 }
 
-// Warp-aggregated append of cell index v to a queue.
-__device__ __forceinline__ void warp_append(bool take, unsigned v, unsigned* queue, unsigned* count) {
+// Append of cell index v to a queue, one atomic for the block's ST threads
+// (all of them call it).  A warp's own atomic for its 32 cells bounded the
+// sort pass: a mesh's go to one address, 65 k of them for 128^3 cells (batch of
+// eight bubbles: 0.287 ms a step, 0.101 so and with interior_offset in 32 bits).
+struct SmemAppend {
+  unsigned count[ST / 32], base[ST / 32];
+};
+__device__ __forceinline__ void block_append(SmemAppend& s, bool take, unsigned v, unsigned* queue, unsigned* count) {
   const unsigned qm = __ballot_sync(0xffffffffu, take);
-  if (!qm) return;
-  const int lane = threadIdx.x & 31;
-  unsigned basei = 0;
-  if (lane == 0) basei = atomicAdd(count, (unsigned)__popc(qm));
-  basei = __shfl_sync(0xffffffffu, basei, 0);
-  if (take) queue[basei + __popc(qm & ((1u << lane) - 1u))] = v;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (lane == 0) s.count[warp] = (unsigned)__popc(qm);
+  __syncthreads();
+  if (warp == 0) {
+    const unsigned c = lane < ST / 32 ? s.count[lane] : 0u;
+    unsigned sum = c;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned below = __shfl_up_sync(0xffffffffu, sum, o);
+      if (lane >= o) sum += below;
+    }
+    unsigned at = 0u;
+    if (lane == 31 && sum) at = atomicAdd(count, sum);
+    at = __shfl_sync(0xffffffffu, at, 31);
+    if (lane < ST / 32) s.base[lane] = at + sum - c;
+  }
+  __syncthreads();
+  if (take) queue[s.base[warp] + __popc(qm & ((1u << lane) - 1u))] = v;
 }
 
 // The counters of the three outcomes (network, fallback, single step).
@@ -185,21 +204,19 @@ __device__ __forceinline__ void add_counts(const SurrogateArgs& sa, unsigned use
   }
 }
 
-__device__ void cool_sort_mesh(const CoolJob& j, double* red, unsigned nblocks, unsigned bid) {
+// Tiles [first, end) of ST queued cells of one mesh (block-uniform).
+__device__ void cool_sort_mesh(const CoolJob& j, double* red, SmemAppend& app, long long first, long long end) {
   const Params& p = j.p;
   const Layout& L = j.L;
   const Clock* clk = j.clk;
-  if (!(clk->t < clk->tfin)) return;  // the step did not run (mainHD.f90:61)
   const long long n = (long long)*j.cqcount;
-  if ((long long)bid * CT >= n) return;  // no queued cell for this block: nothing to fold
   double* __restrict__ U = step_output(j.U0, j.U1, clk, j.it_base);
   const float gm1 = p.f_gamma - 1.0f, gf = p.f_gamma;
   const float dtf = d2f(clk->dt);
   float m0 = 0.f, m1 = 0.f, m2 = 0.f;
   unsigned fell = 0, one = 0;
-  // warp-uniform trip count (the appends are warp-wide)
-  for (long long base = (long long)bid * CT; base < n; base += (long long)nblocks * CT) {
-    const long long q = base + threadIdx.x;
+  for (long long tile = first; tile < end; ++tile) {
+    const long long q = tile * ST + threadIdx.x;
     const bool valid = q < n;
     long long o = 0;
     unsigned cidx = 0;
@@ -224,12 +241,12 @@ __device__ void cool_sort_mesh(const CoolJob& j, double* red, unsigned nblocks, 
       U[4 * L.plane + o] = u[4];
       speeds_max(c.w, gf, m0, m1, m2);
     }
-    warp_append(net, cidx, j.nqueue, j.nqcount);
+    block_append(app, net, cidx, j.nqueue, j.nqcount);
     fell += ext ? 1 : 0;
     one += single ? 1 : 0;
   }
   add_counts(j.sa, 0, fell, one);
-  cfl_contribute<CT>(m0, m1, m2, j.clk, red);
+  cfl_contribute<ST>(m0, m1, m2, j.clk, red);
 }
 
 // A network cell: the prediction y's change where the residual check accepts
@@ -259,26 +276,23 @@ __device__ __forceinline__ bool cool_net_cell(const Params& p, CellCool& c, doub
   return ok;
 }
 
-__device__ void cool_net_mesh(const CoolJob& j, umma::Smem& S, double* red, unsigned nblocks, unsigned bid) {
+// Tiles [first, end) of 128 queued cells of one mesh (block-uniform).
+__device__ void cool_net_mesh(const CoolJob& j, umma::Smem& S, double* red, long long first, long long end, bool& tc,
+                              uint32_t& phase) {
   const Params& p = j.p;
   const Layout& L = j.L;
   const Clock* clk = j.clk;
   const SurrogateArgs& sa = j.sa;
-  if (!(clk->t < clk->tfin)) return;
   const long long n = (long long)*j.nqcount;
-  if ((long long)bid * CT >= n) return;  // no network cell for this block: no weights, nothing to fold
   double* __restrict__ U = step_output(j.U0, j.U1, clk, j.it_base);
   umma::load_weights(sa.img, S);
-  umma::setup(S);
+  __syncthreads();
   const float gf = p.f_gamma;
   const float dtf = d2f(clk->dt);
   float m0 = 0.f, m1 = 0.f, m2 = 0.f;
   unsigned used = 0, fell = 0;
-  uint32_t phase = 0;
-  bool tc = true;  // the tensor-core path is healthy (block-wide)
-  // block-uniform trip count: one 128-row MMA tile per iteration
-  for (long long base = (long long)bid * CT; base < n; base += (long long)nblocks * CT) {
-    const long long q = base + threadIdx.x;
+  for (long long tile = first; tile < end; ++tile) {
+    const long long q = tile * CT + threadIdx.x;
     const bool valid = q < n;
     long long o = 0;
     unsigned cidx = 0;
@@ -302,32 +316,78 @@ __device__ void cool_net_mesh(const CoolJob& j, umma::Smem& S, double* red, unsi
     used += ok ? 1 : 0;
     fell += (valid && !ok) ? 1 : 0;
   }
-  if (!tc) {
-    // an MMA wait ran out: the cells above took the exact integrator; the
-    // step reports the timeout
-    if (threadIdx.x == 0) atomicOr(&const_cast<Clock*>(clk)->status, ST_TIMEOUT);
-    umma::drain(S, phase);
-  }
-  umma::teardown(S);
+  // an MMA wait ran out: the cells above took the exact integrator; the step
+  // reports the timeout
+  if (!tc && threadIdx.x == 0) atomicOr(&const_cast<Clock*>(clk)->status, ST_TIMEOUT);
   add_counts(sa, used, fell, 0);
   cfl_contribute<CT>(m0, m1, m2, j.clk, red);
 }
 
-// The sort and network passes of njobs meshes, each on its own range of the
-// grid's blocks.
-__global__ void __launch_bounds__(CT) k_cool_sort(const CoolJob* __restrict__ jobs, int njobs) {
-  __shared__ double red[96];
-  __shared__ SmemJob sj;
-  const CoolJob& j = stage_job(sj, job_of_block(jobs, njobs, blockIdx.x));
-  cool_sort_mesh(j, red, j.nblk, blockIdx.x - j.blk0);
+// The meshes' tiles (TILE cells of a queue, its length at *count(job)) end
+// to end, an equal run of them to each block of NT threads: run(job, first,
+// end) for each mesh in this block's run, after begin().  (A mesh whose step
+// does not run, mainHD.f90:61, has empty queues.)  Returns whether the block
+// had any.  On ranges of blocks by the meshes' sizes half of the blocks were
+// idle on average, the queues differing widely: batch of eight bubbles, the
+// network pass 0.79 ms a step, 0.47 so (the sort pass 0.10 both ways).
+template <int NT, int TILE, class Count, class Begin, class Run>
+__device__ __forceinline__ bool for_runs(const CoolJob* __restrict__ jobs, int njobs, SmemJob& sj, Count count,
+                                         Begin begin, Run run) {
+  __shared__ unsigned tiles[NT];
+  __shared__ unsigned long long total;
+  const int tid = threadIdx.x;
+  auto tiles_of = [&](int q) { return q < njobs ? (*count(jobs[q]) + TILE - 1u) / TILE : 0u; };
+  if (tid == 0) total = 0ull;
+  __syncthreads();
+  unsigned mine = 0u;
+  for (int q = tid; q < njobs; q += NT) mine += tiles_of(q);
+  mine = __reduce_add_sync(0xffffffffu, mine);
+  if ((tid & 31) == 0 && mine) atomicAdd(&total, (unsigned long long)mine);
+  __syncthreads();
+  const long long T = (long long)total, B = gridDim.x, b = blockIdx.x;
+  const long long lo = T * b / B, hi = T * (b + 1) / B;  // this block's tiles
+  if (lo == hi) return false;
+  begin();
+  long long at = 0;  // tiles of the meshes before
+  for (int q0 = 0; q0 < njobs && at < hi; q0 += NT) {
+    __syncthreads();
+    tiles[tid] = tiles_of(q0 + tid);
+    __syncthreads();
+    for (int q = q0; q < min(q0 + NT, njobs) && at < hi; ++q) {
+      const long long nt = tiles[q - q0];
+      if (nt && at + nt > lo) {
+        __syncthreads();  // the mesh before is done
+        run(stage_job(sj, &jobs[q]), max(lo - at, 0LL), min(hi - at, nt));
+      }
+      at += nt;
+    }
+  }
+  return true;
 }
 
+// The sort pass of njobs meshes.
+__global__ void __launch_bounds__(ST) k_cool_sort(const CoolJob* __restrict__ jobs, int njobs) {
+  __shared__ double red[96];
+  __shared__ SmemAppend app;
+  __shared__ SmemJob sj;
+  for_runs<ST, ST>(
+      jobs, njobs, sj, [](const CoolJob& j) { return j.cqcount; }, [] {},
+      [&](const CoolJob& j, long long first, long long end) { cool_sort_mesh(j, red, app, first, end); });
+}
+
+// The network pass.
 __global__ void __launch_bounds__(CT, 3) k_cool_net(const CoolJob* __restrict__ jobs, int njobs) {
   __shared__ umma::Smem S;
   __shared__ double red[96];
   __shared__ SmemJob sj;
-  const CoolJob& j = stage_job(sj, job_of_block(jobs, njobs, blockIdx.x));
-  cool_net_mesh(j, S, red, j.nblk, blockIdx.x - j.blk0);
+  bool tc = true;  // the tensor-core path is healthy (block-wide)
+  uint32_t phase = 0;
+  const bool any = for_runs<CT, CT>(
+      jobs, njobs, sj, [](const CoolJob& j) { return j.nqcount; }, [&] { umma::setup(S); },
+      [&](const CoolJob& j, long long first, long long end) { cool_net_mesh(j, S, red, first, end, tc, phase); });
+  if (!any) return;
+  if (!tc) umma::drain(S, phase);
+  umma::teardown(S);
 }
 
 __device__ void cool_dt_mesh(const CoolJob& j, double* red, int* flag, unsigned nblocks) {
@@ -502,7 +562,7 @@ int cool_pass_blocks(const Params& p) { return pass_blocks(p); }
 
 cudaError_t launch_cool_mlp_dt_batch(const void* jobs, int njobs, int nblocks, cudaStream_t s) {
   const CoolJob* d = static_cast<const CoolJob*>(jobs);
-  k_cool_sort<<<nblocks, CT, 0, s>>>(d, njobs);
+  k_cool_sort<<<nblocks, ST, 0, s>>>(d, njobs);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   k_cool_net<<<nblocks, CT, 0, s>>>(d, njobs);
