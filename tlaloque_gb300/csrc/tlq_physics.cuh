@@ -436,16 +436,23 @@ __device__ __forceinline__ void winds_cell(const Params& p, int i, int j, int k,
 // returns the same index as the reference's linear scan on an ascending
 // table); held at the last entry above the table (undefined there in the
 // reference).
+//   10^x as exp10, a third of pow's FP64 operations; the search compares the
+// bits, in the numbers' order, off the FP64 pipe.  Bubble 128^3 FP64: stage 2 3.37 -> 2.99 ms.
+__device__ __forceinline__ long long order_key(double x) {
+  const long long b = __double_as_longlong(x);
+  return b ^ ((b >> 63) & 0x7fffffffffffffffLL);
+}
 __device__ __forceinline__ double cool_coef(const CoolTable& t, double temp) {
   int lo = 1, hi = t.n;  // search i in [1, n-1] (0-based) with T[i] > temp
+  const long long key = order_key(temp);
   while (lo < hi) {
     int mid = (lo + hi) >> 1;
-    if (t.T[mid] > temp) hi = mid; else lo = mid + 1;
+    if (order_key(t.T[mid]) > key) hi = mid; else lo = mid + 1;
   }
-  if (lo >= t.n) return pow(10.0, t.C[t.n - 1]);
+  if (lo >= t.n) return exp10(t.C[t.n - 1]);
   const double T0 = t.logT[lo - 1], C0 = t.C[lo - 1];
   const double T1 = t.logT[lo], C1 = t.C[lo];
-  return pow(10.0, quot(C1 - C0, T1 - T0) * (log10(temp) - T0) + C0);
+  return exp10(quot(C1 - C0, T1 - T0) * (log10(temp) - T0) + C0);
 }
 
 // The exact integrator (COOL_EXACT): the temperature after a step of
