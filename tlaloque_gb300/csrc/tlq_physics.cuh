@@ -9,6 +9,7 @@
 // tlaloque source tree.
 #pragma once
 
+#include <cstring>
 #include <cstdint>
 
 #include "tlq_softfp.cuh"
@@ -47,6 +48,44 @@ constexpr int COOL_NONE = 0, COOL_REF = 1, COOL_SUBCYCLE = 2, COOL_MLP = 3, COOL
 // states); SIGN(1.0, a) with gfortran's default signed-zero semantics.
 template <class R> __host__ __device__ __forceinline__ R mn(R a, R b) { return (b < a) ? b : a; }
 template <class R> __host__ __device__ __forceinline__ R mx(R a, R b) { return (b > a) ? b : a; }
+// Signs of doubles on their bits, off the FP64 pipe (a compare takes one of
+// its slots): the operators' results for every operand.  (Minima and maxima
+// so too: 1 % slower.)
+__host__ __device__ __forceinline__ unsigned bits_hi(double x) {
+#ifdef __CUDA_ARCH__
+  return (unsigned)__double2hiint(x);
+#else
+  unsigned long long b;
+  memcpy(&b, &x, 8);
+  return (unsigned)(b >> 32);
+#endif
+}
+__host__ __device__ __forceinline__ unsigned bits_lo(double x) {
+#ifdef __CUDA_ARCH__
+  return (unsigned)__double2loint(x);
+#else
+  unsigned long long b;
+  memcpy(&b, &x, 8);
+  return (unsigned)b;
+#endif
+}
+// The numbers' order as signed integers (-0 below +0; not for NaNs).
+__host__ __device__ __forceinline__ long long order_key(double x) {
+  const long long b = (long long)((unsigned long long)bits_hi(x) << 32 | bits_lo(x));
+  return b ^ ((b >> 63) & 0x7fffffffffffffffLL);
+}
+__host__ __device__ __forceinline__ bool is_zero(double x) { return ((bits_hi(x) & 0x7fffffffu) | bits_lo(x)) == 0u; }
+// x > 0: the bits in 1 .. infinity's
+__host__ __device__ __forceinline__ bool gt0(double x) {
+  const unsigned h = bits_hi(x), l = bits_lo(x);
+  return (h | l) != 0u && (h < 0x7ff00000u || (h == 0x7ff00000u && l == 0u));
+}
+__host__ __device__ __forceinline__ bool lt0(double x) {
+  const unsigned h = bits_hi(x) ^ 0x80000000u, l = bits_lo(x);
+  return (h | l) != 0u && (h < 0x7ff00000u || (h == 0x7ff00000u && l == 0u));
+}
+__host__ __device__ __forceinline__ bool ge0(double x) { return is_zero(x) || gt0(x); }
+__host__ __device__ __forceinline__ bool le0(double x) { return is_zero(x) || lt0(x); }
 __device__ __forceinline__ double sgn1(double a) { return copysign(1.0, a); }
 __device__ __forceinline__ float sgn1(float a) { return copysignf(1.0f, a); }
 
@@ -180,7 +219,7 @@ __device__ __forceinline__ R average(R a, R b, int opt) {
         return __fdividef(xy * (x + y), fmaf(x, x, y * y)) * __uint_as_float(eb);
       } else {
         const R ab = prod(a, b);
-        if (ab <= R(0.0)) return R(0.0);
+        if (le0(ab)) return R(0.0);
         return quot(prod(ab, a + b), prod(a, a) + prod(b, b));
       }
     case LIM_MINMOD:
@@ -438,10 +477,6 @@ __device__ __forceinline__ void winds_cell(const Params& p, int i, int j, int k,
 // reference).
 //   10^x as exp10, a third of pow's FP64 operations; the search compares the
 // bits, in the numbers' order, off the FP64 pipe.  Bubble 128^3 FP64: stage 2 3.37 -> 2.99 ms.
-__device__ __forceinline__ long long order_key(double x) {
-  const long long b = __double_as_longlong(x);
-  return b ^ ((b >> 63) & 0x7fffffffffffffffLL);
-}
 __device__ __forceinline__ double cool_coef(const CoolTable& t, double temp) {
   int lo = 1, hi = t.n;  // search i in [1, n-1] (0-based) with T[i] > temp
   const long long key = order_key(temp);

@@ -213,8 +213,8 @@ __device__ __forceinline__ void face_flux(const Params& p, double* ff, const dou
   const double sr = mx(ul + cl, ur + cr);
   const double ml = prod(wl[0], ul), mr = prod(wr[0], ur);
   if (SOLV == SOLVER_HLL || (SOLV < 0 && p.solver == SOLVER_HLL)) {
-    if (sl >= 0.0 || sr <= 0.0) {
-      const bool left = sl >= 0.0;
+    if (ge0(sl) || le0(sr)) {
+      const bool left = ge0(sl);
       double w[5];
 #pragma unroll
       for (int e = 0; e < 5; ++e) w[e] = left ? wl[e] : wr[e];
@@ -237,10 +237,10 @@ __device__ __forceinline__ void face_flux(const Params& p, double* ff, const dou
   // Branch order of the reference: sl>=0, sr<=0, sst>=0, sst<=0; a face with
   // NaN speeds takes none (NaN here)
   bool star, left;
-  if (sl >= 0.0) { star = false; left = true; }
-  else if (sr <= 0.0) { star = false; left = false; }
-  else if (sst >= 0.0) { star = true; left = true; }
-  else if (sst <= 0.0) { star = true; left = false; }
+  if (ge0(sl)) { star = false; left = true; }
+  else if (le0(sr)) { star = false; left = false; }
+  else if (ge0(sst)) { star = true; left = true; }
+  else if (le0(sst)) { star = true; left = false; }
   else {
 #pragma unroll
     for (int e = 0; e < 5; ++e) ff[e] = NAN;
@@ -282,12 +282,13 @@ __device__ __forceinline__ void face_flux(const Params& p, double* ff, const dou
 // cell's left x, lower y and upper z face, one warp in turn the tile's right
 // and upper edges -- through one copy of the code, then the cells' update.
 // The z flux stays in its thread.
-//   Measured, Sedov 128^3, 8-plane chunks: stage 1 2.90 -> 1.02 ms, stage 2
-// 5.09 -> 2.12 ms per launch against one face task list with the limiter and
+//   Measured, Sedov 128^3, 8-plane chunks: stage 1 2.90 -> 0.98 ms, stage 2
+// 5.09 -> 1.90 ms per launch against one face task list with the limiter and
 // sound speeds per face and hardware divisions (1.44 and 2.80 ms with those
-// off the FP64 pipe).  Now 159 FP64 operations per cell in stage 1 and 365 in
-// stage 2 at 75-80 % of that pipe's rate, beside 5,400 and 9,300 integer and
-// other instructions per warp of cells.  Which multiplications go to the
+// off the FP64 pipe; 1.01 and 2.08 before the sign tests moved to the bits
+// and the z differences were carried).  The FP64 pipe's counter: 197
+// instructions a cell in stage 1 and 407 in stage 2 before those two, at 70-73
+// % of its rate, in a quarter of the issue slots.  Which multiplications go to the
 // integer pipe is measured too: all of them, or none, is 3-12 % slower than
 // the star state's, the wave speeds', the limiter's and the update's.
 template <int STAGE, int LIM, int SOLV>
@@ -385,6 +386,7 @@ __global__ void __launch_bounds__(NT, STAGE == 1 ? 4 : 3)
   // the column's primitives of plane k and k+1, its slope of plane k in z
   // (stage 2) and its lower z flux
   double w0[NP], w1[NP], sz[5], fz[5];
+  double dz[5];  // w1 - w0 (stage 2)
 #pragma unroll
   for (int e = 0; e < 5; ++e) sz[e] = fz[e] = 0.0;
   bool aborted = false;
@@ -397,6 +399,10 @@ __global__ void __launch_bounds__(NT, STAGE == 1 ? 4 : 3)
   if (STAGE == 1) {
 #pragma unroll
     for (int e = 0; e < NP; ++e) w0[e] = w1[e];
+  }
+  if (STAGE == 2) {
+#pragma unroll
+    for (int e = 0; e < 5; ++e) dz[e] = w1[e] - w0[e];
   }
   unsigned long long m0 = 0ull, m1 = 0ull, m2 = 0ull;  // CFL maxima as max_key keys (STAGE 2)
 
@@ -443,8 +449,9 @@ __global__ void __launch_bounds__(NT, STAGE == 1 ? 4 : 3)
         if (r == 3) {
 #pragma unroll
           for (int e = 0; e < 5; ++e) {
-            dm[e] = w1[e] - w0[e];
+            dm[e] = dz[e];
             dp[e] = w2[e] - w1[e];
+            dz[e] = dp[e];
           }
         } else {
           // the own cell's x, its y, and the cells beside the tile (48 tasks,
@@ -590,14 +597,14 @@ __global__ void __launch_bounds__(NT, STAGE == 1 ? 4 : 3)
 #pragma unroll
         for (int e = 0; e < 5; ++e) {
           const double* uo = a.uold + e * L.plane + c;
-          un[e] = up[e] + prod(p.eta, uo[1] + uo[-1] + uo[L.px] + uo[-L.px] + uo[pxy] + uo[-pxy] - 6.0 * uc[e]);
+          un[e] = up[e] + prod(p.eta, uo[1] + uo[-1] + uo[L.px] + uo[-L.px] + uo[pxy] + uo[-pxy] - prod(6.0, uc[e]));
         }
         cons2prim(p.gamma, un, w);  // calc_prims(UPrim, U)
         if (p.cooling != COOL_NONE) {
           cool_cell(p, w, un[4], dtstep);
           a.pout[c] = w[4];
         }
-        if (!(un[0] > 0.0)) atomicOr(&clk->status, ST_NEG_DENSITY);
+        if (!gt0(un[0])) atomicOr(&clk->status, ST_NEG_DENSITY);
 #pragma unroll
         for (int e = 0; e < 5; ++e) a.out[e * L.plane + c] = un[e];
         double v3[3];
