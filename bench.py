@@ -67,17 +67,19 @@ FP64_OPS_PER_ZONE = {
 }
 
 
-def fp64_pipe_bound(ops: dict, rate: dict) -> dict:
-    """The plain FP64 step's compute roofline from the op counts and the FP64
-    pipe's measured rates (tlq_measure_fp64_rate): every add, multiply and
-    comparison takes one FMA slot (the FP64 kernels are built without
-    contraction), an IEEE division or square root the FMA-slot cost measured
-    for it; zone-updates/s at a fully busy pipe = FMA rate / slots."""
-    div_cost = rate["fma_per_s"] / rate["div_per_s"]
-    sqrt_cost = rate["fma_per_s"] / rate["sqrt_per_s"]
-    slots = ops["add"] + ops["mul"] + ops["cmp"] + ops["div"] * div_cost + ops["sqrt"] * sqrt_cost
-    return {"fma_slots_per_zone": slots, "div_fma_slots": div_cost, "sqrt_fma_slots": sqrt_cost,
-            "zone_updates_per_s_bound": rate["fma_per_s"] / slots}
+# Warp instructions x 32 per zone-update that the plain step's two kernels
+# issue to the FP64 pipe (ncu: smsp__inst_executed_pipe_fp64.sum of
+# stage_kernel<1> and <2>).  Divisions, square roots and part of the
+# multiplications run on the integer pipe, and what cells share is formed
+# once, so this is below the operation counts above.
+FP64_PIPE_INST_PER_ZONE = {"wind256": 204.1 + 485.4, "sedov128": 186.2 + 351.3}
+
+
+def fp64_pipe_bound(inst: float, rate: dict) -> dict:
+    """The plain FP64 step's compute roofline: zone-updates/s with the FP64
+    pipe busy all the time with the step's own instructions, at the pipe's
+    measured FMA rate (tlq_measure_fp64_rate)."""
+    return {"fp64_pipe_inst_per_zone": inst, "zone_updates_per_s_bound": rate["fma_per_s"] / inst}
 
 
 def load_peaks():
@@ -574,10 +576,10 @@ def main():
     forms["fp64"]["roofline"] = {
         "hbm_achieved_gbs": bpz64["step"] * f64["value"] / 1e9,
         "hbm_frac": bpz64["step"] * f64["value"] / 1e9 / peak}
-    ops = FP64_OPS_PER_ZONE.get(args.workload)
-    if ops:
+    ops, inst = FP64_OPS_PER_ZONE.get(args.workload), FP64_PIPE_INST_PER_ZONE.get(args.workload)
+    if ops and inst:
         rate = tlq.measure_fp64_rate(local)
-        b = fp64_pipe_bound(ops, rate)
+        b = fp64_pipe_bound(inst, rate)
         forms["fp64"]["roofline"].update({
             "bound": "fp64 pipe", "fp64_ops_per_zone": ops,
             "fp64_rate_measured": {**rate, "how": "tlq_measure_fp64_rate: independent FMA / IEEE divide / IEEE "
