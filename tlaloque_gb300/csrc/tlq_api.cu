@@ -327,7 +327,7 @@ int read_clock(tlq_ctx* ctx) {
 // last wave is half empty on average: cost = (z + prologue) (1 + waves), a
 // wave that is not full adding 0.65 of its share in the mixed form.  Fitted to
 // sweeps of 24^3..300^3 meshes in both forms: the choice is within 6 % of
-// the sweep's best (mixed bubble 48^3: 0.066 ms a step, 0.43 with 32-plane
+// the sweep's best (with the stages of that time: mixed bubble 48^3: 0.066 ms a step, 0.43 with 32-plane
 // chunks; 128^3 0.43 and 1.03; plain Sod tube 256x4x4 0.12 and 0.33, Sedov
 // 128^3 3.1 and 4.1 with 64-plane chunks).
 int rule_zlen(const int* tiles, const int* nz, int n, bool mixed) {
