@@ -4,7 +4,8 @@
 // In the step, stage 2 cools the cells the exact integrator takes in one
 // step and leaves the other cells that cool (temp >= the table's first
 // temperature, cooling.f90:71) and the CFL reduction to three passes
-// (k_cool_sort, k_cool_net, k_cool_dt): for a cell inside the training box
+// (k_cool_sort, k_cool_net, k_cool_dt; one launch, k_cool_all, for a single
+// mesh): for a cell inside the training box
 // the network predicts r with ln(T/T_new) = tau (1 + tau r) from
 // (log10 n, log10 T, log10 tau); the prediction is accepted when
 // |T_pred - T_ex| <= tol T, T_ex the exact integrator's temperature (the
