@@ -34,6 +34,9 @@ struct tlq_ctx {
   int* mg_go = nullptr;       // pinned: whether the cycle after an enqueued one runs, by its parity
   cudaEvent_t mg_seen[2] = {};
   void* mg_coarse = nullptr;  // the one-block levels' schedule
+  // [plane or pipe][with the change's sum][log2 cells]: whether that relax's
+  // blocks are all resident on the device (0: not asked yet, 1, -1)
+  signed char mg_fit[2][2][12] = {};
   cudaStream_t mg_body = nullptr;  // captures a V-cycle into a graph's loop body
   double* phig = nullptr;
   double* phit = nullptr;

@@ -1241,79 +1241,73 @@ void launch_half(const MgCtl* c, const MgLevel& lv, int half, double* part, cuda
   }
 }
 
-// Whether a level's relax runs as one cooperative launch: every plane's
-// block resident at once (checked with the occupancy calculator, once per
-// level size; levels of at most 256 cells), unless TLQ_MG_PIPELINE=0 asks
-// for the per-half-sweep kernels.
-template <int NT, int MINB, int HG, int G, int CH, bool TRACK>
-bool pipe_fits(int n, int nt) {
-  static int cached[2048] = {0};  // 0 unknown, 1 fits, 2 does not
-  if (n >= 2048) return false;
-  if (!cached[n]) {
-    int dev = 0, sms = 0, per = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_mg_relax_pipe<NT, MINB, HG, G, CH, TRACK>, nt, pipe_smem(n));
-    cached[n] = (long long)per * sms >= n ? 1 : 2;
-  }
-  return cached[n] == 1;
+int log2i(int n) {
+  int l = 0;
+  while ((1 << l) < n) ++l;
+  return l;
 }
 
-template <int NT, int MINB, int HG, int G, int CH, bool TRACK>
-bool launch_pipe(MgCtl* c, const MgLevel& lv, double* part, cudaStream_t s) {
-  const int nt = (lv.n * HG + 31) / 32 * 32;
-  if (!pipe_fits<NT, MINB, HG, G, CH, TRACK>(lv.n, nt)) return false;
-  k_mg_prog_reset<<<1, 256, 0, s>>>(c, lv.n);
+// Whether a level's relax runs as one cooperative launch: every plane's
+// block resident at once (checked with the occupancy calculator, once per
+// context, level size and kernel: the answer, and the shared memory a kernel
+// may use, belong to the context's device; levels of at most 256 cells),
+// unless TLQ_MG_PIPELINE=0 asks for the per-half-sweep kernels.
+bool resident(signed char* fit, const void* kernel, int n, int threads, size_t smem) {
+  if (!*fit) {
+    int dev = 0, sms = 0, per = 0;
+    bool ok = cudaGetDevice(&dev) == cudaSuccess &&
+              cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess;
+    ok = ok && cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess;
+    ok = ok && cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, threads, smem) == cudaSuccess;
+    if (!ok) cudaGetLastError();
+    *fit = (ok && (long long)per * sms >= n) ? 1 : -1;
+  }
+  return *fit > 0;
+}
+
+// A relax's cooperative launch; false (and no error left behind) if refused.
+template <class Kernel, class... Args>
+bool launch_resident(Kernel kernel, int n, int threads, size_t smem, cudaStream_t s, Args... args) {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(lv.n);
-  cfg.blockDim = dim3(nt);
-  cfg.dynamicSmemBytes = pipe_smem(lv.n);
+  cfg.gridDim = dim3(n);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeCooperative;
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, k_mg_relax_pipe<NT, MINB, HG, G, CH, TRACK>, c, lv, part) == cudaSuccess;
+  if (cudaLaunchKernelEx(&cfg, kernel, args...) == cudaSuccess) return true;
+  cudaGetLastError();
+  return false;
+}
+
+template <int NT, int MINB, int HG, int G, int CH, bool TRACK>
+bool launch_pipe(tlq_ctx* ctx, MgCtl* c, const MgLevel& lv, double* part, cudaStream_t s) {
+  const int nt = (lv.n * HG + 31) / 32 * 32;
+  const auto kernel = k_mg_relax_pipe<NT, MINB, HG, G, CH, TRACK>;
+  if (!resident(&ctx->mg_fit[1][TRACK][log2i(lv.n)], (const void*)kernel, lv.n, nt, pipe_smem(lv.n))) return false;
+  k_mg_prog_reset<<<1, 256, 0, s>>>(c, lv.n);
+  return launch_resident(kernel, lv.n, nt, pipe_smem(lv.n), s, c, lv, part);
 }
 
 // The shared-memory-plane relax: one block per plane, all resident at once.
 template <int N, bool TRACK>
-bool launch_plane(MgCtl* c, const MgLevel& lv, int leg, double* part, cudaStream_t s) {
+bool launch_plane(tlq_ctx* ctx, MgCtl* c, const MgLevel& lv, int leg, double* part, cudaStream_t s) {
   using G = PlaneGeo<N>;
-  static int state = 0;  // 0 unknown, 1 fits, 2 does not
-  if (!state) {
-    int dev = 0, sms = 0, per = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    bool ok = cudaFuncSetAttribute(k_mg_relax_plane<N, TRACK>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)G::smem) == cudaSuccess;
-    ok = ok && cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_mg_relax_plane<N, TRACK>, G::NT + G::NH, G::smem) ==
-                   cudaSuccess;
-    if (!ok) cudaGetLastError();
-    state = (ok && (long long)per * sms >= N) ? 1 : 2;
-  }
-  if (state != 1 || !lv.X) return false;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(N);
-  cfg.blockDim = dim3(G::NT + G::NH);
-  cfg.dynamicSmemBytes = G::smem;
-  cfg.stream = s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeCooperative;
-  attr[0].val.cooperative = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, k_mg_relax_plane<N, TRACK>, c, lv, leg, part) == cudaSuccess;
+  const auto kernel = k_mg_relax_plane<N, TRACK>;
+  if (!lv.X || !resident(&ctx->mg_fit[0][TRACK][log2i(N)], (const void*)kernel, N, G::NT + G::NH, G::smem)) return false;
+  return launch_resident(kernel, N, G::NT + G::NH, G::smem, s, c, lv, leg, part);
 }
 
 template <bool TRACK>
-bool launch_plane_any(MgCtl* c, const MgLevel& lv, int leg, double* part, cudaStream_t s) {
+bool launch_plane_any(tlq_ctx* ctx, MgCtl* c, const MgLevel& lv, int leg, double* part, cudaStream_t s) {
   switch (lv.n) {
-    case 16: return launch_plane<16, TRACK>(c, lv, leg, part, s);
-    case 32: return launch_plane<32, TRACK>(c, lv, leg, part, s);
-    case 64: return launch_plane<64, TRACK>(c, lv, leg, part, s);
-    case 128: return launch_plane<128, TRACK>(c, lv, leg, part, s);
+    case 16: return launch_plane<16, TRACK>(ctx, c, lv, leg, part, s);
+    case 32: return launch_plane<32, TRACK>(ctx, c, lv, leg, part, s);
+    case 64: return launch_plane<64, TRACK>(ctx, c, lv, leg, part, s);
+    case 128: return launch_plane<128, TRACK>(ctx, c, lv, leg, part, s);
     default: return false;
   }
 }
@@ -1328,25 +1322,25 @@ bool launch_plane_any(MgCtl* c, const MgLevel& lv, int leg, double* part, cudaSt
 // on 16 (a relax takes 2n + 9 (CH + 1) steps); 256-cell levels need two
 // blocks per SM: 2 x 256, checks every 4 steps.
 template <bool TRACK>
-bool launch_pipe_any(MgCtl* c, const MgLevel& lv, int leg, double* part, cudaStream_t s) {
+bool launch_pipe_any(tlq_ctx* ctx, MgCtl* c, const MgLevel& lv, int leg, double* part, cudaStream_t s) {
   const char* env = std::getenv("TLQ_MG_PLANE");
   const bool plane = !(env && env[0] == '0');
-  if (plane && launch_plane_any<TRACK>(c, lv, leg, part, s)) return true;
+  if (plane && launch_plane_any<TRACK>(ctx, c, lv, leg, part, s)) return true;
   switch (lv.n) {
-    case 16: return launch_pipe<160, 1, 10, 1, 2, TRACK>(c, lv, part, s);
-    case 32: return launch_pipe<320, 1, 10, 1, 4, TRACK>(c, lv, part, s);
-    case 64: return launch_pipe<640, 1, 10, 1, 8, TRACK>(c, lv, part, s);
-    case 128: return launch_pipe<640, 1, 5, 1, 8, TRACK>(c, lv, part, s);
-    case 256: return launch_pipe<512, 2, 2, 1, 4, TRACK>(c, lv, part, s);
+    case 16: return launch_pipe<160, 1, 10, 1, 2, TRACK>(ctx, c, lv, part, s);
+    case 32: return launch_pipe<320, 1, 10, 1, 4, TRACK>(ctx, c, lv, part, s);
+    case 64: return launch_pipe<640, 1, 10, 1, 8, TRACK>(ctx, c, lv, part, s);
+    case 128: return launch_pipe<640, 1, 5, 1, 8, TRACK>(ctx, c, lv, part, s);
+    case 256: return launch_pipe<512, 2, 2, 1, 4, TRACK>(ctx, c, lv, part, s);
     default: return false;
   }
 }
 
 // leg: 0 on the way down, 1 on the way up.
-void launch_relax(MgCtl* c, const MgLevel& lv, int leg, double* part, cudaStream_t s) {
+void launch_relax(tlq_ctx* ctx, MgCtl* c, const MgLevel& lv, int leg, double* part, cudaStream_t s) {
   const char* env = std::getenv("TLQ_MG_PIPELINE");
   const bool pipe = !(env && env[0] == '0');
-  if (pipe && (part ? launch_pipe_any<true>(c, lv, leg, part, s) : launch_pipe_any<false>(c, lv, leg, part, s))) return;
+  if (pipe && (part ? launch_pipe_any<true>(ctx, c, lv, leg, part, s) : launch_pipe_any<false>(ctx, c, lv, leg, part, s))) return;
   for (int h = 0; h < 10; ++h) launch_half(c, lv, h & 1, (part && h >= 8) ? part + (h - 8) * lv.n : nullptr, s);
 }
 
@@ -1364,9 +1358,7 @@ int grid_for(long long work, int threads) {
 // block partials.
 int mg_levels_of(const tlq_config& c) {
   if (c.nx != c.ny || c.nx != c.nz || c.nx < 2 || (c.nx & (c.nx - 1))) return -1;
-  int L = 0;
-  while ((1 << L) < c.nx) ++L;
-  return L;
+  return log2i(c.nx);
 }
 
 cudaError_t mg_alloc(tlq_ctx* ctx) {
@@ -1542,7 +1534,7 @@ cudaError_t enqueue_mg(tlq_ctx* ctx, Dens rho, const Clock* clk, double* phit, c
     }
     // down: level 0 .. lc-1 on the large kernels
     for (int l = 0; l < lc; ++l) {
-      launch_relax(c, v.lv[l], 0, nullptr, st);
+      launch_relax(ctx, c, v.lv[l], 0, nullptr, st);
       const int nc = v.lv[l + 1].n, nt = blocks(nc);
       k_mg_resid_restrict<<<(nc * nc * nc + nt - 1) / nt, nt, 0, st>>>(c, v.lv[l], v.lv[l + 1]);
     }
@@ -1553,7 +1545,7 @@ cudaError_t enqueue_mg(tlq_ctx* ctx, Dens rho, const Clock* clk, double* phit, c
       const int nc = v.lv[l + 1].n, nt = blocks(nc);
       k_mg_prolong_add<<<(nc * nc * nc + nt - 1) / nt, nt, 0, st>>>(c, v.lv[l + 1], v.lv[l], l > 0);
       // the last pass of the level-0 relax forms Dif (sources.f90:465-471)
-      launch_relax(c, v.lv[l], 1, l == 0 ? part : nullptr, st);
+      launch_relax(ctx, c, v.lv[l], 1, l == 0 ? part : nullptr, st);
     }
     k_mg_cycle_end<<<1, 32, 0, st>>>(c, 2 * n, loop, h);
   };
