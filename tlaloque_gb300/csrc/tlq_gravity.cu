@@ -44,6 +44,7 @@
 
 #include "tlq_convert.cuh"
 #include "tlq_ctx.h"
+#include "tlq_mg_wait.cuh"
 
 namespace tlq {
 namespace {
@@ -55,11 +56,6 @@ constexpr int MG_PF = 4;            // diagonal steps the smoother's loads run a
 constexpr int MG_MOM_THREADS = 256;
 constexpr int MG_MOM_BLOCKS = 152 * 2;
 constexpr int MG_SOLVE_LIMIT = 100000;  // coarsest-level Gauss-Seidel passes before giving up
-// Polls of a neighbour's progress before a pipelined relax gives up (~1 s);
-// TLQ_MG_WAIT_LIMIT in the environment of tlq_create overrides it (a short
-// limit lets a test make the wait run out and check the error status).
-constexpr long long MG_WAIT_LIMIT = 1LL << 24;
-
 struct MgLevel {
   int n;
   double* E;
@@ -513,12 +509,11 @@ __device__ bool mg_wait(MgCtl* c, int k, int n, int need, int* s_ok) {
   if (threadIdx.x == 0) {
     int ok = 1;
     volatile int* prog = c->prog;
-    volatile int* abort = &c->abort;
     for (int nb = k - 1; nb <= k + 1 && ok; nb += 2) {
       if (nb < 1 || nb > n) continue;
-      long long tries = 0;
+      MgWait wait;
       while (prog[nb] < need) {
-        if (*abort || ++tries > c->wait_limit) {
+        if (wait.out(c)) {
           ok = 0;
           break;
         }
@@ -894,9 +889,9 @@ __global__ void __launch_bounds__(PlaneGeo<N>::NT + PlaneGeo<N>::NH, 1)
         const unsigned hs = cell[w].x >> 16, prev = hs == 0u ? MG_INITIAL : hs - 1u;
         const unsigned long long wu = seq | (top ? MG_INITIAL : prev), wd = seq | (bottom ? MG_INITIAL : prev);
         const Tagged* x = X + (cell[w].y & 0xffffu);
-        long long tries = 0;
+        MgWait wait;
         while (tagged_tag(ru[w]) != wu || tagged_tag(rd[w]) != wd) {
-          if (++tries > c->wait_limit || *(volatile int*)&c->abort) {
+          if (wait.out(c)) {
             *gave_up = 1;
             atomicOr(&c->status, MG_ST_TIMEOUT);
             atomicExch(&c->abort, 1);
