@@ -274,15 +274,18 @@ int tlq_output(tlq_ctx* ctx, int format, const char* outputpath, int nout, int r
 int tlq_output_wait(tlq_ctx* ctx);
 
 /* Stage tiling (no counterpart in the reference): the z-chunk length of the
- * stage grid (>= 8 planes, or nz; the default follows from a cost model of the
- * mesh's tiles and the resident blocks; a mesh too small to fill the GPU with
- * chunks of 8 planes runs shorter ones whatever the choice; results do not
- * depend on it), and the measuring autotuner that picks it -- from the cache file
- * (JSON keyed by GPU name, mesh size and form; NULL = no cache) or timed now
- * over `steps` steps per candidate (8, 16, 32, 64, 128) from the current
- * state, which is restored afterwards. */
+ * stage grid (>= 8 planes, or nz).  A length that is set runs as it is.  The
+ * default follows from a cost model of the mesh's tiles and the resident
+ * blocks; a mesh too small to fill the GPU with chunks of 8 planes runs shorter
+ * ones by default (tlq_get_tiling then gives 8, or nz; tlq_running_tiling the
+ * length that runs).  Results do not depend on it.  The measuring autotuner
+ * picks it -- from the cache file (JSON keyed by GPU name, mesh size and form,
+ * "zlen" 0 for the default; NULL = no cache) or timed now over `steps` steps
+ * per candidate (the default, 8, 16, 32, 64, 128) from the current state, which
+ * is restored afterwards. */
 int tlq_set_tiling(tlq_ctx* ctx, int zlen);
 int tlq_get_tiling(const tlq_ctx* ctx, int* zlen);
+int tlq_running_tiling(const tlq_ctx* ctx, int* zlen);
 int tlq_autotune(tlq_ctx* ctx, const char* cache_path, int steps, int* chosen);
 
 /* ---- Batched ensemble (no counterpart in the reference, which runs one mesh
@@ -312,10 +315,11 @@ int tlq_batch_create(const tlq_config* cfgs, int nmembers, tlq_batch** out);
 int tlq_batch_destroy(tlq_batch* b);
 int tlq_batch_size(const tlq_batch* b);
 tlq_ctx* tlq_batch_member(tlq_batch* b, int i);
-/* z-chunk length (planes per tile, >= 8) of member i; the default by the same
- * model over all members' tiles. */
+/* z-chunk length (planes per tile, >= 8) of member i, and the one that runs;
+ * the default by the same model over all members' tiles. */
 int tlq_batch_set_tiling(tlq_batch* b, int i, int zlen);
 int tlq_batch_get_tiling(const tlq_batch* b, int i, int* zlen);
+int tlq_batch_running_tiling(tlq_batch* b, int i, int* zlen);
 /* Autotuner: per distinct mesh size, the z-chunk length from the cache file
  * (JSON, keyed by GPU name and size; NULL = no cache) or measured now over
  * `steps` steps from the members' current state (restored afterwards);

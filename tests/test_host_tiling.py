@@ -1,0 +1,118 @@
+"""The z-chunk length: a length that is set is the one that runs, the default
+is split for meshes too small to fill the GPU, and the autotuners try the
+default beside the lengths.  Host side only, on a fake CUDA runtime whose
+launches take a time set per number of blocks."""
+import json
+
+import numpy as np
+import pytest
+
+from tests import fakecuda
+from tlaloque_gb300 import problems, tlq
+
+
+@pytest.fixture(scope="module")
+def fake_lib(tmp_path_factory):
+    return fakecuda.link(tmp_path_factory.mktemp("fakecuda"))
+
+
+def config(shape, precision=tlq.PREC_FP64):
+    nx, ny, nz = shape
+    return tlq.Config(nx=nx, ny=ny, nz=nz, precision=precision)
+
+
+def uploaded(cfg):
+    ctx = tlq.Context(cfg)
+    ctx.upload(np.ones(cfg.shape, order="F"))
+    return ctx
+
+
+def chunks(fake, ctx):
+    """The z extent of the two stages' grids in one step."""
+    fake.lib.fake_reset()
+    ctx.advance(1)
+    z = {g[2] for k, g, _ in fake.launches("stage_kernel")}
+    assert len(z) == 1 and len(fake.launches("stage_kernel")) == 2
+    return z.pop()
+
+
+@pytest.mark.parametrize("precision", [tlq.PREC_FP64, tlq.PREC_MIXED])
+@pytest.mark.parametrize("shape", [(16, 8, 9), (33, 20, 25), (48, 48, 48), (64, 64, 70), (150, 150, 150)])
+def test_a_length_that_is_set_runs(fake_lib, shape, precision):
+    nz = shape[2]
+    with fakecuda.loaded(fake_lib) as fake:
+        ctx = uploaded(config(shape, precision))
+        run = ctx.running_tiling()
+        assert chunks(fake, ctx) == -(-nz // run)
+        assert ctx.tiling() >= run and ctx.tiling() >= min(8, nz)
+        assert run < 8 or shape[0] >= 100
+        for z in (8, 16, nz, nz + 5):
+            ctx.set_tiling(z)
+            assert ctx.tiling() == ctx.running_tiling() == min(z, nz)
+            assert chunks(fake, ctx) == -(-nz // min(z, nz))
+        for z in (-1, 0, 1, 7):
+            with pytest.raises(tlq.TlqError):
+                ctx.set_tiling(z)
+        ctx.close()
+
+
+def blocks(shape, z):
+    return -(-shape[0] // 16) * -(-shape[1] // 8) * -(-shape[2] // z)
+
+
+@pytest.mark.parametrize("shape", [(48, 48, 48), (150, 150, 150)])
+@pytest.mark.parametrize("winner", ["default", 8, 16, 32])
+def test_autotune_tries_the_default(fake_lib, tmp_path, shape, winner):
+    cache = str(tmp_path / "tune.json")
+    with fakecuda.loaded(fake_lib) as fake:
+        ctx = uploaded(config(shape, tlq.PREC_MIXED))
+        default, nominal = ctx.running_tiling(), ctx.tiling()
+        run = default if winner == "default" else winner
+        ctx.set_tiling(shape[2])  # (not where the tuner starts from)
+        fake.set_cost(blocks(shape, run), 0.25)
+        got = ctx.autotune(cache, steps=2)
+        assert ctx.running_tiling() == run
+        assert got == ctx.tiling() == (nominal if winner == "default" else winner)
+        (entry,) = json.load(open(cache))["tuned"].values()
+        assert entry["zlen"] == (0 if winner == "default" else winner)
+        ctx.close()
+        ctx = uploaded(config(shape, tlq.PREC_MIXED))
+        fake.lib.fake_reset()
+        assert ctx.autotune(cache, steps=2) == got and ctx.running_tiling() == run
+        assert not fake.launches("stage_kernel")  # (from the cache)
+        ctx.close()
+
+
+@pytest.mark.parametrize("winner", ["default", 8, 16])
+def test_batch_autotune_tries_the_default(fake_lib, tmp_path, winner):
+    cache = str(tmp_path / "tune.json")
+    shapes = [(48, 48, 48), (32, 32, 32), (48, 48, 48)]
+    with fakecuda.loaded(fake_lib) as fake:
+        def batch():
+            b = tlq.Batch([config(s, tlq.PREC_MIXED) for s in shapes])
+            for m in b.members:
+                m.upload(np.ones(m.cfg.shape, order="F"))
+            return b
+
+        b = batch()
+        default = b.running_tiling()
+        assert max(default) < 8 and b.tiling() == [8, 8, 8]
+        for size, members in ((48, (0, 2)), (32, (1,))):  # a size's members run together
+            z = default[members[0]] if winner == "default" else winner
+            fake.set_cost(len(members) * blocks((size,) * 3, z), 0.25)
+        got = b.autotune(cache, steps=2)
+        assert got == b.tiling() == ([8] * 3 if winner == "default" else [winner] * 3)
+        assert b.running_tiling() == (default if winner == "default" else [winner] * 3)
+        assert {e["zlen"] for e in json.load(open(cache))["tuned"].values()} == {0 if winner == "default" else winner}
+        b.set_tiling(1, 16)
+        assert b.tiling()[1] == b.running_tiling()[1] == 16
+        fake.lib.fake_reset()
+        b.run(1)
+        items = {g[0] for k, g, _ in fake.launches("stage_kernel_mixed_batch")}
+        assert items == {sum(blocks(s, z) for s, z in zip(shapes, b.running_tiling()))}
+        b.close()
+        b = batch()
+        fake.lib.fake_reset()
+        assert b.autotune(cache, steps=2) == got
+        assert not fake.launches("stage_kernel")
+        b.close()

@@ -349,22 +349,32 @@ int rule_zlen(const int* tiles, const int* nz, int n, bool mixed) {
   return best;
 }
 
-// The chunk length that runs for a chosen one: the choice, except that a mesh
-// too small to fill the GPU with chunks of 8 planes (the shortest choice) is
-// split to the rule's length; chunks of equal length.
-int split_zlen(int zlen, int rule, int nz) {
-  const int z = rule < 8 ? std::min(zlen, rule) : zlen;
-  const int chunks = (nz + z - 1) / z;
+// The rule's length for nz planes, in chunks of equal length.
+int split_zlen(int rule, int nz) {
+  const int chunks = (nz + rule - 1) / rule;
   return (nz + chunks - 1) / chunks;
 }
 
+// What a mesh without a choice reports as its length: the shortest choice
+// where the rule's is below it.
+int nominal_zlen(int rule, int nz) { return std::min(nz, std::max(8, rule)); }
+
+namespace {
+int ctx_rule(const tlq_ctx* ctx) {
+  const int tiles = (int)(ctx->grid.x * ctx->grid.y);
+  return rule_zlen(&tiles, &ctx->cfg.nz, 1, ctx->cfg.precision == TLQ_PREC_MIXED);
+}
+}  // namespace
+
+// zlen 0: the default.  A choice runs as it is: a mesh too small to fill the
+// GPU with chunks of 8 planes (the shortest choice) goes below them only by
+// default.
 int ctx_set_zlen(tlq_ctx* ctx, int zlen) {
   const int nz = ctx->cfg.nz;
   zlen = std::min(zlen, nz);
-  if (zlen < 8 && zlen != nz) return fail(ctx, TLQ_ERR_ARG, "z-chunk length must be >= 8 planes (or nz)");
+  if (zlen != 0 && zlen < 8 && zlen != nz) return fail(ctx, TLQ_ERR_ARG, "z-chunk length must be >= 8 planes (or nz)");
   ctx->zlen = zlen;
-  const int tiles = (int)(ctx->grid.x * ctx->grid.y);
-  ctx->zrun = split_zlen(zlen, rule_zlen(&tiles, &nz, 1, ctx->cfg.precision == TLQ_PREC_MIXED), nz);
+  ctx->zrun = zlen ? zlen : split_zlen(ctx_rule(ctx), nz);
   ctx->grid.z = (unsigned)((nz + ctx->zrun - 1) / ctx->zrun);
   invalidate_graphs(ctx);
   return TLQ_OK;
@@ -374,12 +384,19 @@ extern "C" {
 
 int tlq_set_tiling(tlq_ctx* ctx, int zlen) {
   if (!ctx) return TLQ_ERR_ARG;
+  if (zlen < 1) return fail(ctx, TLQ_ERR_ARG, "z-chunk length must be >= 8 planes (or nz)");
   return ctx_set_zlen(ctx, zlen);
 }
 
 int tlq_get_tiling(const tlq_ctx* ctx, int* zlen) {
   if (!ctx || !zlen) return TLQ_ERR_ARG;
-  *zlen = ctx->zlen;
+  *zlen = ctx->zlen ? ctx->zlen : nominal_zlen(ctx_rule(ctx), ctx->cfg.nz);
+  return TLQ_OK;
+}
+
+int tlq_running_tiling(const tlq_ctx* ctx, int* zlen) {
+  if (!ctx || !zlen) return TLQ_ERR_ARG;
+  *zlen = ctx->zrun;
   return TLQ_OK;
 }
 
@@ -479,8 +496,7 @@ int tlq_create(const tlq_config* cfg, tlq_ctx** out) {
   const int tx_ = cfg->precision == TLQ_PREC_MIXED ? MTX : TX, ty_ = cfg->precision == TLQ_PREC_MIXED ? MTY : TY;
   const int gx = (cfg->nx + tx_ - 1) / tx_, gy = (cfg->ny + ty_ - 1) / ty_;
   ctx->grid = dim3(gx, gy, 1);
-  const int tiles = gx * gy;
-  ctx_set_zlen(ctx, std::max(8, rule_zlen(&tiles, &cfg->nz, 1, cfg->precision == TLQ_PREC_MIXED)));
+  ctx_set_zlen(ctx, 0);
   const int nb = init_blocks(ctx->P);
   if (cudaMalloc(&ctx->sums_partials, sizeof(double) * 5 * (size_t)nb) || cudaMalloc(&ctx->sums_out, sizeof(double) * 5))
     return bail(TLQ_ERR_NOMEM);

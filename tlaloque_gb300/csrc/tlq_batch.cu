@@ -117,7 +117,7 @@ using tlq::MemberDesc;
 
 struct tlq_batch {
   std::vector<tlq_ctx*> m;
-  std::vector<int> zlen;            // chosen z-chunk length per member
+  std::vector<int> zlen;            // chosen z-chunk length per member (0: none, the default runs)
   std::vector<int> zrun;            // the one that runs (set_zrun)
   std::vector<unsigned> gen_seen;   // member set-up generation the graph was built for
   cudaStream_t stream = nullptr;
@@ -170,7 +170,13 @@ int batch_rule(const tlq_batch* b) {
 
 void set_zrun(tlq_batch* b) {
   const int rule = batch_rule(b);
-  for (size_t i = 0; i < b->m.size(); ++i) b->zrun[i] = split_zlen(b->zlen[i], rule, b->m[i]->cfg.nz);
+  for (size_t i = 0; i < b->m.size(); ++i)
+    b->zrun[i] = b->zlen[i] ? b->zlen[i] : split_zlen(rule, b->m[i]->cfg.nz);
+}
+
+// What member i reports as its length.
+int reported_zlen(const tlq_batch* b, int i) {
+  return b->zlen[i] ? b->zlen[i] : nominal_zlen(batch_rule(b), b->m[i]->cfg.nz);
 }
 
 void fill_desc(tlq_batch* b, int i) {
@@ -408,11 +414,9 @@ int tlq_batch_create(const tlq_config* cfgs, int n, tlq_batch** out) {
     b->m.push_back(c);
     b->gen_seen.push_back(~0u);
   }
-  const int rule = std::max(8, batch_rule(b));
-  for (tlq_ctx* c : b->m) {
-    b->zlen.push_back(std::min(rule, c->cfg.nz));
-    b->zrun.push_back(b->zlen.back());
-  }
+  b->zlen.assign(n, 0);
+  b->zrun.assign(n, 0);
+  set_zrun(b);
   if (cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) != cudaSuccess) return bail(TLQ_ERR_CUDA);
   for (tlq_ctx* c : b->m)
     if (tlq_set_stream(c, b->stream) != TLQ_OK) return bail(TLQ_ERR_CUDA);
@@ -462,7 +466,14 @@ int tlq_batch_set_tiling(tlq_batch* b, int i, int zlen) {
 
 int tlq_batch_get_tiling(const tlq_batch* b, int i, int* zlen) {
   if (!b || i < 0 || i >= (int)b->m.size() || !zlen) return TLQ_ERR_ARG;
-  *zlen = b->zlen[i];
+  *zlen = reported_zlen(b, i);
+  return TLQ_OK;
+}
+
+int tlq_batch_running_tiling(tlq_batch* b, int i, int* zlen) {
+  if (!b || i < 0 || i >= (int)b->m.size() || !zlen) return TLQ_ERR_ARG;
+  set_zrun(b);
+  *zlen = b->zrun[i];
   return TLQ_OK;
 }
 
@@ -544,11 +555,12 @@ int tlq_batch_stats_get(tlq_batch* b, tlq_batch_stats* s) {
 }
 
 // For each distinct mesh size: the cached z-chunk length, or one measured
-// now.  Every candidate (8, 16, 32, 64, 128 planes, at most nz) is timed over
+// now.  Every candidate (the default, 8, 16, 32, 64, 128 planes, at most nz) is timed over
 // `steps` steps (after one warm-up step) of the batch restricted to the
 // members of that size, starting each time from the members' current state,
 // which is restored afterwards (state, clock).  The winner is written to
-// the cache (one JSON object per file, keyed by the GPU's name).
+// the cache (one JSON object per file, keyed by the GPU's name; the default
+// as length 0).
 int tlq_batch_autotune(tlq_batch* b, const char* cache_path, int steps, int* chosen) {
   if (!b || steps < 1) return TLQ_ERR_ARG;
   for (size_t i = 0; i < b->m.size(); ++i)
@@ -569,7 +581,7 @@ int tlq_batch_autotune(tlq_batch* b, const char* cache_path, int steps, int* cho
     const std::vector<int>& mem = kv.second;
     auto hit = cache.find(kv.first);
     if (hit != cache.end()) {
-      for (int i : mem) b->zlen[i] = std::min(hit->second.first, b->m[i]->cfg.nz);
+      for (int i : mem) b->zlen[i] = std::max(0, std::min(hit->second.first, b->m[i]->cfg.nz));
       continue;
     }
     // snapshot the members' current state and clocks
@@ -591,7 +603,7 @@ int tlq_batch_autotune(tlq_batch* b, const char* cache_path, int steps, int* cho
     const int nz = b->m[mem[0]]->cfg.nz;
     int best = b->zlen[mem[0]];
     double best_ms = 1e300;
-    for (int z : {8, 16, 32, 64, 128}) {
+    for (int z : {0, 8, 16, 32, 64, 128}) {
       if (z > nz && z != 8) continue;
       for (int i : mem) b->zlen[i] = std::min(z, b->m[i]->cfg.nz);
       int rc = refresh_desc(b, mem);
@@ -636,12 +648,12 @@ int tlq_batch_autotune(tlq_batch* b, const char* cache_path, int steps, int* cho
     b->graph = nullptr;
   }
   if (chosen)
-    for (size_t i = 0; i < b->m.size(); ++i) chosen[i] = b->zlen[i];
+    for (size_t i = 0; i < b->m.size(); ++i) chosen[i] = reported_zlen(b, (int)i);
   return TLQ_OK;
 }
 
-// The same tuner for one context: the z-chunk length of its stage grid,
-// from the cache or measured over `steps` steps from the current state
+// The same tuner for one context: the z-chunk length of its stage grid (or
+// its default), from the cache or measured over `steps` steps from the current state
 // (restored afterwards), keyed by mesh size and form (mixed / fp64).
 int tlq_autotune(tlq_ctx* ctx, const char* cache_path, int steps, int* chosen) {
   if (!ctx || steps < 1) return TLQ_ERR_ARG;
@@ -683,7 +695,7 @@ int tlq_autotune(tlq_ctx* ctx, const char* cache_path, int steps, int* chosen) {
     cudaStreamSynchronize(ctx->stream);
     const long long steps0 = ctx->steps;
     double best_ms = 1e300;
-    for (int z : {8, 16, 32, 64, 128}) {
+    for (int z : {0, 8, 16, 32, 64, 128}) {
       if (z > c.nz && z != 8) continue;
       rc = ctx_set_zlen(ctx, std::min(z, c.nz));
       if (rc == TLQ_OK) rc = tlq_advance(ctx, 1);  // warm-up
@@ -723,8 +735,7 @@ int tlq_autotune(tlq_ctx* ctx, const char* cache_path, int steps, int* chosen) {
   }
   const int rc = ctx_set_zlen(ctx, best);
   if (rc != TLQ_OK) return rc;
-  if (chosen) *chosen = ctx->zlen;
-  return TLQ_OK;
+  return chosen ? tlq_get_tiling(ctx, chosen) : TLQ_OK;
 }
 
 }  // extern "C"

@@ -62,8 +62,8 @@ struct tlq_ctx {
   Clock* rclk = nullptr;
   // stage launch geometry and tensor maps
   dim3 grid{};
-  int zlen = 0;  // the chosen z-chunk length
-  int zrun = 0;  // the one that runs (split_zlen)
+  int zlen = 0;  // the chosen z-chunk length (0: none, the default runs)
+  int zrun = 0;  // the one that runs
   CUtensorMap tm_U[2]{}, tm_UPP{}, tm_P{};
   // run state
   int cur = 0;  // U[cur] holds the current state
@@ -109,14 +109,16 @@ void output_free(tlq_ctx* ctx);  // waits for a pending output, frees its buffer
 // Drops the captured step graphs and bumps the set-up generation (tlq_api.cu).
 void invalidate_graphs(tlq_ctx* c);
 
-// Z-chunk length of the stage grid (>= 8 planes, or nz): regrids and drops
-// the captured graphs (tlq_api.cu).
+// Z-chunk length of the stage grid (>= 8 planes, or nz; 0: the default):
+// regrids and drops the captured graphs (tlq_api.cu).
 int ctx_set_zlen(tlq_ctx* ctx, int zlen);
 
-// The default z-chunk length for meshes that step together, and the one that
-// runs for a chosen length (tlq_api.cu).
+// The default z-chunk length for meshes that step together (rule_zlen), split
+// evenly over a mesh's planes (split_zlen), and what is reported for it
+// (nominal_zlen) (tlq_api.cu).
 int rule_zlen(const int* tiles, const int* nz, int n, bool mixed);
-int split_zlen(int zlen, int rule, int nz);
+int split_zlen(int rule, int nz);
+int nominal_zlen(int rule, int nz);
 
 // Self-gravity (tlq_gravity.cu).  mg_levels_of: L with nx = ny = nz = 2^L,
 // else -1.  enqueue_multigrid_soa: one MultiGrid call on the density of the

@@ -36,8 +36,8 @@ EXPORTS = (
     "tlq_time_step_noalloc", "tlq_measure_fp64_rate",
     "tlq_surrogate_opts_default", "tlq_train_cooling_surrogate", "tlq_get_cooling_surrogate",
     "tlq_set_cooling_surrogate", "tlq_cooling_pairs", "tlq_mlp_loss_grad", "tlq_mlp_infer",
-    "tlq_set_tfin", "tlq_set_plane_winds", "tlq_output", "tlq_output_wait", "tlq_set_tiling", "tlq_get_tiling", "tlq_autotune", "tlq_batch_create", "tlq_batch_destroy", "tlq_batch_size", "tlq_batch_member",
-    "tlq_batch_set_tiling", "tlq_batch_get_tiling", "tlq_batch_autotune", "tlq_batch_run", "tlq_batch_synchronize",
+    "tlq_set_tfin", "tlq_set_plane_winds", "tlq_output", "tlq_output_wait", "tlq_set_tiling", "tlq_get_tiling", "tlq_running_tiling", "tlq_autotune", "tlq_batch_create", "tlq_batch_destroy", "tlq_batch_size", "tlq_batch_member",
+    "tlq_batch_set_tiling", "tlq_batch_get_tiling", "tlq_batch_running_tiling", "tlq_batch_autotune", "tlq_batch_run", "tlq_batch_synchronize",
     "tlq_batch_status", "tlq_batch_enable_timing", "tlq_batch_stats_get", "tlq_batch_last_error",
 )
 
@@ -134,6 +134,7 @@ def load_library(path: str = LIB_PATH):
         "tlq_output_wait": (I, [V]),
         "tlq_set_tiling": (I, [V, I]),
         "tlq_get_tiling": (I, [V, C.POINTER(I)]),
+        "tlq_running_tiling": (I, [V, C.POINTER(I)]),
         "tlq_autotune": (I, [V, C.c_char_p, I, C.POINTER(I)]),
         "tlq_batch_create": (I, [C.POINTER(CConfig), I, C.POINTER(V)]),
         "tlq_batch_destroy": (I, [V]),
@@ -141,6 +142,7 @@ def load_library(path: str = LIB_PATH):
         "tlq_batch_member": (V, [V, I]),
         "tlq_batch_set_tiling": (I, [V, I, I]),
         "tlq_batch_get_tiling": (I, [V, I, C.POINTER(I)]),
+        "tlq_batch_running_tiling": (I, [V, I, C.POINTER(I)]),
         "tlq_batch_autotune": (I, [V, C.c_char_p, I, C.POINTER(I)]),
         "tlq_batch_run": (I, [V, I]),
         "tlq_batch_synchronize": (I, [V]),
@@ -422,6 +424,12 @@ class Context:
         self._check(self.L.tlq_get_tiling(self.h, C.byref(z)), "get_tiling")
         return z.value
 
+    def running_tiling(self) -> int:
+        """The z-chunk length that runs: tiling(), or the default's, which may be below 8."""
+        z = C.c_int()
+        self._check(self.L.tlq_running_tiling(self.h, C.byref(z)), "running_tiling")
+        return z.value
+
     def autotune(self, cache_path: str | None = None, steps: int = 3) -> int:
         z = C.c_int()
         self._check(self.L.tlq_autotune(self.h, cache_path.encode() if cache_path else None, int(steps), C.byref(z)),
@@ -645,6 +653,15 @@ class Batch:
         for q in range(len(self.members)):
             z = C.c_int()
             self._check(self.L.tlq_batch_get_tiling(self.h, q, C.byref(z)), "batch_get_tiling")
+            out.append(z.value)
+        return out
+
+    def running_tiling(self):
+        """The members' z-chunk lengths that run: tiling(), or the default's, which may be below 8."""
+        out = []
+        for q in range(len(self.members)):
+            z = C.c_int()
+            self._check(self.L.tlq_batch_running_tiling(self.h, q, C.byref(z)), "batch_running_tiling")
             out.append(z.value)
         return out
 
