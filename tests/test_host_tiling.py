@@ -116,3 +116,39 @@ def test_batch_autotune_tries_the_default(fake_lib, tmp_path, winner):
         assert b.autotune(cache, steps=2) == got
         assert not fake.launches("stage_kernel")
         b.close()
+
+
+def stages(fake):
+    return len(fake.launches("stage_kernel"))
+
+
+def test_equal_launches_are_timed_once(fake_lib, tmp_path):
+    """Each running length once (64 planes: the default is one of the lengths),
+    nothing timed or cached where there is one, and a hopeless candidate left
+    after its first step."""
+    cache = tmp_path / "tune.json"
+    with fakecuda.loaded(fake_lib) as fake:
+        ctx = uploaded(config((128, 128, 128), tlq.PREC_MIXED))
+        assert ctx.running_tiling() == 8
+        fake.lib.fake_reset()
+        ctx.autotune(str(cache), steps=4)
+        # captured per candidate and parity, launched 1 + 4 times
+        assert stages(fake) == 5 * 2 * 2 and len({g for _, g, _ in fake.launches("stage_kernel")}) == 5
+        ctx.close()
+        ctx = uploaded(config((512, 256, 8)))
+        assert ctx.running_tiling() == 8
+        fake.lib.fake_reset()
+        assert ctx.autotune(str(tmp_path / "none.json"), steps=4) == 8
+        assert stages(fake) == 0 and not (tmp_path / "none.json").exists()
+        ctx.close()
+        shape = (48, 48, 48)
+        b = tlq.Batch([config(shape, tlq.PREC_MIXED)])
+        b.members[0].upload(np.ones(b.members[0].cfg.shape, order="F"))
+        default = b.running_tiling()[0]
+        fake.lib.fake_reset()
+        fake.set_cost(blocks(shape, default), 0.25)
+        fake.set_cost(blocks(shape, 16), 0.45)
+        b.autotune(None, steps=4)
+        # the default and 16 planes: 1 + 4 steps; 8 and 32 planes: 1 step
+        assert b.running_tiling() == [default] and stages(fake) == 2 * (5 + 5 + 1 + 1)
+        b.close()

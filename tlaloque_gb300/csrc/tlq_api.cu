@@ -366,6 +366,8 @@ int ctx_rule(const tlq_ctx* ctx) {
 }
 }  // namespace
 
+int ctx_default_zlen(const tlq_ctx* ctx) { return split_zlen(ctx_rule(ctx), ctx->cfg.nz); }
+
 // zlen 0: the default.  A choice runs as it is: a mesh too small to fill the
 // GPU with chunks of 8 planes (the shortest choice) goes below them only by
 // default.
@@ -374,7 +376,7 @@ int ctx_set_zlen(tlq_ctx* ctx, int zlen) {
   zlen = std::min(zlen, nz);
   if (zlen != 0 && zlen < 8 && zlen != nz) return fail(ctx, TLQ_ERR_ARG, "z-chunk length must be >= 8 planes (or nz)");
   ctx->zlen = zlen;
-  ctx->zrun = zlen ? zlen : split_zlen(ctx_rule(ctx), nz);
+  ctx->zrun = zlen ? zlen : ctx_default_zlen(ctx);
   ctx->grid.z = (unsigned)((nz + ctx->zrun - 1) / ctx->zrun);
   invalidate_graphs(ctx);
   return TLQ_OK;

@@ -393,6 +393,19 @@ int write_cache(const char* path, const std::string& gpu, const std::map<std::st
   return std::rename(tmp.c_str(), path) == 0 ? TLQ_OK : TLQ_ERR_ARG;
 }
 
+// The tuners' candidates for a mesh of nz planes whose default runs `run`
+// planes: the default (0), and of 8 (or nz) and 16 .. 128 (up to nz) those that
+// run another length.
+std::vector<int> tuning_candidates(int nz, int run) {
+  std::vector<int> z = {0};
+  for (int c : {8, 16, 32, 64, 128})
+    if ((c <= nz || c == 8) && std::min(c, nz) != run) z.push_back(std::min(c, nz));
+  return z;
+}
+// A candidate whose first step takes more than this many times the best one's
+// is not timed further (the longest chunks on small meshes take several).
+constexpr double TUNING_HOPELESS = 2.0;
+
 }  // namespace
 
 extern "C" {
@@ -555,12 +568,11 @@ int tlq_batch_stats_get(tlq_batch* b, tlq_batch_stats* s) {
 }
 
 // For each distinct mesh size: the cached z-chunk length, or one measured
-// now.  Every candidate (the default, 8, 16, 32, 64, 128 planes, at most nz) is timed over
-// `steps` steps (after one warm-up step) of the batch restricted to the
-// members of that size, starting each time from the members' current state,
-// which is restored afterwards (state, clock).  The winner is written to
-// the cache (one JSON object per file, keyed by the GPU's name; the default
-// as length 0).
+// now.  Every candidate (tuning_candidates) is timed over `steps` steps (after
+// one warm-up step) of the batch restricted to the members of that size,
+// starting each time from the members' current state, which is restored
+// afterwards (state, clock).  The winner is written to the cache (one JSON
+// object per file, keyed by the GPU's name; the default as length 0).
 int tlq_batch_autotune(tlq_batch* b, const char* cache_path, int steps, int* chosen) {
   if (!b || steps < 1) return TLQ_ERR_ARG;
   for (size_t i = 0; i < b->m.size(); ++i)
@@ -584,6 +596,12 @@ int tlq_batch_autotune(tlq_batch* b, const char* cache_path, int steps, int* cho
       for (int i : mem) b->zlen[i] = std::max(0, std::min(hit->second.first, b->m[i]->cfg.nz));
       continue;
     }
+    const int nz = b->m[mem[0]]->cfg.nz;
+    const std::vector<int> candidates = tuning_candidates(nz, split_zlen(batch_rule(b), nz));
+    if (candidates.size() == 1) {  // nothing to choose
+      for (int i : mem) b->zlen[i] = 0;
+      continue;
+    }
     // snapshot the members' current state and clocks
     std::vector<double*> snap(mem.size(), nullptr);
     std::vector<tlq::Clock> clk(mem.size());
@@ -600,29 +618,36 @@ int tlq_batch_autotune(tlq_batch* b, const char* cache_path, int steps, int* cho
       BCK(cudaMemcpyAsync(&clk[q], c->clk, sizeof(tlq::Clock), cudaMemcpyDeviceToHost, b->stream));
     }
     BCK(cudaStreamSynchronize(b->stream));
-    const int nz = b->m[mem[0]]->cfg.nz;
-    int best = b->zlen[mem[0]];
+    int best = 0;
     double best_ms = 1e300;
-    for (int z : {0, 8, 16, 32, 64, 128}) {
-      if (z > nz && z != 8) continue;
-      for (int i : mem) b->zlen[i] = std::min(z, b->m[i]->cfg.nz);
+    for (int z : candidates) {
+      for (int i : mem) b->zlen[i] = z;
       int rc = refresh_desc(b, mem);
       if (!rc) rc = upload_items(b, make_items(b, mem));
       if (rc) return rc;
-      for (int w = 0; w < steps + 1; ++w) {
-        if (w == 1) BCK(cudaEventRecord(b->ev[0], b->stream));
-        rc = enqueue_batch_step(b);
-        if (rc) return rc;
+      auto time = [&](int n, double* per) -> int {
+        BCK(cudaEventRecord(b->ev[0], b->stream));
+        for (int w = 0; w < n; ++w) {
+          const int r = enqueue_batch_step(b);
+          if (r) return r;
+        }
+        BCK(cudaEventRecord(b->ev[1], b->stream));
+        BCK(cudaEventSynchronize(b->ev[1]));
+        float ms = 0.f;
+        cudaEventElapsedTime(&ms, b->ev[0], b->ev[1]);
+        *per = ms / n;
+        return TLQ_OK;
+      };
+      double per = 0.0;
+      rc = time(1, &per);  // warm-up
+      if (!rc && per < TUNING_HOPELESS * best_ms) {
+        rc = time(steps, &per);
+        if (per < best_ms) {
+          best_ms = per;
+          best = z;
+        }
       }
-      BCK(cudaEventRecord(b->ev[1], b->stream));
-      BCK(cudaEventSynchronize(b->ev[1]));
-      float ms = 0.f;
-      cudaEventElapsedTime(&ms, b->ev[0], b->ev[1]);
-      const double per = ms / steps;
-      if (per < best_ms) {
-        best_ms = per;
-        best = z;
-      }
+      if (rc) return rc;
       // back to the snapshot
       for (size_t q = 0; q < mem.size(); ++q) {
         tlq_ctx* c = b->m[mem[q]];
@@ -637,7 +662,7 @@ int tlq_batch_autotune(tlq_batch* b, const char* cache_path, int steps, int* cho
       tlq_ctx* c = b->m[mem[q]];
       if (c->cool_counts) cudaMemsetAsync(c->cool_counts, 0, 3 * sizeof(unsigned long long), b->stream);
     }
-    for (int i : mem) b->zlen[i] = std::min(best, b->m[i]->cfg.nz);
+    for (int i : mem) b->zlen[i] = best;
     cache[kv.first] = {best, best_ms};
     wrote = true;
   }
@@ -668,10 +693,11 @@ int tlq_autotune(tlq_ctx* ctx, const char* cache_path, int steps, int* chosen) {
                           (c.precision == TLQ_PREC_MIXED ? "/mixed" : "/fp64") +
                           (c.cooling == TLQ_COOL_MLP ? "_mlp" : "");
   auto hit = cache.find(key);
-  int best = ctx->zlen;
+  const std::vector<int> candidates = tuning_candidates(c.nz, ctx_default_zlen(ctx));
+  int best = 0;
   if (hit != cache.end()) {
     best = hit->second.first;
-  } else {
+  } else if (candidates.size() > 1) {
     double t, dt;
     int it;
     int rc = tlq_get_time(ctx, &t, &it, &dt);
@@ -695,23 +721,29 @@ int tlq_autotune(tlq_ctx* ctx, const char* cache_path, int steps, int* chosen) {
     cudaStreamSynchronize(ctx->stream);
     const long long steps0 = ctx->steps;
     double best_ms = 1e300;
-    for (int z : {0, 8, 16, 32, 64, 128}) {
-      if (z > c.nz && z != 8) continue;
-      rc = ctx_set_zlen(ctx, std::min(z, c.nz));
-      if (rc == TLQ_OK) rc = tlq_advance(ctx, 1);  // warm-up
-      if (rc == TLQ_OK) rc = tlq_enable_timing(ctx, 1);
-      if (rc == TLQ_OK) rc = tlq_advance(ctx, steps);
-      tlq_stats s{};
-      if (rc == TLQ_OK) rc = tlq_stats_get(ctx, &s);
-      tlq_enable_timing(ctx, 0);
+    for (int z : candidates) {
+      rc = ctx_set_zlen(ctx, z);
+      auto time = [&](int n, double* per) -> int {
+        int r = tlq_enable_timing(ctx, 1);
+        if (r == TLQ_OK) r = tlq_advance(ctx, n);
+        tlq_stats s{};
+        if (r == TLQ_OK) r = tlq_stats_get(ctx, &s);
+        tlq_enable_timing(ctx, 0);
+        *per = s.ms_stage1 + s.ms_stage2 + s.ms_cool + s.ms_grav;
+        return r;
+      };
+      double ms = 0.0;
+      if (rc == TLQ_OK) rc = time(1, &ms);  // warm-up
+      if (rc == TLQ_OK && ms < TUNING_HOPELESS * best_ms) {
+        rc = time(steps, &ms);
+        if (ms < best_ms) {
+          best_ms = ms;
+          best = z;
+        }
+      }
       if (rc != TLQ_OK) {
         cudaFree(snap);
         return rc;
-      }
-      const double ms = s.ms_stage1 + s.ms_stage2 + s.ms_cool + s.ms_grav;
-      if (ms < best_ms) {
-        best_ms = ms;
-        best = std::min(z, c.nz);
       }
       // back to the snapshot
       cudaMemcpyAsync(ctx->U[cur], snap, bytes, cudaMemcpyDeviceToDevice, ctx->stream);

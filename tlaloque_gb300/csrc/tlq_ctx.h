@@ -115,10 +115,11 @@ int ctx_set_zlen(tlq_ctx* ctx, int zlen);
 
 // The default z-chunk length for meshes that step together (rule_zlen), split
 // evenly over a mesh's planes (split_zlen), and what is reported for it
-// (nominal_zlen) (tlq_api.cu).
+// (nominal_zlen); the default of a mesh that steps alone (tlq_api.cu).
 int rule_zlen(const int* tiles, const int* nz, int n, bool mixed);
 int split_zlen(int rule, int nz);
 int nominal_zlen(int rule, int nz);
+int ctx_default_zlen(const tlq_ctx* ctx);
 
 // Self-gravity (tlq_gravity.cu).  mg_levels_of: L with nx = ny = nz = 2^L,
 // else -1.  enqueue_multigrid_soa: one MultiGrid call on the density of the
