@@ -652,13 +652,18 @@ int tlq_set_plane_winds(tlq_ctx* ctx, const tlq_plane_wind* w, int n) {
 
 int tlq_set_winds(tlq_ctx* ctx, const tlq_wind* w, int n) {
   if (!ctx || n < 0 || (n > 0 && !w)) return TLQ_ERR_ARG;
-  cudaFree(ctx->dwinds);
-  cudaFree(ctx->dwind_tab);
-  ctx->dwinds = nullptr;
-  ctx->dwind_tab = nullptr;
+  CK(cudaStreamSynchronize(ctx->stream));  // (the steps in flight read the winds)
+  invalidate_graphs(ctx);
   ctx->P.nwinds = 0;
   ctx->P.winds = nullptr;
-  if (n > 0) {
+  if (n == 0) {
+    cudaFree(ctx->dwinds);
+    cudaFree(ctx->dwind_tab);
+    ctx->dwinds = nullptr;
+    ctx->dwind_tab = nullptr;
+    ctx->cap_winds = 0;
+    ctx->cap_wind_cells = 0;
+  } else {
     std::vector<Wind> hw(n);
     const Params& p = ctx->P;
     for (int q = 0; q < n; ++q) {
@@ -674,34 +679,49 @@ int tlq_set_winds(tlq_ctx* ctx, const tlq_wind* w, int n) {
       d.jlo = std::max(-1, lo(d.yc, d.radius, p.yl, p.dy)); d.jhi = std::min(p.ny + 2, hi(d.yc, d.radius, p.yl, p.dy));
       d.klo = std::max(-1, lo(d.zc, d.radius, p.zl, p.dz)); d.khi = std::min(p.nz + 2, hi(d.zc, d.radius, p.zl, p.dz));
     }
-    // the tables of the winds' cells, until their common size is reached
-    auto tabled = [](const Wind& d) {
-      return d.ihi >= d.ilo && d.jhi >= d.jlo && d.khi >= d.klo &&
-             (long long)(d.ihi - d.ilo + 1) * (d.jhi - d.jlo + 1) * (d.khi - d.klo + 1) <= tlq::WIND_TABLE_CELLS;
-    };
-    long long cells = 0;
-    for (Wind& d : hw) {
-      d.tab = nullptr;
-      if (tabled(d) && cells + d.cells() <= tlq::WIND_TABLE_CELLS) cells += d.cells();
+    // Both buffers are kept while they are large enough, and one launch forms
+    // every wind's table: a driver may move its winds each step (a call with
+    // one wind: 8 us before there were tables, 26 with an allocation, a launch
+    // per wind and a wait for them, 6 so).
+    if (n > ctx->cap_winds) {
+      cudaFree(ctx->dwinds);
+      ctx->dwinds = nullptr;
+      ctx->cap_winds = 0;
+      CK(cudaMalloc(&ctx->dwinds, n * sizeof(Wind)));
+      ctx->cap_winds = n;
     }
-    const bool room = cells > 0 && cudaMalloc(&ctx->dwind_tab, 6 * cells * sizeof(double)) == cudaSuccess;
-    if (!room) cudaGetLastError();  // (without tables the stages evaluate the winds)
-    cells = 0;
-    for (Wind& d : hw) {
-      if (!room || !tabled(d) || cells + d.cells() > tlq::WIND_TABLE_CELLS) continue;
-      double* t = ctx->dwind_tab + 6 * cells;
-      CK(ctx->cfg.precision == TLQ_PREC_MIXED ? launch_wind_table_mixed(p, d, t, ctx->stream)
-                                              : launch_wind_table(p, d, t, ctx->stream));
-      d.tab = t;
-      cells += d.cells();
+    // the winds whose cells have a table, until the tables' common size is reached
+    long long cells = 0, largest = 0;
+    std::vector<long long> at(n, -1);
+    for (int q = 0; q < n; ++q) {
+      const Wind& d = hw[q];
+      if (d.ihi < d.ilo || d.jhi < d.jlo || d.khi < d.klo) continue;
+      const long long c = (long long)(d.ihi - d.ilo + 1) * (d.jhi - d.jlo + 1) * (d.khi - d.klo + 1);
+      if (cells + c > tlq::WIND_TABLE_CELLS) continue;
+      at[q] = cells;
+      cells += c;
+      largest = std::max(largest, c);
     }
-    CK(cudaStreamSynchronize(ctx->stream));
-    CK(cudaMalloc(&ctx->dwinds, n * sizeof(Wind)));
-    CK(cudaMemcpy(ctx->dwinds, hw.data(), n * sizeof(Wind), cudaMemcpyHostToDevice));
+    if (cells > ctx->cap_wind_cells) {
+      cudaFree(ctx->dwind_tab);
+      ctx->dwind_tab = nullptr;
+      ctx->cap_wind_cells = 0;
+      if (cudaMalloc(&ctx->dwind_tab, 6 * cells * sizeof(double)) == cudaSuccess)
+        ctx->cap_wind_cells = cells;
+      else
+        cudaGetLastError();  // (without tables the stages evaluate the winds)
+    }
+    const bool tables = cells > 0 && cells <= ctx->cap_wind_cells;
+    for (int q = 0; q < n; ++q) hw[q].tab = tables && at[q] >= 0 ? ctx->dwind_tab + 6 * at[q] : nullptr;
+    // (on the context's stream: a copy from pageable memory may still be under
+    // way when the call returns, and the stream does not wait for others)
+    CK(cudaMemcpyAsync(ctx->dwinds, hw.data(), n * sizeof(Wind), cudaMemcpyHostToDevice, ctx->stream));
+    if (tables)
+      CK(ctx->cfg.precision == TLQ_PREC_MIXED ? launch_wind_tables_mixed(p, ctx->dwinds, n, (int)largest, ctx->stream)
+                                              : launch_wind_tables(p, ctx->dwinds, n, (int)largest, ctx->stream));
     ctx->P.nwinds = n;
     ctx->P.winds = ctx->dwinds;
   }
-  invalidate_graphs(ctx);
   return TLQ_OK;
 }
 

@@ -53,6 +53,8 @@ struct tlq_ctx {
   float *dslopef = nullptr, *dgcumf = nullptr;
   Wind* dwinds = nullptr;
   double* dwind_tab = nullptr;  // the winds' tables (Wind::tab)
+  int cap_winds = 0;            // and how many winds, and cells of tables, the two hold
+  long long cap_wind_cells = 0;
   double* dmasses = nullptr;
   int nmasses = 0;
   std::vector<double> masses_host;

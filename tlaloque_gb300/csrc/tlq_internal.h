@@ -41,9 +41,10 @@ cudaError_t prepare_batch_kernels();  // tlq_batch.cu
 size_t mixed_smem_bytes(int stage);
 cudaError_t launch_stage_mixed(int stage, const CUtensorMap& tm_in, const StageArgs& a, dim3 grid, cudaStream_t s);
 // The first dt of the mixed form (its FP32 signal speeds; tlq_mixed.cu).
-// One wind's table (Wind::tab) in the plain and in the mixed form's arithmetic.
-cudaError_t launch_wind_table(const Params& p, const Wind& w, double* tab, cudaStream_t s);
-cudaError_t launch_wind_table_mixed(const Params& p, const Wind& w, double* tab, cudaStream_t s);
+// The tables (Wind::tab) of n winds on the device that have one, of at most
+// `cells` cells each, in the plain and in the mixed form's arithmetic.
+cudaError_t launch_wind_tables(const Params& p, const Wind* winds, int n, int cells, cudaStream_t s);
+cudaError_t launch_wind_tables_mixed(const Params& p, const Wind* winds, int n, int cells, cudaStream_t s);
 cudaError_t launch_init_dt_mixed(const Params& p, const Layout& L, const double* U, Clock* clk, int nblocks,
                                  cudaStream_t s);
 

@@ -605,13 +605,16 @@ cudaError_t launch_borders_aos(const Params& p, const Aos& A, double* U, int ord
   return cudaGetLastError();
 }
 namespace {
-__global__ void __launch_bounds__(BT) k_wind_table(Params p, Wind w, double* tab) {
+__global__ void __launch_bounds__(BT) k_wind_tables(Params p, const Wind* __restrict__ winds, int n) {
   const int q = blockIdx.x * BT + threadIdx.x;
-  if (q < w.cells()) wind_table_cell(p, w, q, tab);
+  for (int s = blockIdx.y; s < n; s += gridDim.y) {
+    const Wind w = winds[s];
+    if (w.tab && q < w.cells()) wind_table_cell(p, w, q, const_cast<double*>(w.tab));
+  }
 }
 }  // namespace
-cudaError_t launch_wind_table(const Params& p, const Wind& w, double* tab, cudaStream_t s) {
-  k_wind_table<<<(w.cells() + BT - 1) / BT, BT, 0, s>>>(p, w, tab);
+cudaError_t launch_wind_tables(const Params& p, const Wind* winds, int n, int cells, cudaStream_t s) {
+  k_wind_tables<<<dim3((cells + BT - 1) / BT, std::min(n, 65535)), BT, 0, s>>>(p, winds, n);
   return cudaGetLastError();
 }
 cudaError_t launch_winds_aos(const Params& p, const Aos& A, double* U, cudaStream_t s) {

@@ -2,6 +2,8 @@
 // fluxes and sources; FP64 accumulation).  Built with --use_fast_math: FP32
 // division and square root are the approximate hardware forms, FP32
 // subnormals flush to zero; FP64 arithmetic is unaffected.
+#include <algorithm>
+
 #include "tlq_internal.h"
 #include "tlq_stage_mixed.cuh"
 
@@ -75,13 +77,16 @@ __global__ void __launch_bounds__(RED_THREADS) k_init_dt_mixed(Params p, Layout 
 }
 
 namespace {
-__global__ void __launch_bounds__(128) k_wind_table_mixed(Params p, Wind w, double* tab) {
+__global__ void __launch_bounds__(128) k_wind_tables_mixed(Params p, const Wind* __restrict__ winds, int n) {
   const int q = blockIdx.x * 128 + threadIdx.x;
-  if (q < w.cells()) wind_table_cell(p, w, q, tab);
+  for (int s = blockIdx.y; s < n; s += gridDim.y) {
+    const Wind w = winds[s];
+    if (w.tab && q < w.cells()) wind_table_cell(p, w, q, const_cast<double*>(w.tab));
+  }
 }
 }  // namespace
-cudaError_t launch_wind_table_mixed(const Params& p, const Wind& w, double* tab, cudaStream_t s) {
-  k_wind_table_mixed<<<(w.cells() + 127) / 128, 128, 0, s>>>(p, w, tab);
+cudaError_t launch_wind_tables_mixed(const Params& p, const Wind* winds, int n, int cells, cudaStream_t s) {
+  k_wind_tables_mixed<<<dim3((cells + 127) / 128, std::min(n, 65535)), 128, 0, s>>>(p, winds, n);
   return cudaGetLastError();
 }
 

@@ -384,7 +384,7 @@ __device__ __forceinline__ bool wind_lookup(const Params& p, const Wind& w, int 
   return true;
 }
 
-// Entry q of wind w's table (w.tab null).
+// Entry q of wind w's table.
 __device__ __forceinline__ void wind_table_cell(const Params& p, const Wind& w, int q, double* tab) {
   const int ni = w.ihi - w.ilo + 1, nj = w.jhi - w.jlo + 1, n = w.cells();
   double u[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
