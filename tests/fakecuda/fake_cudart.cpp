@@ -6,6 +6,10 @@
 //   Devices: FAKE_DEVICES equal ones; a function's attributes belong to the
 // device current when they are set, and a launch with more dynamic shared
 // memory than the attribute (48 KB unless raised) fails, as on real devices.
+//   Order: a copying call from (pageable) host memory may return before the
+// device has the data, and the library's streams do not wait for the legacy
+// stream: a launch on one of them after such a call is counted as
+// "fake_unordered".
 //   Time: a launch advances the clock by 1 ms, or by what fake_set_cost says
 // for its number of blocks.
 #include <cuda.h>
@@ -50,6 +54,7 @@ std::map<std::string, long long> g_calls;
 std::vector<Launch> g_launches;
 std::map<void*, size_t> g_sizes;
 long long g_bytes = 0;
+bool g_copying = false;  // a copy from the host on the legacy stream may be under way
 std::string g_fail;
 Stream g_legacy;
 
@@ -72,6 +77,7 @@ cudaError_t launch(const void* f, dim3 grid, size_t smem, cudaStream_t s) {
   if (!g_fail.empty() && name.find(g_fail) != std::string::npos) return done(cudaErrorInvalidConfiguration);
   const auto it = g_smem.find({g_device, f});
   if (smem > (size_t)(it == g_smem.end() ? 48 * 1024 : it->second)) return done(cudaErrorInvalidValue);
+  if (s && g_copying) ++g_calls["fake_unordered"];
   g_launches.push_back(Launch{name, {grid.x, grid.y, grid.z}, g_device});
   const auto c = g_cost.find((long long)grid.x * grid.y * grid.z);
   enqueue(s, Op{nullptr, c == g_cost.end() ? 1.0 : c->second});
@@ -112,6 +118,7 @@ void fake_reset() {
   g_fail.clear();
   g_last = cudaSuccess;
   g_device = 0;
+  g_copying = false;
 }
 long long fake_calls(const char* name) { return g_calls[name]; }
 long long fake_bytes() { return g_bytes; }
@@ -205,7 +212,12 @@ cudaError_t cudaFree(void* p) {
   return release(p);
 }
 cudaError_t cudaFreeHost(void* p) { CALL; return release(p); }
-cudaError_t cudaMemcpy(void* d, const void* s, size_t n, enum cudaMemcpyKind) { CALL; std::memmove(d, s, n); return cudaSuccess; }
+cudaError_t cudaMemcpy(void* d, const void* s, size_t n, enum cudaMemcpyKind k) {
+  CALL;
+  g_copying = k == cudaMemcpyHostToDevice;  // (a copy to the host waits for those before it)
+  std::memmove(d, s, n);
+  return cudaSuccess;
+}
 cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, enum cudaMemcpyKind, cudaStream_t) {
   CALL;
   std::memmove(d, s, n);
@@ -228,8 +240,16 @@ cudaError_t cudaGetDriverEntryPointByVersion(const char*, void** f, unsigned, un
   *q = cudaDriverEntryPointSuccess;
   return cudaSuccess;
 }
-cudaError_t cudaDeviceSynchronize() { CALL; return cudaSuccess; }
-cudaError_t cudaStreamSynchronize(cudaStream_t) { CALL; return cudaSuccess; }
+cudaError_t cudaDeviceSynchronize() {
+  CALL;
+  g_copying = false;
+  return cudaSuccess;
+}
+cudaError_t cudaStreamSynchronize(cudaStream_t s) {
+  CALL;
+  if (!s) g_copying = false;
+  return cudaSuccess;
+}
 cudaError_t cudaStreamCreateWithFlags(cudaStream_t* s, unsigned) {
   *s = reinterpret_cast<cudaStream_t>(new Stream());
   return cudaSuccess;

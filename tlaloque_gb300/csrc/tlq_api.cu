@@ -563,16 +563,19 @@ int tlq_set_cooling_table(tlq_ctx* ctx, const double* T, const double* logL, int
     if (!(T[q] >= T[q - 1])) return fail(ctx, TLQ_ERR_ARG, "cooling table temperatures must be ascending");
   std::vector<double> lt(n);
   for (int q = 0; q < n; ++q) lt[q] = std::log10(T[q]);
+  // (the copies here and in the calls below on the context's stream, which
+  // waits for no other: one from pageable memory may still be under way when a
+  // copying call returns)
   cudaFree(ctx->dT); cudaFree(ctx->dlogT); cudaFree(ctx->dC);
   ctx->dT = ctx->dlogT = ctx->dC = nullptr;
   CK(cudaMalloc(&ctx->dT, n * sizeof(double)));
   CK(cudaMalloc(&ctx->dlogT, n * sizeof(double)));
   CK(cudaMalloc(&ctx->dC, n * sizeof(double)));
-  CK(cudaMemcpy(ctx->dT, T, n * sizeof(double), cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(ctx->dC, logL, n * sizeof(double), cudaMemcpyHostToDevice));
+  CK(cudaMemcpyAsync(ctx->dT, T, n * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
+  CK(cudaMemcpyAsync(ctx->dC, logL, n * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
   // log10 of the table temperatures is evaluated on the device, like the
   // reference does at each lookup (cooling.f90:135,137).
-  CK(cudaMemcpy(ctx->dlogT, T, n * sizeof(double), cudaMemcpyHostToDevice));
+  CK(cudaMemcpyAsync(ctx->dlogT, T, n * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
   CK(launch_log10_inplace(ctx->dlogT, n, ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
   // FP32 copies for the mixed-precision step
@@ -585,9 +588,9 @@ int tlq_set_cooling_table(tlq_ctx* ctx, const double* T, const double* logL, int
   CK(cudaMalloc(&ctx->dTf, n * sizeof(float)));
   CK(cudaMalloc(&ctx->dlogTf, n * sizeof(float)));
   CK(cudaMalloc(&ctx->dCf, n * sizeof(float)));
-  CK(cudaMemcpy(ctx->dTf, fT.data(), n * sizeof(float), cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(ctx->dlogTf, flt.data(), n * sizeof(float), cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(ctx->dCf, fC.data(), n * sizeof(float), cudaMemcpyHostToDevice));
+  CK(cudaMemcpyAsync(ctx->dTf, fT.data(), n * sizeof(float), cudaMemcpyHostToDevice, ctx->stream));
+  CK(cudaMemcpyAsync(ctx->dlogTf, flt.data(), n * sizeof(float), cudaMemcpyHostToDevice, ctx->stream));
+  CK(cudaMemcpyAsync(ctx->dCf, fC.data(), n * sizeof(float), cudaMemcpyHostToDevice, ctx->stream));
   // The exact integrator's closed form (COOL_EXACT, and the surrogate's
   // fallback and check): per segment the power law's slope, in find_coef's
   // form (cooling.f90:137-140), 0 above the last node; at each node G(T_i),
@@ -612,10 +615,10 @@ int tlq_set_cooling_table(tlq_ctx* ctx, const double* T, const double* logL, int
   CK(cudaMalloc(&ctx->dgcum, n * sizeof(double)));
   CK(cudaMalloc(&ctx->dslopef, n * sizeof(float)));
   CK(cudaMalloc(&ctx->dgcumf, n * sizeof(float)));
-  CK(cudaMemcpy(ctx->dslope, sl.data(), n * sizeof(double), cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(ctx->dgcum, gc.data(), n * sizeof(double), cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(ctx->dslopef, slf.data(), n * sizeof(float), cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(ctx->dgcumf, gcf.data(), n * sizeof(float), cudaMemcpyHostToDevice));
+  CK(cudaMemcpyAsync(ctx->dslope, sl.data(), n * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
+  CK(cudaMemcpyAsync(ctx->dgcum, gc.data(), n * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
+  CK(cudaMemcpyAsync(ctx->dslopef, slf.data(), n * sizeof(float), cudaMemcpyHostToDevice, ctx->stream));
+  CK(cudaMemcpyAsync(ctx->dgcumf, gcf.data(), n * sizeof(float), cudaMemcpyHostToDevice, ctx->stream));
   // nodes uniform in log10 T (each within a third of a step of the line
   // through the first and last): the FP32 searches guess the segment
   float lt0 = 0.0f, dl_inv = 0.0f;
@@ -634,8 +637,9 @@ int tlq_set_cooling_table(tlq_ctx* ctx, const double* T, const double* logL, int
   ctx->P.c_edge_rho = T[0] * KB;
   if (!ctx->cool_counts) {
     CK(cudaMalloc(&ctx->cool_counts, 3 * sizeof(unsigned long long)));
-    CK(cudaMemset(ctx->cool_counts, 0, 3 * sizeof(unsigned long long)));
+    CK(cudaMemsetAsync(ctx->cool_counts, 0, 3 * sizeof(unsigned long long), ctx->stream));
   }
+  CK(cudaStreamSynchronize(ctx->stream));
   invalidate_graphs(ctx);
   return TLQ_OK;
 }
@@ -664,7 +668,8 @@ int tlq_set_winds(tlq_ctx* ctx, const tlq_wind* w, int n) {
     ctx->cap_winds = 0;
     ctx->cap_wind_cells = 0;
   } else {
-    std::vector<Wind> hw(n);
+    std::vector<Wind>& hw = ctx->winds_host;  // (read by the copy below)
+    hw.assign(n, Wind{});
     const Params& p = ctx->P;
     for (int q = 0; q < n; ++q) {
       Wind& d = hw[q];
@@ -734,7 +739,7 @@ int tlq_set_point_masses(tlq_ctx* ctx, const double* xyzm, int n) {
   CK(cudaMemsetAsync(ctx->phi, 0, (size_t)ctx->L.plane * 8, ctx->stream));
   if (n > 0) {
     CK(cudaMalloc(&ctx->dmasses, 4 * n * sizeof(double)));
-    CK(cudaMemcpy(ctx->dmasses, xyzm, 4 * n * sizeof(double), cudaMemcpyHostToDevice));
+    CK(cudaMemcpyAsync(ctx->dmasses, xyzm, 4 * n * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
     ctx->nmasses = n;
     ctx->P.gravity = 1;
     CK(launch_point_potential_soa(ctx->P, ctx->L, ctx->dmasses, n, ctx->phi, ctx->stream));

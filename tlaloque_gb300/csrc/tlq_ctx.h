@@ -53,6 +53,7 @@ struct tlq_ctx {
   float *dslopef = nullptr, *dgcumf = nullptr;
   Wind* dwinds = nullptr;
   double* dwind_tab = nullptr;  // the winds' tables (Wind::tab)
+  std::vector<Wind> winds_host;
   int cap_winds = 0;            // and how many winds, and cells of tables, the two hold
   long long cap_wind_cells = 0;
   double* dmasses = nullptr;

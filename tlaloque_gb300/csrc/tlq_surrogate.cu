@@ -820,7 +820,8 @@ int tlq_set_cooling_surrogate(tlq_ctx* ctx, const float* params, const float* no
   if (!ctx || !params || !norm6 || !box6) return TLQ_ERR_ARG;
   ctx->mlp_ready = false;  // until the parameters and their image are the new network's
   if (!ctx->mlp_params) SCK(cudaMalloc(&ctx->mlp_params, tlq::mlp::NPARAM * sizeof(float)));
-  SCK(cudaMemcpy(ctx->mlp_params, params, tlq::mlp::NPARAM * sizeof(float), cudaMemcpyHostToDevice));
+  // (on the stream of the kernel that packs them: see tlq_set_cooling_table)
+  SCK(cudaMemcpyAsync(ctx->mlp_params, params, tlq::mlp::NPARAM * sizeof(float), cudaMemcpyHostToDevice, ctx->stream));
   if (!ctx->mlp_image) SCK(cudaMalloc(&ctx->mlp_image, tlq::mlp_image_bytes()));
   SCK(tlq::launch_pack_weights(ctx->mlp_params, ctx->mlp_image, ctx->stream));
   SCK(cudaStreamSynchronize(ctx->stream));
