@@ -250,7 +250,7 @@ int enqueue_step(tlq_ctx* ctx, int par, bool timed) {
   if (ctx->cfg.cooling == TLQ_COOL_MLP)
     CK(launch_cool_mlp_dt(ctx->P, ctx->L, ctx->U[0], ctx->U[1], ctx->it_base, ctx->clk, ctx->mlp_image,
                           ctx->mlp_norm, ctx->mlp_box, ctx->cool_counts, ctx->mlp_cqueue, ctx->mlp_qcount + 1,
-                          ctx->mlp_nqueue, ctx->mlp_qcount + 2, ctx->stream));
+                          ctx->stream));
   if (timed) CK(cudaEventRecordWithFlags(ctx->ev[3], ctx->stream, cudaEventRecordExternal));
   return TLQ_OK;
 }
@@ -484,8 +484,7 @@ int tlq_create(const tlq_config* cfg, tlq_ctx** out) {
   }
   if (cfg->cooling == TLQ_COOL_MLP) {
     const size_t ncell = (size_t)cfg->nx * cfg->ny * cfg->nz;
-    if (cudaMalloc(&ctx->mlp_cqueue, ncell * sizeof(unsigned)) ||
-        cudaMalloc(&ctx->mlp_nqueue, ncell * sizeof(unsigned)) || cudaMalloc(&ctx->mlp_qcount, 3 * sizeof(unsigned)))
+    if (cudaMalloc(&ctx->mlp_cqueue, ncell * sizeof(unsigned)) || cudaMalloc(&ctx->mlp_qcount, 3 * sizeof(unsigned)))
       return bail(TLQ_ERR_NOMEM);
     cudaMemset(ctx->mlp_qcount, 0, 3 * sizeof(unsigned));
   }

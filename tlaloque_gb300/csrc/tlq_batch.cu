@@ -426,6 +426,9 @@ int tlq_batch_create(const tlq_config* cfgs, int n, tlq_batch** out) {
     if (rc != TLQ_OK) return bail(rc);
     b->m.push_back(c);
     b->gen_seen.push_back(~0u);
+    if (c->cfg.cooling == TLQ_COOL_MLP &&
+        cudaMalloc(&c->mlp_nqueue, (size_t)c->cfg.nx * c->cfg.ny * c->cfg.nz * sizeof(unsigned)) != cudaSuccess)
+      return bail(TLQ_ERR_NOMEM);
   }
   b->zlen.assign(n, 0);
   b->zrun.assign(n, 0);

@@ -94,7 +94,7 @@ struct tlq_ctx {
                                               // a single step
   double cool_tmin = 0.0;                  // the table's first temperature
   unsigned* mlp_cqueue = nullptr;          // cells that cool, queued by stage 2 (capacity nx ny nz)
-  unsigned* mlp_nqueue = nullptr;          // cells for the network (capacity nx ny nz)
+  unsigned* mlp_nqueue = nullptr;          // a batch member's cells for the network (capacity nx ny nz)
   unsigned* mlp_qcount = nullptr;          // [1]: cooling queue length, [2]: network queue length (zero
                                            // between steps; [0] unused)
   // output path (tlq_output.cu): device snapshot, page-locked copy, writer thread

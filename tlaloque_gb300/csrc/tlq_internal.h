@@ -90,12 +90,12 @@ cudaError_t launch_normalise(float* X, long long N, const float norm[6], cudaStr
 // (nqueue) and cools the others with the exact integrator; the network pass
 // cools its cells (its prediction, or the exact integrator's where the
 // residual check fails); the dt pass finishes the dt reduction: one launch for
-// a single mesh (k_cool_all).  Queues: capacity nx ny nz; counts zero between
-// steps.
+// a single mesh (k_cool_all, which needs no nqueue).  Queues: capacity nx ny nz;
+// counts zero between steps.
 cudaError_t launch_cool_mlp_dt(const Params& p, const Layout& L, double* U0, double* U1, long long it_base,
                                Clock* clk, const void* img, const float norm[6], const double box[6],
                                unsigned long long* counts, const unsigned* cqueue, unsigned* cqcount,
-                               unsigned* nqueue, unsigned* nqcount, cudaStream_t s);
+                               cudaStream_t s);
 // The three passes for several meshes in three launches: fill_cool_job
 // writes one mesh's arguments (cool_job_bytes() of them) into a host array
 // that is copied to the device; mesh m's blocks of the dt pass are [blk0,

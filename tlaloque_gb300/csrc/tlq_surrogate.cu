@@ -540,13 +540,13 @@ void fill_cool_job(void* dst, const Params& p, const Layout& L, double* U0, doub
 cudaError_t launch_cool_mlp_dt(const Params& p, const Layout& L, double* U0, double* U1, long long it_base,
                                Clock* clk, const void* img, const float norm[6], const double box[6],
                                unsigned long long* counts, const unsigned* cqueue, unsigned* cqcount,
-                               unsigned* nqueue, unsigned* nqcount, cudaStream_t s) {
+                               cudaStream_t s) {
   // a 128-cell tile for every 512 cells (a tenth to a quarter of a clumpy
   // medium is queued), at most one resident wave (2 blocks per SM)
   const long long n = (long long)p.nx * p.ny * p.nz;
   const int nb = (int)std::min<long long>((n + 511) / 512, 152 * 2);
   CoolJob j;
-  fill_cool_job(&j, p, L, U0, U1, it_base, clk, img, norm, box, counts, cqueue, cqcount, nqueue, nqcount, 0, nb);
+  fill_cool_job(&j, p, L, U0, U1, it_base, clk, img, norm, box, counts, cqueue, cqcount, nullptr, nullptr, 0, nb);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(nb);
   cfg.blockDim = dim3(2 * CT);
