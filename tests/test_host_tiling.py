@@ -152,3 +152,17 @@ def test_equal_launches_are_timed_once(fake_lib, tmp_path):
         # the default and 16 planes: 1 + 4 steps; 8 and 32 planes: 1 step
         assert b.running_tiling() == [default] and stages(fake) == 2 * (5 + 5 + 1 + 1)
         b.close()
+
+
+@pytest.mark.parametrize("share,kept", [(0.99, True), (0.975, True), (0.965, False), (0.9, False)])
+def test_batch_keeps_the_default_for_a_small_gain(fake_lib, share, kept):
+    """A size's members are timed alone: a length has to gain more than 3 %."""
+    shape = (48, 48, 48)
+    with fakecuda.loaded(fake_lib) as fake:
+        b = tlq.Batch([config(shape, tlq.PREC_MIXED)])
+        b.members[0].upload(np.ones(b.members[0].cfg.shape, order="F"))
+        default = b.running_tiling()[0]
+        fake.set_cost(blocks(shape, 16), share)
+        b.autotune(None, steps=3)
+        assert b.running_tiling() == [default if kept else 16]
+        b.close()
