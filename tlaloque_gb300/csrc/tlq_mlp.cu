@@ -93,17 +93,6 @@ __device__ __forceinline__ void frag_plain(uint32_t a[4][4], const float d[8][4]
   }
 }
 
-// 1 / x for x >= 1 without the division's branch, which kept a thread's 32
-// sigmoids of a layer from overlapping: the approximate reciprocal and one
-// Newton step in fused arithmetic (correctly rounded but for rare ties,
-// Markstein 1990).  Where 1 / x is subnormal, and for infinity, the
-// approximation alone (0).
-__device__ __forceinline__ float recip_ge1(float x) {
-  float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-  return x < 0x1p126f ? fmaf(r, fmaf(-x, r, 1.0f), r) : r;
-}
-
 // z -> silu(z) and silu'(z), with one sigmoid.
 __device__ __forceinline__ void silu_both(float h[8][4], float ds[8][4], const float z[8][4]) {
 #pragma unroll

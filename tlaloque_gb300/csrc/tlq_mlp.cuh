@@ -51,6 +51,18 @@ __device__ __forceinline__ void mma_bf16(float* d, const uint32_t* a, uint32_t b
 
 __device__ __forceinline__ float sigmoid_f(float z) { return 1.0f / (1.0f + __expf(-z)); }
 __device__ __forceinline__ float silu_f(float z) { return z * sigmoid_f(z); }
+
+// 1 / x for x >= 1 without the division's branch, which kept a thread's 32
+// sigmoids of a layer from overlapping: the approximate reciprocal and one
+// Newton step in fused arithmetic (correctly rounded but for rare ties,
+// Markstein 1990).  Where 1 / x is subnormal, and for infinity, the
+// approximation alone (0).
+__device__ __forceinline__ float recip_ge1(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return x < 0x1p126f ? fmaf(r, fmaf(-x, r, 1.0f), r) : r;
+}
+
 // Load the FP32 master parameters into the BF16 shared layout (all threads).
 __device__ inline void load_weights(const float* __restrict__ P, SmemWeights& W) {
   for (int q = threadIdx.x; q < HID * 4; q += blockDim.x) {
