@@ -317,28 +317,6 @@ __global__ void k_adam(float* P, float* m, float* v, const float* grad, int n, f
   P[q] -= lr * (mq / c1) / (sqrtf(vq / c2) + eps);
 }
 
-// Batch inference (features normalised, 3 per sample) -> y.
-__global__ void __launch_bounds__(TT) k_mlp_infer(const float* __restrict__ P, const float* __restrict__ X, int n,
-                                                  float* __restrict__ Yout) {
-  __shared__ SmemWeights W;
-  load_weights(P, W);
-  __syncthreads();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, tig = lane & 3;
-  const int ntiles = (n + TS - 1) / TS;
-  for (int tile = blockIdx.x * TW + warp; tile < ntiles; tile += gridDim.x * TW) {
-    const int r0 = tile * TS + g, r1 = r0 + 8;
-    float xg[3] = {0.f, 0.f, 0.f}, xg8[3] = {0.f, 0.f, 0.f};
-    if (r0 < n) for (int f = 0; f < 3; ++f) xg[f] = X[3 * r0 + f];
-    if (r1 < n) for (int f = 0; f < 3; ++f) xg8[f] = X[3 * r1 + f];
-    float y[2];
-    forward_tile(W, xg, xg8, g, tig, y);
-    if (tig == 0) {
-      if (r0 < n) Yout[r0] = y[0];
-      if (r1 < n) Yout[r1] = y[1];
-    }
-  }
-}
-
 // Batch inference on the tcgen05 path of the step's network pass
 // (tlq_umma.cuh): 128 samples per tile, one per thread.  A tile whose MMA
 // wait ran out writes NaN (the caller sees it), and the block stops.
@@ -538,14 +516,6 @@ cudaError_t launch_mlp_infer(const float* P, const float* X, int n, float* Y, cu
   const int tiles = (n + umma::ROWS - 1) / umma::ROWS;
   const int blocks = std::max(1, std::min(tiles, 152 * 3));
   mlp::k_mlp_infer_umma<<<blocks, umma::ROWS, 0, s>>>(P, X, n, Y);
-  return cudaGetLastError();
-}
-
-// The mma.sync forward pass (the training kernels' own), for comparison.
-cudaError_t launch_mlp_infer_sync(const float* P, const float* X, int n, float* Y, cudaStream_t s) {
-  const int tiles = (n + mlp::TS - 1) / mlp::TS;
-  const int blocks = std::max(1, std::min((tiles + mlp::TW - 1) / mlp::TW, 152 * 8));
-  mlp::k_mlp_infer<<<blocks, mlp::TT, 0, s>>>(P, X, n, Y);
   return cudaGetLastError();
 }
 

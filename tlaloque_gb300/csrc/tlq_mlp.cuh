@@ -1,13 +1,15 @@
 // tlq_mlp.cuh -- the learned cooling surrogate: a 3-64-64-64-1 SiLU MLP run
 // on the tensor cores with BF16 operands and FP32 accumulation.
 //
-// One warp evaluates 32 samples (two m16 row tiles) with mma.sync
-// m16n8k16.bf16.  The FP32 accumulator fragment of a layer is, element for
-// element, the A-operand fragment of the next layer (the thread that holds
-// output columns 16kt..16kt+15 of a row holds exactly the operand slice of
-// k-tile kt), so activations never leave registers in the forward pass.
-// Weights live in shared memory as BF16, rows padded to 72 (conflict-free
-// 32-bit operand loads).  The 3 -> 64 input layer and the 64 -> 1 output
+// What training (tlq_mlp.cu) and the step's network pass (tlq_umma.cuh) share:
+// the parameters' order, the weights' layout, and the pieces of the training
+// kernel's mma.sync m16n8k16.bf16 pass, a warp per 16 samples.  There the FP32
+// accumulator fragment of a layer is, element for element, the A-operand
+// fragment of the next layer (the thread that holds output columns
+// 16kt..16kt+15 of a row holds exactly the operand slice of k-tile kt), so
+// activations never leave registers in the forward pass.  Weights live in
+// shared memory as BF16, rows padded to 72 (operand loads free of bank
+// conflicts).  The 3 -> 64 input layer and the 64 -> 1 output
 // layer are FP32 dot products (FP32 weights, inputs and activations): they
 // are 4 % of the work, and BF16 inputs (2^-9 of the normalised log features,
 // i.e. 1-2 % in T and tau) or a BF16 output would cost the most accuracy.
@@ -84,28 +86,6 @@ __device__ inline void load_weights(const float* __restrict__ P, SmemWeights& W)
   if (threadIdx.x == 0) W.b4 = P[OFF_B4];
 }
 
-// A block's copy of a network image that pack_weights (tlq_mlp.cu) formed
-// once in device memory with load_weights: 16-byte loads, all of a thread's
-// issued before the first store, instead of load_weights' scalar gathers
-// and conversions in every block.  Same bytes, so the same results.
-template <int NT>
-__device__ __forceinline__ void copy_weights(const SmemWeights* __restrict__ img, SmemWeights& W) {
-  constexpr int NV = (int)(sizeof(SmemWeights) / 16), R = (NV + NT - 1) / NT;
-  const uint4* __restrict__ src = reinterpret_cast<const uint4*>(img);
-  uint4* dst = reinterpret_cast<uint4*>(&W);
-  uint4 v[R];
-#pragma unroll
-  for (int r = 0; r < R; ++r) {
-    const int q = (int)threadIdx.x + r * NT;
-    if (q < NV) v[r] = __ldg(src + q);
-  }
-#pragma unroll
-  for (int r = 0; r < R; ++r) {
-    const int q = (int)threadIdx.x + r * NT;
-    if (q < NV) dst[q] = v[r];
-  }
-}
-
 // Input layer in FP32 for one m16 tile, straight into the accumulator
 // layout: acc[j] = (rows g, g+8) x (columns 8j+2tig, 8j+2tig+1).
 __device__ __forceinline__ void input_layer(float acc[8][4], const SmemWeights& W, const float* xg, const float* xg8,
@@ -120,65 +100,6 @@ __device__ __forceinline__ void input_layer(float acc[8][4], const SmemWeights& 
       acc[j][2 + h] = W.b1[c] + w.x * xg8[0] + w.y * xg8[1] + w.z * xg8[2];
     }
   }
-}
-
-// One dense layer with K = 16*KT inputs and 64 outputs for one m16 tile:
-// acc[j][0..3] = bias + A x W^T (n-tile j = output columns 8j..8j+7).
-template <int KT, int LDW>
-__device__ __forceinline__ void dense64(float acc[8][4], const uint32_t (*a)[4], const __nv_bfloat16 (*w)[LDW],
-                                        const float* bias, int g, int tig) {
-#pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    const float b0 = bias ? bias[8 * j + 2 * tig] : 0.0f, b1v = bias ? bias[8 * j + 2 * tig + 1] : 0.0f;
-    acc[j][0] = b0; acc[j][1] = b1v; acc[j][2] = b0; acc[j][3] = b1v;
-#pragma unroll
-    for (int kt = 0; kt < KT; ++kt) {
-      const uint32_t bb0 = *reinterpret_cast<const uint32_t*>(&w[8 * j + g][16 * kt + 2 * tig]);
-      const uint32_t bb1 = *reinterpret_cast<const uint32_t*>(&w[8 * j + g][16 * kt + 2 * tig + 8]);
-      mma_bf16(acc[j], a[kt], bb0, bb1);
-    }
-  }
-}
-
-// Accumulator fragments (pre-activation z) -> SiLU -> next layer's operand
-// fragments (BF16).
-__device__ __forceinline__ void act_to_frag(uint32_t a[4][4], const float z[8][4]) {
-#pragma unroll
-  for (int kt = 0; kt < 4; ++kt) {
-    const float* c0 = z[2 * kt];
-    const float* c1 = z[2 * kt + 1];
-    a[kt][0] = pack_bf16(silu_f(c0[0]), silu_f(c0[1]));
-    a[kt][1] = pack_bf16(silu_f(c0[2]), silu_f(c0[3]));
-    a[kt][2] = pack_bf16(silu_f(c1[0]), silu_f(c1[1]));
-    a[kt][3] = pack_bf16(silu_f(c1[2]), silu_f(c1[3]));
-  }
-}
-
-// Forward pass of one m16 tile; returns the outputs of rows g and g+8 in
-// y[0], y[1] (in all four lanes of the group g).
-__device__ __forceinline__ void forward_tile(const SmemWeights& W, const float* xg, const float* xg8, int g, int tig,
-                                             float* y) {
-  float acc[8][4];
-  input_layer(acc, W, xg, xg8, tig);
-  uint32_t a[4][4];
-  act_to_frag(a, acc);
-  dense64<4, LD>(acc, a, W.w2, W.b2, g, tig);
-  act_to_frag(a, acc);
-  dense64<4, LD>(acc, a, W.w3, W.b3, g, tig);
-  // output layer in FP32: this lane's 16 columns, then the sum over tig
-  float s0 = 0.0f, s1 = 0.0f;
-#pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    const int c = 8 * j + 2 * tig;
-    s0 += W.w4[c] * silu_f(acc[j][0]) + W.w4[c + 1] * silu_f(acc[j][1]);
-    s1 += W.w4[c] * silu_f(acc[j][2]) + W.w4[c + 1] * silu_f(acc[j][3]);
-  }
-  s0 += __shfl_xor_sync(0xffffffffu, s0, 1);
-  s1 += __shfl_xor_sync(0xffffffffu, s1, 1);
-  s0 += __shfl_xor_sync(0xffffffffu, s0, 2);
-  s1 += __shfl_xor_sync(0xffffffffu, s1, 2);
-  y[0] = W.b4 + s0;  // row g
-  y[1] = W.b4 + s1;  // row g + 8
 }
 
 }  // namespace mlp
