@@ -280,7 +280,7 @@ int tlq_output_wait(tlq_ctx* ctx);
  * ones by default (tlq_get_tiling then gives 8, or nz; tlq_running_tiling the
  * length that runs).  Results do not depend on it.  The measuring autotuner
  * picks it -- from the cache file (JSON keyed by GPU name, mesh size and form,
- * "zlen" 0 for the default; NULL = no cache) or timed now over `steps` steps
+ * "zlen" "default" for the default; NULL = no cache) or timed now over `steps` steps
  * per candidate (the default, 8, 16, 32, 64, 128) from the current state, which
  * is restored afterwards. */
 int tlq_set_tiling(tlq_ctx* ctx, int zlen);

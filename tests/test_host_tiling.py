@@ -74,7 +74,7 @@ def test_autotune_tries_the_default(fake_lib, tmp_path, shape, winner):
         assert ctx.running_tiling() == run
         assert got == ctx.tiling() == (nominal if winner == "default" else winner)
         (entry,) = json.load(open(cache))["tuned"].values()
-        assert entry["zlen"] == (0 if winner == "default" else winner)
+        assert entry["zlen"] == winner
         ctx.close()
         ctx = uploaded(config(shape, tlq.PREC_MIXED))
         fake.lib.fake_reset()
@@ -97,13 +97,12 @@ def test_batch_autotune_tries_the_default(fake_lib, tmp_path, winner):
         b = batch()
         default = b.running_tiling()
         assert max(default) < 8 and b.tiling() == [8, 8, 8]
-        for size, members in ((48, (0, 2)), (32, (1,))):  # a size's members run together
-            z = default[members[0]] if winner == "default" else winner
-            fake.set_cost(len(members) * blocks((size,) * 3, z), 0.25)
+        wins = default if winner == "default" else [winner] * 3
+        fake.set_cost(sum(blocks(s, z) for s, z in zip(shapes, wins)), 0.25)
         got = b.autotune(cache, steps=2)
         assert got == b.tiling() == ([8] * 3 if winner == "default" else [winner] * 3)
         assert b.running_tiling() == (default if winner == "default" else [winner] * 3)
-        assert {e["zlen"] for e in json.load(open(cache))["tuned"].values()} == {0 if winner == "default" else winner}
+        assert {e["zlen"] for e in json.load(open(cache))["tuned"].values()} == {winner}
         b.set_tiling(1, 16)
         assert b.tiling()[1] == b.running_tiling()[1] == 16
         fake.lib.fake_reset()
@@ -149,14 +148,13 @@ def test_equal_launches_are_timed_once(fake_lib, tmp_path):
         fake.set_cost(blocks(shape, default), 0.25)
         fake.set_cost(blocks(shape, 16), 0.45)
         b.autotune(None, steps=4)
-        # the default and 16 planes: 1 + 4 steps; 8 and 32 planes: 1 step
-        assert b.running_tiling() == [default] and stages(fake) == 2 * (5 + 5 + 1 + 1)
+        # the default: 1 + 4 steps; 8, 16 and 32 planes: 1 step
+        assert b.running_tiling() == [default] and stages(fake) == 2 * (5 + 1 + 1 + 1)
         b.close()
 
 
-@pytest.mark.parametrize("share,kept", [(0.99, True), (0.975, True), (0.965, False), (0.9, False)])
+@pytest.mark.parametrize("share,kept", [(0.995, True), (0.985, False), (0.9, False)])
 def test_batch_keeps_the_default_for_a_small_gain(fake_lib, share, kept):
-    """A size's members are timed alone: a length has to gain more than 3 %."""
     shape = (48, 48, 48)
     with fakecuda.loaded(fake_lib) as fake:
         b = tlq.Batch([config(shape, tlq.PREC_MIXED)])
@@ -165,4 +163,42 @@ def test_batch_keeps_the_default_for_a_small_gain(fake_lib, share, kept):
         fake.set_cost(blocks(shape, 16), share)
         b.autotune(None, steps=3)
         assert b.running_tiling() == [default if kept else 16]
+        b.close()
+
+
+def test_batch_is_timed_with_all_members(fake_lib, tmp_path):
+    """Every timed launch holds all members' tiles; after one length for all
+    sizes, a size may take half or twice of it; a size in the cache keeps its."""
+    cache = tmp_path / "tune.json"
+    shapes = [(64, 64, 64), (32, 32, 32), (48, 48, 48)]
+
+    def items(z):
+        return sum(blocks(s, q) for s, q in zip(shapes, z))
+
+    with fakecuda.loaded(fake_lib) as fake:
+        b = tlq.Batch([config(s, tlq.PREC_MIXED) for s in shapes])
+        for m in b.members:
+            m.upload(np.ones(m.cfg.shape, order="F"))
+        default = b.running_tiling()
+        fake.set_cost(items([16, 16, 16]), 0.5)
+        fake.set_cost(items([32, 16, 16]), 0.25)
+        fake.set_cost(items([16, 8, 16]), 0.4999)  # (not gain enough)
+        before = len(fake.launches("stage_kernel"))
+        assert b.autotune(str(cache), steps=2) == [32, 16, 16] == b.running_tiling()
+        timed = {g[0] for k, g, _ in fake.launches("stage_kernel")[before:]}
+        lengths = [default] + [[min(z, s[2]) for s in shapes] for z in (8, 16, 32, 64)]
+        lengths += [[16, 8, 16], [16, 32, 16], [16, 16, 8], [16, 16, 32], [8, 16, 16], [32, 16, 16]]
+        assert timed == {items(z) for z in lengths}
+        b.close()
+        doc = json.load(open(cache))
+        del doc["tuned"]["48x48x48/batch_mixed"]
+        lines = ",\n".join(f'    "{k}": {{"zlen": {v["zlen"]}, "ms_per_step": {v["ms_per_step"]:.6f}}}'
+                           for k, v in doc["tuned"].items())
+        cache.write_text('{\n  "gpu": "fake",\n  "tuned": {\n' + lines + "\n  }\n}\n")
+        fake.reset()
+        fake.set_cost(items([32, 16, 8]), 0.25)
+        b = tlq.Batch([config(s, tlq.PREC_MIXED) for s in shapes])
+        for m in b.members:
+            m.upload(np.ones(m.cfg.shape, order="F"))
+        assert b.autotune(str(cache), steps=2) == [32, 16, 8]
         b.close()

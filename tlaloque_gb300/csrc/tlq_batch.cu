@@ -157,8 +157,7 @@ int member_tiles(const tlq_ctx* c) {
 }
 
 // The rule's chunk length for the batch: its members share the persistent
-// launches (the autotuner, which runs one size's members at a time, keeps it
-// too, so that what it times is what the batch runs).
+// launches.
 int batch_rule(const tlq_batch* b) {
   std::vector<int> tiles, nz;
   for (const tlq_ctx* c : b->m) {
@@ -211,14 +210,12 @@ void fill_desc(tlq_batch* b, int i) {
   d.gz = tiles_z(c, b->zrun[i]);
 }
 
-// Work list of the members in `which` (all when empty), most planes per tile
-// first so that the persistent blocks' static stride mixes long and short
-// tiles evenly.
-std::vector<Item> make_items(const tlq_batch* b, const std::vector<int>& which) {
+// Work list, most planes per tile first so that the persistent blocks' static
+// stride mixes long and short tiles evenly.
+std::vector<Item> make_items(const tlq_batch* b) {
   std::vector<Item> v;
-  std::vector<int> ms = which;
-  if (ms.empty())
-    for (int i = 0; i < (int)b->m.size(); ++i) ms.push_back(i);
+  std::vector<int> ms;
+  for (int i = 0; i < (int)b->m.size(); ++i) ms.push_back(i);
   std::stable_sort(ms.begin(), ms.end(), [&](int x, int y) { return b->zrun[x] > b->zrun[y]; });
   for (int i : ms) {
     const tlq_ctx* c = b->m[i];
@@ -255,8 +252,8 @@ int upload_items(tlq_batch* b, const std::vector<Item>& v) {
 }
 
 // Descriptors of all members, and the cooling-pass arguments of the
-// surrogate members in `which` (all when empty).
-int refresh_desc(tlq_batch* b, const std::vector<int>& which = {}) {
+// surrogate members.
+int refresh_desc(tlq_batch* b) {
   set_zrun(b);
   for (int i = 0; i < (int)b->m.size(); ++i) fill_desc(b, i);
   BCK(cudaMemcpyAsync(b->d_desc, b->h_desc.data(), b->h_desc.size() * sizeof(MemberDesc), cudaMemcpyHostToDevice,
@@ -270,7 +267,6 @@ int refresh_desc(tlq_batch* b, const std::vector<int>& which = {}) {
   for (int i = 0; i < (int)b->m.size(); ++i) {
     tlq_ctx* c = b->m[i];
     if (c->cfg.cooling != TLQ_COOL_MLP) continue;
-    if (!which.empty() && std::find(which.begin(), which.end(), i) == which.end()) continue;
     cool.push_back(i);
     cells += (long long)c->cfg.nx * c->cfg.ny * c->cfg.nz;
   }
@@ -292,10 +288,10 @@ int refresh_desc(tlq_batch* b, const std::vector<int>& which = {}) {
   return TLQ_OK;
 }
 
-// One batched step of the members the item list holds: the two persistent
-// stage launches, then the surrogate's three cooling passes over the members
-// that use it (their stage 2 queued the cooling cells and left the dt
-// reduction to them; refresh_desc wrote their arguments).
+// One batched step: the two persistent stage launches, then the surrogate's
+// three cooling passes over the members that use it (their stage 2 queued the
+// cooling cells and left the dt reduction to them; refresh_desc wrote their
+// arguments).
 int enqueue_batch_step(tlq_batch* b) {
   const size_t smem1 = sizeof(tlq::BatchSmem<1>), smem2 = sizeof(tlq::BatchSmem<2>);
   // the specialised kernels when every member uses their limiter and solver
@@ -329,7 +325,7 @@ int build_batch_graph(tlq_batch* b) {
     cudaGraphExecDestroy(b->graph);
     b->graph = nullptr;
   }
-  int rc = upload_items(b, make_items(b, {}));
+  int rc = upload_items(b, make_items(b));
   if (rc) return rc;
   cudaGraph_t g = nullptr;
   BCK(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
@@ -348,6 +344,8 @@ int build_batch_graph(tlq_batch* b) {
 }
 
 // ---- autotuner cache: one JSON object, one entry per line ----------------
+// (length 0, the default, as "default": versions that know lengths only skip
+// such an entry)
 std::string device_name() {
   int dev = 0;
   cudaGetDevice(&dev);
@@ -370,8 +368,13 @@ std::map<std::string, std::pair<int, double>> read_cache(const char* path, const
     double ms;
     char form[16];
     if (std::sscanf(line, " \"%dx%dx%d/%15[a-z0-9_]\": {\"zlen\": %d, \"ms_per_step\": %lf", &nx, &ny, &nz, form, &z,
-                    &ms) == 6)
-      m[std::to_string(nx) + "x" + std::to_string(ny) + "x" + std::to_string(nz) + "/" + form] = {z, ms};
+                    &ms) != 6) {
+      z = 0;
+      if (std::sscanf(line, " \"%dx%dx%d/%15[a-z0-9_]\": {\"zlen\": \"default\", \"ms_per_step\": %lf", &nx, &ny, &nz,
+                      form, &ms) != 5)
+        continue;
+    }
+    m[std::to_string(nx) + "x" + std::to_string(ny) + "x" + std::to_string(nz) + "/" + form] = {z, ms};
   }
   std::fclose(f);
   if (!same_gpu) m.clear();
@@ -386,8 +389,9 @@ int write_cache(const char* path, const std::string& gpu, const std::map<std::st
   std::fprintf(f, "{\n  \"gpu\": \"%s\",\n  \"tuned\": {\n", gpu.c_str());
   size_t q = 0;
   for (const auto& kv : m)
-    std::fprintf(f, "    \"%s\": {\"zlen\": %d, \"ms_per_step\": %.6f}%s\n", kv.first.c_str(), kv.second.first,
-                 kv.second.second, ++q < m.size() ? "," : "");
+    std::fprintf(f, "    \"%s\": {\"zlen\": %s, \"ms_per_step\": %.6f}%s\n", kv.first.c_str(),
+                 kv.second.first ? std::to_string(kv.second.first).c_str() : "\"default\"", kv.second.second,
+                 ++q < m.size() ? "," : "");
   std::fprintf(f, "  }\n}\n");
   std::fclose(f);
   return std::rename(tmp.c_str(), path) == 0 ? TLQ_OK : TLQ_ERR_ARG;
@@ -405,12 +409,9 @@ std::vector<int> tuning_candidates(int nz, int run) {
 // A candidate whose first step takes more than this many times the best one's
 // is not timed further (the longest chunks on small meshes take several).
 constexpr double TUNING_HOPELESS = 2.0;
-// A batch's candidate replaces the default when the members of its size, timed
-// alone, gain more than this share.  The default is the model's for all members
-// together, as they run: five meshes of 48 to 128 cells that took 16 planes for
-// the 96^3 one on a few percent of its own time stepped in 0.714 ms, 0.675 with
-// the default throughout.
-constexpr double TUNING_GAIN = 0.03;
+// A batch's lengths replace the ones before when its step gains more than this
+// share (timings of one launch differ by a few tenths of a percent).
+constexpr double TUNING_GAIN = 0.01;
 
 }  // namespace
 
@@ -576,114 +577,141 @@ int tlq_batch_stats_get(tlq_batch* b, tlq_batch_stats* s) {
   return TLQ_OK;
 }
 
-// For each distinct mesh size: the cached z-chunk length, or one measured
-// now.  Every candidate (tuning_candidates) is timed over `steps` steps (after
-// one warm-up step) of the batch restricted to the members of that size,
-// starting each time from the members' current state, which is restored
-// afterwards (state, clock).  The winner is written to the cache (one JSON
-// object per file, keyed by the GPU's name; the default as length 0).
+// For each distinct mesh size: the cached z-chunk length, or one measured now,
+// with all members running, as the batch runs them.  (Timed alone, a size's
+// members chose lengths that made the step of 48 bubbles of 48 to 128 cells 4.70
+// ms where the default takes 4.37: tiles of several lengths fill the blocks'
+// static stride less evenly.)  First one length for all open sizes: the default,
+// and 8, 16, 32, 64, 128 planes; then, size by size, half and twice the length
+// that won.  A choice is timed over one step and, where that gains, over `steps`.
+// Every step starts from the members' current state, which it only reads: the
+// clocks are set back, the state needs no copy.  The winners are written to the
+// cache (one JSON object per file, keyed by the GPU's name).
 int tlq_batch_autotune(tlq_batch* b, const char* cache_path, int steps, int* chosen) {
   if (!b || steps < 1) return TLQ_ERR_ARG;
-  for (size_t i = 0; i < b->m.size(); ++i)
+  const int n = (int)b->m.size();
+  for (int i = 0; i < n; ++i)
     if (!b->m[i]->uploaded) return bfail(b, TLQ_ERR_STATE, "autotune needs every member's state (tlq_upload)");
-  for (size_t i = 0; i < b->m.size(); ++i)
+  for (int i = 0; i < n; ++i)
     if (b->m[i]->cfg.cooling == TLQ_COOL_MLP && !b->m[i]->mlp_ready)
       return bfail(b, TLQ_ERR_STATE, "member " + std::to_string(i) + " uses the cooling surrogate but has no network");
   const std::string gpu = device_name();
   auto cache = read_cache(cache_path, gpu);
-  std::map<std::string, std::vector<int>> classes;
-  for (size_t i = 0; i < b->m.size(); ++i) {
+  std::map<std::string, std::vector<int>> classes, open;
+  for (int i = 0; i < n; ++i) {
     const tlq_config& c = b->m[i]->cfg;
-    classes[std::to_string(c.nx) + "x" + std::to_string(c.ny) + "x" + std::to_string(c.nz) + "/batch_mixed"].push_back(
-        (int)i);
+    classes[std::to_string(c.nx) + "x" + std::to_string(c.ny) + "x" + std::to_string(c.nz) + "/batch_mixed"].push_back(i);
   }
-  bool wrote = false;
   for (auto& kv : classes) {
-    const std::vector<int>& mem = kv.second;
     auto hit = cache.find(kv.first);
-    if (hit != cache.end()) {
-      for (int i : mem) b->zlen[i] = std::max(0, std::min(hit->second.first, b->m[i]->cfg.nz));
-      continue;
+    if (hit == cache.end()) open.insert(kv);
+    for (int i : kv.second)
+      b->zlen[i] = hit == cache.end() ? 0 : std::max(0, std::min(hit->second.first, b->m[i]->cfg.nz));
+  }
+  // the lengths per member, and those that run, of the choices to time
+  std::vector<std::vector<int>> choices, runs;
+  auto add = [&](const std::vector<int>& zlen) {
+    const std::vector<int> keep = b->zlen;
+    b->zlen = zlen;
+    set_zrun(b);
+    const bool known = std::find(runs.begin(), runs.end(), b->zrun) != runs.end();
+    if (!known) {
+      choices.push_back(zlen);
+      runs.push_back(b->zrun);
     }
-    const int nz = b->m[mem[0]]->cfg.nz;
-    const std::vector<int> candidates = tuning_candidates(nz, split_zlen(batch_rule(b), nz));
-    if (candidates.size() == 1) {  // nothing to choose
-      for (int i : mem) b->zlen[i] = 0;
-      continue;
-    }
-    // snapshot the members' current state and clocks
-    std::vector<double*> snap(mem.size(), nullptr);
-    std::vector<tlq::Clock> clk(mem.size());
-    std::vector<int> cur(mem.size());
-    for (size_t q = 0; q < mem.size(); ++q) {
-      tlq_ctx* c = b->m[mem[q]];
+    b->zlen = keep;
+  };
+  add(b->zlen);
+  for (int z : {8, 16, 32, 64, 128}) {
+    std::vector<int> zlen = b->zlen;
+    bool fits = z == 8;  // (lengths up to some size's planes)
+    for (auto& kv : open)
+      for (int i : kv.second) {
+        zlen[i] = std::min(z, b->m[i]->cfg.nz);
+        fits = fits || z <= b->m[i]->cfg.nz;
+      }
+    if (fits) add(zlen);
+  }
+  if (choices.size() > 1) {  // (else there is nothing to choose)
+    std::vector<tlq::Clock> clk(n);
+    std::vector<unsigned long long> counts(3 * n, 0ull);
+    for (int i = 0; i < n; ++i) {
+      tlq_ctx* c = b->m[i];
       double t, dt;
       int it;
       tlq_get_time(c, &t, &it, &dt);  // settles c->cur
-      cur[q] = c->cur;
-      BCK(cudaMalloc(&snap[q], (size_t)c->L.plane * 5 * sizeof(double)));
-      BCK(cudaMemcpyAsync(snap[q], c->U[cur[q]], (size_t)c->L.plane * 5 * sizeof(double), cudaMemcpyDeviceToDevice,
-                          b->stream));
-      BCK(cudaMemcpyAsync(&clk[q], c->clk, sizeof(tlq::Clock), cudaMemcpyDeviceToHost, b->stream));
+      BCK(cudaMemcpyAsync(&clk[i], c->clk, sizeof(tlq::Clock), cudaMemcpyDeviceToHost, b->stream));
+      if (c->cool_counts)
+        BCK(cudaMemcpyAsync(&counts[3 * i], c->cool_counts, 3 * sizeof counts[0], cudaMemcpyDeviceToHost, b->stream));
     }
     BCK(cudaStreamSynchronize(b->stream));
-    int best = 0;
-    double best_ms = 1e300, bar = 1e300;
-    for (int z : candidates) {
-      for (int i : mem) b->zlen[i] = z;
-      int rc = refresh_desc(b, mem);
-      if (!rc) rc = upload_items(b, make_items(b, mem));
-      if (rc) return rc;
-      auto time = [&](int n, double* per) -> int {
+    auto set_back = [&]() -> int {
+      for (int i = 0; i < n; ++i)
+        BCK(cudaMemcpyAsync(b->m[i]->clk, &clk[i], sizeof(tlq::Clock), cudaMemcpyHostToDevice, b->stream));
+      return TLQ_OK;
+    };
+    auto time = [&](int reps, double* per) -> int {  // the lengths of b->zlen
+      int rc = refresh_desc(b);
+      if (!rc) rc = upload_items(b, make_items(b));
+      *per = 0.0;
+      for (int w = 0; w < reps && !rc; ++w) {
         BCK(cudaEventRecord(b->ev[0], b->stream));
-        for (int w = 0; w < n; ++w) {
-          const int r = enqueue_batch_step(b);
-          if (r) return r;
-        }
+        rc = enqueue_batch_step(b);
         BCK(cudaEventRecord(b->ev[1], b->stream));
-        BCK(cudaEventSynchronize(b->ev[1]));
+        if (!rc) rc = set_back();
+        BCK(cudaStreamSynchronize(b->stream));
         float ms = 0.f;
         cudaEventElapsedTime(&ms, b->ev[0], b->ev[1]);
-        *per = ms / n;
-        return TLQ_OK;
-      };
+        *per += ms / reps;
+      }
+      return rc;
+    };
+    double best = 0.0;
+    int rc = time(1, &best);  // warm-up
+    if (!rc) rc = time(steps, &best);
+    auto try_choice = [&](const std::vector<int>& zlen) {
+      const std::vector<int> keep = b->zlen;
+      b->zlen = zlen;
       double per = 0.0;
-      rc = time(1, &per);  // warm-up
-      if (!rc && per < TUNING_HOPELESS * best_ms) {
-        rc = time(steps, &per);
-        if (per < bar) {
-          best_ms = per;
-          best = z;
-          bar = z == 0 ? per * (1.0 - TUNING_GAIN) : per;
+      if (!rc) rc = time(1, &per);
+      if (!rc && per < best * (1.0 - TUNING_GAIN)) rc = time(steps, &per);
+      if (!rc && per < best * (1.0 - TUNING_GAIN))
+        best = per;
+      else
+        b->zlen = keep;
+    };
+    for (size_t q = 1; q < choices.size(); ++q) try_choice(choices[q]);
+    if (classes.size() > 1)
+      for (auto& kv : open)
+        for (int twice = 0; twice < 2; ++twice) {
+          set_zrun(b);
+          const int nz = b->m[kv.second[0]]->cfg.nz, run = b->zrun[kv.second[0]];
+          const int z = std::min(nz, twice ? std::max(8, 2 * run) : run / 2);
+          if (z < 8 && z != nz) continue;
+          std::vector<int> zlen = b->zlen;
+          for (int i : kv.second) zlen[i] = z;
+          const size_t before = choices.size();
+          add(zlen);
+          if (choices.size() > before) try_choice(zlen);
         }
-      }
-      if (rc) return rc;
-      // back to the snapshot
-      for (size_t q = 0; q < mem.size(); ++q) {
-        tlq_ctx* c = b->m[mem[q]];
-        BCK(cudaMemcpyAsync(c->U[cur[q]], snap[q], (size_t)c->L.plane * 5 * sizeof(double),
-                            cudaMemcpyDeviceToDevice, b->stream));
-        BCK(cudaMemcpyAsync(c->clk, &clk[q], sizeof(tlq::Clock), cudaMemcpyHostToDevice, b->stream));
-      }
-      BCK(cudaStreamSynchronize(b->stream));
+    if (rc) return rc;
+    for (auto& kv : open) {
+      for (int i : kv.second) std::fill_n(&counts[3 * i], 3, 0ull);  // (a tuned member's counters start anew)
+      cache[kv.first] = {b->zlen[kv.second[0]], best};
     }
-    for (size_t q = 0; q < mem.size(); ++q) {
-      cudaFree(snap[q]);
-      tlq_ctx* c = b->m[mem[q]];
-      if (c->cool_counts) cudaMemsetAsync(c->cool_counts, 0, 3 * sizeof(unsigned long long), b->stream);
-    }
-    for (int i : mem) b->zlen[i] = best;
-    cache[kv.first] = {best, best_ms};
-    wrote = true;
+    for (int i = 0; i < n; ++i)
+      if (b->m[i]->cool_counts)
+        BCK(cudaMemcpyAsync(b->m[i]->cool_counts, &counts[3 * i], 3 * sizeof counts[0], cudaMemcpyHostToDevice, b->stream));
+    BCK(cudaStreamSynchronize(b->stream));
+    if (write_cache(cache_path, gpu, cache) != TLQ_OK)
+      return bfail(b, TLQ_ERR_ARG, std::string("cannot write the tuning cache ") + (cache_path ? cache_path : ""));
   }
-  if (wrote && write_cache(cache_path, gpu, cache) != TLQ_OK)
-    return bfail(b, TLQ_ERR_ARG, std::string("cannot write the tuning cache ") + (cache_path ? cache_path : ""));
   if (b->graph) {
     cudaGraphExecDestroy(b->graph);
     b->graph = nullptr;
   }
   if (chosen)
-    for (size_t i = 0; i < b->m.size(); ++i) chosen[i] = reported_zlen(b, (int)i);
+    for (int i = 0; i < n; ++i) chosen[i] = reported_zlen(b, i);
   return TLQ_OK;
 }
 
