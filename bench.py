@@ -69,16 +69,16 @@ FP64_OPS_PER_ZONE = {
 
 # Warp instructions x 32 per zone-update that the plain step's two kernels
 # issue to the FP64 pipe (ncu: smsp__inst_executed_pipe_fp64.sum of
-# stage_kernel<1> and <2>).  Divisions, square roots and part of the
-# multiplications run on the integer pipe, and what cells share is formed
-# once, so this is below the operation counts above.
+# stage_kernel<1> and <2>, a count of these kernels).  Divisions, square roots
+# and part of the multiplications run on the integer pipe, and what cells share
+# is formed once, so this is below the operation counts above.
 FP64_PIPE_INST_PER_ZONE = {"wind256": 204.1 + 485.4, "sedov128": 186.2 + 351.3}
 
 
 def fp64_pipe_bound(inst: float, rate: dict) -> dict:
-    """The plain FP64 step's compute roofline: zone-updates/s with the FP64
-    pipe busy all the time with the step's own instructions, at the pipe's
-    measured FMA rate (tlq_measure_fp64_rate)."""
+    """zone-updates/s with the FP64 pipe busy all the time with the step's own
+    instructions, at the pipe's measured FMA rate (tlq_measure_fp64_rate): how
+    busy these kernels keep the pipe, not a bound on the work."""
     return {"fp64_pipe_inst_per_zone": inst, "zone_updates_per_s_bound": rate["fma_per_s"] / inst}
 
 
@@ -573,8 +573,9 @@ def main():
     mix = measure(tlq.PREC_MIXED, args.steps, not cooling)
     forms = {"fp64": form(f64), "mixed": form(mix), "speedup_mixed_vs_fp64": mix["value"] / f64["value"],
              "mixed_vs_fp64": accuracy(mix, f64)}
-    # the plain form's bound: the FP64 pipe (measured here, with the oracle's
-    # op counts) next to its HBM fraction
+    # the plain form's bound: the FP64 pipe (its rate measured here) next to
+    # its HBM fraction: how busy the kernels' own instructions keep it, and the
+    # step against the oracle's additions alone, which stay on that pipe
     bpz64 = bytes_per_zone(cfg)["alg"]
     forms["fp64"]["roofline"] = {
         "hbm_achieved_gbs": bpz64["step"] * f64["value"] / 1e9,
@@ -587,7 +588,8 @@ def main():
             "bound": "fp64 pipe", "fp64_ops_per_zone": ops,
             "fp64_rate_measured": {**rate, "how": "tlq_measure_fp64_rate: independent FMA / IEEE divide / IEEE "
                                                  "square-root chains, 8 blocks of 256 threads per SM, CUDA events"},
-            **b, "fp64_pipe_frac": f64["value"] / b["zone_updates_per_s_bound"]})
+            **b, "fp64_pipe_frac": f64["value"] / b["zone_updates_per_s_bound"],
+            "fp64_additions_frac": f64["value"] * ops["add"] / rate["fma_per_s"]})
     head = mix
     surrogate = None
     if cooling:

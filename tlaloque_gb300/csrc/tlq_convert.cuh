@@ -33,7 +33,7 @@ __device__ __forceinline__ float d2f(double d) {
 // range are looked for once for all five (the largest magnitude), so that
 // each conversion is 10 integer operations instead of 16; the rounding's
 // increment is a carry: the 29 dropped bits at the top of a word plus
-// 0x7fffffff and the kept lsb.  (Mixed stage 1, issue-bound, of the bubble
+// 0x7fffffff and the kept lsb.  (Mixed stage 1 of the bubble
 // 256^3: 0.837 -> 0.820 ms; two, three or five of them as F2F: 0.842, 0.866
 // and 0.947.)
 __device__ __forceinline__ void d2f5(const double* u, long long vs, float* f) {

@@ -1079,7 +1079,7 @@ __global__ void k_mg_prolong_add(const MgCtl* c, MgLevel co, MgLevel f, bool gho
 // in a table, packed: at most 128 of them on 8 cells, one per thread, so
 // that four warps' FP64 operations (8 x 4 x 19 cycles a step) take no longer
 // than one cell's chain of eight (8 x 79), which bounds it.  Levels 8 to 1:
-// 140 us a cycle (from level arrays, wave after wave: 195 us for 4 to 1
+// 130 us a cycle (from level arrays, wave after wave: 195 us for 4 to 1
 // alone, and 68 us and four launches more for the 8-cell level's relaxes).
 // ---------------------------------------------------------------------------
 constexpr int MG_CT = 128;

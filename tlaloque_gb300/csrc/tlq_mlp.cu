@@ -136,8 +136,10 @@ __device__ __forceinline__ void add_column_sums(float acc[2], const float v[16],
 // accumulator starts at zero).  Each pre-activation's sigmoid is evaluated
 // once, for the activation and its derivative.  262,144 samples: 637 us with
 // shared-memory atomics for every 16 samples' gradient, a sum over lanes per
-// column and three sigmoids, 105 us now, bound by issue (sigmoids and their
-// divisions, products, column sums).
+// column and three sigmoids, 105 us now.  Latency bounds it: one block of 8
+// warps an SM (255 registers a thread) uses 46 % of the issue slots, the tensor
+// pipe is 22 % busy, and a warp waits on fixed latencies (0.83 of its cycles per
+// issue) and on loads (0.78).
 __global__ void __launch_bounds__(TT) k_mlp_grad(const float* __restrict__ P, const float* __restrict__ X,
                                                  const float* __restrict__ Y, const float* __restrict__ Wt, int nb,
                                                  float* grad, float* loss) {

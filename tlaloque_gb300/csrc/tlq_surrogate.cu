@@ -418,7 +418,7 @@ __global__ void __launch_bounds__(FT) k_cool_dt(const CoolJob* __restrict__ jobs
 // cools the others), so sorting them first gains no density here, and the
 // passes were latency: three launches of a few tiles each, 49 us of a 48^3
 // clumpy step (the stages take 56) and 72 us at 128^3.  (The batched step
-// keeps the three passes: its members' queues differ widely in length.)
+// keeps the three passes; one launch over its members' queues is not tried.)
 __global__ void __launch_bounds__(2 * CT, 2) k_cool_all(const __grid_constant__ CoolJob j) {
   __shared__ umma::Smem S;
   __shared__ float x3[3][CT], acc[CT];
