@@ -1,4 +1,4 @@
-"""tlq_set_winds called again and again (a driver that moves its winds each
+"""tlq_set_winds called again and again (a program that moves its winds each
 step): buffers kept while they are large enough, one launch, one wait.  Host
 side only, on a fake CUDA runtime."""
 import pytest

@@ -684,7 +684,7 @@ int tlq_set_winds(tlq_ctx* ctx, const tlq_wind* w, int n) {
       d.klo = std::max(-1, lo(d.zc, d.radius, p.zl, p.dz)); d.khi = std::min(p.nz + 2, hi(d.zc, d.radius, p.zl, p.dz));
     }
     // Both buffers are kept while they are large enough, and one launch forms
-    // every wind's table: a driver may move its winds each step (a call with
+    // every wind's table: a program may move its winds each step (a call with
     // one wind: 8 us before there were tables, 26 with an allocation, a launch
     // per wind and a wait for them, 6 so).
     if (n > ctx->cap_winds) {
